@@ -25,8 +25,6 @@ namespace lg {
 
 namespace {
 
-constexpr int kMaxL = 128;
-
 struct GridX {  // FP64 reciprocal metrics and FP32 metric differences of the FP64 parts
   const double *inv_dx, *inv_dy, *inv_dz, *inv_volume, *inv_area_z;
   // FP32: 1/volume, 1/area_z, and at w level jl (2..nl) z_scalar(jl-1)-z_scalar(jl) and
@@ -476,17 +474,28 @@ __device__ __forceinline__ float div_col(const Dims& D, const Grid<float>& G, co
   return (comp_h + comp_v) * X.inv_volume_f[q];
 }
 
-// div_h of a stored horizontal vector field (the third-order theta chain)
+// the levels l0..l1 of a marching thread: the column cut into gridDim.z chunks of equal length
+// (a chunk forms h of the layer above it anew, so every cell has the bits of a whole column's walk)
+struct LevelChunk { int l0, l1; };
+__device__ __forceinline__ LevelChunk level_chunk(const Dims& D) {
+  const int len = (D.nl + (int)gridDim.z - 1) / (int)gridDim.z;
+  return LevelChunk{(int)blockIdx.z * len + 1, min(D.nl, ((int)blockIdx.z + 1) * len)};
+}
+
+// div_h of a stored horizontal vector field (the third-order theta chain); blockIdx.z is the
+// chunk of levels (level_chunks)
 __global__ void __launch_bounds__(128) ks_div_h(Dims D, Grid<float> GF, GridX X, const float* vx, const float* vy,
                                                 float* out) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
+  const LevelChunk lc = level_chunk(D);
   auto fx = [&](int i, int j, int k) { return vx[IX(D, i, j, k)]; };
   auto fy = [&](int i, int j, int k) { return vy[IX(D, i, j, k)]; };
-  LayerFaces cur = layer_faces(D, GF, fx, fy, ji, jk, 1), nxt{};
+  LayerFaces cur = layer_faces(D, GF, fx, fy, ji, jk, lc.l0), nxt{};
   float h_prev = 0.f;
-  for (int jl = 1; jl <= D.nl; ++jl) {
+  if (lc.l0 - 1 >= D.nf + 1) h_prev = layer_faces(D, GF, fx, fy, ji, jk, lc.l0 - 1).h;
+  for (int jl = lc.l0; jl <= lc.l1; ++jl) {
     nxt.h = 0.f;
     if (jl < D.nl || jl == D.nf) nxt = layer_faces(D, GF, fx, fy, ji, jk, jl + 1);
     out[IX(D, ji, jk, jl)] = div_col(D, GF, X, cur, vert_faces(D, h_prev, cur.h, nxt.h, jl), ji, jk, jl);
@@ -505,15 +514,20 @@ __global__ void __launch_bounds__(128) ks_gas_div(Dims D, Grid<float> GF, GridX 
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
+  const LevelChunk lc = level_chunk(D);
   const long long goff = (long long)(D.g - 1) * D.fstride;
   auto fx = [&](int i, int j, int k) { return fu[IX(D, i, j, k)]; };
   auto fy = [&](int i, int j, int k) { return fv[IX(D, i, j, k)]; };
   auto gx = [&](int i, int j, int k) { return gu[IX(D, i, j, k)]; };
   auto gy = [&](int i, int j, int k) { return gv[IX(D, i, j, k)]; };
-  LayerFaces mc = layer_faces(D, GF, fx, fy, ji, jk, 1), mn{};
-  LayerFaces tc = layer_faces(D, GF, gx, gy, ji, jk, 1), tn{};
+  LayerFaces mc = layer_faces(D, GF, fx, fy, ji, jk, lc.l0), mn{};
+  LayerFaces tc = layer_faces(D, GF, gx, gy, ji, jk, lc.l0), tn{};
   float mh_prev = 0.f, th_prev = 0.f;
-  for (int jl = 1; jl <= D.nl; ++jl) {
+  if (lc.l0 - 1 >= D.nf + 1) {
+    mh_prev = layer_faces(D, GF, fx, fy, ji, jk, lc.l0 - 1).h;
+    th_prev = layer_faces(D, GF, gx, gy, ji, jk, lc.l0 - 1).h;
+  }
+  for (int jl = lc.l0; jl <= lc.l1; ++jl) {
     const long long q = IX(D, ji, jk, jl);
     mn.h = 0.f;
     tn.h = 0.f;
@@ -737,16 +751,22 @@ __global__ void ks_tend_wind(Dims D, State So, State Sn, Tend<float> Tn, Carried
 }
 
 // ---- three_band_solver_ver, mo_column_solvers.F90:21-351 --------------------------------
-// The reference's implicit system for the vertical mass-flux increments at levels 2..nl,
-// one thread per column, streamed top to bottom.  C = float (LGAME_PRECISION_SPLIT): from the
-// FP32 mirror, the partial derivatives alpha, beta, gamma, the interface theta and density
-// weights, the matrix and its elimination multipliers; FP64: the explicit predictions of theta'
-// and exner', the right-hand side (where the pressure-gradient and buoyancy terms balance), the
-// forward and back substitution, and the new rho_g, rho*theta_v, exner', w; theta' is formed as
-// (rho*theta_v - theta_bg*rho)/rho with the small numerator in FP64.  C = double
-// (LGAME_PRECISION_SPLIT_FP64_COLUMN): the same from the FP64 state, FP64 metric differences and
-// reciprocals, with FP64 coefficients, multipliers and quotients -- the column solve wholly in
-// FP64 (only the explicit tendencies it reads are FP32).
+// The reference's implicit system for the vertical mass-flux increments at levels 2..nl of a
+// column.  C = float (LGAME_PRECISION_SPLIT): from the FP32 mirror, the partial derivatives
+// alpha, beta, gamma, the interface theta and density weights, the matrix and its elimination
+// multipliers; FP64: the explicit predictions of theta' and exner', the right-hand side (where
+// the pressure-gradient and buoyancy terms balance), the forward and back substitution, and the
+// new rho_g, rho*theta_v, exner', w; theta' is formed as (rho*theta_v - theta_bg*rho)/rho with
+// the small numerator in FP64.  C = double (LGAME_PRECISION_SPLIT_FP64_COLUMN): the same from
+// the FP64 state, FP64 metric differences and reciprocals, with FP64 coefficients, multipliers
+// and quotients -- the column solve wholly in FP64 (only the explicit tendencies it reads are
+// FP32).
+//
+// Two kernels (the rule between them stands at their launch in split_step).  Large grids:
+// ks_column_ver, one thread per column, streamed top to bottom and back; every warp issues FP64
+// work all the time, which is what bounds it (about 26 FP64 operations a cell).  Small grids:
+// ks_column_ver_tile below.
+constexpr int kMaxLayers = 128;  // layers a context may have (lgame_gpu_create)
 template <class C>
 __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
                                                      State Sn, StateF Mo, StateF Mn, Tend<float> Tn, int rk_step) {
@@ -821,10 +841,10 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
     *rhe = L.ro + dtf * tr;
   };
 
-  C epr[kMaxL + 1];       // elimination multipliers
-  double rpr[kMaxL + 1];  // substituted right-hand side, then the solution (FP64)
-  C tis[kMaxL + 1];       // interface theta
-  C gs[kMaxL + 1];        // gamma of each layer
+  C epr[kMaxLayers + 1];       // elimination multipliers
+  double rpr[kMaxLayers + 1];  // substituted right-hand side, then the solution (FP64)
+  C tis[kMaxLayers + 1];       // interface theta
+  C gs[kMaxLayers + 1];        // gamma of each layer
   Lay L0 = layer(1), L1 = layer(2), L2{};
   double tpe0, epe0, tpe1, epe1, tpe2 = 0.0, epe2 = 0.0;
   C rhe0, rhe1, rhe2 = C(0);
@@ -960,6 +980,304 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
     Mn.w[IX(D, ji, jk, m + 1)] = narrow(wf);
   }
 }
+
+// the same operators as functions of the column, for ks_column_ver_tile (in ks_column_ver they
+// stand in the loop: with these functions there it took 3.47 instead of 3.15 ms at 768 x 768 x 80)
+template <class C>
+struct ColVer {
+  static constexpr bool F64 = sizeof(C) == 8;
+  const Dims& D;
+  const Grid<double>& G;
+  const Grid<float>& GF;
+  const GridX& X;
+  const State &So, &Sn, &Su;  // Su: state_new_used, mo_column_solvers.F90:69-73
+  const StateF &Mo, &Mn, &Mu;
+  const Tend<float>& Tn;
+  const int rk_step, ji, jk;
+  const long long goff;
+  const C dtf, idtf, rdcv, ic2, ic1;
+  const double idtd;
+
+  __device__ __forceinline__ ColVer(const Dims& D_, const Grid<double>& G_, const Grid<float>& GF_, const GridX& X_,
+                                    const State& So_, const State& Sn_, const StateF& Mo_, const StateF& Mn_,
+                                    const Tend<float>& Tn_, int rk, int i, int j)
+      : D(D_), G(G_), GF(GF_), X(X_), So(So_), Sn(Sn_), Su(rk == 1 ? So_ : Sn_), Mo(Mo_), Mn(Mn_),
+        Mu(rk == 1 ? Mo_ : Mn_), Tn(Tn_), rk_step(rk), ji(i), jk(j), goff((long long)(D_.g - 1) * D_.fstride),
+        dtf(C(D_.dtime)), idtf(C(1.0 / D_.dtime)), rdcv(C(kR_D / kC_D_V)),
+        ic2(C(1.0 / (kIMPL_THERMO_WEIGHT * (D_.dtime * D_.dtime) * kC_D_P))),
+        ic1(C(1.0 / (kIMPL_THERMO_WEIGHT * D_.dtime * kC_D_P))), idtd(1.0 / D_.dtime) {}
+
+  // the inputs of the coefficients, from the FP32 mirror or the FP64 state and metrics
+  __device__ C rho_o(long long i) const { if constexpr (F64) return So.rho[goff + i]; else return Mo.rho[goff + i]; }
+  __device__ C rt_o(long long i) const { if constexpr (F64) return So.rt[i]; else return Mo.rt[i]; }
+  __device__ C ep_o(long long i) const { if constexpr (F64) return So.ep[i]; else return Mo.ep[i]; }
+  __device__ C rho_u(long long i) const { if constexpr (F64) return Su.rho[goff + i]; else return Mu.rho[goff + i]; }
+  __device__ C rt_u(long long i) const { if constexpr (F64) return Su.rt[i]; else return Mu.rt[i]; }
+  __device__ C ep_u(long long i) const { if constexpr (F64) return Su.ep[i]; else return Mu.ep[i]; }
+  __device__ C w_o(long long i) const { if constexpr (F64) return So.w[i]; else return Mo.w[i]; }
+  __device__ C ebg(long long i) const { if constexpr (F64) return G.exner_bg[i]; else return GF.exner_bg[i]; }
+  __device__ C ivol(long long i) const { if constexpr (F64) return X.inv_volume[i]; else return X.inv_volume_f[i]; }
+  __device__ C iarz(long long i) const { if constexpr (F64) return X.inv_area_z[i]; else return X.inv_area_z_f[i]; }
+  __device__ C damp(long long i) const { if constexpr (F64) return G.damp[i]; else return GF.damp[i]; }
+  // at w level jl (2..nl): z_scalar(jl-1) - z_scalar(jl) and exner_bg(jl-1) - exner_bg(jl)
+  __device__ C dzs(long long i) const {
+    if constexpr (F64) return G.z_scalar[i - D.plane] - G.z_scalar[i]; else return X.dzs_f[i];
+  }
+  __device__ C debg(long long i) const {
+    if constexpr (F64) return G.exner_bg[i - D.plane] - G.exner_bg[i]; else return X.deb_f[i];
+  }
+  static __device__ double W(C x) { if constexpr (F64) return x; else return wide(x); }
+  static __device__ double quot(double x, C d) { if constexpr (F64) return x / d; else return div_f(x, d); }
+
+  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
+  // state, where theta * d(exner')/dz carries the whole hydrostatic balance); with predict() the
+  // explicit predictions of theta_v' and exner' (FP64 state plus increments) and of rho_g
+  struct Lay { C a, b, g, th, ro, iv, rhe; double thd, tpe, epe; };
+  __device__ __forceinline__ Lay layer(int jl) const {
+    const long long i = IX(D, ji, jk, jl);
+    Lay L{};
+    L.thd = D.luse_bg ? 0.0 : Su.rt[i] / Su.rho[goff + i];
+    const C ro = rho_o(i), rto = rt_o(i);
+    const C iro = C(1) / ro, irto = C(1) / rto;
+    L.a = -rto * iro * iro;
+    L.b = iro;
+    L.g = rdcv * irto * (ebg(i) + ep_o(i));
+    if (rk_step == 2) {
+      const C ru = rho_u(i), rtu = rt_u(i);
+      const C iru = C(1) / ru, irtu = C(1) / rtu;
+      L.a = C(0.5) * (L.a - rtu * iru * iru);
+      L.b = C(0.5) * (L.b + iru);
+      L.g = C(0.5) * (L.g + rdcv * irtu * (ebg(i) + ep_u(i)));
+      L.th = rtu * iru;
+    } else {
+      L.th = rto * iro;
+    }
+    L.ro = ro;
+    L.iv = ivol(i);
+    return L;
+  }
+  __device__ __forceinline__ void predict(int jl, Lay& L) const {
+    const long long i = IX(D, ji, jk, jl);
+    const C tr = C(Tn.rho[goff + i]), trt = C(Tn.rt[i]);
+    L.tpe = So.tp[i] + W(dtf * (L.a * tr + L.b * trt));
+    L.epe = So.ep[i] + W(dtf * L.g * trt);
+    L.rhe = L.ro + dtf * tr;
+  }
+
+  // row jl: level jl+1 between layers jl (L0) and jl+1 (L1); the couplings with row jl+1 (layer
+  // jl+1's derivatives) need layer jl+2 (L2) and are 0 in the last row
+  struct Row { C dv, cv, ev, ti; double rv; };
+  __device__ __forceinline__ Row row(int jl, const Lay& L0, const Lay& L1, const Lay& L2) const {
+    Row r;
+    const long long ib = IX(D, ji, jk, jl + 1);
+    const C ti = C(0.5) * (L0.th + L1.th);
+    r.ti = ti;
+    const C irio = C(2) / (L0.ro + L1.ro);
+    const C dz = dzs(ib), deb = debg(ib), dp = damp(ib);
+    const double wo = So.w[ib];
+    const C wof = w_o(ib);
+    const C al0 = L0.a * L0.iv, al1 = L1.a * L1.iv, be0 = L0.b * L0.iv, be1 = L1.b * L1.iv;
+    const C ga0 = L0.g * L0.iv, ga1 = L1.g * L1.iv;
+    r.dv = -(ti * ti) * (ga0 + ga1) + C(0.5) * deb * (al1 - al0 + ti * (be1 - be0))
+           - dz * ic2 * irio * (C(2) * iarz(ib) + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
+    const C rie = C(0.5) * (L0.rhe + L1.rhe);
+    double rv = (wo + W(dtf * C(Tn.w[ib]))) * W(-dz * ic2);
+    rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
+    rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
+    r.rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
+    r.cv = r.ev = C(0);
+    if (jl < D.nl - 1) {
+      const long long ic = IX(D, ji, jk, jl + 2);
+      const C ti_n = C(0.5) * (L1.th + L2.th);
+      const C irio_n = C(2) / (L1.ro + L2.ro);
+      r.cv = ti_n * ga1 * ti + C(0.5) * debg(ic) * (al1 + be1 * ti)
+             - dzs(ic) * ic1 * C(0.5) * w_o(ic) * L1.iv * irio_n * damp(ic);
+      r.ev = ti * ga1 * ti_n - C(0.5) * deb * (al1 + be1 * ti_n) + dz * ic1 * C(0.5) * wof * L1.iv * irio * dp;
+    }
+    return r;
+  }
+
+  // the new state, mo_column_solvers.F90:300-345: layer jl from the solutions s0, s1 at the
+  // interfaces above and below it (w levels jl, jl+1) and their interface theta t0, t1; w at level
+  // jl+1 from the new densities of layers jl and jl+1
+  struct StateIn { double rt, rho, ep, bg, w; C ivf, iaz, mro; float trho, trt; };
+  __device__ __forceinline__ StateIn state_in(int m) const {
+    StateIn r;
+    const long long p = IX(D, ji, jk, m);
+    r.rt = So.rt[p];
+    r.rho = So.rho[goff + p];
+    r.ep = So.ep[p];
+    r.bg = G.theta_v_bg[p];
+    r.w = So.w[p];
+    r.ivf = ivol(p);
+    r.iaz = iarz(p);
+    r.mro = rho_o(p);
+    r.trho = Tn.rho[goff + p];
+    r.trt = Tn.rt[p];
+    return r;
+  }
+  __device__ __forceinline__ double new_rho(const StateIn& c, double s0, double s1) const {
+    return fma(W(dtf * c.ivf), s1 - s0, c.rho + W(dtf * C(c.trho)));
+  }
+  // new rho_g in the type of the coefficients (FP32: rounded)
+  static __device__ __forceinline__ C rho_c(double rn) { if constexpr (F64) return rn; else return narrow(rn); }
+  // returns rho_c of the layer's new density; below: the layer below and its rho_c
+  __device__ __forceinline__ C new_state(int jl, const StateIn& c, const StateIn& below, C rnc_below, double s0,
+                                         double s1, C t0, C t1, C g) const {
+    const long long i = IX(D, ji, jk, jl);
+    const double dtv = W(dtf * c.ivf);
+    const double rn = new_rho(c, s0, s1);
+    const double rt_e = c.rt + W(dtf * C(c.trt));
+    const double rtn = fma(dtv, fma(-W(t0), s0, W(t1) * s1), rt_e);
+    const double epn = fma(W(g), rtn - c.rt, c.ep);
+    const float rnf = narrow(rn);
+    const C rnc = F64 ? C(rn) : C(rnf);
+    if constexpr (F64) {
+      const double tpn = fma(-c.bg, rn, rtn) / rn;
+      Sn.tp[i] = tpn;
+      Mn.tp[i] = narrow(tpn);
+    } else {
+      const float tpf = narrow(fma(-c.bg, rn, rtn)) / rnf;
+      Sn.tp[i] = wide(tpf);
+      Mn.tp[i] = tpf;
+    }
+    Sn.rho[goff + i] = rn;
+    Sn.rt[i] = rtn;
+    Sn.ep[i] = epn;
+    Mn.rho[goff + i] = rnf;
+    Mn.rt[i] = narrow(rtn);
+    Mn.ep[i] = narrow(epn);
+    if (jl < D.nl) {
+      const long long ib = i + D.plane;
+      const C rin = C(0.5) * (rnc + rnc_below);
+      const C irio = C(2) / (c.mro + below.mro);
+      const double wn = fma(-W(rin), below.w, W(C(2) * below.iaz) * s1) * W(irio);
+      Sn.w[ib] = wn;
+      Mn.w[ib] = narrow(wn);
+    }
+    return rnc;
+  }
+  // w_free_slip, mo_inner_product.F90:52-75, with the new u, v
+  __device__ __forceinline__ void free_slip() const {
+    const int m = D.nl;
+    const double wf =
+        G.ipw[0][IX(D, ji, jk, m)] * Sn.u[IX(D, ji, jk + 1, m)] * G.slope_x[IX(D, ji, jk + 1, m)]
+      + G.ipw[1][IX(D, ji, jk, m)] * Sn.v[IX(D, ji, jk, m)] * G.slope_y[IX(D, ji, jk, m)]
+      + G.ipw[2][IX(D, ji, jk, m)] * Sn.u[IX(D, ji, jk, m)] * G.slope_x[IX(D, ji, jk, m)]
+      + G.ipw[3][IX(D, ji, jk, m)] * Sn.v[IX(D, ji + 1, jk, m)] * G.slope_y[IX(D, ji + 1, jk, m)];
+    Sn.w[IX(D, ji, jk, m + 1)] = wf;
+    Mn.w[IX(D, ji, jk, m + 1)] = narrow(wf);
+  }
+};
+
+// Small grids: a block owns TC columns and NW chunks of levels (a lane per column, chunk w of a
+// column in thread w*TC + lane), in phases:
+//   1. every thread forms the rows of its chunk (matrix, right-hand side) into shared memory;
+//   2. the first TC threads run the factorisation (pivot p, upper factor e/p, lower factor c/p,
+//      type C) and the forward substitution y = r - (c/p)*y, one multiply-add a row in the chain;
+//   3. every thread its rows' y/p;  4. the first TC threads the back substitution;
+//   5. every thread the new state of its chunk of layers.
+// The chain of levels then waits on shared memory and arithmetic alone, and the levels' loads and
+// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 34 against 280
+// us at 4 x 256 x 60, 150 against 381 us at 128 x 128 x 80; equal (460 us) at 256 x 256 x 80, and
+// slower above (3.6 against 3.2 ms at 768 x 768 x 80), where the phases in which one warp works
+// cost more than the latency they hide.
+template <class C, int TC, int NW>
+__global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
+    ks_column_ver_tile(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So, State Sn, StateF Mo, StateF Mn,
+                       Tend<float> Tn, int rk_step) {
+  using Cv = ColVer<C>;
+  constexpr int kRow = 5 * TC;  // coefficients of one level of the block's columns in shared memory
+  const int lane = threadIdx.x % TC, w = threadIdx.x / TC;
+  const int col = blockIdx.x * TC + lane;
+  const bool valid = col < D.ny * D.nx;
+  const Cv V(D, G, GF, X, So, Sn, Mo, Mn, Tn, rk_step, valid ? col % D.ny + 1 : 1, valid ? col / D.ny + 1 : 1);
+  const int nl = D.nl, n = nl - 1;
+  extern __shared__ __align__(16) unsigned char smem_cv[];
+  double* const sr = (double*)smem_cv + lane;             // right-hand side, y, then the solution
+  C* const sc = (C*)((double*)smem_cv + TC * nl) + lane;  // per row: diagonal (then the pivot), c, e (then
+                                                          // e/p), interface theta, gamma of layer jl
+  const int chunk = (n + NW - 1) / NW, r0 = w * chunk + 1, r1 = min(n, (w + 1) * chunk);
+  if (valid && r0 <= r1) {
+    typename Cv::Lay L0 = V.layer(r0), L1 = V.layer(r0 + 1), L2{};
+    V.predict(r0, L0);
+    V.predict(r0 + 1, L1);
+    for (int jl = r0; jl <= r1; ++jl) {
+      if (jl < n) {
+        L2 = V.layer(jl + 2);
+        if (jl < r1) V.predict(jl + 2, L2);
+      }
+      const typename Cv::Row q = V.row(jl, L0, L1, L2);
+      C* const row = sc + kRow * (jl - 1);
+      row[0] = q.dv;
+      row[TC] = q.cv;
+      row[2 * TC] = q.ev;
+      row[3 * TC] = q.ti;
+      row[4 * TC] = L0.g;
+      if (jl == n) row[kRow + 4 * TC] = L1.g;
+      sr[TC * (jl - 1)] = q.rv;
+      L0 = L1; L1 = L2;
+    }
+  }
+  __syncthreads();
+  if (w == 0 && valid) {
+    C cv_prev = C(0), epr_prev = C(0), f = C(0);
+    double y = 0.0;
+    C* row = sc;
+    double* r = sr;
+#pragma unroll 4
+    for (int jl = 1; jl <= n; ++jl, row += kRow, r += TC) {
+      const C piv = row[0] - epr_prev * cv_prev;
+      y = fma(-Cv::W(f), y, r[0]);
+      r[0] = y;
+      epr_prev = row[2 * TC] / piv;
+      cv_prev = row[TC];
+      f = cv_prev / piv;
+      row[0] = piv;
+      row[2 * TC] = epr_prev;
+    }
+  }
+  __syncthreads();
+  if (valid)
+    for (int jl = r0; jl <= r1; ++jl) sr[TC * (jl - 1)] = Cv::quot(sr[TC * (jl - 1)], sc[kRow * (jl - 1)]);
+  __syncthreads();
+  if (w == 0 && valid) {
+    C* row = sc + kRow * (n - 2);
+    double* r = sr + TC * (n - 2);
+    double s = r[TC];
+#pragma unroll 4
+    for (int jl = n - 1; jl >= 1; --jl, row -= kRow, r -= TC) {
+      s = fma(-Cv::W(row[2 * TC]), s, r[0]);
+      r[0] = s;
+    }
+  }
+  __syncthreads();
+  // the new state, each chunk of layers bottom to top; the chunk's first layer needs the new
+  // density of the layer below it, formed anew
+  const int lchunk = (nl + NW - 1) / NW, l0 = w * lchunk + 1, l1 = min(nl, (w + 1) * lchunk);
+  if (!valid || l0 > l1) return;
+  // solution and interface theta of row m (w level m+1), 0 at the model top and surface
+  auto sol = [&](int m) -> double { return (m >= 1 && m <= n) ? sr[TC * (m - 1)] : 0.0; };
+  auto tif = [&](int m) -> C { return (m >= 1 && m <= n) ? sc[kRow * (m - 1) + 3 * TC] : C(0); };
+  typename Cv::StateIn in_cur = V.state_in(l1), in_up{}, in_below{};
+  double s1 = sol(l1);
+  C rnf_below = C(0);
+  if (l1 < nl) {
+    in_below = V.state_in(l1 + 1);
+    rnf_below = Cv::rho_c(V.new_rho(in_below, s1, sol(l1 + 1)));
+  }
+  for (int jl = l1; jl >= l0; --jl) {
+    if (jl > l0) in_up = V.state_in(jl - 1);
+    const double s0 = sol(jl - 1);
+    rnf_below = V.new_state(jl, in_cur, in_below, rnf_below, s0, s1, tif(jl - 1), tif(jl), sc[kRow * (jl - 1) + 4 * TC]);
+    s1 = s0;
+    in_below = in_cur;
+    in_cur = in_up;
+  }
+  if (D.freeslip && l1 == nl) V.free_slip();
+}
+template <class C, int TC>
+constexpr size_t column_ver_smem(int nl) { return (size_t)nl * TC * (sizeof(double) + 5 * sizeof(C)); }
 
 // ---- three_band_solver_gen_densities, mo_column_solvers.F90:353-604 ----------------------
 // The reference's system per (column, tracer)  d_l s_l + e_l s_{l+1} + c_{l-1} s_{l-1} = rho_l + inc_l
@@ -1240,7 +1558,7 @@ __device__ __forceinline__ void tracer_block(const Dims& D, const Grid<float>& G
     for (int q = 0; q < kTrSet; ++q) update(jl, q, So.rho[tq[q] + (jl - 1) * pl]);
 }
 
-// grid (2 tracer sets, row tiles, nx), 256 threads, dynamic shared memory tracer_smem(D);
+// grid (2 tracer sets, row tiles, nx), 256 threads, dynamic shared memory tracer_smem(D.nl);
 // HEAT: the first substep
 template <bool HEAT>
 __global__ void __launch_bounds__(kTrWarps * 32, 2) ks_column_tracers(Dims D, Grid<float> GF, GridX X, State So,
@@ -1264,7 +1582,18 @@ __global__ void ks_csh_sum(Dims D, const float* csh_part, float* csh) {
 }
 
 // dynamic shared memory of ks_column_tracers: alpha, beta and e' of three tracers, 32 columns
-size_t tracer_smem(const Dims& D) { return (size_t)D.nl * kTrRow * sizeof(float); }
+size_t tracer_smem(int nl) { return (size_t)nl * kTrRow * sizeof(float); }
+
+// dynamic shared memory of ks_column_ver: right-hand side and five coefficients per level, 32 columns
+// the tile kernel's shared memory is allowed for the most layers a context may have: contexts of
+// different heights share the function's attribute
+template <class C, int TC, int NW>
+bool column_ver_attr() {
+  return cudaFuncSetAttribute(ks_column_ver_tile<C, TC, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)column_ver_smem<C, TC>(kMaxLayers)) == cudaSuccess;
+}
+
+constexpr int kSMs = 152;  // streaming multiprocessors of the GB300
 
 dim3 sblk() { return dim3(32, 8, 1); }
 // x: row tiles, y: levels, z: column tiles (see LG_IDX3)
@@ -1274,6 +1603,18 @@ dim3 sgrd(int rows, int cols, int levs) {
 // column kernels: 128 threads, 32 rows x 4 columns
 dim3 cblk() { return dim3(32, 4, 1); }
 dim3 cgrd(int rows, int cols) { return dim3((unsigned)((rows + 31) / 32), (unsigned)((cols + 3) / 4), 1u); }
+// the marching divergences: the column in as many chunks as give the device about 128 warps an SM,
+// of at least 4 levels.  (One chunk: ks_gas_div 187, 421, 505, 1772 us at 4x256x60, 128x128x80,
+// 256x256x80, 768x768x80; so: 24, 62, 245, 1718 us.  64 warps an SM: 72 us at 128x128x80, 1899 us at
+// 768x768x80; two levels a chunk at least: 64 us at 128x128x80.)
+dim3 cgrd_levels(const Dims& D) {
+  dim3 g = cgrd(D.ny, D.nx);
+  const long long warps = 4LL * g.x * g.y;
+  const int chunks = (int)std::min<long long>((kSMs * 128LL + warps - 1) / warps, D.nl);
+  const int len = std::max((D.nl + chunks - 1) / chunks, 4);
+  g.z = (unsigned)((D.nl + len - 1) / len);
+  return g;
+}
 
 }  // namespace
 
@@ -1284,13 +1625,18 @@ int split_create(const Dims& D, bool column_fp64, const SplitDiff& diff, const S
     return LGAME_ERR_UNSUPPORTED;
   }
   if (D.ncons > 1 &&
-      (D.nl > 128 ||
+      (D.nl > kMaxLayers ||
        cudaFuncSetAttribute(ks_column_tracers<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)tracer_smem(D)) != cudaSuccess ||
+                            (int)tracer_smem(kMaxLayers)) != cudaSuccess ||
        cudaFuncSetAttribute(ks_column_tracers<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)tracer_smem(D)) != cudaSuccess)) {
+                            (int)tracer_smem(kMaxLayers)) != cudaSuccess)) {
     lgame_set_error("split precision: the tracer solver supports at most 128 layers");
     return LGAME_ERR_UNSUPPORTED;
+  }
+  if (!(column_fp64 ? column_ver_attr<double, 8, 32>() && column_ver_attr<double, 16, 16>()
+                    : column_ver_attr<float, 8, 32>() && column_ver_attr<float, 32, 12>())) {
+    lgame_set_error("split precision: shared memory of the vertical solver refused");
+    return LGAME_ERR_CUDA;
   }
   if (diff.mom_h &&
       (cudaFuncSetAttribute(k_diff_scalar_col<7, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1643,7 +1989,7 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
                      float* pv) -> int {
     SL("ks_grad_vert", (k_grad_vert<float, float>), sgrd(D.ny, D.nx, D.nl - 1), B, D, GF, tp, s->gz);
     SL("ks_grad_hor", (k_grad_hor<float, float>), sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, tp, s->gz, s->gx, s->gy);
-    SL("ks_div_h", ks_div_h, cgrd(D.ny, D.nx), cblk(), D, GF, s->GX, s->gx, s->gy, s->divf);
+    SL("ks_div_h", ks_div_h, cgrd_levels(D), cblk(), D, GF, s->GX, s->gx, s->gy, s->divf);
     SL("ks_theta_edges", ks_theta_edges, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, tp, s->divf, s->dbg, s->tbu, s->tbv, u,
        v, ou, ov, pu, pv);
     return LGAME_OK;
@@ -1788,16 +2134,34 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
         return LGAME_ERR_CUDA;
       }
     }
-    SL("ks_gas_div", ks_gas_div, cgrd(D.ny, D.nx), cblk(), D, GF, s->GX, Ms, s->fu, s->fv, s->gu, s->gv,
+    SL("ks_gas_div", ks_gas_div, cgrd_levels(D), cblk(), D, GF, s->GX, Ms, s->fu, s->fv, s->gu, s->gv,
        C.temperature, C.hdiss, C.rad, C.csh, T.rho, T.rt, mdt, tdh, ptr, pth);
     if (SF.sens || SF.soil)
       SL("ks_sfc_column", k_sfc_column_split<float>, sgrd(D.ny, D.nx, 1), B, D, G, So, rk == 1 ? So : Sn, T.rt,
          SF.buf, SF.par, SF.tsoil[so], SF.tsoil[rk == 1 ? so : sn], SF.tsoil[sn]);
-    const dim3 gc = cgrd(D.ny, D.nx);
-    if (s->column_fp64)
-      SL("ks_column_ver", ks_column_ver<double>, gc, cblk(), D, G, GF, s->GX, So, Sn, Mo, Mn, T, rk);
-    else
-      SL("ks_column_ver", ks_column_ver<float>, gc, cblk(), D, G, GF, s->GX, So, Sn, Mo, Mn, T, rk);
+    // The vertical solve by the number of columns: up to 8 columns an SM, 8 a block with 32 chunks of
+    // levels (34 us at 1,024 columns of 60 layers; 54 with 32 x 12); up to the size that gives
+    // every SM sub-partition three warps of columns, 32 a block with 12 chunks (150 us at 16,384
+    // columns of 80 layers; 216 with 8 x 32); above, a thread a column (461 us at 65,536 columns
+    // of 80 layers; 502 with 32 x 12).  The FP64-coefficient solve keeps twice the shared memory
+    // a column and takes 16 columns a block.
+    const long long cols = (long long)D.ny * D.nx;
+#define CV_ARGS D, G, GF, s->GX, So, Sn, Mo, Mn, T, rk
+#define CV_TILE(C, TC, NW)                                                                              \
+  SLS("ks_column_ver", (ks_column_ver_tile<C, TC, NW>), dim3((unsigned)((cols + TC - 1) / TC)), dim3(TC * NW), \
+      (column_ver_smem<C, TC>(D.nl)), CV_ARGS)
+    const bool tiny = cols <= kSMs * 8LL, small = cols <= kSMs * 4LL * 32 * 3;
+    if (s->column_fp64) {
+      if (tiny) CV_TILE(double, 8, 32);
+      else if (small) CV_TILE(double, 16, 16);
+      else SL("ks_column_ver", ks_column_ver<double>, cgrd(D.ny, D.nx), cblk(), CV_ARGS);
+    } else {
+      if (tiny) CV_TILE(float, 8, 32);
+      else if (small) CV_TILE(float, 32, 12);
+      else SL("ks_column_ver", ks_column_ver<float>, cgrd(D.ny, D.nx), cblk(), CV_ARGS);
+    }
+#undef CV_TILE
+#undef CV_ARGS
     if (tracers) {
       // the two tracer sets fastest (the blocks of a row tile run together), row tiles, columns
       const dim3 gt(2u, (unsigned)((D.ny + 31) / 32), (unsigned)D.nx);
@@ -1807,7 +2171,7 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
         // tracer densities and csh, beside the second substep's vorticity and wind update
         SYNC(after(side, stream, EV_C));
         cur = side;
-        SLS("ks_column_tracers", ks_column_tracers<true>, gt, dim3(kTrWarps * 32), tracer_smem(D), D, GF, s->GX, So,
+        SLS("ks_column_tracers", ks_column_tracers<true>, gt, dim3(kTrWarps * 32), tracer_smem(D.nl), D, GF, s->GX, So,
             Sn, Mo, Mn, T.rho, C.temperature, s->csh_part);
         if (D.nc > 0) SL("ks_csh_sum", ks_csh_sum, sgrd(D.ny, D.nx, D.nl), B, D, s->csh_part, C.csh);
         if (conc && cudaEventRecord(s->ev[EV_CSH], side) != cudaSuccess) {
@@ -1817,7 +2181,7 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
         cur = stream;
       } else {
         SYNC(after(stream, side, EV_END));
-        SLS("ks_column_tracers", ks_column_tracers<false>, gt, dim3(kTrWarps * 32), tracer_smem(D), D, GF, s->GX, So,
+        SLS("ks_column_tracers", ks_column_tracers<false>, gt, dim3(kTrWarps * 32), tracer_smem(D.nl), D, GF, s->GX, So,
             Sn, Mo, Mn, T.rho, C.temperature, s->csh_part);
       }
     }
