@@ -750,7 +750,13 @@ __global__ void k_pgrad(Dims D, Grid<double> G, State S, const double* gx, const
                         const double* tvu, const double* tvv, const double* tpu, const double* tpv, PGrad<double> P,
                         int lfirst);
 __global__ void k_column_ver(Dims D, Grid<double> G, State So, State Sn, Tend<double> Tn, int rk_step);
-__global__ void k_column_tracers(Dims D, Grid<double> G, State So, State Sn, const double* t_rho, const double* T,
-                                 double* csh, int rk_step);
+// once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
+// and c_p of ice and water
+__global__ void k_moist_aux(Dims D, Grid<double> G, State So, const double* T, double* vcloud, double* cpi, double* cpw);
+// the tracer solve: rvol = 1/volume, itwdtv = 0.5*dtime/volume; csh is written at rk_step 1
+int column_tracers_prepare();
+void launch_column_tracers(const Dims& D, const Grid<double>& G, const State& So, const State& Sn, const double* t_rho,
+                           const double* T, const double* rvol, const double* itwdtv, const double* vcloud,
+                           const double* cpi, const double* cpw, double* csh, int rk_step, cudaStream_t st);
 
 }  // namespace lg

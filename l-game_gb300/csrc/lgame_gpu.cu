@@ -85,6 +85,8 @@ struct lgame_gpu {
   bool phase = false;
   double *ptr = nullptr, *pth = nullptr;
   // scratch
+  double *rvol = nullptr, *itwdtv = nullptr;  // FP64 step: 1/volume and 0.5*dtime/volume
+  double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
   double* staging = nullptr;
   size_t staging_elems = 0;
@@ -280,6 +282,14 @@ __global__ void k_split_ipw(Dims D, const double* src, double* w1, double* w2, d
   const size_t h = 6 * ((size_t)(ji - 1) + (size_t)D.ny * ((size_t)(jk - 1) + (size_t)D.nx * (size_t)(jl - 1)));
   const long long q = IX(D, ji, jk, jl);
   w1[q] = src[h]; w2[q] = src[h + 1]; w3[q] = src[h + 2]; w4[q] = src[h + 3]; w5[q] = src[h + 4]; w6[q] = src[h + 5];
+}
+
+__global__ void k_volume_recip(Dims D, const double* volume, double* rvol, double* itwdtv) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl);
+  rvol[q] = 1.0 / volume[q];
+  itwdtv[q] = 0.5 * D.dtime / volume[q];
 }
 
 __global__ void k_check_finite(Dims D, State S, int* flag) {
@@ -513,7 +523,7 @@ const auto k_tracers = lg::k_tracers<double>;
 const auto k_gas_theta = lg::k_gas_theta<double>;
 const auto k_pgrad = lg::k_pgrad;
 const auto k_column_ver = lg::k_column_ver;
-const auto k_column_tracers = lg::k_column_tracers;
+const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
 const auto k_diff_visc = lg::k_diff_visc<double, double>;
 const auto k_diff_zeta = lg::k_diff_zeta<double, double>;
@@ -550,6 +560,16 @@ int klaunch_check(lgame_gpu* c, const char* what) {
     if (tr_ >= 0) lg::trace_end(c, tr_);                                       \
     int rc_ = klaunch_check(c, #kernel);                                       \
     if (rc_ != LGAME_OK) return rc_;                                           \
+  } while (0)
+
+// the same around a function that launches one kernel
+#define LAUNCH_FN(name, call)                                        \
+  do {                                                               \
+    const int tr_ = c->profiling ? lg::trace_begin(c, name) : -1;    \
+    call;                                                            \
+    if (tr_ >= 0) lg::trace_end(c, tr_);                             \
+    int rc_ = klaunch_check(c, name);                                \
+    if (rc_ != LGAME_OK) return rc_;                                 \
   } while (0)
 
 // theta_v_adv_3rd_order (mo_multiplications.F90:116-204) of theta = theta_v_bg + tp
@@ -656,6 +676,9 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
       LAUNCH(kd::k_grad_hor, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So.ep, c->gz, c->gx, c->gy);
       LAUNCH(kd::k_pgrad, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So, c->gx, c->gy, c->gz, c->tvu, c->tvv, c->tpu, c->tpv,
              P, step == 0 ? 1 : 0);
+      // into the edge arrays of theta', which nothing reads after k_pgrad, and cpw
+      if (D.ncons > 1)
+        LAUNCH(kd::k_moist_aux, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature, c->tpu, c->tpv, c->cpw);
     }
     if (rk == 2 || step == 0) {
       int rc = advection(c, Sv);
@@ -704,7 +727,9 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
                c->tsoil[so], c->tsoil[rk == 1 ? so : sn], c->tsoil[sn]);
       dim3 g2((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 7) / 8), 1);
       LAUNCH(kd::k_column_ver, g2, D, G, So, Sn, T, rk);
-      if (D.ncons > 1) LAUNCH(kd::k_column_tracers, g2, D, G, So, Sn, T.rho, c->temperature, c->csh, rk);
+      if (D.ncons > 1)
+        LAUNCH_FN("k_column_tracers", lg::launch_column_tracers(D, G, So, Sn, T.rho, c->temperature, c->rvol, c->itwdtv,
+                                                                c->tpu, c->tpv, c->cpw, c->csh, rk, c->stream));
     }
   }
   return LGAME_OK;
@@ -916,6 +941,11 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
   double** scratch[] = {&c->theta, &c->gz, &c->gx, &c->gy, &c->divf, &c->tvu, &c->tvv, &c->tpu, &c->tpv,
                         &c->ex, &c->ey, &c->ez, &c->uph, &c->vph, &c->wph, &c->vsq};
   for (double** p : scratch) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
+  if (cfg->precision == LGAME_PRECISION_FP64) {
+    if ((rc = dalloc(c, &c->rvol, F)) || (rc = dalloc(c, &c->itwdtv, F))) return fail(rc);
+    if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
+    if (column_tracers_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the tracer solver refused"));
+  }
   // diffusion closure: the carried diagnostics always, the work arrays when a part is on
   {
     DiffBuf<double>& B = c->dbuf;
@@ -1082,6 +1112,10 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     for (size_t p = 0; p < n2; ++p) sum = sum + az[p];
     c->dpar.mva = 2.0 * sum / (double)n2;
     if (c->split) split_set_diff_par(c->split, c->dpar);
+  }
+  if (c->rvol) {
+    k_volume_recip<<<grd(D, D.ny, D.nx, D.nl), blk(), 0, c->stream>>>(D, c->G.volume, c->rvol, c->itwdtv);
+    CK(cudaGetLastError());
   }
   if (c->split) {
     if ((rc = split_set_grid(c->split, c->D, c->G, c->stream)) != LGAME_OK) return rc;
