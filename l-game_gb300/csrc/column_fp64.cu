@@ -1,153 +1,250 @@
-// column_fp64.cu -- the vertically implicit part of the HEVI step, FP64, one thread per
-// column (compiled with -fmad=false).
+// column_fp64.cu -- the vertically implicit part of the HEVI step, FP64 (compiled with
+// -fmad=false: only the fma written out are fused).
 //
-// A warp owns 32 adjacent columns of one x-row, so every level load of every field is
-// one coalesced 256-byte access.  Each thread runs the Thomas algorithm of its column
-// (mo_column_solvers.F90:606-640); the forward sweep and the back substitution are
-// sequential in the level index, which is why the work is spread over the ~10^6
-// columns of the domain instead of over the levels (parallel cyclic reduction would
-// multiply the FP64 divisions by log2(n_layers), and FP64 throughput is the scarce
-// resource of this GPU).
+// A block owns a tile of columns, numbered through the plane, and cuts them into chunks of levels:
+// what can be formed level by level is (matrices, right-hand sides, new state), and only the
+// Thomas algorithm (mo_column_solvers.F90:606-640) is sequential in the level index, one thread
+// per column from shared memory.  (Parallel cyclic reduction would multiply the FP64 divisions by
+// log2(n_layers), and FP64 throughput is the scarce resource of this GPU.)
 #include "kernels.cuh"
 
 namespace lg {
 
 constexpr int kMaxLayers = 128;
 
-// a/b rounded to nearest for y = 1/b rounded to nearest: quotient, exact remainder, correction
-// (Markstein, IBM J. Res. Dev. 34, 1990): three FP64-pipe operations instead of about seven.  The
-// result is the correctly rounded quotient, except that a quotient within 2^-52 of its last place
-// from the middle of two doubles may round the other way; a zero quotient's sign is not kept, and
-// an infinite a gives NaN.
+// a/b rounded to nearest for y within two units of the last place of 1/b: quotient, remainder,
+// correction (Markstein, IBM J. Res. Dev. 34, 1990): three FP64-pipe operations instead of about
+// seven.  The result is the correctly rounded quotient, except that a quotient within 2^-50 of its
+// last place from the middle of two doubles may round the other way; a zero quotient's sign is not
+// kept, and an infinite a gives NaN.
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
   const double q = a * y;
   return fma(fma(-b, q, a), y, q);
 }
 
-// the Thomas algorithm of mo_column_solvers.F90:606-640 (arrays 1-based)
-__device__ __forceinline__ void thomas(const double* c, const double* d, const double* e, const double* r,
-                                       double* sol, double* ep, double* rp, int n) {
-  ep[1] = e[1] / d[1];
-  rp[1] = r[1] / d[1];
-  for (int jl = 2; jl <= n; ++jl) {
-    const double den = d[jl] - ep[jl - 1] * c[jl - 1];
-    if (jl <= n - 1) ep[jl] = e[jl] / den;
-    rp[jl] = (r[jl] - rp[jl - 1] * c[jl - 1]) / den;
-  }
-  sol[n] = rp[n];
-  for (int jl = n - 1; jl >= 1; --jl) sol[jl] = rp[jl] - ep[jl] * sol[jl + 1];
-}
-
 // three_band_solver_ver, mo_column_solvers.F90:21-351, plus the array-wide update of
 // theta_v_pert (:346-349) and w_free_slip (mo_inner_product.F90:52-75) of this column,
-// both of which only touch the column itself.
-__global__ void k_column_ver(Dims D, Grid<double> G, State So, State Sn, Tend<double> Tn, int rk_step) {
-  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (ji > D.ny || jk > D.nx) return;
-  const int nl = D.nl;
-  const double dtime = D.dtime;
-  const long long goff = (long long)(D.g - 1) * D.fstride;
-  const State& Su = (rk_step == 1) ? So : Sn;  // state_new_used
+// both of which only touch the column itself, with the reference's operations in its order.
+//
+// A block owns kCvCols columns and kCvChunks chunks of levels: every thread forms its chunk's rows
+// (matrix and right-hand side) into shared memory, one thread a column runs the Thomas algorithm
+// (mo_column_solvers.F90:606-640), every thread the new state of its chunk.  FP64 operations bound it
+// on large grids: grid-only factors come from arrays formed once (ColumnGrid), the reciprocals of
+// rho and of the interface density are formed once and divide by div_rn.  One thread per column with
+// fourteen arrays in local memory took 788, 2116 us a launch at 65x97x33, 192x192x80.
+constexpr int kCvCols = 16, kCvChunks = 16;
+constexpr int kCvArrays = 7;  // c (then c of the row above), d, e (then e/den), r (then the solution), interface
+                              // theta, gamma, 1/(interface density)
+
+template <int RK>
+__global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
+    k_column_ver(Dims D, Grid<double> G, ColumnGrid X, State So, State Sn, Tend<double> Tn) {
+  extern __shared__ __align__(16) double sm_cv[];
+  constexpr int S = kCvCols;
+  const int lane = threadIdx.x % S, w = threadIdx.x / S;
+  const int col = blockIdx.x * S + lane;
+  const bool valid = col < D.ny * D.nx;
+  const int ji = valid ? col % D.ny + 1 : 1, jk = valid ? col / D.ny + 1 : 1;
+  const int nl = D.nl, n = nl - 1;
+  const double dtime = D.dtime, rdt = X.rdt;
+  const long long goff = (long long)(D.g - 1) * D.fstride, pl = D.plane, c0 = IX(D, ji, jk, 1);
+  const State& Su = (RK == 1) ? So : Sn;  // state_new_used
   const double* rho_o = So.rho + goff;
   const double* rho_u = Su.rho + goff;
   double* rho_n = Sn.rho + goff;
   const double* t_rho = Tn.rho + goff;
   const double pdw = 0.5;
-
-  double alpha[kMaxLayers + 1], beta[kMaxLayers + 1], gammaa[kMaxLayers + 1];
-  double rho_expl[kMaxLayers + 1], rt_expl[kMaxLayers + 1], ep_expl[kMaxLayers + 1], tp_expl[kMaxLayers + 1];
-  double rio[kMaxLayers + 1], rie[kMaxLayers + 1], ti[kMaxLayers + 1];
-  double cv[kMaxLayers + 1], dv[kMaxLayers + 1], evec[kMaxLayers + 1], rv[kMaxLayers + 1];
-  double sol[kMaxLayers + 1], epr[kMaxLayers + 1], rpr[kMaxLayers + 1];
-
-  for (int jl = 1; jl <= nl; ++jl) {
-    const long long i = IX(D, ji, jk, jl);
-    const double V = G.volume[i];
-    rho_expl[jl] = rho_o[i] + dtime * t_rho[i];
-    rt_expl[jl] = So.rt[i] + dtime * Tn.rt[i];
-    if (rk_step == 1) {
-      alpha[jl] = -So.rt[i] / (rho_o[i] * rho_o[i]) / V;
-      beta[jl] = 1.0 / rho_o[i] / V;
-      gammaa[jl] = kR_D / (kC_D_V * So.rt[i]) * (G.exner_bg[i] + So.ep[i]) / V;
-    } else {
-      const double alpha_old = -So.rt[i] / (rho_o[i] * rho_o[i]);
-      const double beta_old = 1.0 / rho_o[i];
-      const double gamma_old = kR_D / (kC_D_V * So.rt[i]) * (G.exner_bg[i] + So.ep[i]);
-      const double alpha_new = -Su.rt[i] / (rho_u[i] * rho_u[i]);
-      const double beta_new = 1.0 / rho_u[i];
-      const double gamma_new = kR_D / (kC_D_V * Su.rt[i]) * (G.exner_bg[i] + Su.ep[i]);
-      alpha[jl] = ((1.0 - pdw) * alpha_old + pdw * alpha_new) / V;
-      beta[jl] = ((1.0 - pdw) * beta_old + pdw * beta_new) / V;
-      gammaa[jl] = ((1.0 - pdw) * gamma_old + pdw * gamma_new) / V;
-    }
-    tp_expl[jl] = So.tp[i] + dtime * V * (alpha[jl] * t_rho[i] + beta[jl] * Tn.rt[i]);
-    ep_expl[jl] = So.ep[i] + dtime * V * gammaa[jl] * Tn.rt[i];
-  }
-  for (int jl = 1; jl <= nl - 1; ++jl) {
-    const long long a = IX(D, ji, jk, jl), b = IX(D, ji, jk, jl + 1);
-    rio[jl] = 0.5 * (rho_o[a] + rho_o[b]);
-    rie[jl] = 0.5 * (rho_expl[jl] + rho_expl[jl + 1]);
-    ti[jl] = 0.5 * (Su.rt[a] / rho_u[a] + Su.rt[b] / rho_u[b]);
-  }
+  double* const sc = sm_cv + lane;               // row jl at S*(jl-1)
+  double* const sd = sm_cv + S * nl + lane;
+  double* const se = sm_cv + 2 * S * nl + lane;
+  double* const sr = sm_cv + 3 * S * nl + lane;
+  double* const st = sm_cv + 4 * S * nl + lane;
+  double* const sg = sm_cv + 5 * S * nl + lane;  // layer jl
+  double* const sy = sm_cv + 6 * S * nl + lane;
   const double c_imp2 = kIMPL_THERMO_WEIGHT * (dtime * dtime) * kC_D_P;
-  const double c_imp1 = kIMPL_THERMO_WEIGHT * dtime * kC_D_P;
-  for (int jl = 1; jl <= nl - 1; ++jl) {
-    const long long a = IX(D, ji, jk, jl), b = IX(D, ji, jk, jl + 1);
-    const double zs0 = G.z_scalar[a], zs1 = G.z_scalar[b];
-    const double eb0 = G.exner_bg[a], eb1 = G.exner_bg[b];
-    const double dp = G.damp[b];  // prefactor at level jl+1
-    const double wo = So.w[b];
-    const double t = ti[jl];
-    dv[jl] = -(t * t) * (gammaa[jl] + gammaa[jl + 1])
-           + 0.5 * (eb0 - eb1) * (alpha[jl + 1] - alpha[jl] + t * (beta[jl + 1] - beta[jl]))
-           - (zs0 - zs1) / (c_imp2 * rio[jl])
-           * (2.0 / G.area_z[b] + dtime * wo * 0.5 * (-1.0 / G.volume[a] + 1.0 / G.volume[b])) * dp;
-    rv[jl] = -(wo + dtime * Tn.w[b]) * (zs0 - zs1) / c_imp2
-           + t * (ep_expl[jl] - ep_expl[jl + 1]) / dtime
-           + 0.5 / dtime * (tp_expl[jl] + tp_expl[jl + 1]) * (eb0 - eb1)
-           - (zs0 - zs1) / c_imp2 * wo * rie[jl] / rio[jl];
+
+  // alpha, beta, gamma over the volume, theta of state_new_used, explicit predictions
+  struct Lay { double al, be, ga, th, ro, rhe, tpe, epe, V, rV; };
+  auto layer = [&](int jl, bool predict) {
+    Lay L{};
+    const long long i = c0 + (long long)(jl - 1) * pl;
+    L.V = G.volume[i];
+    L.rV = X.rvol[i];
+    const double ro = rho_o[i], rto = So.rt[i];
+    L.ro = ro;
+    const double yo = __drcp_rn(ro);
+    double alpha = div_rn(-rto, ro * ro, yo * yo), beta = yo;
+    double gamma = kR_D / (kC_D_V * rto) * (G.exner_bg[i] + So.ep[i]);
+    if (RK == 2) {
+      const double ru = rho_u[i], rtu = Su.rt[i];
+      const double yu = __drcp_rn(ru);
+      const double alpha_new = div_rn(-rtu, ru * ru, yu * yu);
+      const double gamma_new = kR_D / (kC_D_V * rtu) * (G.exner_bg[i] + Su.ep[i]);
+      alpha = (1.0 - pdw) * alpha + pdw * alpha_new;
+      beta = (1.0 - pdw) * beta + pdw * yu;
+      gamma = (1.0 - pdw) * gamma + pdw * gamma_new;
+      L.th = div_rn(rtu, ru, yu);
+    } else {
+      L.th = div_rn(rto, ro, yo);
+    }
+    L.al = div_rn(alpha, L.V, L.rV);
+    L.be = div_rn(beta, L.V, L.rV);
+    L.ga = div_rn(gamma, L.V, L.rV);
+    if (predict) {
+      const double tr = t_rho[i], trt = Tn.rt[i], dtv = dtime * L.V;
+      L.rhe = ro + dtime * tr;
+      L.tpe = So.tp[i] + dtv * (L.al * tr + L.be * trt);
+      L.epe = So.ep[i] + dtv * L.ga * trt;
+    }
+    return L;
+  };
+
+  const int chunk = (n + kCvChunks - 1) / kCvChunks, r0 = w * chunk + 1, r1 = min(n, (w + 1) * chunk);
+  if (valid && r0 <= r1) {
+    Lay L0 = layer(r0, true), L1 = layer(r0 + 1, true), L2{};
+    double rio = 0.5 * (L0.ro + L1.ro), yrio = __drcp_rn(rio);
+    double t = 0.5 * (L0.th + L1.th);
+    for (int jl = r0; jl <= r1; ++jl) {
+      const long long b = c0 + (long long)jl * pl;  // layer jl+1 and w level jl+1
+      const double zs = X.zs[b], hdeb = X.hdeb[b], dp = G.damp[b], wo = So.w[b];
+      const double rie = 0.5 * (L0.rhe + L1.rhe);
+      const double dv = -(t * t) * (L0.ga + L1.ga) + hdeb * (L1.al - L0.al + t * (L1.be - L0.be))
+                      - div_rn(zs, c_imp2 * rio, X.rc_imp2 * yrio)
+                      * (2.0 * X.raz[b] + dtime * wo * 0.5 * (-L0.rV + L1.rV)) * dp;
+      // (0.5/dtime * (...) * d(exner_bg), with hdeb half that difference: powers of two are exact)
+      const double rv = div_rn(-(wo + dtime * Tn.w[b]) * zs, c_imp2, X.rc_imp2)
+                      + div_rn(t * (L0.epe - L1.epe), dtime, rdt)
+                      + 2.0 * (0.5 / dtime) * (L0.tpe + L1.tpe) * hdeb
+                      - div_rn(X.zs_c2[b] * wo * rie, rio, yrio);
+      double cv = 0.0, ev = 0.0, rio_n = 0.0, yrio_n = 0.0, tn = 0.0;
+      if (jl < n) {
+        L2 = layer(jl + 2, jl < r1);
+        const long long cc = b + pl;
+        tn = 0.5 * (L1.th + L2.th);
+        rio_n = 0.5 * (L1.ro + L2.ro);
+        yrio_n = __drcp_rn(rio_n);
+        cv = tn * L1.ga * t + X.hdeb[cc] * (L1.al + L1.be * t)
+           - div_rn(X.zs_c1h[cc] * So.w[cc], L1.V * rio_n, L1.rV * yrio_n) * G.damp[cc];
+        ev = t * L1.ga * tn - hdeb * (L1.al + L1.be * tn)
+           + div_rn(X.zs_c1h[b] * wo, L1.V * rio, L1.rV * yrio) * dp;
+      }
+      sc[S * (jl - 1)] = cv;
+      sd[S * (jl - 1)] = dv;
+      se[S * (jl - 1)] = ev;
+      sr[S * (jl - 1)] = rv;
+      st[S * (jl - 1)] = t;
+      sg[S * (jl - 1)] = L0.ga;
+      if (jl == n) sg[S * n] = L1.ga;
+      sy[S * (jl - 1)] = yrio;
+      L0 = L1;
+      L1 = L2;
+      rio = rio_n;
+      yrio = yrio_n;
+      t = tn;
+    }
   }
-  for (int jl = 1; jl <= nl - 2; ++jl) {
-    const long long a = IX(D, ji, jk, jl), b = IX(D, ji, jk, jl + 1), c = IX(D, ji, jk, jl + 2);
-    cv[jl] = ti[jl + 1] * gammaa[jl + 1] * ti[jl]
-           + 0.5 * (G.exner_bg[b] - G.exner_bg[c]) * (alpha[jl + 1] + beta[jl + 1] * ti[jl])
-           - (G.z_scalar[b] - G.z_scalar[c]) / c_imp1 * 0.5 * So.w[c] / (G.volume[b] * rio[jl + 1]) * G.damp[c];
-    evec[jl] = ti[jl] * gammaa[jl + 1] * ti[jl + 1]
-             - 0.5 * (G.exner_bg[a] - G.exner_bg[b]) * (alpha[jl + 1] + beta[jl + 1] * ti[jl + 1])
-             + (G.z_scalar[a] - G.z_scalar[b]) / c_imp1 * 0.5 * So.w[b] / (G.volume[b] * rio[jl]) * G.damp[b];
+  __syncthreads();
+  if (valid && w == 0) {
+    double y = __drcp_rn(sd[0]);
+    double ep = div_rn(se[0], sd[0], y), rp = div_rn(sr[0], sd[0], y);
+    se[0] = ep;
+    sr[0] = rp;
+#pragma unroll 2
+    for (int jl = 2; jl <= n; ++jl) {
+      const double c = sc[S * (jl - 2)];
+      const double den = sd[S * (jl - 1)] - ep * c;
+      y = __drcp_rn(den);
+      ep = div_rn(se[S * (jl - 1)], den, y);  // (0 in the last row)
+      rp = div_rn(sr[S * (jl - 1)] - rp * c, den, y);
+      se[S * (jl - 1)] = ep;
+      sr[S * (jl - 1)] = rp;
+    }
+#pragma unroll 4
+    for (int jl = n - 1; jl >= 1; --jl) {
+      rp = sr[S * (jl - 1)] - se[S * (jl - 1)] * rp;
+      sr[S * (jl - 1)] = rp;
+    }
   }
-  thomas(cv, dv, evec, rv, sol, epr, rpr, nl - 1);
-  for (int jl = 2; jl <= nl - 1; ++jl) {
-    const long long i = IX(D, ji, jk, jl);
-    rho_n[i] = rho_expl[jl] + dtime * (-sol[jl - 1] + sol[jl]) / G.volume[i];
-    Sn.rt[i] = rt_expl[jl] + dtime * (-(ti[jl - 1] * sol[jl - 1]) + ti[jl] * sol[jl]) / G.volume[i];
+  __syncthreads();
+  const int lchunk = (nl + kCvChunks - 1) / kCvChunks, l0 = w * lchunk + 1, l1 = min(nl, (w + 1) * lchunk);
+  if (!valid || l0 > l1) return;
+  auto new_rho = [&](int jl, double V, double rV) {
+    const long long i = c0 + (long long)(jl - 1) * pl;
+    const double rhe = rho_o[i] + dtime * t_rho[i];
+    if (jl == 1) return rhe + div_rn(dtime * sr[0], V, rV);
+    if (jl == nl) return rhe - div_rn(dtime * sr[S * (n - 1)], V, rV);
+    return rhe + div_rn(dtime * (-sr[S * (jl - 2)] + sr[S * (jl - 1)]), V, rV);
+  };
+  double rn_up = 0.0, ro_up = 0.0;
+  if (l0 > 1) {
+    const long long a = c0 + (long long)(l0 - 2) * pl;
+    rn_up = new_rho(l0 - 1, G.volume[a], X.rvol[a]);
+    ro_up = rho_o[a];
   }
-  {
-    const long long i1 = IX(D, ji, jk, 1), iN = IX(D, ji, jk, nl);
-    rho_n[i1] = rho_expl[1] + dtime * sol[1] / G.volume[i1];
-    Sn.rt[i1] = rt_expl[1] + dtime * ti[1] * sol[1] / G.volume[i1];
-    rho_n[iN] = rho_expl[nl] - dtime * sol[nl - 1] / G.volume[iN];
-    Sn.rt[iN] = rt_expl[nl] - dtime * ti[nl - 1] * sol[nl - 1] / G.volume[iN];
+  for (int jl = l0; jl <= l1; ++jl) {
+    const long long i = c0 + (long long)(jl - 1) * pl;
+    const double V = G.volume[i], rV = X.rvol[i], rto = So.rt[i], ro = rho_o[i];
+    const double rn = new_rho(jl, V, rV);
+    const double rte = rto + dtime * Tn.rt[i];
+    double rtn;
+    if (jl == 1) rtn = rte + div_rn(dtime * st[0] * sr[0], V, rV);
+    else if (jl == nl) rtn = rte - div_rn(dtime * st[S * (n - 1)] * sr[S * (n - 1)], V, rV);
+    else rtn = rte + div_rn(dtime * (-(st[S * (jl - 2)] * sr[S * (jl - 2)]) + st[S * (jl - 1)] * sr[S * (jl - 1)]), V, rV);
+    const double epn = So.ep[i] + V * sg[S * (jl - 1)] * (rtn - rto);
+    const double tpn = rtn / rn - G.theta_v_bg[i];
+    if (jl >= 2) {
+      const double rin = 0.5 * (rn_up + rn);
+      Sn.w[i] = div_rn(div_rn(2.0 * sr[S * (jl - 2)], G.area_z[i], X.raz[i]) - rin * So.w[i], 0.5 * (ro_up + ro),
+                       sy[S * (jl - 2)]);
+    }
+    rho_n[i] = rn;
+    Sn.rt[i] = rtn;
+    Sn.ep[i] = epn;
+    Sn.tp[i] = tpn;
+    rn_up = rn;
+    ro_up = ro;
   }
-  for (int jl = 2; jl <= nl; ++jl) {
-    const long long i = IX(D, ji, jk, jl);
-    const double rin = 0.5 * (rho_n[IX(D, ji, jk, jl - 1)] + rho_n[i]);
-    Sn.w[i] = (2.0 * sol[jl - 1] / G.area_z[i] - rin * So.w[i]) / rio[jl - 1];
+  if (D.freeslip && l1 == nl) {
+    Sn.w[IX(D, ji, jk, nl + 1)] =
+        W_(1, ji, jk, nl) * Sn.u[IX(D, ji, jk + 1, nl)] * G.slope_x[IX(D, ji, jk + 1, nl)]
+      + W_(2, ji, jk, nl) * Sn.v[IX(D, ji, jk, nl)] * G.slope_y[IX(D, ji, jk, nl)]
+      + W_(3, ji, jk, nl) * Sn.u[IX(D, ji, jk, nl)] * G.slope_x[IX(D, ji, jk, nl)]
+      + W_(4, ji, jk, nl) * Sn.v[IX(D, ji + 1, jk, nl)] * G.slope_y[IX(D, ji + 1, jk, nl)];
   }
-  for (int jl = 1; jl <= nl; ++jl) {
-    const long long i = IX(D, ji, jk, jl);
-    Sn.ep[i] = So.ep[i] + G.volume[i] * gammaa[jl] * (Sn.rt[i] - So.rt[i]);
-    Sn.tp[i] = Sn.rt[i] / rho_n[i] - G.theta_v_bg[i];
-  }
-  if (D.freeslip) {
-    const int n = nl;
-    Sn.w[IX(D, ji, jk, n + 1)] =
-        W_(1, ji, jk, n) * Sn.u[IX(D, ji, jk + 1, n)] * G.slope_x[IX(D, ji, jk + 1, n)]
-      + W_(2, ji, jk, n) * Sn.v[IX(D, ji, jk, n)] * G.slope_y[IX(D, ji, jk, n)]
-      + W_(3, ji, jk, n) * Sn.u[IX(D, ji, jk, n)] * G.slope_x[IX(D, ji, jk, n)]
-      + W_(4, ji, jk, n) * Sn.v[IX(D, ji + 1, jk, n)] * G.slope_y[IX(D, ji + 1, jk, n)];
-  }
+}
+
+// the grid-only factors of the vertical solve, at w level jl = 2..nl (index of layer jl) and, the
+// reciprocal of the volume, at every layer
+__global__ void k_column_grid(Dims D, Grid<double> G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
+                              double* zs_c1h, double* hdeb, double* raz) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl), a = q - D.plane;
+  rvol[q] = 1.0 / G.volume[q];
+  itwdtv[q] = 0.5 * D.dtime / G.volume[q];
+  if (jl == 1) return;
+  const double c_imp2 = kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P;
+  const double c_imp1 = kIMPL_THERMO_WEIGHT * D.dtime * kC_D_P;
+  const double z = G.z_scalar[a] - G.z_scalar[q];
+  zs[q] = z;
+  zs_c2[q] = z / c_imp2;
+  zs_c1h[q] = z / c_imp1 * 0.5;
+  hdeb[q] = 0.5 * (G.exner_bg[a] - G.exner_bg[q]);
+  raz[q] = 1.0 / G.area_z[q];
+}
+
+void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
+                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st) {
+  const dim3 g((unsigned)((D.ny + 31) / 32), (unsigned)D.nl, (unsigned)((D.nx + 7) / 8));
+  k_column_grid<<<g, dim3(32, 8), 0, st>>>(D, G, rvol, itwdtv, zs, zs_c2, zs_c1h, hdeb, raz);
+}
+
+void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,
+                       const Tend<double>& Tn, int rk_step, cudaStream_t st) {
+  const unsigned nb = (unsigned)(((long long)D.ny * D.nx + kCvCols - 1) / kCvCols);
+  const size_t sm = (size_t)kCvArrays * kCvCols * D.nl * sizeof(double);
+  if (rk_step == 1) k_column_ver<1><<<nb, kCvCols * kCvChunks, sm, st>>>(D, G, X, So, Sn, Tn);
+  else k_column_ver<2><<<nb, kCvCols * kCvChunks, sm, st>>>(D, G, X, So, Sn, Tn);
 }
 
 // x < 0 by the bits (a comparison issues on the FP64 pipe); -0 counts as negative, NaN does not
@@ -388,7 +485,11 @@ __global__ void __launch_bounds__(kTcCols* kTcChunks, 2)
 #undef TC_GROUP
 }
 
-int column_tracers_prepare() {
+int column_prepare() {
+  for (auto k : {k_column_ver<1>, k_column_ver<2>})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kCvArrays * kCvCols * kMaxLayers * (int)sizeof(double)) != cudaSuccess)
+      return 1;
   for (auto k : {k_column_tracers<true>, k_column_tracers<false>})
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kTcArrays * kTcCols * kMaxLayers * (int)sizeof(double)) != cudaSuccess)

@@ -749,12 +749,23 @@ __global__ void k_gas_theta(Dims D, Grid<T> G, StateT<V> Ss, const V* u_new, con
 __global__ void k_pgrad(Dims D, Grid<double> G, State S, const double* gx, const double* gy, const double* gz,
                         const double* tvu, const double* tvv, const double* tpu, const double* tpv, PGrad<double> P,
                         int lfirst);
-__global__ void k_column_ver(Dims D, Grid<double> G, State So, State Sn, Tend<double> Tn, int rk_step);
+// grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of
+// layer jl) z_scalar(jl-1) - z_scalar(jl), that over c_imp2 and half of it over c_imp1 (c_imp2 =
+// impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -
+// exner_bg(jl), 1/area_z; 1/c_imp2 and 1/dtime
+struct ColumnGrid {
+  const double *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
+  double rc_imp2, rdt;
+};
+void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
+                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st);
+int column_prepare();
+void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,
+                       const Tend<double>& Tn, int rk_step, cudaStream_t st);
 // once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
 // and c_p of ice and water
 __global__ void k_moist_aux(Dims D, Grid<double> G, State So, const double* T, double* vcloud, double* cpi, double* cpw);
 // the tracer solve: rvol = 1/volume, itwdtv = 0.5*dtime/volume; csh is written at rk_step 1
-int column_tracers_prepare();
 void launch_column_tracers(const Dims& D, const Grid<double>& G, const State& So, const State& Sn, const double* t_rho,
                            const double* T, const double* rvol, const double* itwdtv, const double* vcloud,
                            const double* cpi, const double* cpw, double* csh, int rk_step, cudaStream_t st);

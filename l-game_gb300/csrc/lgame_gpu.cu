@@ -85,7 +85,10 @@ struct lgame_gpu {
   bool phase = false;
   double *ptr = nullptr, *pth = nullptr;
   // scratch
-  double *rvol = nullptr, *itwdtv = nullptr;  // FP64 step: 1/volume and 0.5*dtime/volume
+  // FP64 step: grid-only factors of the column solves (ColumnGrid), 0.5*dtime/volume
+  double *rvol = nullptr, *itwdtv = nullptr, *zs = nullptr, *zs_c2 = nullptr, *zs_c1h = nullptr, *hdeb = nullptr,
+         *raz = nullptr;
+  ColumnGrid colg{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
   double* staging = nullptr;
@@ -282,14 +285,6 @@ __global__ void k_split_ipw(Dims D, const double* src, double* w1, double* w2, d
   const size_t h = 6 * ((size_t)(ji - 1) + (size_t)D.ny * ((size_t)(jk - 1) + (size_t)D.nx * (size_t)(jl - 1)));
   const long long q = IX(D, ji, jk, jl);
   w1[q] = src[h]; w2[q] = src[h + 1]; w3[q] = src[h + 2]; w4[q] = src[h + 3]; w5[q] = src[h + 4]; w6[q] = src[h + 5];
-}
-
-__global__ void k_volume_recip(Dims D, const double* volume, double* rvol, double* itwdtv) {
-  LG_IDX3;
-  if (ji > D.ny || jk > D.nx) return;
-  const long long q = IX(D, ji, jk, jl);
-  rvol[q] = 1.0 / volume[q];
-  itwdtv[q] = 0.5 * D.dtime / volume[q];
 }
 
 __global__ void k_check_finite(Dims D, State S, int* flag) {
@@ -522,7 +517,6 @@ const auto k_tend_wind = lg::k_tend_wind<double>;
 const auto k_tracers = lg::k_tracers<double>;
 const auto k_gas_theta = lg::k_gas_theta<double>;
 const auto k_pgrad = lg::k_pgrad;
-const auto k_column_ver = lg::k_column_ver;
 const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
 const auto k_diff_visc = lg::k_diff_visc<double, double>;
@@ -725,8 +719,7 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
       if (c->sfc_sens || c->sfc_soil)
         LAUNCH(kd::k_sfc_column, grd(D, D.ny, D.nx, 1), D, G, So, rk == 1 ? So : Sn, T.rt, c->sbuf, c->spar,
                c->tsoil[so], c->tsoil[rk == 1 ? so : sn], c->tsoil[sn]);
-      dim3 g2((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 7) / 8), 1);
-      LAUNCH(kd::k_column_ver, g2, D, G, So, Sn, T, rk);
+      LAUNCH_FN("k_column_ver", lg::launch_column_ver(D, G, c->colg, So, Sn, T, rk, c->stream));
       if (D.ncons > 1)
         LAUNCH_FN("k_column_tracers", lg::launch_column_tracers(D, G, So, Sn, T.rho, c->temperature, c->rvol, c->itwdtv,
                                                                 c->tpu, c->tpv, c->cpw, c->csh, rk, c->stream));
@@ -942,9 +935,12 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
                         &c->ex, &c->ey, &c->ez, &c->uph, &c->vph, &c->wph, &c->vsq};
   for (double** p : scratch) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
   if (cfg->precision == LGAME_PRECISION_FP64) {
-    if ((rc = dalloc(c, &c->rvol, F)) || (rc = dalloc(c, &c->itwdtv, F))) return fail(rc);
+    double** colg[] = {&c->rvol, &c->itwdtv, &c->zs, &c->zs_c2, &c->zs_c1h, &c->hdeb, &c->raz};
+    for (double** p : colg) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
     if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
-    if (column_tracers_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the tracer solver refused"));
+    c->colg = ColumnGrid{c->rvol, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz,
+                         1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
+    if (column_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the column solvers refused"));
   }
   // diffusion closure: the carried diagnostics always, the work arrays when a part is on
   {
@@ -1114,7 +1110,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     if (c->split) split_set_diff_par(c->split, c->dpar);
   }
   if (c->rvol) {
-    k_volume_recip<<<grd(D, D.ny, D.nx, D.nl), blk(), 0, c->stream>>>(D, c->G.volume, c->rvol, c->itwdtv);
+    launch_column_grid(D, c->G, c->rvol, c->itwdtv, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz, c->stream);
     CK(cudaGetLastError());
   }
   if (c->split) {
