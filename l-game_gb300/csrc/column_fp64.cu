@@ -6,21 +6,11 @@
 // Thomas algorithm (mo_column_solvers.F90:606-640) is sequential in the level index, one thread
 // per column from shared memory.  (Parallel cyclic reduction would multiply the FP64 divisions by
 // log2(n_layers), and FP64 throughput is the scarce resource of this GPU.)
-#include "kernels.cuh"
+#include "fp64.cuh"
 
 namespace lg {
 
 constexpr int kMaxLayers = 128;
-
-// a/b rounded to nearest for y within two units of the last place of 1/b: quotient, remainder,
-// correction (Markstein, IBM J. Res. Dev. 34, 1990): three FP64-pipe operations instead of about
-// seven.  The result is the correctly rounded quotient, except that a quotient within 2^-50 of its
-// last place from the middle of two doubles may round the other way; a zero quotient's sign is not
-// kept, and an infinite a gives NaN.
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-  const double q = a * y;
-  return fma(fma(-b, q, a), y, q);
-}
 
 // three_band_solver_ver, mo_column_solvers.F90:21-351, plus the array-wide update of
 // theta_v_pert (:346-349) and w_free_slip (mo_inner_product.F90:52-75) of this column,
@@ -245,12 +235,6 @@ void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X
   const size_t sm = (size_t)kCvArrays * kCvCols * D.nl * sizeof(double);
   if (rk_step == 1) k_column_ver<1><<<nb, kCvCols * kCvChunks, sm, st>>>(D, G, X, So, Sn, Tn);
   else k_column_ver<2><<<nb, kCvCols * kCvChunks, sm, st>>>(D, G, X, So, Sn, Tn);
-}
-
-// x < 0 by the bits (a comparison issues on the FP64 pipe); -0 counts as negative, NaN does not
-__device__ __forceinline__ bool negative(double x) {
-  const unsigned u = (unsigned)__double2hiint(x) - 0x80000000u;
-  return u < 0x7FF00000u || (u == 0x7FF00000u && __double2loint(x) == 0);
 }
 
 // v_fall_liquid, mo_derived.F90:218-263 (state_old, diag%temperature)

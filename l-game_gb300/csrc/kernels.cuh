@@ -60,44 +60,6 @@ __device__ __forceinline__ bool grad_y_cov(const Dims& D, const Grid<T>& G, cons
   return true;
 }
 
-// theta_v_adv_3rd_order x edge, mo_multiplications.F90:136-183
-template <class T, class V>
-__device__ __forceinline__ bool theta_edge_u(const Dims& D, const T* th, const T* Dv, const V* u,
-                                             T c, int ji, int jk, int jl, T* out) {
-  if (jk >= 2 && jk <= D.nx) {
-    T t = T(0.5) * (th[IX(D, ji, jk - 1, jl)] + th[IX(D, ji, jk, jl)]);
-    if (u[IX(D, ji, jk, jl)] >= V(0)) t = t - c * Dv[IX(D, ji, jk - 1, jl)];
-    else t = t - c * Dv[IX(D, ji, jk, jl)];
-    *out = t;
-    return true;
-  }
-  if (!D.periodic) return false;
-  T t = T(0.5) * (th[IX(D, ji, D.nx, jl)] + th[IX(D, ji, 1, jl)]);
-  if (u[IX(D, ji, 1, jl)] >= V(0)) t = t - c * Dv[IX(D, ji, D.nx, jl)];
-  else t = t - c * Dv[IX(D, ji, 1, jl)];
-  *out = t;
-  return true;
-}
-
-// theta_v_adv_3rd_order y edge, mo_multiplications.F90:152-200
-template <class T, class V>
-__device__ __forceinline__ bool theta_edge_v(const Dims& D, const T* th, const T* Dv, const V* v,
-                                             T c, int ji, int jk, int jl, T* out) {
-  if (ji >= 2 && ji <= D.ny) {
-    T t = T(0.5) * (th[IX(D, ji, jk, jl)] + th[IX(D, ji - 1, jk, jl)]);
-    if (v[IX(D, ji, jk, jl)] >= V(0)) t = t - c * Dv[IX(D, ji, jk, jl)];
-    else t = t - c * Dv[IX(D, ji - 1, jk, jl)];
-    *out = t;
-    return true;
-  }
-  if (!D.periodic) return false;
-  T t = T(0.5) * (th[IX(D, 1, jk, jl)] + th[IX(D, D.ny, jk, jl)]);
-  if (v[IX(D, 1, jk, jl)] >= V(0)) t = t - c * Dv[IX(D, 1, jk, jl)];
-  else t = t - c * Dv[IX(D, D.ny, jk, jl)];
-  *out = t;
-  return true;
-}
-
 // scalar_times_vector_h, mo_multiplications.F90:34-54 (state scalar and vector)
 template <class T, class V>
 __device__ __forceinline__ bool stv_h_x(const Dims& D, const V* s, const V* vx, int ji, int jk, int jl, T* r) {
@@ -119,48 +81,6 @@ __device__ __forceinline__ bool stv_h_y(const Dims& D, const V* s, const V* vy, 
   *r = T(0.5) * (T(s[IX(D, 1, jk, jl)]) + T(s[IX(D, D.ny, jk, jl)])) * T(vy[IX(D, 1, jk, jl)]);
   return true;
 }
-// the same with the scalar and the vector given as functions of the index
-template <class T, class FS, class FV>
-__device__ __forceinline__ bool stv_h_x_fn(const Dims& D, FS s, FV vx, int ji, int jk, int jl, T* r) {
-  if (jk >= 2 && jk <= D.nx) { *r = T(0.5) * (s(ji, jk - 1, jl) + s(ji, jk, jl)) * vx(ji, jk, jl); return true; }
-  if (!D.periodic) return false;
-  *r = T(0.5) * (s(ji, 1, jl) + s(ji, D.nx, jl)) * vx(ji, 1, jl);
-  return true;
-}
-template <class T, class FS, class FV>
-__device__ __forceinline__ bool stv_h_y_fn(const Dims& D, FS s, FV vy, int ji, int jk, int jl, T* r) {
-  if (ji >= 2 && ji <= D.ny) { *r = T(0.5) * (s(ji - 1, jk, jl) + s(ji, jk, jl)) * vy(ji, jk, jl); return true; }
-  if (!D.periodic) return false;
-  *r = T(0.5) * (s(1, jk, jl) + s(D.ny, jk, jl)) * vy(1, jk, jl);
-  return true;
-}
-
-// scalar_times_vector_h_upstream, mo_multiplications.F90:222-285
-template <class T, class V>
-__device__ __forceinline__ bool upstream_x(const Dims& D, const V* s, const V* vx, int ji, int jk, int jl, T* r) {
-  if (jk >= 2 && jk <= D.nx) {
-    const V u = vx[IX(D, ji, jk, jl)];
-    *r = (u >= V(0)) ? T(s[IX(D, ji, jk - 1, jl)]) * T(u) : T(s[IX(D, ji, jk, jl)]) * T(u);
-    return true;
-  }
-  if (!D.periodic) return false;
-  const V u = vx[IX(D, ji, 1, jl)];
-  *r = (u >= V(0)) ? T(s[IX(D, ji, D.nx, jl)]) * T(u) : T(s[IX(D, ji, 1, jl)]) * T(u);
-  return true;
-}
-template <class T, class V>
-__device__ __forceinline__ bool upstream_y(const Dims& D, const V* s, const V* vy, int ji, int jk, int jl, T* r) {
-  if (ji >= 2 && ji <= D.ny) {
-    const V v = vy[IX(D, ji, jk, jl)];
-    *r = (v >= V(0)) ? T(s[IX(D, ji, jk, jl)]) * T(v) : T(s[IX(D, ji - 1, jk, jl)]) * T(v);
-    return true;
-  }
-  if (!D.periodic) return false;
-  const V v = vy[IX(D, 1, jk, jl)];
-  *r = (v >= V(0)) ? T(s[IX(D, 1, jk, jl)]) * T(v) : T(s[IX(D, D.ny, jk, jl)]) * T(v);
-  return true;
-}
-
 // sum(state%rho(:,:,:,1:nc+1),4) in constituent order
 template <class T, class V>
 __device__ __forceinline__ T rho_sum_cond_gas(const Dims& D, const V* rho, long long q) {
@@ -467,22 +387,6 @@ __global__ void k_div_h(Dims D, Grid<T> G, const T* vx, const T* vy, T* out) {
   out[IX(D, ji, jk, jl)] = div_h_at<T>(D, G, fx, fy, ji, jk, jl);
 }
 
-// theta_v_adv_3rd_order edge values, mo_multiplications.F90:134-202
-template <class T, class V = double>
-__global__ void k_theta_edges(Dims D, Grid<T> G, const T* th, const T* Dv, const V* u, const V* v,
-                              T* tvu, T* tvv) {
-  LG_IDX3;
-  const T c = cvt<T>(D.theta_edge_c);
-  if (ji <= D.ny && jk <= D.nx + 1) {
-    T t;
-    if (theta_edge_u<T>(D, th, Dv, u, c, ji, jk, jl, &t)) tvu[IX(D, ji, jk, jl)] = t;
-  }
-  if (ji <= D.ny + 1 && jk <= D.nx) {
-    T t;
-    if (theta_edge_v<T>(D, th, Dv, v, c, ji, jk, jl, &t)) tvv[IX(D, ji, jk, jl)] = t;
-  }
-}
-
 // calc_pot_vort, mo_vorticities.F90:189-421 with rel_vort :19-187 inlined:
 // eta_x (ny+1,nx,nl+1) and eta_y (ny,nx+1,nl+1)
 template <class T, class V = double>
@@ -641,114 +545,7 @@ __global__ void k_tend_wind(Dims D, State So, State Sn, Tend<T> Tn, Carried<T> C
   }
 }
 
-// scalar_tend_expl for every constituent other than the gas, mo_scalar_tend_expl.F90:102-128
-// with scalar_times_vector_h_upstream (mo_multiplications.F90:206-287) and div_h_tracers
-// (mo_divergence_operators.F90:70-147) evaluated inline.
-template <class T, class V = double>
-__device__ __forceinline__ void tracers_body(const Dims& D, const Grid<T>& G, const StateT<V>& Ss, const V* u_new,
-                                             const V* v_new, T* t_rho, int rk_step, const T* mdt,
-                                             const T* ptr) {
-  LG_IDX3;
-  if (ji > D.ny || jk > D.nx) return;
-  const long long q = IX(D, ji, jk, jl);
-  auto wx = [&](int i, int j, int k) { return T(u_new[IX(D, i, j, k)]); };
-  auto wy = [&](int i, int j, int k) { return T(v_new[IX(D, i, j, k)]); };
-  // contravariant vertical velocity corrections do not depend on the constituent
-  T cu = T(0), cl = T(0);
-  if (jl == D.nf) cl = vcc<T>(D, G, wx, wy, ji, jk, jl + 1);
-  else if (jl == D.nl) cu = vcc<T>(D, G, wx, wy, ji, jk, jl);
-  else if (jl > D.nf) { cu = vcc<T>(D, G, wx, wy, ji, jk, jl); cl = vcc<T>(D, G, wx, wy, ji, jk, jl + 1); }
-  const T new_weight = (rk_step == 2) ? T(0.5) : T(1);
-  const T old_weight = T(1) - new_weight;
-  for (int jc = 1; jc <= D.ncons; ++jc) {
-    if (jc == D.g) continue;
-    const V* r = Ss.rho + (long long)(jc - 1) * D.fstride;
-    auto fx = [&](int i, int j, int k) { T f; return upstream_x<T>(D, r, u_new, i, j, k, &f) ? f : T(0); };
-    auto fy = [&](int i, int j, int k) { T f; return upstream_y<T>(D, r, v_new, i, j, k, &f) ? f : T(0); };
-    const T comp_h = fx(ji, jk + 1, jl) * G.area_x[IX(D, ji, jk + 1, jl)]
-                   + fy(ji, jk, jl) * G.area_y[IX(D, ji, jk, jl)]
-                   - fx(ji, jk, jl) * G.area_x[IX(D, ji, jk, jl)]
-                   - fy(ji + 1, jk, jl) * G.area_y[IX(D, ji + 1, jk, jl)];
-    T comp_v = T(0);
-    if (jl == D.nf) {
-      const T dl = (cl <= T(0)) ? T(r[IX(D, ji, jk, jl)]) : T(r[IX(D, ji, jk, jl + 1)]);
-      comp_v = -dl * cl * G.area_z[IX(D, ji, jk, jl + 1)];
-    } else if (jl == D.nl) {
-      const T du = (cu <= T(0)) ? T(r[IX(D, ji, jk, jl - 1)]) : T(r[IX(D, ji, jk, jl)]);
-      comp_v = du * cu * G.area_z[IX(D, ji, jk, jl)];
-    } else if (jl > D.nf) {
-      const T du = (cu <= T(0)) ? T(r[IX(D, ji, jk, jl - 1)]) : T(r[IX(D, ji, jk, jl)]);
-      const T dl = (cl <= T(0)) ? T(r[IX(D, ji, jk, jl)]) : T(r[IX(D, ji, jk, jl + 1)]);
-      comp_v = du * cu * G.area_z[IX(D, ji, jk, jl)] - dl * cl * G.area_z[IX(D, ji, jk, jl + 1)];
-    }
-    const T div = (comp_h + comp_v) / G.volume[q];
-    T* t = t_rho + (long long)(jc - 1) * D.fstride;
-    T f = -div;
-    if (mdt) f = f + mdt[q + (long long)(jc - 1) * D.fstride];  // mass diffusion
-    // phase transitions (null: off, the reference's zero); vapour takes rate nc+1
-    if (ptr) f = f + ptr[q + (long long)((jc < D.g ? jc : D.g) - 1) * D.fstride];
-    t[q] = old_weight * t[q] + new_weight * f;
-  }
-}
-
-template <class T, class V = double>
-__global__ void k_tracers(Dims D, Grid<T> G, StateT<V> Ss, const V* u_new, const V* v_new, T* t_rho, int rk_step,
-                          const T* mdt, const T* ptr) {
-  tracers_body<T, V>(D, G, Ss, u_new, v_new, t_rho, rk_step, mdt, ptr);
-}
-
-// scalar_tend_expl for the gas and the rho*theta_v tendency, mo_scalar_tend_expl.F90:106-177
-template <class T, class V = double>
-__global__ void k_gas_theta(Dims D, Grid<T> G, StateT<V> Ss, const V* u_new, const V* v_new, const T* tvu,
-                            const T* tvv, const T* Tm, const T* hd, const T* rad, const T* csh, T* t_rho,
-                            T* t_rt, const T* mdt, const T* tdh, const T* ptr, const T* pth) {
-  LG_IDX3;
-  if (ji > D.ny || jk > D.nx) return;
-  const long long q = IX(D, ji, jk, jl);
-  const V* rg = Ss.rho + (long long)(D.g - 1) * D.fstride;
-  auto fx = [&](int i, int j, int k) { T f; return stv_h_x<T>(D, rg, u_new, i, j, k, &f) ? f : T(0); };
-  auto fy = [&](int i, int j, int k) { T f; return stv_h_y<T>(D, rg, v_new, i, j, k, &f) ? f : T(0); };
-  const T div_m = div_h_at<T>(D, G, fx, fy, ji, jk, jl);
-  // old_weight 0, new_weight 1 for the gas; mass diffusion and the phase transitions' vapour
-  // rate (null: off)
-  const T mdg = mdt ? mdt[q + (long long)(D.g - 1) * D.fstride] : T(0);
-  const T ptg = ptr ? ptr[q + (long long)(D.g - 1) * D.fstride] : T(0);
-  T tg = mdt ? -div_m + mdg : -div_m;
-  if (ptr) tg = tg + ptg;
-  t_rho[q + (long long)(D.g - 1) * D.fstride] = tg;
-  T div_t;
-  if (D.theta_order == 2) {
-    auto th = [&](int i, int j, int k) { const long long p = IX(D, i, j, k); return G.theta_v_bg[p] + T(Ss.tp[p]); };
-    auto gx = [&](int i, int j, int k) { T f; return stv_h_x_fn<T>(D, th, fx, i, j, k, &f) ? f : T(0); };
-    auto gy = [&](int i, int j, int k) { T f; return stv_h_y_fn<T>(D, th, fy, i, j, k, &f) ? f : T(0); };
-    div_t = div_h_at<T>(D, G, gx, gy, ji, jk, jl);
-  } else {
-    auto gx = [&](int i, int j, int k) { return tvu[IX(D, i, j, k)] * fx(i, j, k); };
-    auto gy = [&](int i, int j, int k) { return tvv[IX(D, i, j, k)] * fy(i, j, k); };
-    div_t = div_h_at<T>(D, G, gx, gy, ji, jk, jl);
-  }
-  // dissipative heating, radiation, phase transitions (null: off), sediment heating and
-  // temperature diffusion, in the reference's order
-  T heat = hd[q] + rad[q];
-  if (pth) heat = heat + pth[q];
-  heat = heat + csh[q];
-  if (tdh) heat = heat + tdh[q];
-  T x = T(0);
-  if (heat != T(0)) {
-    const T cv = c_v_mass_weighted_air<T>(D, Ss.rho, Tm, q);
-    x = T(kC_D_V) * T(rg[q]) / cv * heat / (T(kC_D_P) * (G.exner_bg[q] + T(Ss.ep[q])));
-  }
-  T r = -div_t + x;
-  // (phase transition rate + mass diffusion of the gas) * theta_v
-  if (ptr) r = r + (ptg + mdg) * (G.theta_v_bg[q] + T(Ss.tp[q]));
-  else if (mdt) r = r + mdg * (G.theta_v_bg[q] + T(Ss.tp[q]));
-  t_rt[q] = r;
-}
-
-// ---- FP64-only kernels (kernels_fp64.cu, column_fp64.cu) -------------------------------
-__global__ void k_pgrad(Dims D, Grid<double> G, State S, const double* gx, const double* gy, const double* gz,
-                        const double* tvu, const double* tvv, const double* tpu, const double* tpv, PGrad<double> P,
-                        int lfirst);
+// ---- FP64-only kernels (column_fp64.cu; the explicit ones: fp64.cuh) --------------------
 // grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of
 // layer jl) z_scalar(jl-1) - z_scalar(jl), that over c_imp2 and half of it over c_imp1 (c_imp2 =
 // impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -

@@ -1,26 +1,411 @@
-// kernels_fp64.cu -- the FP64 pressure-gradient kernel of the HEVI step (compiled with
-// -fmad=false).  The other explicit kernels are templates in kernels.cuh, instantiated
-// for double by lgame_gpu.cu (same compiler flags).
-#include "kernels.cuh"
+// kernels_fp64.cu -- explicit kernels of the FP64 step (compiled with -fmad=false: only the fma
+// written out are fused), in the reference's operand order, so with its bits.
+//
+// All are bound by the FP64 pipe (fp64.cuh), so each is written for few of its operations: a
+// product that two cells or two interfaces share is formed once (at the face, or carried down the
+// column), metrics divide by their stored reciprocals, halves are taken in the exponent, and sums do
+// not start with 0 + x.
+#include "fp64.cuh"
 
 namespace lg {
 
-// manage_p_grad, mo_p_grad.F90:20-104, after the gradients of exner_pert (gx,gy,gz)
-// and, for theta_adv_order 3, the edge values of theta (tvu,tvv) and theta' (tpu,tpv)
-// are known; also calc_p_grad_condensates_v, mo_p_grad.F90:106-120 (identical at both
-// substeps because it always reads state_old).
-__global__ void k_pgrad(Dims D, Grid<double> G, State S, const double* gx, const double* gy, const double* gz,
-                        const double* tvu, const double* tvv, const double* tpu, const double* tpv,
-                        PGrad<double> P, int lfirst) {
+namespace {
+
+constexpr int kMarch = 8;  // levels of a marching thread's chunk (blockIdx.z)
+dim3 march_grid(const Dims& D) {
+  return dim3((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 3) / 4), (unsigned)((D.nl + kMarch - 1) / kMarch));
+}
+dim3 cell_grid(int rows, int cols, int levs) {
+  return dim3((unsigned)((rows + 31) / 32), (unsigned)levs, (unsigned)((cols + 7) / 8));
+}
+const dim3 kMarchBlock(32, 4), kCellBlock(32, 8);
+
+__global__ void k64_recip(Dims D, Grid<double> G, double* rdx, double* rdy, double* rdz) {
+  LG_IDX3;
+  const long long q = IX(D, ji, jk, jl);
+  if (ji <= D.ny && jk <= D.nx + 1) rdx[q] = 1.0 / G.dx[q];
+  if (ji <= D.ny + 1 && jk <= D.nx) rdy[q] = 1.0 / G.dy[q];
+  if (ji <= D.ny && jk <= D.nx) rdz[q] = 1.0 / G.dz[q];
+}
+
+// ---- gradient of a scalar, mo_gradient_operators.F90:17-130 -----------------------------------------
+// The vertical gradient gz at w levels 2..nl and, in the terrain-following layers, each column's
+// two products of the remap to the horizontal faces (mo_averaging.F90:56-136), W5(l)*gz(l) and
+// W6(l)*gz(l+1), which the four faces of the column share.  gz_sfc: gz at level nl+1 (never written
+// by grad_vert) as the array holds it.
+__global__ void __launch_bounds__(128) k64_grad_vert(Dims D, Grid<double> G, const double* rdz, const double* s, double* gz,
+                                                     double* w5, double* w6) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  long long q = IX(D, ji, jk, l0);
+  double cur = s[q];
+  double g = (l0 >= 2) ? div_rn(s[q - D.plane] - cur, G.dz[q], rdz[q]) : 0.0;
+  for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
+    double gn = 0.0;
+    if (jl < D.nl) {
+      const double nxt = s[q + D.plane];
+      gn = div_rn(cur - nxt, G.dz[q + D.plane], rdz[q + D.plane]);
+      cur = nxt;
+    }
+    if (jl >= 2) gz[q] = g;
+    if (jl > D.nf) {
+      w5[q] = G.ipw[4][q] * g;
+      if (jl < D.nl) w6[q] = G.ipw[5][q] * gn;
+      else if (D.freeslip) w6[q] = G.ipw[5][q] * gz[q + D.plane];
+    }
+    g = gn;
+  }
+}
+
+// the horizontal gradient at u and v points; false where the reference leaves the point untouched
+__device__ __forceinline__ bool grad_x64(const Dims& D, const Grid<double>& G, const double* rdx, const double* s,
+                                         const double* w5, const double* w6, int ji, int jk, int jl, double* r) {
+  const bool inner = jk >= 2 && jk <= D.nx;
+  if (!inner && !D.periodic) return false;
+  const long long a = IX(D, ji, inner ? jk - 1 : D.nx, jl), b = IX(D, ji, inner ? jk : 1, jl);
+  double g = div_rn(s[b] - s[a], G.dx[b], rdx[b]);
+  if (jl > D.nf) {
+    double m = w5[a] + w5[b];
+    if (jl < D.nl || D.freeslip) m = m + w6[a] + w6[b];
+    g = g - G.slope_x[IX(D, ji, jk, jl)] * half(m);
+  }
+  *r = g;
+  return true;
+}
+__device__ __forceinline__ bool grad_y64(const Dims& D, const Grid<double>& G, const double* rdy, const double* s,
+                                         const double* w5, const double* w6, int ji, int jk, int jl, double* r) {
+  const bool inner = ji >= 2 && ji <= D.ny;
+  if (!inner && !D.periodic) return false;
+  const long long a = IX(D, inner ? ji - 1 : D.ny, jk, jl), b = IX(D, inner ? ji : 1, jk, jl);
+  double g = div_rn(s[a] - s[b], G.dy[b], rdy[b]);
+  if (jl > D.nf) {
+    double m = w5[a] + w5[b];
+    if (jl < D.nl || D.freeslip) m = m + w6[a] + w6[b];
+    g = g - G.slope_y[IX(D, ji, jk, jl)] * half(m);
+  }
+  *r = g;
+  return true;
+}
+__global__ void k64_grad_hor(Dims D, Grid<double> G, Recip R, const double* s, const double* w5, const double* w6,
+                             double* rx, double* ry) {
+  LG_IDX3;
+  double r;
+  if (ji <= D.ny && jk <= D.nx + 1 && grad_x64(D, G, R.dx, s, w5, w6, ji, jk, jl, &r)) rx[IX(D, ji, jk, jl)] = r;
+  if (ji <= D.ny + 1 && jk <= D.nx && grad_y64(D, G, R.dy, s, w5, w6, ji, jk, jl, &r)) ry[IX(D, ji, jk, jl)] = r;
+}
+
+// ---- divergence of a horizontal vector, mo_divergence_operators.F90:16-68 ---------------------------
+// A face hands its two cells the flux f*area and, in the terrain-following layers, the slope term
+// 0.5*f*slope of the contravariant vertical velocity (mo_averaging.F90:16-54).  The faces of a
+// non-periodic boundary, which the reference leaves untouched at 0, are written as 0: the arrays serve
+// several fields in turn.
+__device__ __forceinline__ void face_x(const Dims& D, const Grid<double>& G, double f, const Faces& F, int jl, long long q) {
+  F.px[q] = f * G.area_x[q];
+  if (jl > D.nf) F.hx[q] = half(f) * G.slope_x[q];
+}
+__device__ __forceinline__ void face_y(const Dims& D, const Grid<double>& G, double f, const Faces& F, int jl, long long q) {
+  F.py[q] = f * G.area_y[q];
+  if (jl > D.nf) F.hy[q] = half(f) * G.slope_y[q];
+}
+
+// the vertical part of a column's divergence, walked down: the reference's sum at an interface runs
+// over the four slope terms of the layer above and then of the layer below, so the sum over a layer's
+// own terms serves as the start of the interface below it
+struct SlopeTerms { double a, b, c, d; };
+__device__ __forceinline__ SlopeTerms slope_terms(const Dims& D, const Grid<double>& G, const double* hx, const double* hy,
+                                                  long long q) {
+  return SlopeTerms{hx[q + D.P] * G.ipw[0][q], hy[q] * G.ipw[1][q], hx[q] * G.ipw[2][q], hy[q + 1] * G.ipw[3][q]};
+}
+__device__ __forceinline__ double own_sum(const SlopeTerms& t) { return -t.a - t.b - t.c - t.d; }
+__device__ __forceinline__ double join(double above, const SlopeTerms& t) { return above - t.a - t.b - t.c - t.d; }
+
+// the contravariant correction at interface l = nf+1..nl of the layers above and below it
+struct Contra {
+  double sum;  // own_sum of the current layer
+  // at the chunk's first level l0 (> nf): the correction at its upper interface
+  __device__ __forceinline__ double start(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, long long q,
+                                          int l0) {
+    const SlopeTerms t = slope_terms(D, G, hx, hy, q);
+    sum = own_sum(t);
+    if (l0 == D.nf + 1) return sum;
+    return join(own_sum(slope_terms(D, G, hx, hy, q - D.plane)), t);
+  }
+  // the correction at the lower interface of layer jl (jl == nf, or nf < jl < nl); q: layer jl
+  __device__ __forceinline__ double below(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, long long q,
+                                          int jl) {
+    const SlopeTerms t = slope_terms(D, G, hx, hy, q + D.plane);
+    const double r = (jl == D.nf) ? own_sum(t) : join(sum, t);
+    sum = own_sum(t);
+    return r;
+  }
+};
+struct ColumnDiv {
+  Contra c;
+  double up;  // correction times area at the upper interface
+  __device__ __forceinline__ void start(const Dims& D, const Grid<double>& G, const Faces& F, long long q, int l0) {
+    up = 0.0;
+    c.sum = 0.0;
+    if (l0 > D.nf) up = c.start(D, G, F.hx, F.hy, q, l0) * G.area_z[q];
+  }
+  // divergence of layer jl
+  __device__ __forceinline__ double step(const Dims& D, const Grid<double>& G, const Faces& F, double V, double rV, long long q,
+                                         int jl) {
+    double s = F.px[q + D.P] + F.py[q] - F.px[q] - F.py[q + 1];
+    double lo = 0.0;
+    if (jl == D.nf || (jl > D.nf && jl < D.nl)) lo = c.below(D, G, F.hx, F.hy, q, jl) * G.area_z[q + D.plane];
+    if (jl == D.nf) s = s - lo;
+    else if (jl == D.nl) s = s + up;
+    else if (jl > D.nf) s = s + (up - lo);
+    up = lo;
+    return div_rn(s, V, rV);
+  }
+};
+
+// faces of the gradient of a scalar, and their divergence (theta_v_adv_3rd_order)
+__global__ void k64_grad_faces(Dims D, Grid<double> G, Recip R, const double* s, const double* w5, const double* w6, Faces F) {
+  LG_IDX3;
+  double r;
+  if (ji <= D.ny && jk <= D.nx + 1)
+    face_x(D, G, grad_x64(D, G, R.dx, s, w5, w6, ji, jk, jl, &r) ? r : 0.0, F, jl, IX(D, ji, jk, jl));
+  if (ji <= D.ny + 1 && jk <= D.nx)
+    face_y(D, G, grad_y64(D, G, R.dy, s, w5, w6, ji, jk, jl, &r) ? r : 0.0, F, jl, IX(D, ji, jk, jl));
+}
+__global__ void __launch_bounds__(128) k64_div(Dims D, Grid<double> G, const double* rvol, Faces F, double* out) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  long long q = IX(D, ji, jk, l0);
+  ColumnDiv c;
+  c.start(D, G, F, q, l0);
+  for (int jl = l0; jl <= l1; ++jl, q += D.plane) out[q] = c.step(D, G, F, G.volume[q], rvol[q], q, jl);
+}
+
+// theta_v_adv_3rd_order edge values, mo_multiplications.F90:134-202
+__global__ void k64_theta_edges(Dims D, const double* th, const double* Dv, const double* u, const double* v, double* tvu,
+                                double* tvv) {
+  LG_IDX3;
+  const double c = D.theta_edge_c;
+  if (ji <= D.ny && jk <= D.nx + 1) {
+    const bool inner = jk >= 2 && jk <= D.nx;
+    if (inner || D.periodic) {
+      const long long a = IX(D, ji, inner ? jk - 1 : D.nx, jl), b = IX(D, ji, inner ? jk : 1, jl);
+      tvu[IX(D, ji, jk, jl)] = half(th[a] + th[b]) - c * Dv[upwind(u[b]) ? a : b];
+    }
+  }
+  if (ji <= D.ny + 1 && jk <= D.nx) {
+    const bool inner = ji >= 2 && ji <= D.ny;
+    if (inner || D.periodic) {
+      const long long a = IX(D, inner ? ji : 1, jk, jl), b = IX(D, inner ? ji - 1 : D.ny, jk, jl);
+      tvv[IX(D, ji, jk, jl)] = half(th[a] + th[b]) - c * Dv[upwind(v[a]) ? a : b];
+    }
+  }
+}
+
+// ---- scalar tendencies, mo_scalar_tend_expl.F90:106-177 ---------------------------------------------
+// faces of the gas mass flux and of the theta_v flux (theta_order 3: edge values tvu, tvv; 2: the
+// mean of the two cells)
+__global__ void k64_gas_faces(Dims D, Grid<double> G, StateT<double> Ss, const double* u_new, const double* v_new,
+                              const double* tvu, const double* tvv, Faces M, Faces T) {
+  LG_IDX3;
+  const double* rg = Ss.rho + (long long)(D.g - 1) * D.fstride;
+  auto th = [&](long long p) { return G.theta_v_bg[p] + Ss.tp[p]; };
+  if (ji <= D.ny && jk <= D.nx + 1) {
+    const bool inner = jk >= 2 && jk <= D.nx;
+    const long long q = IX(D, ji, jk, jl);
+    double f = 0.0, g = 0.0;  // (a non-periodic boundary's faces carry no flux)
+    if (inner || D.periodic) {
+      const long long a = IX(D, ji, inner ? jk - 1 : D.nx, jl), b = IX(D, ji, inner ? jk : 1, jl);
+      f = half(rg[a] + rg[b]) * u_new[b];
+      g = D.theta_order == 2 ? half(th(a) + th(b)) * f : tvu[q] * f;
+    }
+    face_x(D, G, f, M, jl, q);
+    face_x(D, G, g, T, jl, q);
+  }
+  if (ji <= D.ny + 1 && jk <= D.nx) {
+    const bool inner = ji >= 2 && ji <= D.ny;
+    const long long q = IX(D, ji, jk, jl);
+    double f = 0.0, g = 0.0;
+    if (inner || D.periodic) {
+      const long long a = IX(D, inner ? ji - 1 : D.ny, jk, jl), b = IX(D, inner ? ji : 1, jk, jl);
+      f = half(rg[a] + rg[b]) * v_new[b];
+      g = D.theta_order == 2 ? half(th(a) + th(b)) * f : tvv[q] * f;
+    }
+    face_y(D, G, f, M, jl, q);
+    face_y(D, G, g, T, jl, q);
+  }
+}
+
+// their divergences and the diabatic term: the gas and rho*theta_v tendencies (k_gas_theta<double>
+// formed every face two to five times and c_p of every condensate anew: 2084 us a launch at
+// 192x192x80)
+__global__ void __launch_bounds__(128) k64_gas_theta(Dims D, Grid<double> G, StateT<double> Ss, const double* rvol, Faces M,
+                                                     Faces T, const double* cpi, const double* cpw, const double* hd,
+                                                     const double* rad, const double* csh, double* t_rho, double* t_rt,
+                                                     const double* mdt, const double* tdh, const double* ptr,
+                                                     const double* pth) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  const long long goff = (long long)(D.g - 1) * D.fstride;
+  long long q = IX(D, ji, jk, l0);
+  ColumnDiv cm, ct;
+  cm.start(D, G, M, q, l0);
+  ct.start(D, G, T, q, l0);
+  for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
+    const double V = G.volume[q], rV = rvol[q];
+    const double div_m = cm.step(D, G, M, V, rV, q, jl), div_t = ct.step(D, G, T, V, rV, q, jl);
+    double heat = hd[q] + rad[q];
+    if (pth) heat = heat + pth[q];
+    heat = heat + csh[q];
+    if (tdh) heat = heat + tdh[q];
+    double r = -div_t;
+    if (nonzero(heat)) {
+      const double rg = Ss.rho[q + goff];
+      double cv;  // c_v_mass_weighted_air, mo_derived.F90:157-187 (odd constituents are ice)
+      if (D.lmoist) {
+        const double ci = cpi[q], cw = cpw[q];
+        cv = Ss.rho[q] * ci;
+        for (int jc = 2; jc <= D.nc; ++jc) cv = cv + Ss.rho[q + (long long)(jc - 1) * D.fstride] * ((jc & 1) ? ci : cw);
+        const double rv = Ss.rho[q + goff + D.fstride];
+        cv = cv + (rg - rv) * kC_D_V;
+        cv = cv + rv * kC_V_V;
+      } else {
+        cv = rg * kC_D_V;
+      }
+      r = r + kC_D_V * rg / cv * heat / (kC_D_P * (G.exner_bg[q] + Ss.ep[q]));
+    }
+    double tg = -div_m;
+    if (mdt) tg = tg + mdt[q + goff];
+    if (ptr) {
+      const double ptg = ptr[q + goff];
+      tg = tg + ptg;
+      r = r + (mdt ? ptg + mdt[q + goff] : ptg) * (G.theta_v_bg[q] + Ss.tp[q]);
+    } else if (mdt) {
+      r = r + mdt[q + goff] * (G.theta_v_bg[q] + Ss.tp[q]);
+    }
+    t_rho[q + goff] = tg;
+    t_rt[q] = r;
+  }
+}
+
+// the contravariant correction of the new wind at the interfaces nf+1..nl, for the tracers
+__global__ void __launch_bounds__(128) k64_contra(Dims D, Grid<double> G, const double* hx, const double* hy, double* cw) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = max((int)blockIdx.z * kMarch + 1, D.nf + 1), l1 = min(D.nl, (int)(blockIdx.z + 1) * kMarch);
+  if (l0 > l1) return;
+  long long q = IX(D, ji, jk, l0);
+  Contra c;
+  cw[q] = c.start(D, G, hx, hy, q, l0);
+  for (int jl = l0 + 1; jl <= l1; ++jl) {
+    cw[q + D.plane] = c.below(D, G, hx, hy, q, jl - 1);
+    q += D.plane;
+  }
+}
+__global__ void k64_wind_slopes(Dims D, Grid<double> G, const double* u, const double* v, double* hx, double* hy) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.z * blockDim.y + threadIdx.y + 1;
-  const int jl = blockIdx.y + 1;
-  const double use_bg_switch = D.luse_bg ? 1.0 : 0.0;
-  auto theta = [&](int i, int j, int k) { const long long q = IX(D, i, j, k); return G.theta_v_bg[q] + S.tp[q]; };
-  auto thetap = [&](int i, int j, int k) { return S.tp[IX(D, i, j, k)]; };
-  auto decel = [&](int i, int j, int k) {
-    const long long q = IX(D, i, j, k);
-    return kC_D_P * S.rho[q + (long long)(D.g - 1) * D.fstride] / rho_sum_cond_gas<double>(D, S.rho, q);
+  const int jl = blockIdx.y + D.nf + 1;
+  const long long q = IX(D, ji, jk, jl);
+  if (ji <= D.ny && jk <= D.nx + 1) hx[q] = half(u[q]) * G.slope_x[q];
+  if (ji <= D.ny + 1 && jk <= D.nx) hy[q] = half(v[q]) * G.slope_y[q];
+}
+
+// scalar_tend_expl for the tracers, mo_scalar_tend_expl.F90:24-104, with
+// scalar_times_vector_h_upstream (mo_multiplications.F90:206-287) and div_h_tracers
+// (mo_divergence_operators.F90:70-147): velocity, area and upwind cell of each of a cell's six faces
+// are found once for all tracers.  At the first substep the old tendency has weight 0 and is not read.
+__global__ void __launch_bounds__(256) k64_tracers(Dims D, Grid<double> G, const double* rvol, StateT<double> Ss,
+                                                   const double* u_new, const double* v_new, const double* cw, double* t_rho,
+                                                   int rk_step, const double* mdt, const double* ptr) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl);
+  struct F { double v, a; long long i; };
+  auto fx = [&](int kf) {
+    const bool inner = kf >= 2 && kf <= D.nx;
+    F f{0.0, 0.0, q};
+    if (!inner && !D.periodic) return f;
+    f.v = u_new[IX(D, ji, inner ? kf : 1, jl)];
+    f.a = G.area_x[IX(D, ji, kf, jl)];
+    f.i = IX(D, ji, upwind(f.v) ? (inner ? kf - 1 : D.nx) : (inner ? kf : 1), jl);
+    return f;
+  };
+  auto fy = [&](int i_f) {
+    const bool inner = i_f >= 2 && i_f <= D.ny;
+    F f{0.0, 0.0, q};
+    if (!inner && !D.periodic) return f;
+    f.v = v_new[IX(D, inner ? i_f : 1, jk, jl)];
+    f.a = G.area_y[IX(D, i_f, jk, jl)];
+    f.i = IX(D, upwind(f.v) ? (inner ? i_f : 1) : (inner ? i_f - 1 : D.ny), jk, jl);
+    return f;
+  };
+  const F e = fx(jk + 1), n = fy(ji), w = fx(jk), s = fy(ji + 1);
+  const bool has_up = jl > D.nf, has_lo = jl == D.nf || (jl > D.nf && jl < D.nl);
+  double cu = 0.0, cl = 0.0, au = 0.0, al = 0.0;
+  long long iu = q, il = q;
+  if (has_up) {
+    cu = cw[q];
+    au = G.area_z[q];
+    if (!positive(cu)) iu = q - D.plane;
+  }
+  if (has_lo) {
+    cl = cw[q + D.plane];
+    al = G.area_z[q + D.plane];
+    if (positive(cl)) il = q + D.plane;
+  }
+  const double V = G.volume[q], rV = rvol[q];
+  for (int jc = 1; jc <= D.ncons; ++jc) {
+    if (jc == D.g) continue;
+    const double* r = Ss.rho + (long long)(jc - 1) * D.fstride;
+    double c = r[e.i] * e.v * e.a + r[n.i] * n.v * n.a - r[w.i] * w.v * w.a - r[s.i] * s.v * s.a;
+    if (has_up && has_lo && jl != D.nf) c = c + (r[iu] * cu * au - r[il] * cl * al);
+    else if (has_lo) c = c - r[il] * cl * al;
+    else if (has_up) c = c + r[iu] * cu * au;
+    double f = -div_rn(c, V, rV);
+    if (mdt) f = f + mdt[q + (long long)(jc - 1) * D.fstride];
+    if (ptr) f = f + ptr[q + (long long)((jc < D.g ? jc : D.g) - 1) * D.fstride];
+    double* t = t_rho + (long long)(jc - 1) * D.fstride;
+    t[q] = (rk_step == 1) ? f : half(t[q]) + half(f);
+  }
+}
+
+// what the pressure gradient reads of a cell: theta_v, c_d_p*rho_g/sum(rho) and rho_g/sum(rho) - 1
+__global__ void k64_pgrad_cells(Dims D, Grid<double> G, StateT<double> S, double* th, double* decel, double* cond) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl);
+  th[q] = G.theta_v_bg[q] + S.tp[q];
+  double sum = S.rho[q];
+  for (int jc = 1; jc <= D.nc; ++jc) sum = sum + S.rho[q + (long long)jc * D.fstride];
+  const double rg = S.rho[q + (long long)(D.g - 1) * D.fstride], y = __drcp_rn(sum);
+  decel[q] = div_rn(kC_D_P * rg, sum, y);
+  cond[q] = div_rn(rg, sum, y) - 1.0;
+}
+// manage_p_grad, mo_p_grad.F90:20-104, after the gradients of exner_pert (gx,gy,gz) and, for
+// theta_adv_order 3, the edge values of theta (tvu,tvv) and theta' (tpu,tpv) are known; also
+// calc_p_grad_condensates_v, mo_p_grad.F90:106-120 (identical at both substeps because it always
+// reads state_old).  (With theta and both quotients formed at each of a cell's six faces: 902 us
+// at 192x192x80.)
+__global__ void k64_pgrad(Dims D, Grid<double> G, StateT<double> S, const double* gx, const double* gy, const double* gz,
+                          const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
+                          const double* tpu, const double* tpv, PGrad<double> P, int lfirst) {
+  LG_IDX3;
+  auto negsum = [&](double nl, double l) { return D.luse_bg ? -nl - l : -nl; };
+  // one face between cells a and b: point q, evaluated at qr
+  auto face = [&](long long q, long long qr, long long a, long long b, const double* g, const double* tv, const double* tp,
+                  const double* eg, double* nl, double* l, double* old) {
+    if (!lfirst) old[q] = negsum(nl[q], D.luse_bg ? l[q] : 0.0);
+    const double de = half(decel[a] + decel[b]);
+    const double nlv = de * ((D.theta_order == 2 ? half(th[a] + th[b]) : tv[qr]) * g[qr]);
+    double lv = 0.0;
+    nl[q] = nlv;
+    if (D.luse_bg) {
+      lv = de * ((D.theta_order == 2 ? half(S.tp[a] + S.tp[b]) : tp[qr]) * eg[qr]);
+      l[q] = lv;
+    }
+    if (lfirst) old[q] = negsum(nlv, lv);
   };
   // u points.  Periodic jk = nx+1 ends as a copy of jk = 1 (scalar_times_vector_h2
   // copies it last), so it is evaluated from column 1.  Non-periodic boundary edges stay
@@ -29,75 +414,88 @@ __global__ void k_pgrad(Dims D, Grid<double> G, State S, const double* gx, const
   if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
     const long long q = IX(D, ji, jk, jl);
     const bool inner = jk >= 2 && jk <= D.nx;
-    const double nl_prev = P.nl_u[q], l_prev = P.l_u[q];
-    if (!lfirst) P.old_u[q] = -nl_prev - use_bg_switch * l_prev;
-    if (inner || D.periodic) {
-      const int kk = inner ? jk : 1;
-      const int ka = inner ? jk - 1 : D.nx, kb = kk;
-      const long long qr = IX(D, ji, kk, jl);
-      double nlv = gx[qr];
-      if (D.theta_order == 2) nlv = 0.5 * (theta(ji, ka, jl) + theta(ji, kb, jl)) * nlv;
-      else nlv = tvu[qr] * nlv;
-      double lv = l_prev;
-      if (D.luse_bg) {
-        if (D.theta_order == 2) lv = 0.5 * (thetap(ji, ka, jl) + thetap(ji, kb, jl)) * G.egu[qr];
-        else lv = tpu[qr] * G.egu[qr];
-      }
-      const double de = 0.5 * (decel(ji, ka, jl) + decel(ji, kb, jl));
-      nlv = de * nlv;
-      if (D.luse_bg) lv = de * lv;
-      P.nl_u[q] = nlv;
-      if (D.luse_bg) P.l_u[q] = lv;
-      if (lfirst) P.old_u[q] = -nlv - use_bg_switch * lv;
-    } else if (lfirst) {
-      P.old_u[q] = -nl_prev - use_bg_switch * l_prev;
-    }
+    if (inner || D.periodic)
+      face(q, IX(D, ji, inner ? jk : 1, jl), IX(D, ji, inner ? jk - 1 : D.nx, jl), IX(D, ji, inner ? jk : 1, jl), gx, tvu, tpu,
+           G.egu, P.nl_u, P.l_u, P.old_u);
+    else
+      P.old_u[q] = negsum(P.nl_u[q], P.l_u[q]);
   }
   // v points (periodic ji = ny+1 from row 1)
   if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
     const long long q = IX(D, ji, jk, jl);
     const bool inner = ji >= 2 && ji <= D.ny;
-    const double nl_prev = P.nl_v[q], l_prev = P.l_v[q];
-    if (!lfirst) P.old_v[q] = -nl_prev - use_bg_switch * l_prev;
-    if (inner || D.periodic) {
-      const int ii = inner ? ji : 1;
-      const int ia = inner ? ji - 1 : 1, ib = inner ? ji : D.ny;  // periodic: s(1)+s(ny)
-      const long long qr = IX(D, ii, jk, jl);
-      double nlv = gy[qr];
-      if (D.theta_order == 2) nlv = 0.5 * (theta(ia, jk, jl) + theta(ib, jk, jl)) * nlv;
-      else nlv = tvv[qr] * nlv;
-      double lv = l_prev;
-      if (D.luse_bg) {
-        if (D.theta_order == 2) lv = 0.5 * (thetap(ia, jk, jl) + thetap(ib, jk, jl)) * G.egv[qr];
-        else lv = tpv[qr] * G.egv[qr];
-      }
-      const double de = 0.5 * (decel(ia, jk, jl) + decel(ib, jk, jl));
-      nlv = de * nlv;
-      if (D.luse_bg) lv = de * lv;
-      P.nl_v[q] = nlv;
-      if (D.luse_bg) P.l_v[q] = lv;
-      if (lfirst) P.old_v[q] = -nlv - use_bg_switch * lv;
-    } else if (lfirst) {
-      P.old_v[q] = -nl_prev - use_bg_switch * l_prev;
-    }
+    if (inner || D.periodic)
+      face(q, IX(D, inner ? ji : 1, jk, jl), IX(D, inner ? ji - 1 : 1, jk, jl), IX(D, inner ? ji : D.ny, jk, jl), gy, tvv, tpv,
+           G.egv, P.nl_v, P.l_v, P.old_v);
+    else
+      P.old_v[q] = negsum(P.nl_v[q], P.l_v[q]);
   }
   // w points, levels 2..nl
   if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    double nlv = 0.5 * (theta(ji, jk, jl - 1) + theta(ji, jk, jl)) * gz[q];
-    const double de = 0.5 * (decel(ji, jk, jl - 1) + decel(ji, jk, jl));
-    nlv = de * nlv;
-    P.nl_w[q] = nlv;
-    if (D.luse_bg) {
-      double lv = 0.5 * (thetap(ji, jk, jl - 1) + thetap(ji, jk, jl)) * G.egw[q];
-      P.l_w[q] = de * lv;
-    }
-    // p_grad_condensates_w
-    const long long qa = IX(D, ji, jk, jl - 1);
-    const double da = S.rho[qa + (long long)(D.g - 1) * D.fstride] / rho_sum_cond_gas<double>(D, S.rho, qa) - 1.0;
-    const double db = S.rho[q + (long long)(D.g - 1) * D.fstride] / rho_sum_cond_gas<double>(D, S.rho, q) - 1.0;
-    P.pgcw[q] = 0.5 * (da + db) * G.gm[q];
+    const long long q = IX(D, ji, jk, jl), qa = q - D.plane;
+    const double de = half(decel[qa] + decel[q]);
+    P.nl_w[q] = de * (half(th[qa] + th[q]) * gz[q]);
+    if (D.luse_bg) P.l_w[q] = de * (half(S.tp[qa] + S.tp[q]) * G.egw[q]);
+    P.pgcw[q] = half(cond[qa] + cond[q]) * G.gm[q];  // p_grad_condensates_w
   }
+}
+
+}  // namespace
+
+void launch64_pgrad_cells(const Dims& D, const Grid<double>& G, const State& S, double* th, double* decel, double* cond,
+                          cudaStream_t st) {
+  k64_pgrad_cells<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, G, S, th, decel, cond);
+}
+void launch64_pgrad(const Dims& D, const Grid<double>& G, const State& S, const double* gx, const double* gy, const double* gz,
+                    const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
+                    const double* tpu, const double* tpv, const PGrad<double>& P, int lfirst, cudaStream_t st) {
+  k64_pgrad<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, S, gx, gy, gz, th, decel, cond, tvu, tvv, tpu,
+                                                                       tpv, P, lfirst);
+}
+void launch64_recip(const Dims& D, const Grid<double>& G, double* rdx, double* rdy, double* rdz, cudaStream_t st) {
+  k64_recip<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, rdx, rdy, rdz);
+}
+void launch64_grad_vert(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, double* gz, double* w5,
+                        double* w6, cudaStream_t st) {
+  k64_grad_vert<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, R.dz, s, gz, w5, w6);
+}
+void launch64_grad_hor(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
+                       const double* w6, double* rx, double* ry, cudaStream_t st) {
+  k64_grad_hor<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, R, s, w5, w6, rx, ry);
+}
+void launch64_grad_faces(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
+                         const double* w6, const Faces& F, cudaStream_t st) {
+  k64_grad_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, R, s, w5, w6, F);
+}
+void launch64_div(const Dims& D, const Grid<double>& G, const Recip& R, const Faces& F, double* out, cudaStream_t st) {
+  k64_div<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, R.vol, F, out);
+}
+void launch64_theta_edges(const Dims& D, const double* th, const double* dv, const double* u, const double* v, double* tvu,
+                          double* tvv, cudaStream_t st) {
+  k64_theta_edges<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, th, dv, u, v, tvu, tvv);
+}
+void launch64_gas_faces(const Dims& D, const Grid<double>& G, const State& Ss, const double* u_new, const double* v_new,
+                        const double* tvu, const double* tvv, const Faces& M, const Faces& T, cudaStream_t st) {
+  k64_gas_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, Ss, u_new, v_new, tvu, tvv, M, T);
+}
+void launch64_gas_theta(const Dims& D, const Grid<double>& G, const Recip& R, const State& Ss, const Faces& M, const Faces& T,
+                        const double* cpi, const double* cpw, const double* hd, const double* rad, const double* csh,
+                        double* t_rho, double* t_rt, const double* mdt, const double* tdh, const double* ptr,
+                        const double* pth, cudaStream_t st) {
+  k64_gas_theta<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, Ss, R.vol, M, T, cpi, cpw, hd, rad, csh, t_rho, t_rt, mdt, tdh,
+                                                       ptr, pth);
+}
+void launch64_wind_slopes(const Dims& D, const Grid<double>& G, const double* u, const double* v, double* hx, double* hy,
+                          cudaStream_t st) {
+  k64_wind_slopes<<<cell_grid(D.ny + 1, D.nx + 1, D.nl - D.nf), kCellBlock, 0, st>>>(D, G, u, v, hx, hy);
+}
+void launch64_contra(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, double* cw, cudaStream_t st) {
+  k64_contra<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, hx, hy, cw);
+}
+void launch64_tracers(const Dims& D, const Grid<double>& G, const Recip& R, const State& Ss, const double* u_new,
+                      const double* v_new, const double* cw, double* t_rho, int rk_step, const double* mdt, const double* ptr,
+                      cudaStream_t st) {
+  k64_tracers<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, G, R.vol, Ss, u_new, v_new, cw, t_rho, rk_step, mdt, ptr);
 }
 
 }  // namespace lg

@@ -4,6 +4,7 @@
 #include "lgame_emulator.h"
 #include "common.h"
 #include "emulator.cuh"
+#include "fp64.cuh"
 #include "diffusion.cuh"
 #include "kernels.cuh"
 #include "phase.cuh"
@@ -89,6 +90,11 @@ struct lgame_gpu {
   double *rvol = nullptr, *itwdtv = nullptr, *zs = nullptr, *zs_c2 = nullptr, *zs_c1h = nullptr, *hdeb = nullptr,
          *raz = nullptr;
   ColumnGrid colg{};
+  // reciprocals of the metrics of the explicit kernels, and the faces of the mass flux and of theta_v's
+  // flux or gradient
+  double *rdx = nullptr, *rdy = nullptr, *rdz = nullptr;
+  Recip recip{};
+  Faces fcm{}, fct{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
   double* staging = nullptr;
@@ -504,19 +510,12 @@ int preload_budget_scratch() {
 namespace kd {
 const auto k_temperature = lg::k_temperature<double>;
 const auto k_theta = lg::k_theta<double>;
-const auto k_grad_vert = lg::k_grad_vert<double, double>;
-const auto k_grad_hor = lg::k_grad_hor<double, double>;
-const auto k_div_h = lg::k_div_h<double>;
-const auto k_theta_edges = lg::k_theta_edges<double>;
 const auto k_eta_xy = lg::k_eta_xy<double>;
 const auto k_eta_z = lg::k_eta_z<double>;
 const auto k_mass_flux = lg::k_mass_flux<double>;
 const auto k_vort_flux = lg::k_vort_flux<double>;
 const auto k_ke = lg::k_ke<double>;
 const auto k_tend_wind = lg::k_tend_wind<double>;
-const auto k_tracers = lg::k_tracers<double>;
-const auto k_gas_theta = lg::k_gas_theta<double>;
-const auto k_pgrad = lg::k_pgrad;
 const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
 const auto k_diff_visc = lg::k_diff_visc<double, double>;
@@ -571,10 +570,17 @@ int klaunch_check(lgame_gpu* c, const char* what) {
 int theta3(lgame_gpu* c, const double* tp, int mode, const double* u, const double* v, double* ou, double* ov) {
   const Dims& D = c->D;
   LAUNCH(kd::k_theta, grd(D, D.ny, D.nx, D.nl), D, c->G, tp, c->theta, mode);
-  LAUNCH(kd::k_grad_vert, grd(D, D.ny, D.nx, D.nl - 1), D, c->G, c->theta, c->gz);
-  LAUNCH(kd::k_grad_hor, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, c->theta, c->gz, c->gx, c->gy);
-  LAUNCH(kd::k_div_h, grd(D, D.ny, D.nx, D.nl), D, c->G, c->gx, c->gy, c->divf);
-  LAUNCH(kd::k_theta_edges, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, c->theta, c->divf, u, v, ou, ov);
+  LAUNCH_FN("k_grad_vert", launch64_grad_vert(D, c->G, c->recip, c->theta, c->gz, c->ex, c->ey, c->stream));
+  LAUNCH_FN("k_grad_faces", launch64_grad_faces(D, c->G, c->recip, c->theta, c->ex, c->ey, c->fct, c->stream));
+  LAUNCH_FN("k_div_h", launch64_div(D, c->G, c->recip, c->fct, c->divf, c->stream));
+  LAUNCH_FN("k_theta_edges", launch64_theta_edges(D, c->theta, c->divf, u, v, ou, ov, c->stream));
+  return LGAME_OK;
+}
+// the gradient of a scalar: the vertical one into gz, the horizontal one into (gx, gy)
+int gradient(lgame_gpu* c, const double* f, double* gx, double* gy, double* gz) {
+  const Dims& D = c->D;
+  LAUNCH_FN("k_grad_vert", launch64_grad_vert(D, c->G, c->recip, f, gz, c->ex, c->ey, c->stream));
+  LAUNCH_FN("k_grad_hor", launch64_grad_hor(D, c->G, c->recip, f, c->ex, c->ey, gx, gy, c->stream));
   return LGAME_OK;
 }
 
@@ -589,8 +595,9 @@ int advection(lgame_gpu* c, const State& S) {
          c->pvt_x, c->pvt_y, c->pvt_z);
   if (!D.llinear) {
     LAUNCH(kd::k_ke, grd(D, D.ny, D.nx, D.nl), D, c->G, S, c->vsq);
-    LAUNCH(kd::k_grad_vert, grd(D, D.ny, D.nx, D.nl - 1), D, c->G, c->vsq, c->vsg_z);
-    LAUNCH(kd::k_grad_hor, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, c->vsq, c->vsg_z, c->vsg_x, c->vsg_y);
+    // (the vorticity flux above was the last to read ex and ey, which carry the column products here)
+    const int rc = gradient(c, c->vsq, c->vsg_x, c->vsg_y, c->vsg_z);
+    if (rc != LGAME_OK) return rc;
   }
   return LGAME_OK;
 }
@@ -666,10 +673,14 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
         if (rc != LGAME_OK) return rc;
         if (D.luse_bg) { rc = theta3(c, So.tp, 1, So.u, So.v, c->tpu, c->tpv); if (rc != LGAME_OK) return rc; }
       }
-      LAUNCH(kd::k_grad_vert, grd(D, D.ny, D.nx, D.nl - 1), D, G, So.ep, c->gz);
-      LAUNCH(kd::k_grad_hor, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So.ep, c->gz, c->gx, c->gy);
-      LAUNCH(kd::k_pgrad, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So, c->gx, c->gy, c->gz, c->tvu, c->tvv, c->tpu, c->tpv,
-             P, step == 0 ? 1 : 0);
+      {
+        const int rc = gradient(c, So.ep, c->gx, c->gy, c->gz);
+        if (rc != LGAME_OK) return rc;
+      }
+      // (theta_v and the two quotients of every cell in theta and fcm)
+      LAUNCH_FN("k_pgrad_cells", launch64_pgrad_cells(D, G, So, c->theta, c->fcm.px, c->fcm.py, c->stream));
+      LAUNCH_FN("k_pgrad", launch64_pgrad(D, G, So, c->gx, c->gy, c->gz, c->theta, c->fcm.px, c->fcm.py, c->tvu, c->tvv, c->tpu,
+                                          c->tpv, P, step == 0 ? 1 : 0, c->stream));
       // into the edge arrays of theta', which nothing reads after k_pgrad, and cpw
       if (D.ncons > 1)
         LAUNCH(kd::k_moist_aux, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature, c->tpu, c->tpv, c->cpw);
@@ -701,7 +712,11 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
              (const double*)c->tsoil[so], c->cfg.lsfc_phase_trans, D.dtime, c->ptr, c->pth);
     const double* ptr = c->phase ? c->ptr : nullptr;
     const double* pth = c->phase ? c->pth : nullptr;
-    if (D.ncons > 1) LAUNCH(kd::k_tracers, grd(D, D.ny, D.nx, D.nl), D, G, Ss, Sn.u, Sn.v, T.rho, rk, mdt, ptr);
+    if (D.ncons > 1) {  // the slope terms of the new wind in fct, its vertical correction in divf
+      LAUNCH_FN("k_wind_slopes", launch64_wind_slopes(D, G, Sn.u, Sn.v, c->fct.hx, c->fct.hy, c->stream));
+      LAUNCH_FN("k_contra", launch64_contra(D, G, c->fct.hx, c->fct.hy, c->divf, c->stream));
+      LAUNCH_FN("k_tracers", launch64_tracers(D, G, c->recip, Ss, Sn.u, Sn.v, c->divf, T.rho, rk, mdt, ptr, c->stream));
+    }
     // theta_v_adv_3rd_order of the state used here: in the first substep that is state_old,
     // whose edges manage_p_grad's call above already left in tvu/tvv (nothing in between
     // writes state_old or tvu/tvv), so only the second substep recomputes them -- the same
@@ -710,8 +725,9 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
       int rc = theta3(c, Ss.tp, 0, Ss.u, Ss.v, c->tvu, c->tvv);
       if (rc != LGAME_OK) return rc;
     }
-    LAUNCH(kd::k_gas_theta, grd(D, D.ny, D.nx, D.nl), D, G, Ss, Sn.u, Sn.v, c->tvu, c->tvv, c->temperature, c->hdiss,
-           c->rad, c->csh, T.rho, T.rt, mdt, tdh, ptr, pth);
+    LAUNCH_FN("k_gas_faces", launch64_gas_faces(D, G, Ss, Sn.u, Sn.v, c->tvu, c->tvv, c->fcm, c->fct, c->stream));
+    LAUNCH_FN("k_gas_theta", launch64_gas_theta(D, G, c->recip, Ss, c->fcm, c->fct, c->tpv, c->cpw, c->hdiss, c->rad, c->csh,
+                                                T.rho, T.rt, mdt, tdh, ptr, pth, c->stream));
     // three_band_solver_ver (+ w_free_slip), three_band_solver_gen_densities
     {
       // the sensible heat flux and the soil rows of three_band_solver_ver (mo_column_solvers.F90:
@@ -935,11 +951,13 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
                         &c->ex, &c->ey, &c->ez, &c->uph, &c->vph, &c->wph, &c->vsq};
   for (double** p : scratch) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
   if (cfg->precision == LGAME_PRECISION_FP64) {
-    double** colg[] = {&c->rvol, &c->itwdtv, &c->zs, &c->zs_c2, &c->zs_c1h, &c->hdeb, &c->raz};
+    double** colg[] = {&c->rvol, &c->itwdtv, &c->zs, &c->zs_c2, &c->zs_c1h, &c->hdeb, &c->raz, &c->rdx, &c->rdy, &c->rdz,
+                       &c->fcm.px, &c->fcm.py, &c->fcm.hx, &c->fcm.hy, &c->fct.px, &c->fct.py, &c->fct.hx, &c->fct.hy};
     for (double** p : colg) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
     if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
     c->colg = ColumnGrid{c->rvol, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz,
                          1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
+    c->recip = Recip{c->rvol, c->rdx, c->rdy, c->rdz};
     if (column_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the column solvers refused"));
   }
   // diffusion closure: the carried diagnostics always, the work arrays when a part is on
@@ -1110,6 +1128,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     if (c->split) split_set_diff_par(c->split, c->dpar);
   }
   if (c->rvol) {
+    launch64_recip(D, c->G, c->rdx, c->rdy, c->rdz, c->stream);
     launch_column_grid(D, c->G, c->rvol, c->itwdtv, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz, c->stream);
     CK(cudaGetLastError());
   }
