@@ -10,6 +10,9 @@
 
 namespace lg {
 
+// (The products stay the hardware's here: with a few warps an SM between barriers these kernels wait
+// on chains of operations, and mul_int's longer chain made them slower, 1980 against 1811 us and 1716
+// against 1662 us at 192x192x80.)
 constexpr int kMaxLayers = 128;
 
 // three_band_solver_ver, mo_column_solvers.F90:21-351, plus the array-wide update of
@@ -21,16 +24,17 @@ constexpr int kMaxLayers = 128;
 // (mo_column_solvers.F90:606-640), every thread the new state of its chunk.  FP64 operations bound it
 // on large grids: grid-only factors come from arrays formed once (ColumnGrid), the reciprocals of
 // rho and of the interface density are formed once and divide by div_rn.  One thread per column with
-// fourteen arrays in local memory took 788, 2116 us a launch at 65x97x33, 192x192x80.
+// fourteen arrays in local memory took 788, 2116 us a launch at 65x97x33, 192x192x80; two blocks an SM 158,
+// 1591 us; three (80 registers) 139, 1523 us.
 constexpr int kCvCols = 16, kCvChunks = 16;
 constexpr int kCvArrays = 7;  // c (then c of the row above), d, e (then e/den), r (then the solution), interface
                               // theta, gamma, 1/(interface density)
 
 template <int RK>
-__global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
-    k_column_ver(Dims D, Grid<double> G, ColumnGrid X, State So, State Sn, Tend<double> Tn) {
+__global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
+    k_column_ver(Dims D, Grid<double> G, ColumnGrid X, StateT<double> So, StateT<double> Sn, Tend<double> Tn) {
   extern __shared__ __align__(16) double sm_cv[];
-  constexpr int S = kCvCols;
+    constexpr int S = kCvCols;
   const int lane = threadIdx.x % S, w = threadIdx.x / S;
   const int col = blockIdx.x * S + lane;
   const bool valid = col < D.ny * D.nx;
@@ -38,7 +42,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
   const int nl = D.nl, n = nl - 1;
   const double dtime = D.dtime, rdt = X.rdt;
   const long long goff = (long long)(D.g - 1) * D.fstride, pl = D.plane, c0 = IX(D, ji, jk, 1);
-  const State& Su = (RK == 1) ? So : Sn;  // state_new_used
+  const StateT<double>& Su = (RK == 1) ? So : Sn;  // state_new_used
   const double* rho_o = So.rho + goff;
   const double* rho_u = Su.rho + goff;
   double* rho_n = Sn.rho + goff;
@@ -62,14 +66,14 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
     L.rV = X.rvol[i];
     const double ro = rho_o[i], rto = So.rt[i];
     L.ro = ro;
-    const double yo = __drcp_rn(ro);
+    const double yo = rcp(ro);
     double alpha = div_rn(-rto, ro * ro, yo * yo), beta = yo;
-    double gamma = kR_D / (kC_D_V * rto) * (G.exner_bg[i] + So.ep[i]);
+    double gamma = quot(kR_D, kC_D_V * rto) * (G.exner_bg[i] + So.ep[i]);
     if (RK == 2) {
       const double ru = rho_u[i], rtu = Su.rt[i];
-      const double yu = __drcp_rn(ru);
+      const double yu = rcp(ru);
       const double alpha_new = div_rn(-rtu, ru * ru, yu * yu);
-      const double gamma_new = kR_D / (kC_D_V * rtu) * (G.exner_bg[i] + Su.ep[i]);
+      const double gamma_new = quot(kR_D, kC_D_V * rtu) * (G.exner_bg[i] + Su.ep[i]);
       alpha = (1.0 - pdw) * alpha + pdw * alpha_new;
       beta = (1.0 - pdw) * beta + pdw * yu;
       gamma = (1.0 - pdw) * gamma + pdw * gamma_new;
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
   const int chunk = (n + kCvChunks - 1) / kCvChunks, r0 = w * chunk + 1, r1 = min(n, (w + 1) * chunk);
   if (valid && r0 <= r1) {
     Lay L0 = layer(r0, true), L1 = layer(r0 + 1, true), L2{};
-    double rio = 0.5 * (L0.ro + L1.ro), yrio = __drcp_rn(rio);
+    double rio = 0.5 * (L0.ro + L1.ro), yrio = rcp_near(rio);
     double t = 0.5 * (L0.th + L1.th);
     for (int jl = r0; jl <= r1; ++jl) {
       const long long b = c0 + (long long)jl * pl;  // layer jl+1 and w level jl+1
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
         const long long cc = b + pl;
         tn = 0.5 * (L1.th + L2.th);
         rio_n = 0.5 * (L1.ro + L2.ro);
-        yrio_n = __drcp_rn(rio_n);
+        yrio_n = rcp_near(rio_n);
         cv = tn * L1.ga * t + X.hdeb[cc] * (L1.al + L1.be * t)
            - div_rn(X.zs_c1h[cc] * So.w[cc], L1.V * rio_n, L1.rV * yrio_n) * G.damp[cc];
         ev = t * L1.ga * tn - hdeb * (L1.al + L1.be * tn)
@@ -135,7 +139,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
   }
   __syncthreads();
   if (valid && w == 0) {
-    double y = __drcp_rn(sd[0]);
+    double y = rcp_near(sd[0]);
     double ep = div_rn(se[0], sd[0], y), rp = div_rn(sr[0], sd[0], y);
     se[0] = ep;
     sr[0] = rp;
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
     for (int jl = 2; jl <= n; ++jl) {
       const double c = sc[S * (jl - 2)];
       const double den = sd[S * (jl - 1)] - ep * c;
-      y = __drcp_rn(den);
+      y = rcp_near(den);
       ep = div_rn(se[S * (jl - 1)], den, y);  // (0 in the last row)
       rp = div_rn(sr[S * (jl - 1)] - rp * c, den, y);
       se[S * (jl - 1)] = ep;
@@ -181,7 +185,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 2)
     else if (jl == nl) rtn = rte - div_rn(dtime * st[S * (n - 1)] * sr[S * (n - 1)], V, rV);
     else rtn = rte + div_rn(dtime * (-(st[S * (jl - 2)] * sr[S * (jl - 2)]) + st[S * (jl - 1)] * sr[S * (jl - 1)]), V, rV);
     const double epn = So.ep[i] + V * sg[S * (jl - 1)] * (rtn - rto);
-    const double tpn = rtn / rn - G.theta_v_bg[i];
+    const double tpn = quot(rtn, rn) - G.theta_v_bg[i];
     if (jl >= 2) {
       const double rin = 0.5 * (rn_up + rn);
       Sn.w[i] = div_rn(div_rn(2.0 * sr[S * (jl - 2)], G.area_z[i], X.raz[i]) - rin * So.w[i], 0.5 * (ro_up + ro),
@@ -286,9 +290,10 @@ __global__ void k_moist_aux(Dims D, Grid<double> G, State So, const double* T, d
 // thread forms its chunk's rows into shared memory, one thread per column and tracer runs the two
 // sweeps, every thread clips and stores its chunk.  The level's own quantities come from k_moist_aux
 // and from the grid (the reciprocal of the volume and itw*dtime/volume).  One thread per column with
-// its arrays in local memory took 1530, 4887 us a launch at 65x97x33, 192x192x80; this 199, 1814 us.
+// its arrays in local memory took 1530, 4887 us a launch at 65x97x33, 192x192x80; two blocks an SM 187, 1772 us; three (80 registers) 138,
+// 1571 us.
 constexpr int kTcCols = 16, kTcChunks = 16;
-constexpr int kTcArrays = 8;  // k, d, 1/d, right-hand sides of up to three tracers, two heating sums (first substep)
+constexpr int kTcArrays = 6;  // k, d, 1/d, right-hand sides of up to three tracers
 
 template <int GROUP>
 struct TracerGroup {
@@ -300,12 +305,12 @@ struct TracerGroup {
 };
 
 // one group of tracers of the block's columns; HEAT: the first substep, which forms the sediment
-// heating (the sums over the condensates in their order, in hs; graupel's part waits in hx)
+// heating (the sum over the condensates in their order, in csh; graupel's part waits in hx)
 template <int GROUP, bool HEAT>
-__device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& G, const State& So, const State& Sn,
+__device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& G, const StateT<double>& So, const StateT<double>& Sn,
                                              const double* t_rho_all, const double* T, const double* rvol,
                                              const double* itwdtv, const double* vcloud, const double* cpi,
-                                             const double* cpw, double* csh, int ji, int jk, bool valid, int lane, int w,
+                                             const double* cpw, double* csh, double* hx, int ji, int jk, bool valid, int lane, int w,
                                              double* sm) {
   using TG = TracerGroup<GROUP>;
   constexpr int N = TG::n(), S = kTcCols;
@@ -315,8 +320,6 @@ __device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& 
   double* const sd = sm + S * nl + lane;      // diagonal
   double* const sy = sm + 2 * S * nl + lane;  // its reciprocal
   double* const sr = sm + 3 * S * nl + lane;  // right-hand side, then the solution: tracer q at + q*S*nl
-  double* const hs = sm + 6 * S * nl + lane;
-  double* const hx = sm + 7 * S * nl + lane;
   const double dtime = D.dtime;
   const double itw = 0.5, expl_weight = 1.0 - itw;
   const double ewdt = expl_weight * dtime;
@@ -379,7 +382,7 @@ __device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& 
       if (jl > 1 && !negative(up.vfi)) d = d + up.p1;
       if (jl < nl && negative(dn.vfi)) d = d - dn.p0;
       if (jl == nl && TG::cond(0) && GROUP != 1) d = d + div_rn(itw * v_sfc * dtime * az_sfc, V, rV);
-      const double y = __drcp_rn(d);
+      const double y = rcp_near(d);
       sd[S * (jl - 1)] = d;
       sy[S * (jl - 1)] = y;
       // (written as -e/d: e = -(itwdtv*vfi), so k = (itwdtv*vfi)/d)
@@ -406,13 +409,10 @@ __device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& 
         }
         sr[S * (nl * q + jl - 1)] = r;
         if (HEAT && TG::cond(q)) {  // (the thread is the only one to touch its levels' sums)
-          if (TG::jc(q) == 1) hs[S * (jl - 1)] = h;
-          else if (TG::jc(q) == 5) hx[S * (jl - 1)] = h;  // its surface term is 0 (no fall speed)
-          else {
-            const double s = (hs[S * (jl - 1)] + h) - h2;
-            if (TG::jc(q) == 4) csh[i] = s + hx[S * (jl - 1)];
-            else hs[S * (jl - 1)] = s;
-          }
+          if (TG::jc(q) == 1) csh[i] = h;
+          else if (TG::jc(q) == 5) hx[i] = h;  // its surface term is 0 (no fall speed)
+          else if (TG::jc(q) == 4) csh[i] = ((csh[i] + h) - h2) + hx[i];
+          else csh[i] = (csh[i] + h) - h2;
         }
         ro[q] = ro_n[q];
       }
@@ -451,17 +451,17 @@ __device__ __forceinline__ void tracer_group(const Dims& D, const Grid<double>& 
 }
 
 template <bool HEAT>
-__global__ void __launch_bounds__(kTcCols* kTcChunks, 2)
-    k_column_tracers(Dims D, Grid<double> G, State So, State Sn, const double* t_rho_all, const double* T,
+__global__ void __launch_bounds__(kTcCols* kTcChunks, 3)
+    k_column_tracers(Dims D, Grid<double> G, StateT<double> So, StateT<double> Sn, const double* t_rho_all, const double* T,
                      const double* rvol, const double* itwdtv, const double* vcloud, const double* cpi, const double* cpw,
-                     double* csh) {
+                     double* csh, double* hx) {
   extern __shared__ __align__(16) double sm_tc[];
   const int lane = threadIdx.x % kTcCols, w = threadIdx.x / kTcCols;
   const int col = blockIdx.x * kTcCols + lane;
   const bool valid = col < D.ny * D.nx;
   const int ji = valid ? col % D.ny + 1 : 1, jk = valid ? col / D.ny + 1 : 1;
 #define TC_GROUP(g) \
-  tracer_group<g, HEAT>(D, G, So, Sn, t_rho_all, T, rvol, itwdtv, vcloud, cpi, cpw, csh, ji, jk, valid, lane, w, sm_tc)
+  tracer_group<g, HEAT>(D, G, So, Sn, t_rho_all, T, rvol, itwdtv, vcloud, cpi, cpw, csh, hx, ji, jk, valid, lane, w, sm_tc)
   TC_GROUP(0);
   TC_GROUP(1);
   TC_GROUP(2);
@@ -483,15 +483,14 @@ int column_prepare() {
 
 void launch_column_tracers(const Dims& D, const Grid<double>& G, const State& So, const State& Sn, const double* t_rho,
                            const double* T, const double* rvol, const double* itwdtv, const double* vcloud,
-                           const double* cpi, const double* cpw, double* csh, int rk_step, cudaStream_t st) {
+                           const double* cpi, const double* cpw, double* csh, double* hx, int rk_step, cudaStream_t st) {
   const unsigned nb = (unsigned)(((long long)D.ny * D.nx + kTcCols - 1) / kTcCols);
   const dim3 b(kTcCols * kTcChunks);
-  // the second substep keeps no heating sums
-  const size_t lev = (size_t)kTcCols * D.nl * sizeof(double);
+  const size_t sm = (size_t)kTcArrays * kTcCols * D.nl * sizeof(double);
   if (rk_step == 1)
-    k_column_tracers<true><<<nb, b, 8 * lev, st>>>(D, G, So, Sn, t_rho, T, rvol, itwdtv, vcloud, cpi, cpw, csh);
+    k_column_tracers<true><<<nb, b, sm, st>>>(D, G, So, Sn, t_rho, T, rvol, itwdtv, vcloud, cpi, cpw, csh, hx);
   else
-    k_column_tracers<false><<<nb, b, 6 * lev, st>>>(D, G, So, Sn, t_rho, T, rvol, itwdtv, vcloud, cpi, cpw, csh);
+    k_column_tracers<false><<<nb, b, sm, st>>>(D, G, So, Sn, t_rho, T, rvol, itwdtv, vcloud, cpi, cpw, csh, hx);
 }
 
 }  // namespace lg

@@ -74,6 +74,12 @@ __device__ __forceinline__ T cvt(S x) {
   else return T(x);
 }
 
+// a half and a quarter of x (the FP64 step takes them in the exponent: fp64.cuh)
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half_of(double x) { return 0.5 * x; }
+__device__ __forceinline__ float quarter_of(float x) { return 0.25f * x; }
+__device__ __forceinline__ double quarter_of(double x) { return 0.25 * x; }
+
 // Offset of point (i, j, k) in a field.  A field's padded extent (fstride) is below 2^31
 // (lgame_gpu_create checks it), so the offset is formed in 32-bit signed arithmetic: two
 // integer multiply-adds, and the compiler folds the offsets of neighbouring points (+-1, +-P,
@@ -132,19 +138,19 @@ __device__ __forceinline__ T vcc(const Dims& D, const Grid<T>& G, FX vx, FY vy, 
   T r = T(0);
   if (jl >= D.nf + 1) {
     if (jl == D.nf + 1) {
-      r = r - T(0.5) * vx(ji, jk + 1, jl) * G.slope_x[IX(D, ji, jk + 1, jl)] * W_(1, ji, jk, jl)
-            - T(0.5) * vy(ji, jk, jl) * G.slope_y[IX(D, ji, jk, jl)] * W_(2, ji, jk, jl)
-            - T(0.5) * vx(ji, jk, jl) * G.slope_x[IX(D, ji, jk, jl)] * W_(3, ji, jk, jl)
-            - T(0.5) * vy(ji + 1, jk, jl) * G.slope_y[IX(D, ji + 1, jk, jl)] * W_(4, ji, jk, jl);
+      r = r - half_of(vx(ji, jk + 1, jl)) * G.slope_x[IX(D, ji, jk + 1, jl)] * W_(1, ji, jk, jl)
+            - half_of(vy(ji, jk, jl)) * G.slope_y[IX(D, ji, jk, jl)] * W_(2, ji, jk, jl)
+            - half_of(vx(ji, jk, jl)) * G.slope_x[IX(D, ji, jk, jl)] * W_(3, ji, jk, jl)
+            - half_of(vy(ji + 1, jk, jl)) * G.slope_y[IX(D, ji + 1, jk, jl)] * W_(4, ji, jk, jl);
     } else {
-      r = r - T(0.5) * vx(ji, jk + 1, jl - 1) * G.slope_x[IX(D, ji, jk + 1, jl - 1)] * W_(1, ji, jk, jl - 1)
-            - T(0.5) * vy(ji, jk, jl - 1) * G.slope_y[IX(D, ji, jk, jl - 1)] * W_(2, ji, jk, jl - 1)
-            - T(0.5) * vx(ji, jk, jl - 1) * G.slope_x[IX(D, ji, jk, jl - 1)] * W_(3, ji, jk, jl - 1)
-            - T(0.5) * vy(ji + 1, jk, jl - 1) * G.slope_y[IX(D, ji + 1, jk, jl - 1)] * W_(4, ji, jk, jl - 1);
-      r = r - T(0.5) * vx(ji, jk + 1, jl) * G.slope_x[IX(D, ji, jk + 1, jl)] * W_(1, ji, jk, jl)
-            - T(0.5) * vy(ji, jk, jl) * G.slope_y[IX(D, ji, jk, jl)] * W_(2, ji, jk, jl)
-            - T(0.5) * vx(ji, jk, jl) * G.slope_x[IX(D, ji, jk, jl)] * W_(3, ji, jk, jl)
-            - T(0.5) * vy(ji + 1, jk, jl) * G.slope_y[IX(D, ji + 1, jk, jl)] * W_(4, ji, jk, jl);
+      r = r - half_of(vx(ji, jk + 1, jl - 1)) * G.slope_x[IX(D, ji, jk + 1, jl - 1)] * W_(1, ji, jk, jl - 1)
+            - half_of(vy(ji, jk, jl - 1)) * G.slope_y[IX(D, ji, jk, jl - 1)] * W_(2, ji, jk, jl - 1)
+            - half_of(vx(ji, jk, jl - 1)) * G.slope_x[IX(D, ji, jk, jl - 1)] * W_(3, ji, jk, jl - 1)
+            - half_of(vy(ji + 1, jk, jl - 1)) * G.slope_y[IX(D, ji + 1, jk, jl - 1)] * W_(4, ji, jk, jl - 1);
+      r = r - half_of(vx(ji, jk + 1, jl)) * G.slope_x[IX(D, ji, jk + 1, jl)] * W_(1, ji, jk, jl)
+            - half_of(vy(ji, jk, jl)) * G.slope_y[IX(D, ji, jk, jl)] * W_(2, ji, jk, jl)
+            - half_of(vx(ji, jk, jl)) * G.slope_x[IX(D, ji, jk, jl)] * W_(3, ji, jk, jl)
+            - half_of(vy(ji + 1, jk, jl)) * G.slope_y[IX(D, ji + 1, jk, jl)] * W_(4, ji, jk, jl);
     }
   }
   return r;
@@ -170,7 +176,7 @@ __device__ __forceinline__ T remap_x(const Dims& D, const Grid<T>& G, const V* v
       r = r + W_(6, ji, jk, jl) * T(vc[IX(D, ji, jk, jl + 1)]);
     }
   }
-  return T(0.5) * r;
+  return half_of(r);
 }
 
 // remap_ver2hor_y, mo_averaging.F90:97-136
@@ -193,7 +199,7 @@ __device__ __forceinline__ T remap_y(const Dims& D, const Grid<T>& G, const V* v
       r = r + W_(6, ji, jk, jl) * T(vc[IX(D, ji, jk, jl + 1)]);
     }
   }
-  return T(0.5) * r;
+  return half_of(r);
 }
 
 // horizontal_covariant_x/y, mo_averaging.F90:138-176

@@ -129,7 +129,7 @@ __global__ void k_diff_tke(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, DiffPar
     const long long a = IX(D, ji, jk, l - 1), b = IX(D, ji, jk, l);
     const T th_a = G.theta_v_bg[a] + T(S.tp[a]), th_b = G.theta_v_bg[b] + T(S.tp[b]);
     const T grad = (th_a - th_b) / G.dz[b];
-    return G.gm[b] * (T(0.5) * (T(1) / th_a + T(1) / th_b) * grad);
+    return G.gm[b] * (half_of(T(1) / th_a + T(1) / th_b) * grad);
   };
   T nsq;
   if (jl == 1) nsq = nz(1);
@@ -154,7 +154,7 @@ __global__ void k_diff_tke(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, DiffPar
       r = r + W_(5, i, j, l) * gz(i, j, l);
       if (l < D.nl || D.freeslip) { r = r + W_(6, i, j - 1, l) * gz(i, j - 1, l + 1); r = r + W_(6, i, j, l) * gz(i, j, l + 1); }
     }
-    return T(0.5) * r;
+    return half_of(r);
   };
   auto remap_gy = [&](int i, int j, int l) -> T {  // remap_ver2hor_y of gz
     T r = T(0);
@@ -168,7 +168,7 @@ __global__ void k_diff_tke(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, DiffPar
       r = r + W_(5, i, j, l) * gz(i, j, l);
       if (l < D.nl || D.freeslip) { r = r + W_(6, i - 1, j, l) * gz(i - 1, j, l + 1); r = r + W_(6, i, j, l) * gz(i, j, l + 1); }
     }
-    return T(0.5) * r;
+    return half_of(r);
   };
   auto gx = [&](int i, int j, int l) -> T {  // grad_hor x at a u point; non-periodic boundary: 0
     T r;
@@ -213,7 +213,7 @@ __global__ void k_diff_visc(Dims D, Grid<T> G, StateT<V> S, const T* Tm, DiffBuf
     eddy = tke2hor<T>(P, tke);
   } else {
     const T* zz = B.zz;
-    const T vac = T(0.25) * (zz[q] + zz[q + D.P] + zz[q + 1] + zz[q + D.P + 1]);
+    const T vac = quarter_of(zz[q] + zz[q + D.P] + zz[q + 1] + zz[q + D.P + 1]);
     const T a = vac * vac + dv * dv, b = T(P.bg_shear) * T(P.bg_shear);
     eddy = T(P.c_s) * T(P.mva) * dsqrt<T>(a > b ? a : b);
   }
@@ -249,18 +249,18 @@ __global__ void k_diff_vz(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B) {
   const bool in_i = ji >= 2 && ji <= D.ny, in_k = jk >= 2 && jk <= D.nx;
   T vd = T(0);
   if (in_i && in_k) {
-    vd = T(0.25) * (vs(ji - 1, jk - 1) + vs(ji - 1, jk) + vs(ji, jk - 1) + vs(ji, jk));
-    vd = T(0.25) * (rs(ji - 1, jk - 1) + rs(ji - 1, jk) + rs(ji, jk - 1) + rs(ji, jk)) * vd;
+    vd = quarter_of(vs(ji - 1, jk - 1) + vs(ji - 1, jk) + vs(ji, jk - 1) + vs(ji, jk));
+    vd = quarter_of(rs(ji - 1, jk - 1) + rs(ji - 1, jk) + rs(ji, jk - 1) + rs(ji, jk)) * vd;
   } else if (D.periodic) {
     if (in_k) {  // ji = 1 or ny+1 (the copy of 1)
-      vd = T(0.25) * (vs(1, jk - 1) + vs(D.ny, jk - 1) + vs(1, jk) + vs(D.ny, jk));
-      vd = vd * (T(0.25) * (rs(1, jk - 1) + rs(D.ny, jk - 1) + rs(1, jk) + rs(D.ny, jk)));
+      vd = quarter_of(vs(1, jk - 1) + vs(D.ny, jk - 1) + vs(1, jk) + vs(D.ny, jk));
+      vd = vd * (quarter_of(rs(1, jk - 1) + rs(D.ny, jk - 1) + rs(1, jk) + rs(D.ny, jk)));
     } else if (in_i) {  // jk = 1 or nx+1
-      vd = T(0.25) * (vs(ji - 1, D.nx) + vs(ji - 1, 1) + vs(ji, D.nx) + vs(ji, 1));
-      vd = vd * (T(0.25) * (rs(ji - 1, D.nx) + rs(ji - 1, 1) + rs(ji, D.nx) + rs(ji, 1)));
+      vd = quarter_of(vs(ji - 1, D.nx) + vs(ji - 1, 1) + vs(ji, D.nx) + vs(ji, 1));
+      vd = vd * (quarter_of(rs(ji - 1, D.nx) + rs(ji - 1, 1) + rs(ji, D.nx) + rs(ji, 1)));
     } else {  // corners
-      vd = T(0.25) * (vs(1, 1) + vs(D.ny, 1) + vs(1, D.nx) + vs(D.ny, D.nx));
-      vd = vd * (T(0.25) * (rs(D.ny, D.nx) + rs(D.ny, 1) + rs(1, D.nx) + rs(1, 1)));
+      vd = quarter_of(vs(1, 1) + vs(D.ny, 1) + vs(1, D.nx) + vs(D.ny, D.nx));
+      vd = vd * (quarter_of(rs(D.ny, D.nx) + rs(D.ny, 1) + rs(1, D.nx) + rs(1, 1)));
     }
   }
   B.vz[q] = vd * B.zz[q];
@@ -294,12 +294,12 @@ __global__ void k_mom_diff_h(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B) {
       const T dyd = G.dy_dual[q];
       T up = (vz[IX(D, ji + 1, kk, jl)] - vz[IX(D, ji, kk, jl)]) / dyd;
       const T slope = (zd[IX(D, ji + 1, kk, jl)] - zd[IX(D, ji, kk, jl)]) / dyd;
-      const T vg = T(0.5) * (vz[IX(D, ji + 1, kk, ui)] - vz[IX(D, ji + 1, kk, li)])
+      const T vg = half_of(vz[IX(D, ji + 1, kk, ui)] - vz[IX(D, ji + 1, kk, li)])
                      / (zd[IX(D, ji + 1, kk, ui)] - zd[IX(D, ji + 1, kk, li)])
-                 + T(0.5) * (vz[IX(D, ji, kk, ui)] - vz[IX(D, ji, kk, li)])
+                 + half_of(vz[IX(D, ji, kk, ui)] - vz[IX(D, ji, kk, li)])
                      / (zd[IX(D, ji, kk, ui)] - zd[IX(D, ji, kk, li)]);
       up = up - slope * vg;
-      r = (r + up) / (T(0.5) * (rsum(ji, ka, jl) + rsum(ji, kk, jl)));
+      r = (r + up) / (half_of(rsum(ji, ka, jl) + rsum(ji, kk, jl)));
     } else {
       r = B.mdtx[q];
       if (jl > D.nf) r = r - G.slope_x[q] * T(0);
@@ -319,12 +319,12 @@ __global__ void k_mom_diff_h(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B) {
       const T dxd = G.dx_dual[q];
       T vp = (vz[IX(D, ji, jk + 1, jl)] - vz[q]) / dxd;
       const T slope = (zd[IX(D, ji, jk + 1, jl)] - zd[q]) / dxd;
-      const T vg = T(0.5) * (vz[IX(D, ji, jk + 1, ui)] - vz[IX(D, ji, jk + 1, li)])
+      const T vg = half_of(vz[IX(D, ji, jk + 1, ui)] - vz[IX(D, ji, jk + 1, li)])
                      / (zd[IX(D, ji, jk + 1, ui)] - zd[IX(D, ji, jk + 1, li)])
-                 + T(0.5) * (vz[IX(D, ji, jk, ui)] - vz[IX(D, ji, jk, li)])
+                 + half_of(vz[IX(D, ji, jk, ui)] - vz[IX(D, ji, jk, li)])
                      / (zd[IX(D, ji, jk, ui)] - zd[IX(D, ji, jk, li)]);
       vp = vp - slope * vg;
-      r = (r + vp) / (T(0.5) * (rsum(ia, jk, jl) + rsum(ji, jk, jl)));
+      r = (r + vp) / (half_of(rsum(ia, jk, jl) + rsum(ji, jk, jl)));
     } else {
       r = B.mdty[q];
       if (jl > D.nf) r = r - G.slope_y[q] * T(0);
@@ -355,7 +355,7 @@ __global__ void k_mom_diff_v(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B) {
   };
   const long long q = IX(D, ji, jk, jl);
   T m = (sp(jl - 1) - sp(jl)) / G.dz[q];
-  m = m / (T(0.5) * (rho_sum_cond_gas<T, V>(D, S.rho, q - D.plane) + rho_sum_cond_gas<T, V>(D, S.rho, q)));
+  m = m / (half_of(rho_sum_cond_gas<T, V>(D, S.rho, q - D.plane) + rho_sum_cond_gas<T, V>(D, S.rho, q)));
   B.mdtz[q] = m;
 }
 
@@ -455,7 +455,7 @@ __global__ void k_diff_fluxes(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, cons
         r = r + e.w6a * gza1;
         r = r + e.w6b * gzb1;
       }
-      g = g - e.slope * (T(0.5) * r);
+      g = g - e.slope * (half_of(r));
     }
     return g;
   };
@@ -469,7 +469,7 @@ __global__ void k_diff_fluxes(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, cons
     } else {
       // cells west (a = jk-1, periodic nx) and east (b = jk, periodic 1) of the u point
       const long long a = inner ? q - D.P : IX(D, ji, D.nx, jl), b = inner ? q : IX(D, ji, 1, jl);
-      const T h = inner ? T(0.5) * (ch(a) + ch(b)) : T(0.5) * (ch(b) + ch(a));
+      const T h = inner ? half_of(ch(a) + ch(b)) : half_of(ch(b) + ch(a));
       const Edge e = edge(a, b, h, G.dx[b], G.slope_x[q]);
 #pragma unroll
       for (int f = 0; f < nf; ++f) fx[q + (long long)f * D.fstride] = e.h * grad(s0 + (long long)f * D.fstride, e, true);
@@ -484,7 +484,7 @@ __global__ void k_diff_fluxes(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, cons
     } else {
       // cells north (a = ji-1, periodic ny) and south (b = ji, periodic 1) of the v point
       const long long a = inner ? q - 1 : IX(D, D.ny, jk, jl), b = inner ? q : IX(D, 1, jk, jl);
-      const T h = inner ? T(0.5) * (ch(a) + ch(b)) : T(0.5) * (ch(b) + ch(a));
+      const T h = inner ? half_of(ch(a) + ch(b)) : half_of(ch(b) + ch(a));
       const Edge e = edge(a, b, h, G.dy[b], G.slope_y[q]);
 #pragma unroll
       for (int f = 0; f < nf; ++f) fy[q + (long long)f * D.fstride] = e.h * grad(s0 + (long long)f * D.fstride, e, false);
@@ -492,7 +492,7 @@ __global__ void k_diff_fluxes(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, cons
   }
   if (vertical && jl >= 2 && ji <= D.ny && jk <= D.nx) {
     const long long q = IX(D, ji, jk, jl);
-    const T h = T(0.5) * (diff_coeff_v<T, V>(D, G, S, B, kind, q - pl) + diff_coeff_v<T, V>(D, G, S, B, kind, q));
+    const T h = half_of(diff_coeff_v<T, V>(D, G, S, B, kind, q - pl) + diff_coeff_v<T, V>(D, G, S, B, kind, q));
     const T dz = G.dz[q];
 #pragma unroll
     for (int f = 0; f < nf; ++f) {
@@ -538,8 +538,8 @@ __global__ void k_diff_divs(Dims D, Grid<T> G, const T* __restrict__ fx, const T
     const T* Y = fy + o;
     // r - 0.5*vx(e)*slope_x(e)*W1 - 0.5*vy(n)*slope_y(n)*W2 - 0.5*vx(w)*slope_x(w)*W3 - 0.5*vy(s)*slope_y(s)*W4
     auto terms = [&](T r, const LM& m, long long d) {
-      return r - T(0.5) * X[qe + d] * m.sxe * m.w1 - T(0.5) * Y[q + d] * m.sy * m.w2
-               - T(0.5) * X[q + d] * m.sx * m.w3 - T(0.5) * Y[qs + d] * m.sys * m.w4;
+      return r - half_of(X[qe + d]) * m.sxe * m.w1 - half_of(Y[q + d]) * m.sy * m.w2
+               - half_of(X[q + d]) * m.sx * m.w3 - half_of(Y[qs + d]) * m.sys * m.w4;
     };
     // vertical_contravariant_corr at interface jl (cu) and jl+1 (cl)
     T cu = T(0), cl = T(0);

@@ -1,21 +1,49 @@
 // fp64.cuh -- FP64 arithmetic of the FP64 step in fewer operations of the FP64 pipe, which issues
-// 1.7 operations per clock and SM on this GPU against 64 integer ones: with every kernel of the
-// step at 80-88 % of that pipe and below 10 % of everything else, its time is the number of these
-// operations.  Every function returns the bits of the plain expression (exceptions as stated).
+// 1.6 operations per clock and SM on this GPU against 64 integer ones: with plain expressions every
+// kernel of the step had that pipe at 80-88 % and everything else below 10 %, so its time was the
+// number of these operations.  Every function returns the bits of the plain expression (exceptions
+// as stated).
 #pragma once
+
+#include <cstdint>
 
 #include "kernels.cuh"
 
 namespace lg {
 
-// a/b rounded to nearest for y within two units of the last place of 1/b: quotient, remainder,
-// correction (Markstein, IBM J. Res. Dev. 34, 1990): three FP64-pipe operations instead of about
-// seven.  The result is the correctly rounded quotient, except that a quotient within 2^-50 of its
-// last place from the middle of two doubles may round the other way; a zero quotient's sign is not
-// kept, and an infinite a gives NaN.
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-  const double q = a * y;
-  return fma(fma(-b, q, a), y, q);
+// The hardware product, out of line: as a select the compiler would issue it beside the integer path.
+static __device__ __noinline__ double mul_hw(double x, double y) { return x * y; }
+
+// x*y rounded to nearest even in integer operations: the 53-bit mantissas multiplied in four 32 x 32
+// bit products, normalised, the dropped bits folded into one.  On this GPU the FP64 pipe runs beside
+// the integer ones, so a product formed here costs it nothing: chains of a product and a sum run at 3.15
+// operations per clock and SM, against 1.60 with the hardware's product (1.89 for this product
+// alone).  Factors outside 2^-510..2^511 take the hardware's, but zeros.
+__device__ __forceinline__ double mul_int(double x, double y) {
+  const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
+  const uint32_t yh = (uint32_t)__double2hiint(y), yl = (uint32_t)__double2loint(y);
+  const uint32_t xe = xh & 0x7FF00000u, ye = yh & 0x7FF00000u;
+  if (max(xe - (513u << 20), ye - (513u << 20)) >= (1022u << 20)) {
+    const bool x0 = ((xh << 1) | xl) == 0u, y0 = ((yh << 1) | yl) == 0u;
+    if ((x0 && ye < 0x7FF00000u) || (y0 && xe < 0x7FF00000u)) return __hiloint2double((int)((xh ^ yh) & 0x80000000u), 0);
+    return mul_hw(x, y);
+  }
+  // mantissas as a < 2^54 and b < 2^64: the product is in [2^116, 2^118), its upper 64 bits hold 53 or 54
+  const uint32_t ah = (__funnelshift_l(xl, xh, 1) & 0x1FFFFFu) | 0x200000u, al = xl << 1;
+  const uint32_t bh = __funnelshift_l(yl, yh, 11) | 0x80000000u, bl = yl << 11;
+  const uint64_t p00 = (uint64_t)al * bl;
+  const uint64_t p01 = (uint64_t)al * bh + (p00 >> 32);
+  const uint64_t p10 = (uint64_t)ah * bl + (uint32_t)p01;
+  const uint64_t up = (uint64_t)ah * bh + (p01 >> 32) + (p10 >> 32);
+  uint32_t hh = (uint32_t)(up >> 32), hl = (uint32_t)up;
+  const uint32_t big = hh >> 21, sh = 1u - big, mid = (uint32_t)p10;
+  // to 54 bits: the mantissa and the first dropped bit; t rounds (to even at a tie)
+  hh = __funnelshift_l(hl, hh, sh);
+  hl = __funnelshift_l(mid, hl, sh);
+  const uint32_t t = ((hl >> 1) & 1u) | (((mid << sh) | (uint32_t)p00) != 0u ? 1u : 0u);
+  const uint64_t r = ((((uint64_t)hh << 32) | hl) + t) >> 1;
+  const uint32_t e = xe + ye - 0x3FF00000u - 0x00100000u + (big << 20);
+  return __hiloint2double((int)(((uint32_t)(r >> 32) + e) ^ ((xh ^ yh) & 0x80000000u)), (int)(uint32_t)r);
 }
 
 // x < 0 by the bits (a comparison issues on the FP64 pipe); -0 counts as negative, NaN does not
@@ -44,14 +72,74 @@ __device__ __forceinline__ double scale_down(double x) {
 __device__ __forceinline__ double half(double x) { return scale_down<1>(x); }
 __device__ __forceinline__ double quarter(double x) { return scale_down<2>(x); }
 
+// a double whose products are formed by mul_int; sums are the hardware's.  Arrays of
+// double are read and written as arrays of it.
+struct F64 {
+  double v;
+  F64() = default;
+  __host__ __device__ __forceinline__ constexpr F64(double x) : v(x) {}
+};
+__device__ __forceinline__ F64 operator-(F64 a) { return -a.v; }
+__device__ __forceinline__ F64 operator+(F64 a, F64 b) { return a.v + b.v; }
+__device__ __forceinline__ F64 operator-(F64 a, F64 b) { return a.v - b.v; }
+__device__ __forceinline__ F64 operator*(F64 a, F64 b) { return mul_int(a.v, b.v); }
+__device__ __forceinline__ bool operator>(F64 a, F64 b) { return a.v > b.v; }
+__device__ __forceinline__ bool operator<(F64 a, F64 b) { return a.v < b.v; }
+__device__ __forceinline__ bool operator>=(F64 a, F64 b) { return a.v >= b.v; }
+__device__ __forceinline__ F64 half(F64 a) { return half(a.v); }
+__device__ __forceinline__ F64 half_of(F64 a) { return half(a.v); }
+__device__ __forceinline__ F64 quarter_of(F64 a) { return quarter(a.v); }
+__device__ __forceinline__ bool negative(F64 a) { return negative(a.v); }
+__device__ __forceinline__ bool nonzero(F64 a) { return nonzero(a.v); }
+__device__ __forceinline__ bool upwind(F64 a) { return upwind(a.v); }
+__device__ __forceinline__ bool positive(F64 a) { return positive(a.v); }
+// 1/b to about a unit of the last place: the single-precision reciprocal of b's leading bits (to
+// 2^-22) and one step of Halley's iteration, y(1 + e + e^2) with e = 1 - b*y: three operations of the
+// FP64 pipe
+static __device__ __noinline__ double rcp_hw(double b) { return 1.0 / b; }
+__device__ __forceinline__ double rcp_near(double b) {
+  const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
+  if ((hi & 0x7FF00000u) - (923u << 20) >= (200u << 20)) return rcp_hw(b);  // not within 2^-100..2^99
+  const float f = __uint_as_float((hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29)));
+  const double y = wide(__fdividef(1.f, f));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+// 1/b and a/b rounded to nearest for y within two units of the last place of 1/b: value, remainder,
+// correction (Markstein, IBM J. Res. Dev. 34, 1990).  The result is the correctly rounded one, except
+// that a value within 2^-50 of its last place from the middle of two doubles may round the other
+// way; a zero quotient's sign is not kept, and an infinite a gives NaN.
+__device__ __forceinline__ double rcp(double b) {
+  const double y = rcp_near(b);
+  return fma(fma(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ F64 rcp(F64 b) { return rcp(b.v); }
+__device__ __forceinline__ F64 rcp_near(F64 b) { return rcp_near(b.v); }
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ F64 div_rn(F64 a, F64 b, F64 y) {
+  const double q = mul_int(a.v, y.v);
+  return fma(fma(-b.v, q, a.v), y.v, q);
+}
+__device__ __forceinline__ double quot(double a, double b) { return div_rn(a, b, rcp_near(b)); }
+__device__ __forceinline__ F64 operator/(F64 a, F64 b) { return div_rn(a, b, rcp_near(b)); }
+
+// the same arrays, read as F64
+inline const F64* f64(const double* p) { return reinterpret_cast<const F64*>(p); }
+inline F64* f64(double* p) { return reinterpret_cast<F64*>(p); }
+inline const Grid<F64>& f64(const Grid<double>& g) { return reinterpret_cast<const Grid<F64>&>(g); }
+inline const StateT<F64>& f64(const StateT<double>& s) { return reinterpret_cast<const StateT<F64>&>(s); }
+
 // reciprocals of the metrics at their own points, formed once with the grid
 struct Recip {
-  const double *vol, *dx, *dy, *dz;
+  const F64 *vol, *dx, *dy, *dz;
 };
 // what a face hands to the divergences of its two cells: flux times area and the slope term
 // 0.5*f*slope, x at u points, y at v points
 struct Faces {
-  double *px, *py, *hx, *hy;
+  F64 *px, *py, *hx, *hy;
 };
 
 // the explicit kernels (kernels_fp64.cu)
@@ -82,5 +170,25 @@ void launch64_pgrad_cells(const Dims& D, const Grid<double>& G, const State& S, 
 void launch64_pgrad(const Dims& D, const Grid<double>& G, const State& S, const double* gx, const double* gy, const double* gz,
                     const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
                     const double* tpu, const double* tpv, const PGrad<double>& P, int lfirst, cudaStream_t st);
+
+// the column solves (column_fp64.cu)
+// grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of
+// layer jl) z_scalar(jl-1) - z_scalar(jl), that over c_imp2 and half of it over c_imp1 (c_imp2 =
+// impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -
+// exner_bg(jl), 1/area_z; 1/c_imp2 and 1/dtime
+struct ColumnGrid {
+  const double *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
+  double rc_imp2, rdt;
+};
+void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
+                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st);
+int column_prepare();
+void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,
+                       const Tend<double>& Tn, int rk_step, cudaStream_t st);
+// the tracer solve: rvol = 1/volume, itwdtv = 0.5*dtime/volume; csh is written at rk_step 1, with
+// hx as work space
+void launch_column_tracers(const Dims& D, const Grid<double>& G, const State& So, const State& Sn, const double* t_rho,
+                           const double* T, const double* rvol, const double* itwdtv, const double* vcloud,
+                           const double* cpi, const double* cpw, double* csh, double* hx, int rk_step, cudaStream_t st);
 
 }  // namespace lg

@@ -64,21 +64,21 @@ __device__ __forceinline__ bool grad_y_cov(const Dims& D, const Grid<T>& G, cons
 template <class T, class V>
 __device__ __forceinline__ bool stv_h_x(const Dims& D, const V* s, const V* vx, int ji, int jk, int jl, T* r) {
   if (jk >= 2 && jk <= D.nx) {
-    *r = T(0.5) * (T(s[IX(D, ji, jk - 1, jl)]) + T(s[IX(D, ji, jk, jl)])) * T(vx[IX(D, ji, jk, jl)]);
+    *r = half_of(T(s[IX(D, ji, jk - 1, jl)]) + T(s[IX(D, ji, jk, jl)])) * T(vx[IX(D, ji, jk, jl)]);
     return true;
   }
   if (!D.periodic) return false;
-  *r = T(0.5) * (T(s[IX(D, ji, 1, jl)]) + T(s[IX(D, ji, D.nx, jl)])) * T(vx[IX(D, ji, 1, jl)]);
+  *r = half_of(T(s[IX(D, ji, 1, jl)]) + T(s[IX(D, ji, D.nx, jl)])) * T(vx[IX(D, ji, 1, jl)]);
   return true;
 }
 template <class T, class V>
 __device__ __forceinline__ bool stv_h_y(const Dims& D, const V* s, const V* vy, int ji, int jk, int jl, T* r) {
   if (ji >= 2 && ji <= D.ny) {
-    *r = T(0.5) * (T(s[IX(D, ji - 1, jk, jl)]) + T(s[IX(D, ji, jk, jl)])) * T(vy[IX(D, ji, jk, jl)]);
+    *r = half_of(T(s[IX(D, ji - 1, jk, jl)]) + T(s[IX(D, ji, jk, jl)])) * T(vy[IX(D, ji, jk, jl)]);
     return true;
   }
   if (!D.periodic) return false;
-  *r = T(0.5) * (T(s[IX(D, 1, jk, jl)]) + T(s[IX(D, D.ny, jk, jl)])) * T(vy[IX(D, 1, jk, jl)]);
+  *r = half_of(T(s[IX(D, 1, jk, jl)]) + T(s[IX(D, D.ny, jk, jl)])) * T(vy[IX(D, 1, jk, jl)]);
   return true;
 }
 // sum(state%rho(:,:,:,1:nc+1),4) in constituent order
@@ -162,12 +162,12 @@ __device__ __forceinline__ T zeta_x_raw(const Dims& D, const Grid<T>& G, const S
   T r = -G.dy[IX(D, ii, jk, nl)] * hcov_y<T, V>(D, G, v, w, ii, jk, nl);
   if (D.freeslip && (inner || (D.periodic && ii == 1))) {
     const int im = (ii == 1) ? D.ny : ii - 1;
-    r = r + T(0.5) * G.dz[IX(D, im, jk, NL)] * T(w[IX(D, im, jk, NL)])
-          - T(0.5) * G.dz[IX(D, ii, jk, NL)] * T(w[IX(D, ii, jk, NL)])
+    r = r + half_of(G.dz[IX(D, im, jk, NL)]) * T(w[IX(D, im, jk, NL)])
+          - half_of(G.dz[IX(D, ii, jk, NL)]) * T(w[IX(D, ii, jk, NL)])
           + G.dy[IX(D, ii, jk, nl)] * (T(v[IX(D, ii, jk, nl)])
           + (T(v[IX(D, ii, jk, nl - 1)]) - T(v[IX(D, ii, jk, nl)])) / (G.z_v[IX(D, ii, jk, nl - 1)] - G.z_v[IX(D, ii, jk, nl)])
-          * (T(0.5) * (G.z_w[IX(D, im, jk, NL)] + G.z_w[IX(D, ii, jk, NL)]) - G.z_v[IX(D, ii, jk, nl)])
-          + T(0.5) * (T(w[IX(D, im, jk, NL)]) + T(w[IX(D, ii, jk, NL)]))
+          * (half_of(G.z_w[IX(D, im, jk, NL)] + G.z_w[IX(D, ii, jk, NL)]) - G.z_v[IX(D, ii, jk, nl)])
+          + half_of(T(w[IX(D, im, jk, NL)]) + T(w[IX(D, ii, jk, NL)]))
           * (G.z_w[IX(D, im, jk, NL)] - G.z_w[IX(D, ii, jk, NL)]) / G.dy[IX(D, ii, jk, nl)]);
   }
   return r;
@@ -193,12 +193,12 @@ __device__ __forceinline__ T zeta_y_raw(const Dims& D, const Grid<T>& G, const S
   T r = G.dx[IX(D, ji, kk, nl)] * hcov_x<T, V>(D, G, u, w, ji, kk, nl);
   if (D.freeslip && (inner || (D.periodic && kk == 1))) {
     const int km = (kk == 1) ? D.nx : kk - 1;
-    r = r + T(0.5) * G.dz[IX(D, ji, km, NL)] * T(w[IX(D, ji, km, NL)])
-          - T(0.5) * G.dz[IX(D, ji, kk, NL)] * T(w[IX(D, ji, kk, NL)])
+    r = r + half_of(G.dz[IX(D, ji, km, NL)]) * T(w[IX(D, ji, km, NL)])
+          - half_of(G.dz[IX(D, ji, kk, NL)]) * T(w[IX(D, ji, kk, NL)])
           - G.dx[IX(D, ji, kk, nl)] * (T(u[IX(D, ji, kk, nl)])
           + (T(u[IX(D, ji, kk, nl - 1)]) - T(u[IX(D, ji, kk, nl)])) / (G.z_u[IX(D, ji, kk, nl - 1)] - G.z_u[IX(D, ji, kk, nl)])
-          * (T(0.5) * (G.z_w[IX(D, ji, km, NL)] + G.z_w[IX(D, ji, kk, NL)]) - G.z_u[IX(D, ji, kk, nl)])
-          + T(0.5) * (T(w[IX(D, ji, km, NL)]) + T(w[IX(D, ji, kk, NL)]))
+          * (half_of(G.z_w[IX(D, ji, km, NL)] + G.z_w[IX(D, ji, kk, NL)]) - G.z_u[IX(D, ji, kk, nl)])
+          + half_of(T(w[IX(D, ji, km, NL)]) + T(w[IX(D, ji, kk, NL)]))
           * (G.z_w[IX(D, ji, kk, NL)] - G.z_w[IX(D, ji, km, NL)]) / G.dx[IX(D, ji, kk, nl)]);
   }
   return r;
@@ -211,7 +211,7 @@ __device__ __forceinline__ T rho_avg_h(const Dims& D, const Grid<T>& G, const V*
   const T* zs = G.z_scalar;
   auto R = [&](int i, int k, int l) { return T(rho[IX(D, i, k, l)]); };
   if (jl == 1) {
-    return T(0.5) * (R(ia, ka, jl)
+    return half_of(R(ia, ka, jl)
       + (cvt<T>(D.toa) - zs[IX(D, ia, ka, jl)]) * (R(ia, ka, jl) - R(ia, ka, jl + 1))
         / (zs[IX(D, ia, ka, jl)] - zs[IX(D, ia, ka, jl + 1)])
       + R(ib, kb, jl)
@@ -220,14 +220,14 @@ __device__ __forceinline__ T rho_avg_h(const Dims& D, const Grid<T>& G, const V*
   }
   if (jl == D.NL) {
     const T* zw = G.z_w;
-    return T(0.5) * (R(ia, ka, jl - 1)
+    return half_of(R(ia, ka, jl - 1)
       + (zw[IX(D, ia, ka, jl)] - zs[IX(D, ia, ka, jl - 1)]) * (R(ia, ka, jl - 2) - R(ia, ka, jl - 1))
         / (zs[IX(D, ia, ka, jl - 2)] - zs[IX(D, ia, ka, jl - 1)])
       + R(ib, kb, jl - 1)
       + (zw[IX(D, ib, kb, jl)] - zs[IX(D, ib, kb, jl - 1)]) * (R(ib, kb, jl - 2) - R(ib, kb, jl - 1))
         / (zs[IX(D, ib, kb, jl - 2)] - zs[IX(D, ib, kb, jl - 1)]));
   }
-  return T(0.25) * (R(ia, ka, jl - 1) + R(ib, kb, jl - 1) + R(ia, ka, jl) + R(ib, kb, jl));
+  return quarter_of(R(ia, ka, jl - 1) + R(ib, kb, jl - 1) + R(ia, ka, jl) + R(ib, kb, jl));
 }
 
 // eta_x at (ji,jk,jl), jl in 1..nl+1
@@ -280,7 +280,7 @@ __device__ __forceinline__ T eta_z_at(const Dims& D, const Grid<T>& G, const Sta
   if (inner || D.periodic) {
     const V* rg = S.rho + (long long)(D.g - 1) * D.fstride;
     const int km = (jk == 1) ? D.nx : jk - 1, im = (ji == 1) ? D.ny : ji - 1;
-    e = e / (T(0.25) * (T(rg[IX(D, ji, km, jl)]) + T(rg[IX(D, ji, jk, jl)]) + T(rg[IX(D, im, jk, jl)]) +
+    e = e / (quarter_of(T(rg[IX(D, ji, km, jl)]) + T(rg[IX(D, ji, jk, jl)]) + T(rg[IX(D, im, jk, jl)]) +
                         T(rg[IX(D, im, km, jl)])));
   }
   return e;
@@ -292,12 +292,12 @@ __device__ __forceinline__ T trsk_u(const Dims& D, const Grid<T>& G, const T* vp
                                     int ji, int km, int kk, int kp, int jl) {
   const T w1 = G.trsk_u[0][ji - 1], w2 = G.trsk_u[1][ji - 1], w3 = G.trsk_u[2][ji - 1];
 #define EZ(i, k) ez[IX(D, i, k, jl)]
-  return w1 * vp[IX(D, ji, km, jl)] * T(0.25) * (EZ(ji, km) + EZ(ji, kk) + EZ(ji, kk) + EZ(ji + 1, kk))
-       + w2 * up[IX(D, ji, km, jl)] * T(0.25) * (EZ(ji, km) + EZ(ji + 1, km) + EZ(ji, kk) + EZ(ji + 1, kk))
-       + w3 * vp[IX(D, ji + 1, km, jl)] * T(0.25) * (EZ(ji + 1, km) + EZ(ji + 1, kk) + EZ(ji, kk) + EZ(ji + 1, kk))
-       + w3 * vp[IX(D, ji + 1, kk, jl)] * T(0.25) * (EZ(ji + 1, kk) + EZ(ji + 1, kp) + EZ(ji, kk) + EZ(ji + 1, kk))
-       + w2 * up[IX(D, ji, kp, jl)] * T(0.25) * (EZ(ji + 1, kp) + EZ(ji, kp) + EZ(ji, kk) + EZ(ji + 1, kk))
-       + w1 * vp[IX(D, ji, kk, jl)] * T(0.25) * (EZ(ji, kk) + EZ(ji, kp) + EZ(ji, kk) + EZ(ji + 1, kk));
+  return quarter_of(w1 * vp[IX(D, ji, km, jl)]) * (EZ(ji, km) + EZ(ji, kk) + EZ(ji, kk) + EZ(ji + 1, kk))
+       + quarter_of(w2 * up[IX(D, ji, km, jl)]) * (EZ(ji, km) + EZ(ji + 1, km) + EZ(ji, kk) + EZ(ji + 1, kk))
+       + quarter_of(w3 * vp[IX(D, ji + 1, km, jl)]) * (EZ(ji + 1, km) + EZ(ji + 1, kk) + EZ(ji, kk) + EZ(ji + 1, kk))
+       + quarter_of(w3 * vp[IX(D, ji + 1, kk, jl)]) * (EZ(ji + 1, kk) + EZ(ji + 1, kp) + EZ(ji, kk) + EZ(ji + 1, kk))
+       + quarter_of(w2 * up[IX(D, ji, kp, jl)]) * (EZ(ji + 1, kp) + EZ(ji, kp) + EZ(ji, kk) + EZ(ji + 1, kk))
+       + quarter_of(w1 * vp[IX(D, ji, kk, jl)]) * (EZ(ji, kk) + EZ(ji, kp) + EZ(ji, kk) + EZ(ji + 1, kk));
 }
 
 // TRSK term for v, mo_vorticity_flux.F90:72-80 (im, ii: rows ji-1, ji)
@@ -305,10 +305,10 @@ template <class T>
 __device__ __forceinline__ T trsk_v(const Dims& D, const Grid<T>& G, const T* up, const T* ez, int im, int ii, int jk,
                                     int jl) {
   const T w1 = G.trsk_v[0][ii - 1], w2 = G.trsk_v[1][ii - 1];
-  return w1 * up[IX(D, ii, jk, jl)] * T(0.25) * (EZ(ii, jk) + EZ(ii + 1, jk) + EZ(ii, jk) + EZ(ii, jk + 1))
-       + w1 * up[IX(D, ii, jk + 1, jl)] * T(0.25) * (EZ(ii, jk + 1) + EZ(ii + 1, jk + 1) + EZ(ii, jk) + EZ(ii, jk + 1))
-       + w2 * up[IX(D, im, jk + 1, jl)] * T(0.25) * (EZ(im, jk + 1) + EZ(ii, jk + 1) + EZ(ii, jk) + EZ(ii, jk + 1))
-       + w2 * up[IX(D, im, jk, jl)] * T(0.25) * (EZ(im, jk) + EZ(ii, jk) + EZ(ii, jk) + EZ(ii, jk + 1));
+  return quarter_of(w1 * up[IX(D, ii, jk, jl)]) * (EZ(ii, jk) + EZ(ii + 1, jk) + EZ(ii, jk) + EZ(ii, jk + 1))
+       + quarter_of(w1 * up[IX(D, ii, jk + 1, jl)]) * (EZ(ii, jk + 1) + EZ(ii + 1, jk + 1) + EZ(ii, jk) + EZ(ii, jk + 1))
+       + quarter_of(w2 * up[IX(D, im, jk + 1, jl)]) * (EZ(im, jk + 1) + EZ(ii, jk + 1) + EZ(ii, jk) + EZ(ii, jk + 1))
+       + quarter_of(w2 * up[IX(D, im, jk, jl)]) * (EZ(im, jk) + EZ(ii, jk) + EZ(ii, jk) + EZ(ii, jk + 1));
 #undef EZ
 }
 
@@ -420,7 +420,7 @@ __global__ void k_mass_flux(Dims D, Grid<T> G, StateT<V> S, T* uph, T* vph, T* w
   }
   if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
     const long long q = IX(D, ji, jk, jl);
-    wph[q] = T(0.5) * (T(rg[IX(D, ji, jk, jl - 1)]) + T(rg[q])) * T(S.w[q]);
+    wph[q] = half_of(T(rg[IX(D, ji, jk, jl - 1)]) + T(rg[q])) * T(S.w[q]);
   }
 }
 
@@ -447,10 +447,10 @@ __device__ __forceinline__ void vort_flux_body(const Dims& D, const Grid<T>& G, 
     if (inner || D.periodic) {
       const int kk = inner ? jk : 1, km = inner ? jk - 1 : D.nx, kp = kk + 1;
       T r = trsk_u<T>(D, G, vph, uph, ez, ji, km, kk, kp, jl);
-      r = r - T(0.5) * W_(5, ji, km, jl) * wp(ji, km, jl) * ey[IX(D, ji, kk, jl)]
-            - T(0.5) * W_(6, ji, km, jl) * wp(ji, km, jl + 1) * ey[IX(D, ji, kk, jl + 1)]
-            - T(0.5) * W_(5, ji, kk, jl) * wp(ji, kk, jl) * ey[IX(D, ji, kk, jl)]
-            - T(0.5) * W_(6, ji, kk, jl) * wp(ji, kk, jl + 1) * ey[IX(D, ji, kk, jl + 1)];
+      r = r - half_of(W_(5, ji, km, jl)) * wp(ji, km, jl) * ey[IX(D, ji, kk, jl)]
+            - half_of(W_(6, ji, km, jl)) * wp(ji, km, jl + 1) * ey[IX(D, ji, kk, jl + 1)]
+            - half_of(W_(5, ji, kk, jl)) * wp(ji, kk, jl) * ey[IX(D, ji, kk, jl)]
+            - half_of(W_(6, ji, kk, jl)) * wp(ji, kk, jl + 1) * ey[IX(D, ji, kk, jl + 1)];
       px[IX(D, ji, jk, jl)] = r;
     }
   }
@@ -459,15 +459,15 @@ __device__ __forceinline__ void vort_flux_body(const Dims& D, const Grid<T>& G, 
     if (inner || D.periodic) {
       const int ii = inner ? ji : 1, im = inner ? ji - 1 : D.ny;
       T r = trsk_v<T>(D, G, uph, ez, im, ii, jk, jl);
-      r = r + T(0.5) * W_(5, im, jk, jl) * wp(im, jk, jl) * ex[IX(D, ii, jk, jl)]
-            + T(0.5) * W_(6, im, jk, jl) * wp(im, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)]
-            + T(0.5) * W_(5, ii, jk, jl) * wp(ii, jk, jl) * ex[IX(D, ii, jk, jl)]
-            + T(0.5) * W_(6, ii, jk, jl) * wp(ii, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)];
+      r = r + half_of(W_(5, im, jk, jl)) * wp(im, jk, jl) * ex[IX(D, ii, jk, jl)]
+            + half_of(W_(6, im, jk, jl)) * wp(im, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)]
+            + half_of(W_(5, ii, jk, jl)) * wp(ii, jk, jl) * ex[IX(D, ii, jk, jl)]
+            + half_of(W_(6, ii, jk, jl)) * wp(ii, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)];
       py[IX(D, ji, jk, jl)] = r;
     }
   }
   if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
-    pz[IX(D, ji, jk, jl)] = T(0.5) * (
+    pz[IX(D, ji, jk, jl)] = half_of(
         W_(1, ji, jk, jl - 1) * uph[IX(D, ji, jk + 1, jl - 1)] * ey[IX(D, ji, jk + 1, jl)]
       - W_(2, ji, jk, jl - 1) * vph[IX(D, ji, jk, jl - 1)] * ex[IX(D, ji, jk, jl)]
       + W_(3, ji, jk, jl - 1) * uph[IX(D, ji, jk, jl - 1)] * ey[IX(D, ji, jk, jl)]
@@ -516,7 +516,7 @@ __global__ void k_tend_wind(Dims D, State So, State Sn, Tend<T> Tn, Carried<T> C
   };
   if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
     const long long q = IX(D, ji, jk, jl);
-    T f = pg_h(C.old_u, C.nl_u, C.l_u, q) - T(0.5) * C.vsg_x[q] + C.pvt_x[q];
+    T f = pg_h(C.old_u, C.nl_u, C.l_u, q) - half_of(C.vsg_x[q]) + C.pvt_x[q];
     if (C.mdt_x) f = f + C.mdt_x[q];
     const T t = old_weight * Tn.u[q] + new_weight * f;
     Tn.u[q] = t;
@@ -526,7 +526,7 @@ __global__ void k_tend_wind(Dims D, State So, State Sn, Tend<T> Tn, Carried<T> C
   }
   if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
     const long long q = IX(D, ji, jk, jl);
-    T f = pg_h(C.old_v, C.nl_v, C.l_v, q) - T(0.5) * C.vsg_y[q] + C.pvt_y[q];
+    T f = pg_h(C.old_v, C.nl_v, C.l_v, q) - half_of(C.vsg_y[q]) + C.pvt_y[q];
     if (C.mdt_y) f = f + C.mdt_y[q];
     const T t = old_weight * Tn.v[q] + new_weight * f;
     Tn.v[q] = t;
@@ -539,32 +539,15 @@ __global__ void k_tend_wind(Dims D, State So, State Sn, Tend<T> Tn, Carried<T> C
     T pg;
     if (pg32) pg = -(T(cvw_d) * cvt<T>(C.nl_w[q] + C.l_w[q]));
     else pg = cvt<T>(-(cvw_d * (C.nl_w[q] + C.l_w[q])) - no_bg_d * (1.0 - cvw_d) * C.l_w[q]);
-    T f = pg - T(0.5) * C.vsg_z[q] + C.pvt_z[q] + C.pgcw[q];
+    T f = pg - half_of(C.vsg_z[q]) + C.pvt_z[q] + C.pgcw[q];
     if (C.mdt_z) f = f + C.mdt_z[q];
     Tn.w[q] = old_weight * Tn.w[q] + new_weight * f;
   }
 }
 
-// ---- FP64-only kernels (column_fp64.cu; the explicit ones: fp64.cuh) --------------------
-// grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of
-// layer jl) z_scalar(jl-1) - z_scalar(jl), that over c_imp2 and half of it over c_imp1 (c_imp2 =
-// impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -
-// exner_bg(jl), 1/area_z; 1/c_imp2 and 1/dtime
-struct ColumnGrid {
-  const double *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
-  double rc_imp2, rdt;
-};
-void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
-                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st);
-int column_prepare();
-void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,
-                       const Tend<double>& Tn, int rk_step, cudaStream_t st);
+// ---- FP64-only kernels (column_fp64.cu; the others: fp64.cuh) --------------------------
 // once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
 // and c_p of ice and water
 __global__ void k_moist_aux(Dims D, Grid<double> G, State So, const double* T, double* vcloud, double* cpi, double* cpw);
-// the tracer solve: rvol = 1/volume, itwdtv = 0.5*dtime/volume; csh is written at rk_step 1
-void launch_column_tracers(const Dims& D, const Grid<double>& G, const State& So, const State& Sn, const double* t_rho,
-                           const double* T, const double* rvol, const double* itwdtv, const double* vcloud,
-                           const double* cpi, const double* cpw, double* csh, int rk_step, cudaStream_t st);
 
 }  // namespace lg

@@ -7,20 +7,33 @@
 // not start with 0 + x.
 #include "fp64.cuh"
 
+#include <algorithm>
+
 namespace lg {
 
 namespace {
 
-constexpr int kMarch = 8;  // levels of a marching thread's chunk (blockIdx.z)
+struct PGradF { F64 *nl_u, *nl_v, *nl_w, *l_u, *l_v, *l_w, *old_u, *old_v, *pgcw; };
+
+// marching threads: a chunk of the column's levels each (blockIdx.z), of eight levels (the layer above a
+// chunk is formed twice) and of fewer, down to two, where that leaves an SM under 1536 threads
 dim3 march_grid(const Dims& D) {
-  return dim3((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 3) / 4), (unsigned)((D.nl + kMarch - 1) / kMarch));
+  dim3 g((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 3) / 4), 1);
+  const long long cells = 128LL * g.x * g.y * D.nl;
+  const int len = (int)std::min(8LL, std::max(2LL, cells / (152LL * 1536)));
+  g.z = (unsigned)((D.nl + len - 1) / len);
+  return g;
+}
+__device__ __forceinline__ int march_first(const Dims& D, unsigned z) {
+  const int len = (D.nl + (int)gridDim.z - 1) / (int)gridDim.z;
+  return min((int)z * len, D.nl) + 1;
 }
 dim3 cell_grid(int rows, int cols, int levs) {
   return dim3((unsigned)((rows + 31) / 32), (unsigned)levs, (unsigned)((cols + 7) / 8));
 }
 const dim3 kMarchBlock(32, 4), kCellBlock(32, 8);
 
-__global__ void k64_recip(Dims D, Grid<double> G, double* rdx, double* rdy, double* rdz) {
+__global__ void k64_recip(Dims D, Grid<F64> G, F64* rdx, F64* rdy, F64* rdz) {
   LG_IDX3;
   const long long q = IX(D, ji, jk, jl);
   if (ji <= D.ny && jk <= D.nx + 1) rdx[q] = 1.0 / G.dx[q];
@@ -33,18 +46,19 @@ __global__ void k64_recip(Dims D, Grid<double> G, double* rdx, double* rdy, doub
 // two products of the remap to the horizontal faces (mo_averaging.F90:56-136), W5(l)*gz(l) and
 // W6(l)*gz(l+1), which the four faces of the column share.  gz_sfc: gz at level nl+1 (never written
 // by grad_vert) as the array holds it.
-__global__ void __launch_bounds__(128) k64_grad_vert(Dims D, Grid<double> G, const double* rdz, const double* s, double* gz,
-                                                     double* w5, double* w6) {
+__global__ void __launch_bounds__(128) k64_grad_vert(Dims D, Grid<F64> G, const F64* rdz, const F64* s, F64* gz,
+                                                     F64* w5, F64* w6) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
-  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  const int l0 = march_first(D, blockIdx.z), l1 = march_first(D, blockIdx.z + 1) - 1;
+  if (l0 > l1) return;
   long long q = IX(D, ji, jk, l0);
-  double cur = s[q];
-  double g = (l0 >= 2) ? div_rn(s[q - D.plane] - cur, G.dz[q], rdz[q]) : 0.0;
+  F64 cur = s[q];
+  F64 g = (l0 >= 2) ? div_rn(s[q - D.plane] - cur, G.dz[q], rdz[q]) : 0.0;
   for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
-    double gn = 0.0;
+    F64 gn = 0.0;
     if (jl < D.nl) {
-      const double nxt = s[q + D.plane];
+      const F64 nxt = s[q + D.plane];
       gn = div_rn(cur - nxt, G.dz[q + D.plane], rdz[q + D.plane]);
       cur = nxt;
     }
@@ -59,38 +73,38 @@ __global__ void __launch_bounds__(128) k64_grad_vert(Dims D, Grid<double> G, con
 }
 
 // the horizontal gradient at u and v points; false where the reference leaves the point untouched
-__device__ __forceinline__ bool grad_x64(const Dims& D, const Grid<double>& G, const double* rdx, const double* s,
-                                         const double* w5, const double* w6, int ji, int jk, int jl, double* r) {
+__device__ __forceinline__ bool grad_x64(const Dims& D, const Grid<F64>& G, const F64* rdx, const F64* s,
+                                         const F64* w5, const F64* w6, int ji, int jk, int jl, F64* r) {
   const bool inner = jk >= 2 && jk <= D.nx;
   if (!inner && !D.periodic) return false;
   const long long a = IX(D, ji, inner ? jk - 1 : D.nx, jl), b = IX(D, ji, inner ? jk : 1, jl);
-  double g = div_rn(s[b] - s[a], G.dx[b], rdx[b]);
+  F64 g = div_rn(s[b] - s[a], G.dx[b], rdx[b]);
   if (jl > D.nf) {
-    double m = w5[a] + w5[b];
+    F64 m = w5[a] + w5[b];
     if (jl < D.nl || D.freeslip) m = m + w6[a] + w6[b];
     g = g - G.slope_x[IX(D, ji, jk, jl)] * half(m);
   }
   *r = g;
   return true;
 }
-__device__ __forceinline__ bool grad_y64(const Dims& D, const Grid<double>& G, const double* rdy, const double* s,
-                                         const double* w5, const double* w6, int ji, int jk, int jl, double* r) {
+__device__ __forceinline__ bool grad_y64(const Dims& D, const Grid<F64>& G, const F64* rdy, const F64* s,
+                                         const F64* w5, const F64* w6, int ji, int jk, int jl, F64* r) {
   const bool inner = ji >= 2 && ji <= D.ny;
   if (!inner && !D.periodic) return false;
   const long long a = IX(D, inner ? ji - 1 : D.ny, jk, jl), b = IX(D, inner ? ji : 1, jk, jl);
-  double g = div_rn(s[a] - s[b], G.dy[b], rdy[b]);
+  F64 g = div_rn(s[a] - s[b], G.dy[b], rdy[b]);
   if (jl > D.nf) {
-    double m = w5[a] + w5[b];
+    F64 m = w5[a] + w5[b];
     if (jl < D.nl || D.freeslip) m = m + w6[a] + w6[b];
     g = g - G.slope_y[IX(D, ji, jk, jl)] * half(m);
   }
   *r = g;
   return true;
 }
-__global__ void k64_grad_hor(Dims D, Grid<double> G, Recip R, const double* s, const double* w5, const double* w6,
-                             double* rx, double* ry) {
+__global__ void k64_grad_hor(Dims D, Grid<F64> G, Recip R, const F64* s, const F64* w5, const F64* w6,
+                             F64* rx, F64* ry) {
   LG_IDX3;
-  double r;
+  F64 r;
   if (ji <= D.ny && jk <= D.nx + 1 && grad_x64(D, G, R.dx, s, w5, w6, ji, jk, jl, &r)) rx[IX(D, ji, jk, jl)] = r;
   if (ji <= D.ny + 1 && jk <= D.nx && grad_y64(D, G, R.dy, s, w5, w6, ji, jk, jl, &r)) ry[IX(D, ji, jk, jl)] = r;
 }
@@ -100,11 +114,11 @@ __global__ void k64_grad_hor(Dims D, Grid<double> G, Recip R, const double* s, c
 // 0.5*f*slope of the contravariant vertical velocity (mo_averaging.F90:16-54).  The faces of a
 // non-periodic boundary, which the reference leaves untouched at 0, are written as 0: the arrays serve
 // several fields in turn.
-__device__ __forceinline__ void face_x(const Dims& D, const Grid<double>& G, double f, const Faces& F, int jl, long long q) {
+__device__ __forceinline__ void face_x(const Dims& D, const Grid<F64>& G, F64 f, const Faces& F, int jl, long long q) {
   F.px[q] = f * G.area_x[q];
   if (jl > D.nf) F.hx[q] = half(f) * G.slope_x[q];
 }
-__device__ __forceinline__ void face_y(const Dims& D, const Grid<double>& G, double f, const Faces& F, int jl, long long q) {
+__device__ __forceinline__ void face_y(const Dims& D, const Grid<F64>& G, F64 f, const Faces& F, int jl, long long q) {
   F.py[q] = f * G.area_y[q];
   if (jl > D.nf) F.hy[q] = half(f) * G.slope_y[q];
 }
@@ -112,19 +126,19 @@ __device__ __forceinline__ void face_y(const Dims& D, const Grid<double>& G, dou
 // the vertical part of a column's divergence, walked down: the reference's sum at an interface runs
 // over the four slope terms of the layer above and then of the layer below, so the sum over a layer's
 // own terms serves as the start of the interface below it
-struct SlopeTerms { double a, b, c, d; };
-__device__ __forceinline__ SlopeTerms slope_terms(const Dims& D, const Grid<double>& G, const double* hx, const double* hy,
+struct SlopeTerms { F64 a, b, c, d; };
+__device__ __forceinline__ SlopeTerms slope_terms(const Dims& D, const Grid<F64>& G, const F64* hx, const F64* hy,
                                                   long long q) {
   return SlopeTerms{hx[q + D.P] * G.ipw[0][q], hy[q] * G.ipw[1][q], hx[q] * G.ipw[2][q], hy[q + 1] * G.ipw[3][q]};
 }
-__device__ __forceinline__ double own_sum(const SlopeTerms& t) { return -t.a - t.b - t.c - t.d; }
-__device__ __forceinline__ double join(double above, const SlopeTerms& t) { return above - t.a - t.b - t.c - t.d; }
+__device__ __forceinline__ F64 own_sum(const SlopeTerms& t) { return -t.a - t.b - t.c - t.d; }
+__device__ __forceinline__ F64 join(F64 above, const SlopeTerms& t) { return above - t.a - t.b - t.c - t.d; }
 
 // the contravariant correction at interface l = nf+1..nl of the layers above and below it
 struct Contra {
-  double sum;  // own_sum of the current layer
+  F64 sum;  // own_sum of the current layer
   // at the chunk's first level l0 (> nf): the correction at its upper interface
-  __device__ __forceinline__ double start(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, long long q,
+  __device__ __forceinline__ F64 start(const Dims& D, const Grid<F64>& G, const F64* hx, const F64* hy, long long q,
                                           int l0) {
     const SlopeTerms t = slope_terms(D, G, hx, hy, q);
     sum = own_sum(t);
@@ -132,27 +146,27 @@ struct Contra {
     return join(own_sum(slope_terms(D, G, hx, hy, q - D.plane)), t);
   }
   // the correction at the lower interface of layer jl (jl == nf, or nf < jl < nl); q: layer jl
-  __device__ __forceinline__ double below(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, long long q,
+  __device__ __forceinline__ F64 below(const Dims& D, const Grid<F64>& G, const F64* hx, const F64* hy, long long q,
                                           int jl) {
     const SlopeTerms t = slope_terms(D, G, hx, hy, q + D.plane);
-    const double r = (jl == D.nf) ? own_sum(t) : join(sum, t);
+    const F64 r = (jl == D.nf) ? own_sum(t) : join(sum, t);
     sum = own_sum(t);
     return r;
   }
 };
 struct ColumnDiv {
   Contra c;
-  double up;  // correction times area at the upper interface
-  __device__ __forceinline__ void start(const Dims& D, const Grid<double>& G, const Faces& F, long long q, int l0) {
+  F64 up;  // correction times area at the upper interface
+  __device__ __forceinline__ void start(const Dims& D, const Grid<F64>& G, const Faces& F, long long q, int l0) {
     up = 0.0;
     c.sum = 0.0;
     if (l0 > D.nf) up = c.start(D, G, F.hx, F.hy, q, l0) * G.area_z[q];
   }
   // divergence of layer jl
-  __device__ __forceinline__ double step(const Dims& D, const Grid<double>& G, const Faces& F, double V, double rV, long long q,
+  __device__ __forceinline__ F64 step(const Dims& D, const Grid<F64>& G, const Faces& F, F64 V, F64 rV, long long q,
                                          int jl) {
-    double s = F.px[q + D.P] + F.py[q] - F.px[q] - F.py[q + 1];
-    double lo = 0.0;
+    F64 s = F.px[q + D.P] + F.py[q] - F.px[q] - F.py[q + 1];
+    F64 lo = 0.0;
     if (jl == D.nf || (jl > D.nf && jl < D.nl)) lo = c.below(D, G, F.hx, F.hy, q, jl) * G.area_z[q + D.plane];
     if (jl == D.nf) s = s - lo;
     else if (jl == D.nl) s = s + up;
@@ -163,18 +177,19 @@ struct ColumnDiv {
 };
 
 // faces of the gradient of a scalar, and their divergence (theta_v_adv_3rd_order)
-__global__ void k64_grad_faces(Dims D, Grid<double> G, Recip R, const double* s, const double* w5, const double* w6, Faces F) {
+__global__ void k64_grad_faces(Dims D, Grid<F64> G, Recip R, const F64* s, const F64* w5, const F64* w6, Faces F) {
   LG_IDX3;
-  double r;
+  F64 r;
   if (ji <= D.ny && jk <= D.nx + 1)
     face_x(D, G, grad_x64(D, G, R.dx, s, w5, w6, ji, jk, jl, &r) ? r : 0.0, F, jl, IX(D, ji, jk, jl));
   if (ji <= D.ny + 1 && jk <= D.nx)
     face_y(D, G, grad_y64(D, G, R.dy, s, w5, w6, ji, jk, jl, &r) ? r : 0.0, F, jl, IX(D, ji, jk, jl));
 }
-__global__ void __launch_bounds__(128) k64_div(Dims D, Grid<double> G, const double* rvol, Faces F, double* out) {
+__global__ void __launch_bounds__(128) k64_div(Dims D, Grid<F64> G, const F64* rvol, Faces F, F64* out) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
-  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  const int l0 = march_first(D, blockIdx.z), l1 = march_first(D, blockIdx.z + 1) - 1;
+  if (l0 > l1) return;
   long long q = IX(D, ji, jk, l0);
   ColumnDiv c;
   c.start(D, G, F, q, l0);
@@ -182,10 +197,10 @@ __global__ void __launch_bounds__(128) k64_div(Dims D, Grid<double> G, const dou
 }
 
 // theta_v_adv_3rd_order edge values, mo_multiplications.F90:134-202
-__global__ void k64_theta_edges(Dims D, const double* th, const double* Dv, const double* u, const double* v, double* tvu,
-                                double* tvv) {
+__global__ void k64_theta_edges(Dims D, const F64* th, const F64* Dv, const F64* u, const F64* v, F64* tvu,
+                                F64* tvv) {
   LG_IDX3;
-  const double c = D.theta_edge_c;
+  const F64 c = D.theta_edge_c;
   if (ji <= D.ny && jk <= D.nx + 1) {
     const bool inner = jk >= 2 && jk <= D.nx;
     if (inner || D.periodic) {
@@ -205,15 +220,15 @@ __global__ void k64_theta_edges(Dims D, const double* th, const double* Dv, cons
 // ---- scalar tendencies, mo_scalar_tend_expl.F90:106-177 ---------------------------------------------
 // faces of the gas mass flux and of the theta_v flux (theta_order 3: edge values tvu, tvv; 2: the
 // mean of the two cells)
-__global__ void k64_gas_faces(Dims D, Grid<double> G, StateT<double> Ss, const double* u_new, const double* v_new,
-                              const double* tvu, const double* tvv, Faces M, Faces T) {
+__global__ void k64_gas_faces(Dims D, Grid<F64> G, StateT<F64> Ss, const F64* u_new, const F64* v_new,
+                              const F64* tvu, const F64* tvv, Faces M, Faces T) {
   LG_IDX3;
-  const double* rg = Ss.rho + (long long)(D.g - 1) * D.fstride;
+  const F64* rg = Ss.rho + (long long)(D.g - 1) * D.fstride;
   auto th = [&](long long p) { return G.theta_v_bg[p] + Ss.tp[p]; };
   if (ji <= D.ny && jk <= D.nx + 1) {
     const bool inner = jk >= 2 && jk <= D.nx;
     const long long q = IX(D, ji, jk, jl);
-    double f = 0.0, g = 0.0;  // (a non-periodic boundary's faces carry no flux)
+    F64 f = 0.0, g = 0.0;  // (a non-periodic boundary's faces carry no flux)
     if (inner || D.periodic) {
       const long long a = IX(D, ji, inner ? jk - 1 : D.nx, jl), b = IX(D, ji, inner ? jk : 1, jl);
       f = half(rg[a] + rg[b]) * u_new[b];
@@ -225,7 +240,7 @@ __global__ void k64_gas_faces(Dims D, Grid<double> G, StateT<double> Ss, const d
   if (ji <= D.ny + 1 && jk <= D.nx) {
     const bool inner = ji >= 2 && ji <= D.ny;
     const long long q = IX(D, ji, jk, jl);
-    double f = 0.0, g = 0.0;
+    F64 f = 0.0, g = 0.0;
     if (inner || D.periodic) {
       const long long a = IX(D, inner ? ji - 1 : D.ny, jk, jl), b = IX(D, inner ? ji : 1, jk, jl);
       f = half(rg[a] + rg[b]) * v_new[b];
@@ -236,38 +251,39 @@ __global__ void k64_gas_faces(Dims D, Grid<double> G, StateT<double> Ss, const d
   }
 }
 
-// their divergences and the diabatic term: the gas and rho*theta_v tendencies (k_gas_theta<double>
+// their divergences and the diabatic term: the gas and rho*theta_v tendencies (k_gas_theta<F64>
 // formed every face two to five times and c_p of every condensate anew: 2084 us a launch at
 // 192x192x80)
-__global__ void __launch_bounds__(128) k64_gas_theta(Dims D, Grid<double> G, StateT<double> Ss, const double* rvol, Faces M,
-                                                     Faces T, const double* cpi, const double* cpw, const double* hd,
-                                                     const double* rad, const double* csh, double* t_rho, double* t_rt,
-                                                     const double* mdt, const double* tdh, const double* ptr,
-                                                     const double* pth) {
+__global__ void __launch_bounds__(128) k64_gas_theta(Dims D, Grid<F64> G, StateT<F64> Ss, const F64* rvol, Faces M,
+                                                     Faces T, const F64* cpi, const F64* cpw, const F64* hd,
+                                                     const F64* rad, const F64* csh, F64* t_rho, F64* t_rt,
+                                                     const F64* mdt, const F64* tdh, const F64* ptr,
+                                                     const F64* pth) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
-  const int l0 = blockIdx.z * kMarch + 1, l1 = min(D.nl, l0 + kMarch - 1);
+  const int l0 = march_first(D, blockIdx.z), l1 = march_first(D, blockIdx.z + 1) - 1;
+  if (l0 > l1) return;
   const long long goff = (long long)(D.g - 1) * D.fstride;
   long long q = IX(D, ji, jk, l0);
   ColumnDiv cm, ct;
   cm.start(D, G, M, q, l0);
   ct.start(D, G, T, q, l0);
   for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
-    const double V = G.volume[q], rV = rvol[q];
-    const double div_m = cm.step(D, G, M, V, rV, q, jl), div_t = ct.step(D, G, T, V, rV, q, jl);
-    double heat = hd[q] + rad[q];
+    const F64 V = G.volume[q], rV = rvol[q];
+    const F64 div_m = cm.step(D, G, M, V, rV, q, jl), div_t = ct.step(D, G, T, V, rV, q, jl);
+    F64 heat = hd[q] + rad[q];
     if (pth) heat = heat + pth[q];
     heat = heat + csh[q];
     if (tdh) heat = heat + tdh[q];
-    double r = -div_t;
+    F64 r = -div_t;
     if (nonzero(heat)) {
-      const double rg = Ss.rho[q + goff];
-      double cv;  // c_v_mass_weighted_air, mo_derived.F90:157-187 (odd constituents are ice)
+      const F64 rg = Ss.rho[q + goff];
+      F64 cv;  // c_v_mass_weighted_air, mo_derived.F90:157-187 (odd constituents are ice)
       if (D.lmoist) {
-        const double ci = cpi[q], cw = cpw[q];
+        const F64 ci = cpi[q], cw = cpw[q];
         cv = Ss.rho[q] * ci;
         for (int jc = 2; jc <= D.nc; ++jc) cv = cv + Ss.rho[q + (long long)(jc - 1) * D.fstride] * ((jc & 1) ? ci : cw);
-        const double rv = Ss.rho[q + goff + D.fstride];
+        const F64 rv = Ss.rho[q + goff + D.fstride];
         cv = cv + (rg - rv) * kC_D_V;
         cv = cv + rv * kC_V_V;
       } else {
@@ -275,10 +291,10 @@ __global__ void __launch_bounds__(128) k64_gas_theta(Dims D, Grid<double> G, Sta
       }
       r = r + kC_D_V * rg / cv * heat / (kC_D_P * (G.exner_bg[q] + Ss.ep[q]));
     }
-    double tg = -div_m;
+    F64 tg = -div_m;
     if (mdt) tg = tg + mdt[q + goff];
     if (ptr) {
-      const double ptg = ptr[q + goff];
+      const F64 ptg = ptr[q + goff];
       tg = tg + ptg;
       r = r + (mdt ? ptg + mdt[q + goff] : ptg) * (G.theta_v_bg[q] + Ss.tp[q]);
     } else if (mdt) {
@@ -290,10 +306,10 @@ __global__ void __launch_bounds__(128) k64_gas_theta(Dims D, Grid<double> G, Sta
 }
 
 // the contravariant correction of the new wind at the interfaces nf+1..nl, for the tracers
-__global__ void __launch_bounds__(128) k64_contra(Dims D, Grid<double> G, const double* hx, const double* hy, double* cw) {
+__global__ void __launch_bounds__(128) k64_contra(Dims D, Grid<F64> G, const F64* hx, const F64* hy, F64* cw) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
-  const int l0 = max((int)blockIdx.z * kMarch + 1, D.nf + 1), l1 = min(D.nl, (int)(blockIdx.z + 1) * kMarch);
+  const int l0 = max(march_first(D, blockIdx.z), D.nf + 1), l1 = march_first(D, blockIdx.z + 1) - 1;
   if (l0 > l1) return;
   long long q = IX(D, ji, jk, l0);
   Contra c;
@@ -303,7 +319,7 @@ __global__ void __launch_bounds__(128) k64_contra(Dims D, Grid<double> G, const 
     q += D.plane;
   }
 }
-__global__ void k64_wind_slopes(Dims D, Grid<double> G, const double* u, const double* v, double* hx, double* hy) {
+__global__ void k64_wind_slopes(Dims D, Grid<F64> G, const F64* u, const F64* v, F64* hx, F64* hy) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.z * blockDim.y + threadIdx.y + 1;
   const int jl = blockIdx.y + D.nf + 1;
@@ -316,13 +332,13 @@ __global__ void k64_wind_slopes(Dims D, Grid<double> G, const double* u, const d
 // scalar_times_vector_h_upstream (mo_multiplications.F90:206-287) and div_h_tracers
 // (mo_divergence_operators.F90:70-147): velocity, area and upwind cell of each of a cell's six faces
 // are found once for all tracers.  At the first substep the old tendency has weight 0 and is not read.
-__global__ void __launch_bounds__(256) k64_tracers(Dims D, Grid<double> G, const double* rvol, StateT<double> Ss,
-                                                   const double* u_new, const double* v_new, const double* cw, double* t_rho,
-                                                   int rk_step, const double* mdt, const double* ptr) {
+__global__ void __launch_bounds__(256) k64_tracers(Dims D, Grid<F64> G, const F64* rvol, StateT<F64> Ss,
+                                                   const F64* u_new, const F64* v_new, const F64* cw, F64* t_rho,
+                                                   int rk_step, const F64* mdt, const F64* ptr) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
   const long long q = IX(D, ji, jk, jl);
-  struct F { double v, a; long long i; };
+  struct F { F64 v, a; long long i; };
   auto fx = [&](int kf) {
     const bool inner = kf >= 2 && kf <= D.nx;
     F f{0.0, 0.0, q};
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(256) k64_tracers(Dims D, Grid<double> G, const
   };
   const F e = fx(jk + 1), n = fy(ji), w = fx(jk), s = fy(ji + 1);
   const bool has_up = jl > D.nf, has_lo = jl == D.nf || (jl > D.nf && jl < D.nl);
-  double cu = 0.0, cl = 0.0, au = 0.0, al = 0.0;
+  F64 cu = 0.0, cl = 0.0, au = 0.0, al = 0.0;
   long long iu = q, il = q;
   if (has_up) {
     cu = cw[q];
@@ -355,31 +371,31 @@ __global__ void __launch_bounds__(256) k64_tracers(Dims D, Grid<double> G, const
     al = G.area_z[q + D.plane];
     if (positive(cl)) il = q + D.plane;
   }
-  const double V = G.volume[q], rV = rvol[q];
+  const F64 V = G.volume[q], rV = rvol[q];
   for (int jc = 1; jc <= D.ncons; ++jc) {
     if (jc == D.g) continue;
-    const double* r = Ss.rho + (long long)(jc - 1) * D.fstride;
-    double c = r[e.i] * e.v * e.a + r[n.i] * n.v * n.a - r[w.i] * w.v * w.a - r[s.i] * s.v * s.a;
+    const F64* r = Ss.rho + (long long)(jc - 1) * D.fstride;
+    F64 c = r[e.i] * e.v * e.a + r[n.i] * n.v * n.a - r[w.i] * w.v * w.a - r[s.i] * s.v * s.a;
     if (has_up && has_lo && jl != D.nf) c = c + (r[iu] * cu * au - r[il] * cl * al);
     else if (has_lo) c = c - r[il] * cl * al;
     else if (has_up) c = c + r[iu] * cu * au;
-    double f = -div_rn(c, V, rV);
+    F64 f = -div_rn(c, V, rV);
     if (mdt) f = f + mdt[q + (long long)(jc - 1) * D.fstride];
     if (ptr) f = f + ptr[q + (long long)((jc < D.g ? jc : D.g) - 1) * D.fstride];
-    double* t = t_rho + (long long)(jc - 1) * D.fstride;
+    F64* t = t_rho + (long long)(jc - 1) * D.fstride;
     t[q] = (rk_step == 1) ? f : half(t[q]) + half(f);
   }
 }
 
 // what the pressure gradient reads of a cell: theta_v, c_d_p*rho_g/sum(rho) and rho_g/sum(rho) - 1
-__global__ void k64_pgrad_cells(Dims D, Grid<double> G, StateT<double> S, double* th, double* decel, double* cond) {
+__global__ void k64_pgrad_cells(Dims D, Grid<F64> G, StateT<F64> S, F64* th, F64* decel, F64* cond) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
   const long long q = IX(D, ji, jk, jl);
   th[q] = G.theta_v_bg[q] + S.tp[q];
-  double sum = S.rho[q];
+  F64 sum = S.rho[q];
   for (int jc = 1; jc <= D.nc; ++jc) sum = sum + S.rho[q + (long long)jc * D.fstride];
-  const double rg = S.rho[q + (long long)(D.g - 1) * D.fstride], y = __drcp_rn(sum);
+  const F64 rg = S.rho[q + (long long)(D.g - 1) * D.fstride], y = rcp_near(sum);
   decel[q] = div_rn(kC_D_P * rg, sum, y);
   cond[q] = div_rn(rg, sum, y) - 1.0;
 }
@@ -388,18 +404,18 @@ __global__ void k64_pgrad_cells(Dims D, Grid<double> G, StateT<double> S, double
 // calc_p_grad_condensates_v, mo_p_grad.F90:106-120 (identical at both substeps because it always
 // reads state_old).  (With theta and both quotients formed at each of a cell's six faces: 902 us
 // at 192x192x80.)
-__global__ void k64_pgrad(Dims D, Grid<double> G, StateT<double> S, const double* gx, const double* gy, const double* gz,
-                          const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
-                          const double* tpu, const double* tpv, PGrad<double> P, int lfirst) {
+__global__ void k64_pgrad(Dims D, Grid<F64> G, StateT<F64> S, const F64* gx, const F64* gy, const F64* gz,
+                          const F64* th, const F64* decel, const F64* cond, const F64* tvu, const F64* tvv,
+                          const F64* tpu, const F64* tpv, PGradF P, int lfirst) {
   LG_IDX3;
-  auto negsum = [&](double nl, double l) { return D.luse_bg ? -nl - l : -nl; };
+  auto negsum = [&](F64 nl, F64 l) { return D.luse_bg ? -nl - l : -nl; };
   // one face between cells a and b: point q, evaluated at qr
-  auto face = [&](long long q, long long qr, long long a, long long b, const double* g, const double* tv, const double* tp,
-                  const double* eg, double* nl, double* l, double* old) {
+  auto face = [&](long long q, long long qr, long long a, long long b, const F64* g, const F64* tv, const F64* tp,
+                  const F64* eg, F64* nl, F64* l, F64* old) {
     if (!lfirst) old[q] = negsum(nl[q], D.luse_bg ? l[q] : 0.0);
-    const double de = half(decel[a] + decel[b]);
-    const double nlv = de * ((D.theta_order == 2 ? half(th[a] + th[b]) : tv[qr]) * g[qr]);
-    double lv = 0.0;
+    const F64 de = half(decel[a] + decel[b]);
+    const F64 nlv = de * ((D.theta_order == 2 ? half(th[a] + th[b]) : tv[qr]) * g[qr]);
+    F64 lv = 0.0;
     nl[q] = nlv;
     if (D.luse_bg) {
       lv = de * ((D.theta_order == 2 ? half(S.tp[a] + S.tp[b]) : tp[qr]) * eg[qr]);
@@ -433,7 +449,7 @@ __global__ void k64_pgrad(Dims D, Grid<double> G, StateT<double> S, const double
   // w points, levels 2..nl
   if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
     const long long q = IX(D, ji, jk, jl), qa = q - D.plane;
-    const double de = half(decel[qa] + decel[q]);
+    const F64 de = half(decel[qa] + decel[q]);
     P.nl_w[q] = de * (half(th[qa] + th[q]) * gz[q]);
     if (D.luse_bg) P.l_w[q] = de * (half(S.tp[qa] + S.tp[q]) * G.egw[q]);
     P.pgcw[q] = half(cond[qa] + cond[q]) * G.gm[q];  // p_grad_condensates_w
@@ -444,58 +460,58 @@ __global__ void k64_pgrad(Dims D, Grid<double> G, StateT<double> S, const double
 
 void launch64_pgrad_cells(const Dims& D, const Grid<double>& G, const State& S, double* th, double* decel, double* cond,
                           cudaStream_t st) {
-  k64_pgrad_cells<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, G, S, th, decel, cond);
+  k64_pgrad_cells<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(th), f64(decel), f64(cond));
 }
 void launch64_pgrad(const Dims& D, const Grid<double>& G, const State& S, const double* gx, const double* gy, const double* gz,
                     const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
                     const double* tpu, const double* tpv, const PGrad<double>& P, int lfirst, cudaStream_t st) {
-  k64_pgrad<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, S, gx, gy, gz, th, decel, cond, tvu, tvv, tpu,
-                                                                       tpv, P, lfirst);
+  k64_pgrad<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(gx), f64(gy), f64(gz), f64(th), f64(decel), f64(cond), f64(tvu), f64(tvv), f64(tpu),
+                                                                       f64(tpv), PGradF{f64(P.nl_u), f64(P.nl_v), f64(P.nl_w), f64(P.l_u), f64(P.l_v), f64(P.l_w), f64(P.old_u), f64(P.old_v), f64(P.pgcw)}, lfirst);
 }
 void launch64_recip(const Dims& D, const Grid<double>& G, double* rdx, double* rdy, double* rdz, cudaStream_t st) {
-  k64_recip<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, rdx, rdy, rdz);
+  k64_recip<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(rdx), f64(rdy), f64(rdz));
 }
 void launch64_grad_vert(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, double* gz, double* w5,
                         double* w6, cudaStream_t st) {
-  k64_grad_vert<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, R.dz, s, gz, w5, w6);
+  k64_grad_vert<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), R.dz, f64(s), f64(gz), f64(w5), f64(w6));
 }
 void launch64_grad_hor(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
                        const double* w6, double* rx, double* ry, cudaStream_t st) {
-  k64_grad_hor<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, R, s, w5, w6, rx, ry);
+  k64_grad_hor<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), R, f64(s), f64(w5), f64(w6), f64(rx), f64(ry));
 }
 void launch64_grad_faces(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
                          const double* w6, const Faces& F, cudaStream_t st) {
-  k64_grad_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, R, s, w5, w6, F);
+  k64_grad_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), R, f64(s), f64(w5), f64(w6), F);
 }
 void launch64_div(const Dims& D, const Grid<double>& G, const Recip& R, const Faces& F, double* out, cudaStream_t st) {
-  k64_div<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, R.vol, F, out);
+  k64_div<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), R.vol, F, f64(out));
 }
 void launch64_theta_edges(const Dims& D, const double* th, const double* dv, const double* u, const double* v, double* tvu,
                           double* tvv, cudaStream_t st) {
-  k64_theta_edges<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, th, dv, u, v, tvu, tvv);
+  k64_theta_edges<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(th), f64(dv), f64(u), f64(v), f64(tvu), f64(tvv));
 }
 void launch64_gas_faces(const Dims& D, const Grid<double>& G, const State& Ss, const double* u_new, const double* v_new,
                         const double* tvu, const double* tvv, const Faces& M, const Faces& T, cudaStream_t st) {
-  k64_gas_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, G, Ss, u_new, v_new, tvu, tvv, M, T);
+  k64_gas_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(Ss), f64(u_new), f64(v_new), f64(tvu), f64(tvv), M, T);
 }
 void launch64_gas_theta(const Dims& D, const Grid<double>& G, const Recip& R, const State& Ss, const Faces& M, const Faces& T,
                         const double* cpi, const double* cpw, const double* hd, const double* rad, const double* csh,
                         double* t_rho, double* t_rt, const double* mdt, const double* tdh, const double* ptr,
                         const double* pth, cudaStream_t st) {
-  k64_gas_theta<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, Ss, R.vol, M, T, cpi, cpw, hd, rad, csh, t_rho, t_rt, mdt, tdh,
-                                                       ptr, pth);
+  k64_gas_theta<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), f64(Ss), R.vol, M, T, f64(cpi), f64(cpw), f64(hd), f64(rad), f64(csh), f64(t_rho), f64(t_rt), f64(mdt), f64(tdh),
+                                                       f64(ptr), f64(pth));
 }
 void launch64_wind_slopes(const Dims& D, const Grid<double>& G, const double* u, const double* v, double* hx, double* hy,
                           cudaStream_t st) {
-  k64_wind_slopes<<<cell_grid(D.ny + 1, D.nx + 1, D.nl - D.nf), kCellBlock, 0, st>>>(D, G, u, v, hx, hy);
+  k64_wind_slopes<<<cell_grid(D.ny + 1, D.nx + 1, D.nl - D.nf), kCellBlock, 0, st>>>(D, f64(G), f64(u), f64(v), f64(hx), f64(hy));
 }
 void launch64_contra(const Dims& D, const Grid<double>& G, const double* hx, const double* hy, double* cw, cudaStream_t st) {
-  k64_contra<<<march_grid(D), kMarchBlock, 0, st>>>(D, G, hx, hy, cw);
+  k64_contra<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), f64(hx), f64(hy), f64(cw));
 }
 void launch64_tracers(const Dims& D, const Grid<double>& G, const Recip& R, const State& Ss, const double* u_new,
                       const double* v_new, const double* cw, double* t_rho, int rk_step, const double* mdt, const double* ptr,
                       cudaStream_t st) {
-  k64_tracers<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, G, R.vol, Ss, u_new, v_new, cw, t_rho, rk_step, mdt, ptr);
+  k64_tracers<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), R.vol, f64(Ss), f64(u_new), f64(v_new), f64(cw), f64(t_rho), rk_step, f64(mdt), f64(ptr));
 }
 
 }  // namespace lg

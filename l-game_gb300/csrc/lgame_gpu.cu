@@ -94,6 +94,7 @@ struct lgame_gpu {
   // flux or gradient
   double *rdx = nullptr, *rdy = nullptr, *rdz = nullptr;
   Recip recip{};
+  double* fc[8] = {};
   Faces fcm{}, fct{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
@@ -508,13 +509,13 @@ int preload_budget_scratch() {
 // FP64 instantiations of the kernel templates of kernels.cuh (this file is compiled with
 // -fmad=false like the rest of the FP64 step)
 namespace kd {
-const auto k_temperature = lg::k_temperature<double>;
+const auto k_temperature = lg::k_temperature<F64, F64>;
 const auto k_theta = lg::k_theta<double>;
-const auto k_eta_xy = lg::k_eta_xy<double>;
-const auto k_eta_z = lg::k_eta_z<double>;
-const auto k_mass_flux = lg::k_mass_flux<double>;
-const auto k_vort_flux = lg::k_vort_flux<double>;
-const auto k_ke = lg::k_ke<double>;
+const auto k_eta_xy = lg::k_eta_xy<F64, F64>;
+const auto k_eta_z = lg::k_eta_z<F64, F64>;
+const auto k_mass_flux = lg::k_mass_flux<F64, F64>;
+const auto k_vort_flux = lg::k_vort_flux<F64, F64>;
+const auto k_ke = lg::k_ke<F64, F64>;
 const auto k_tend_wind = lg::k_tend_wind<double>;
 const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
@@ -588,13 +589,13 @@ int gradient(lgame_gpu* c, const double* f, double* gx, double* gy, double* gz) 
 int advection(lgame_gpu* c, const State& S) {
   const Dims& D = c->D;
   if (!(!D.llinear || D.lcorio)) return LGAME_OK;
-  LAUNCH(kd::k_eta_xy, grd(D, D.ny + 1, D.nx + 1, D.NL), D, c->G, S, c->ex, c->ey);
-  LAUNCH(kd::k_eta_z, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, S, c->ez);
-  LAUNCH(kd::k_mass_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, S, c->uph, c->vph, c->wph);
-  LAUNCH(kd::k_vort_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, c->G, S, c->ex, c->ey, c->ez, c->uph, c->vph, c->wph,
-         c->pvt_x, c->pvt_y, c->pvt_z);
+  LAUNCH(kd::k_eta_xy, grd(D, D.ny + 1, D.nx + 1, D.NL), D, f64(c->G), f64(S), f64(c->ex), f64(c->ey));
+  LAUNCH(kd::k_eta_z, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->ez));
+  LAUNCH(kd::k_mass_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->uph), f64(c->vph), f64(c->wph));
+  LAUNCH(kd::k_vort_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->ex), f64(c->ey),
+         f64(c->ez), f64(c->uph), f64(c->vph), f64(c->wph), f64(c->pvt_x), f64(c->pvt_y), f64(c->pvt_z));
   if (!D.llinear) {
-    LAUNCH(kd::k_ke, grd(D, D.ny, D.nx, D.nl), D, c->G, S, c->vsq);
+    LAUNCH(kd::k_ke, grd(D, D.ny, D.nx, D.nl), D, f64(c->G), f64(S), f64(c->vsq));
     // (the vorticity flux above was the last to read ex and ey, which carry the column products here)
     const int rc = gradient(c, c->vsq, c->vsg_x, c->vsg_y, c->vsg_z);
     if (rc != LGAME_OK) return rc;
@@ -657,7 +658,7 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
   const State& So = c->st[so];
   const State& Sn = c->st[sn];
   const Grid<double>& G = c->G;
-  LAUNCH(kd::k_temperature, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature);
+  LAUNCH(kd::k_temperature, grd(D, D.ny, D.nx, D.nl), D, f64(G), f64(So), f64(c->temperature));
   // update_sfc_turb_quantities (mo_manage_pchevi.F90:51-53)
   if (c->sfc_turb) LAUNCH(kd::k_sfc_turb, grd(D, D.ny, D.nx, 1), D, G, So, c->vsq, c->sbuf, c->spar);
   PGrad<double> P{c->pg_nl_u, c->pg_nl_v, c->pg_nl_w, c->pg_l_u, c->pg_l_v, c->pg_l_w, c->pg_old_u, c->pg_old_v, c->pgcw};
@@ -678,8 +679,8 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
         if (rc != LGAME_OK) return rc;
       }
       // (theta_v and the two quotients of every cell in theta and fcm)
-      LAUNCH_FN("k_pgrad_cells", launch64_pgrad_cells(D, G, So, c->theta, c->fcm.px, c->fcm.py, c->stream));
-      LAUNCH_FN("k_pgrad", launch64_pgrad(D, G, So, c->gx, c->gy, c->gz, c->theta, c->fcm.px, c->fcm.py, c->tvu, c->tvv, c->tpu,
+      LAUNCH_FN("k_pgrad_cells", launch64_pgrad_cells(D, G, So, c->theta, c->fc[0], c->fc[1], c->stream));
+      LAUNCH_FN("k_pgrad", launch64_pgrad(D, G, So, c->gx, c->gy, c->gz, c->theta, c->fc[0], c->fc[1], c->tvu, c->tvv, c->tpu,
                                           c->tpv, P, step == 0 ? 1 : 0, c->stream));
       // into the edge arrays of theta', which nothing reads after k_pgrad, and cpw
       if (D.ncons > 1)
@@ -713,8 +714,8 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
     const double* ptr = c->phase ? c->ptr : nullptr;
     const double* pth = c->phase ? c->pth : nullptr;
     if (D.ncons > 1) {  // the slope terms of the new wind in fct, its vertical correction in divf
-      LAUNCH_FN("k_wind_slopes", launch64_wind_slopes(D, G, Sn.u, Sn.v, c->fct.hx, c->fct.hy, c->stream));
-      LAUNCH_FN("k_contra", launch64_contra(D, G, c->fct.hx, c->fct.hy, c->divf, c->stream));
+      LAUNCH_FN("k_wind_slopes", launch64_wind_slopes(D, G, Sn.u, Sn.v, c->fc[6], c->fc[7], c->stream));
+      LAUNCH_FN("k_contra", launch64_contra(D, G, c->fc[6], c->fc[7], c->divf, c->stream));
       LAUNCH_FN("k_tracers", launch64_tracers(D, G, c->recip, Ss, Sn.u, Sn.v, c->divf, T.rho, rk, mdt, ptr, c->stream));
     }
     // theta_v_adv_3rd_order of the state used here: in the first substep that is state_old,
@@ -738,7 +739,7 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
       LAUNCH_FN("k_column_ver", lg::launch_column_ver(D, G, c->colg, So, Sn, T, rk, c->stream));
       if (D.ncons > 1)
         LAUNCH_FN("k_column_tracers", lg::launch_column_tracers(D, G, So, Sn, T.rho, c->temperature, c->rvol, c->itwdtv,
-                                                                c->tpu, c->tpv, c->cpw, c->csh, rk, c->stream));
+                                                                c->tpu, c->tpv, c->cpw, c->csh, c->theta, rk, c->stream));
     }
   }
   return LGAME_OK;
@@ -952,12 +953,14 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
   for (double** p : scratch) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
   if (cfg->precision == LGAME_PRECISION_FP64) {
     double** colg[] = {&c->rvol, &c->itwdtv, &c->zs, &c->zs_c2, &c->zs_c1h, &c->hdeb, &c->raz, &c->rdx, &c->rdy, &c->rdz,
-                       &c->fcm.px, &c->fcm.py, &c->fcm.hx, &c->fcm.hy, &c->fct.px, &c->fct.py, &c->fct.hx, &c->fct.hy};
+                       &c->fc[0], &c->fc[1], &c->fc[2], &c->fc[3], &c->fc[4], &c->fc[5], &c->fc[6], &c->fc[7]};
     for (double** p : colg) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
     if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
     c->colg = ColumnGrid{c->rvol, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz,
                          1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
-    c->recip = Recip{c->rvol, c->rdx, c->rdy, c->rdz};
+    c->fcm = Faces{f64(c->fc[0]), f64(c->fc[1]), f64(c->fc[2]), f64(c->fc[3])};
+    c->fct = Faces{f64(c->fc[4]), f64(c->fc[5]), f64(c->fc[6]), f64(c->fc[7])};
+    c->recip = Recip{f64(c->rvol), f64(c->rdx), f64(c->rdy), f64(c->rdz)};
     if (column_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the column solvers refused"));
   }
   // diffusion closure: the carried diagnostics always, the work arrays when a part is on
