@@ -142,7 +142,27 @@ struct Faces {
   F64 *px, *py, *hx, *hy;
 };
 
+// grid-only factors of the vorticity: reciprocals of the dual areas (x and y to level nl+1); in the
+// terrain-following layers, for each side of a dual point, (r_e + z_dual)/(r_e + z_side) times its
+// length, with the side's sign; reciprocals of z(l) - z(l+1) at v and u points
+struct RotGrid {
+  const F64 *radx, *rady, *radz, *m0, *m1, *m2, *m3, *ryv, *ryu;
+};
+
 // the explicit kernels (kernels_fp64.cu)
+void launch64_rot_grid(const Dims& D, const Grid<double>& G, double* const* a, cudaStream_t st);
+void launch64_zeta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* zz, cudaStream_t st);
+void launch64_eta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* ez, cudaStream_t st);
+void launch64_covariant(const Dims& D, const Grid<double>& G, const State& S, double* cx, double* cy, cudaStream_t st);
+void launch64_eta_xy(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, const double* cx, const double* cy,
+                     double* ex, double* ey, cudaStream_t st);
+void launch64_mass_flux(const Dims& D, const Grid<double>& G, const State& S, double* uph, double* vph, double* q5, double* q6,
+                        cudaStream_t st);
+void launch64_vort_flux(const Dims& D, const Grid<double>& G, const double* ex, const double* ey, const double* ez,
+                        const double* uph, const double* vph, const double* q5, const double* q6, double* px, double* py,
+                        double* pz, cudaStream_t st);
+void launch64_tend_wind(const Dims& D, const State& So, const State& Sn, const Tend<double>& Tn, const Carried<double>& C,
+                        int rk_step, cudaStream_t st);
 void launch64_recip(const Dims& D, const Grid<double>& G, double* rdx, double* rdy, double* rdz, cudaStream_t st);
 void launch64_grad_vert(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, double* gz, double* w5,
                         double* w6, cudaStream_t st);

@@ -387,43 +387,6 @@ __global__ void k_div_h(Dims D, Grid<T> G, const T* vx, const T* vy, T* out) {
   out[IX(D, ji, jk, jl)] = div_h_at<T>(D, G, fx, fy, ji, jk, jl);
 }
 
-// calc_pot_vort, mo_vorticities.F90:189-421 with rel_vort :19-187 inlined:
-// eta_x (ny+1,nx,nl+1) and eta_y (ny,nx+1,nl+1)
-template <class T, class V = double>
-__global__ void k_eta_xy(Dims D, Grid<T> G, StateT<V> S, T* ex, T* ey) {
-  LG_IDX3;
-  if (jl > D.NL) return;
-  if (ji <= D.ny + 1 && jk <= D.nx) ex[IX(D, ji, jk, jl)] = eta_x_at<T>(D, G, S, ji, jk, jl);
-  if (ji <= D.ny && jk <= D.nx + 1) ey[IX(D, ji, jk, jl)] = eta_y_at<T>(D, G, S, ji, jk, jl);
-}
-
-// eta_z (ny+1,nx+1,nl)
-template <class T, class V = double>
-__global__ void k_eta_z(Dims D, Grid<T> G, StateT<V> S, T* ez) {
-  LG_IDX3;
-  if (ji > D.ny + 1 || jk > D.nx + 1) return;
-  ez[IX(D, ji, jk, jl)] = eta_z_at<T>(D, G, S, ji, jk, jl);
-}
-
-// mass flux densities, mo_vector_tend_expl.F90:64-66 (scalar_times_vector_h/_v)
-template <class T, class V = double>
-__global__ void k_mass_flux(Dims D, Grid<T> G, StateT<V> S, T* uph, T* vph, T* wph) {
-  LG_IDX3;
-  const V* rg = S.rho + (long long)(D.g - 1) * D.fstride;
-  if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
-    T f;
-    if (stv_h_x<T>(D, rg, S.u, ji, jk, jl, &f)) uph[IX(D, ji, jk, jl)] = f;
-  }
-  if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
-    T f;
-    if (stv_h_y<T>(D, rg, S.v, ji, jk, jl, &f)) vph[IX(D, ji, jk, jl)] = f;
-  }
-  if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    wph[q] = half_of(T(rg[IX(D, ji, jk, jl - 1)]) + T(rg[q])) * T(S.w[q]);
-  }
-}
-
 // calc_vorticity_flux_term, mo_vorticity_flux.F90:16-171
 template <class T, class V = double>
 __device__ __forceinline__ void vort_flux_body(const Dims& D, const Grid<T>& G, const StateT<V>& S, const T* ex,
@@ -479,70 +442,12 @@ __device__ __forceinline__ void vort_flux_body(const Dims& D, const Grid<T>& G, 
   }
 }
 
-template <class T, class V = double>
-__global__ void k_vort_flux(Dims D, Grid<T> G, StateT<V> S, const T* ex, const T* ey, const T* ez, const T* uph,
-                            const T* vph, const T* wph, T* px, T* py, T* pz) {
-  vort_flux_body<T, V>(D, G, S, ex, ey, ez, uph, vph, wph, px, py, pz);
-}
-
 // inner_product of the wind with itself, mo_inner_product.F90:16-50
 template <class T, class V = double>
 __global__ void k_ke(Dims D, Grid<T> G, StateT<V> S, T* out) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
   out[IX(D, ji, jk, jl)] = inner_product_at<T>(D, G, S.u, S.v, S.w, ji, jk, jl);
-}
-
-// combination of the explicit wind tendencies, mo_vector_tend_expl.F90:258-310, and the
-// forward step of the horizontal wind, mo_manage_pchevi.F90:86-89 (in FP64)
-template <class T>
-// mu, mv (may be null): FP32 mirrors of the new u, v, written beside the FP64 values
-__global__ void k_tend_wind(Dims D, State So, State Sn, Tend<T> Tn, Carried<T> C, int rk_step, float* mu, float* mv) {
-  LG_IDX3;
-  const T new_weight = (rk_step == 2) ? T(0.5) : T(1);
-  const T old_weight = T(1) - new_weight;
-  // the pressure-gradient combinations are formed in FP64 (the products are FP64; without a
-  // background state they are O(g) and cancel gravity), in the reference's operation order
-  const double chw_d = 0.5 + kIMPL_THERMO_WEIGHT, ohw_d = 1.0 - (0.5 + kIMPL_THERMO_WEIGHT);
-  const double cvw_d = 1.0 - kIMPL_THERMO_WEIGHT, no_bg_d = D.luse_bg ? 0.0 : 1.0;
-  // FP32 tendencies with a background state: the sum nl + l, where the two products cancel,
-  // is the only FP64 operation; the previous substep's value (already a net force) and that
-  // sum are rounded to FP32 and combined there, as the FP32 tendency is rounded anyway
-  constexpr bool f32 = sizeof(T) == 4;
-  const bool pg32 = f32 && D.luse_bg;
-  auto pg_h = [&](const double* old, const double* nl, const double* l, long long q) -> T {
-    if (pg32) return T(ohw_d) * cvt<T>(old[q]) - T(chw_d) * cvt<T>(nl[q] + l[q]);
-    return cvt<T>(ohw_d * old[q] - chw_d * (nl[q] + l[q]));
-  };
-  if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
-    const long long q = IX(D, ji, jk, jl);
-    T f = pg_h(C.old_u, C.nl_u, C.l_u, q) - half_of(C.vsg_x[q]) + C.pvt_x[q];
-    if (C.mdt_x) f = f + C.mdt_x[q];
-    const T t = old_weight * Tn.u[q] + new_weight * f;
-    Tn.u[q] = t;
-    const double un = So.u[q] + D.dtime * cvt<double>(t);
-    Sn.u[q] = un;
-    if (mu) mu[q] = narrow(un);
-  }
-  if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    T f = pg_h(C.old_v, C.nl_v, C.l_v, q) - half_of(C.vsg_y[q]) + C.pvt_y[q];
-    if (C.mdt_y) f = f + C.mdt_y[q];
-    const T t = old_weight * Tn.v[q] + new_weight * f;
-    Tn.v[q] = t;
-    const double vn = So.v[q] + D.dtime * cvt<double>(t);
-    Sn.v[q] = vn;
-    if (mv) mv[q] = narrow(vn);
-  }
-  if (jl <= D.NL && ji <= D.ny && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    T pg;
-    if (pg32) pg = -(T(cvw_d) * cvt<T>(C.nl_w[q] + C.l_w[q]));
-    else pg = cvt<T>(-(cvw_d * (C.nl_w[q] + C.l_w[q])) - no_bg_d * (1.0 - cvw_d) * C.l_w[q]);
-    T f = pg - half_of(C.vsg_z[q]) + C.pvt_z[q] + C.pgcw[q];
-    if (C.mdt_z) f = f + C.mdt_z[q];
-    Tn.w[q] = old_weight * Tn.w[q] + new_weight * f;
-  }
 }
 
 // ---- FP64-only kernels (column_fp64.cu; the others: fp64.cuh) --------------------------

@@ -13,6 +13,23 @@ namespace lg {
 
 namespace {
 
+struct CarriedF {
+  const F64 *nl_u, *nl_v, *nl_w, *l_u, *l_v, *l_w, *old_u, *old_v, *pgcw, *vsg_x, *vsg_y, *vsg_z, *pvt_x, *pvt_y, *pvt_z,
+      *mdt_x, *mdt_y, *mdt_z;
+};
+// the four sides of a dual point: v, u, v, u points (mo_vorticities.F90:423-538); not in: a non-periodic
+// boundary point, where the vorticity is 0
+struct RotSides { long long v0, u1, v2, u3; bool in; };
+__device__ __forceinline__ RotSides rot_sides(const Dims& D, int ji, int jk, int jl) {
+  const bool edge = ji == 1 || jk == 1 || ji == D.ny + 1 || jk == D.nx + 1;
+  RotSides s;
+  s.in = !edge || D.periodic;
+  s.v0 = IX(D, ji, (jk == D.nx + 1) ? 1 : jk, jl);
+  s.u1 = IX(D, (ji == 1) ? D.ny : ji - 1, jk, jl);
+  s.v2 = IX(D, ji, (jk == 1) ? D.nx : jk - 1, jl);
+  s.u3 = IX(D, (ji == D.ny + 1) ? 1 : ji, jk, jl);
+  return s;
+}
 struct PGradF { F64 *nl_u, *nl_v, *nl_w, *l_u, *l_v, *l_w, *old_u, *old_v, *pgcw; };
 
 // marching threads: a chunk of the column's levels each (blockIdx.z), of eight levels (the layer above a
@@ -456,7 +473,256 @@ __global__ void k64_pgrad(Dims D, Grid<F64> G, StateT<F64> S, const F64* gx, con
   }
 }
 
+// ---- potential vorticity and its flux, mo_vorticities.F90, mo_vorticity_flux.F90 -------------------
+// grid-only factors (RotGrid)
+__global__ void k64_rot_grid(Dims D, Grid<F64> G, F64* radx, F64* rady, F64* radz, F64* m0, F64* m1, F64* m2, F64* m3,
+                             F64* ryv, F64* ryu) {
+  LG_IDX3;
+  const long long q = IX(D, ji, jk, jl);
+  const F64 one = 1.0;
+  if (ji <= D.ny + 1 && jk <= D.nx) radx[q] = one / G.area_dual_x[q];
+  if (ji <= D.ny && jk <= D.nx + 1) rady[q] = one / G.area_dual_y[q];
+  if (jl > D.nl || ji > D.ny + 1 || jk > D.nx + 1) return;
+  radz[q] = one / G.area_dual_z[q];
+  if (jl < D.nl) {
+    if (jk <= D.nx) ryv[q] = one / (G.z_v[q] - G.z_v[q + D.plane]);
+    if (ji <= D.ny) ryu[q] = one / (G.z_u[q] - G.z_u[q + D.plane]);
+  }
+  if (jl > D.nf) {
+    const RotSides n = rot_sides(D, ji, jk, jl);
+    if (n.in) {
+      const F64 up = F64(kR_E) + G.z_area_dual_z[q];
+      m0[q] = up / (F64(kR_E) + G.z_v[n.v0]) * G.dy[n.v0];
+      m1[q] = -(up / (F64(kR_E) + G.z_u[n.u1])) * G.dx[n.u1];
+      m2[q] = -(up / (F64(kR_E) + G.z_v[n.v2])) * G.dy[n.v2];
+      m3[q] = up / (F64(kR_E) + G.z_u[n.u3]) * G.dx[n.u3];
+    }
+  }
+}
+// rel_vort_z_local, mo_vorticities.F90:423-538, over the dual area: the wind of each of the four sides
+// extrapolated to the dual point's height
+__device__ __forceinline__ F64 zeta_z64(const Dims& D, const Grid<F64>& G, const RotGrid& X, const F64* u, const F64* v, int ji,
+                                        int jk, int jl) {
+  const long long q = IX(D, ji, jk, jl), pl = D.plane;
+  const RotSides n = rot_sides(D, ji, jk, jl);
+  F64 r = 0.0;
+  if (!n.in) return r;
+  if (jl <= D.nf) {
+    r = G.dy[n.v0] * v[n.v0] - G.dx[n.u1] * u[n.u1] - G.dy[n.v2] * v[n.v2] + G.dx[n.u3] * u[n.u3];
+  } else {
+    const F64 zd = G.z_area_dual_z[q];
+    auto side = [&](const F64* x, const F64* z, const F64* ry, const F64* m, long long i) {
+      const F64 z0 = z[i], x0 = x[i], dz = zd - z0;
+      const bool above = (positive(dz) || jl == D.nl) && jl != 1;
+      const long long o = above ? i - pl : i + pl;
+      const F64 y = above ? -ry[o] : ry[i];
+      return m[q] * (x0 + dz * div_rn(x0 - x[o], z0 - z[o], y));
+    };
+    r = side(v, G.z_v, X.ryv, X.m0, n.v0) + side(u, G.z_u, X.ryu, X.m1, n.u1) + side(v, G.z_v, X.ryv, X.m2, n.v2)
+      + side(u, G.z_u, X.ryu, X.m3, n.u3);
+  }
+  return div_rn(r, G.area_dual_z[q], X.radz[q]);
+}
+__global__ void k64_zeta_z(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, F64* zz) {
+  LG_IDX3;
+  if (ji <= D.ny + 1 && jk <= D.nx + 1) zz[IX(D, ji, jk, jl)] = zeta_z64(D, G, X, S.u, S.v, ji, jk, jl);
+}
+// eta_z at (ny+1, nx+1, nl)
+__global__ void k64_eta_z(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, F64* ez) {
+  LG_IDX3;
+  if (ji > D.ny + 1 || jk > D.nx + 1) return;
+  const int i = (D.periodic && ji == D.ny + 1) ? 1 : ji, k = (D.periodic && jk == D.nx + 1) ? 1 : jk;
+  F64 e = 0.0;
+  if (!D.llinear) e = zeta_z64(D, G, X, S.u, S.v, i, k, jl);
+  if (D.lcorio) e = e + G.fvec_z[IX(D, i, k, 1)];
+  if (D.periodic || (i >= 2 && i <= D.ny && k >= 2 && k <= D.nx)) {
+    const F64* rg = S.rho + (long long)(D.g - 1) * D.fstride;
+    const int km = (k == 1) ? D.nx : k - 1, im = (i == 1) ? D.ny : i - 1;
+    e = e / quarter_of(rg[IX(D, i, km, jl)] + rg[IX(D, i, k, jl)] + rg[IX(D, im, k, jl)] + rg[IX(D, im, km, jl)]);
+  }
+  ez[IX(D, ji, jk, jl)] = e;
+}
+// dx times the covariant wind (horizontal_covariant_x/y, mo_averaging.F90:138-176) at u and v points,
+// which the two interfaces of the layer share
+__global__ void k64_covariant(Dims D, Grid<F64> G, StateT<F64> S, F64* cx, F64* cy) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl);
+  const F64* w = S.w;
+  const bool lower = jl < D.nl || D.freeslip;
+  auto remap = [&](long long a, long long b) {
+    F64 m = G.ipw[4][a] * w[a] + G.ipw[4][b] * w[b];
+    if (lower) m = m + G.ipw[5][a] * w[a + D.plane] + G.ipw[5][b] * w[b + D.plane];
+    return half(m);
+  };
+  F64 x = S.u[q], y = S.v[q];
+  if (jl > D.nf) {
+    if (jk >= 2 || D.periodic) x = x + G.slope_x[q] * remap(jk >= 2 ? q - D.P : IX(D, ji, D.nx, jl), q);
+    if (ji >= 2 || D.periodic) y = y + G.slope_y[q] * remap(ji >= 2 ? q - 1 : IX(D, D.ny, jk, jl), q);
+  }
+  cx[q] = G.dx[q] * x;
+  cy[q] = G.dy[q] * y;
+}
+// eta_x (ny+1, nx, nl+1) and eta_y (ny, nx+1, nl+1); level 1 takes the vorticity of level 2, and the
+// surface level the general form
+__global__ void k64_eta_xy(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, const F64* cx, const F64* cy, F64* ex, F64* ey) {
+  LG_IDX3;
+  const int lev = max(jl, 2);
+  const F64* rg = S.rho + (long long)(D.g - 1) * D.fstride;
+  if (ji <= D.ny + 1 && jk <= D.nx) {
+    const int i = (D.periodic && ji == D.ny + 1) ? 1 : ji;
+    const bool inner = i >= 2 && i <= D.ny;
+    F64 e = 0.0;
+    if (jl == D.NL) {
+      e = eta_x_at<F64>(D, G, S, i, jk, jl);
+    } else {
+      const long long b = IX(D, inner ? i : 1, jk, lev), a = IX(D, inner ? i - 1 : D.ny, jk, lev), q = IX(D, i, jk, lev);
+      if (!D.llinear && (inner || D.periodic))
+        e = div_rn(G.dz[a] * S.w[a] - cy[b - D.plane] - G.dz[b] * S.w[b] + cy[b], G.area_dual_x[q], X.radx[q]);
+      if (D.lcorio) e = e + G.fvec_x[IX(D, i, jk, 1)];
+      if (inner || D.periodic) e = e / rho_avg_h<F64>(D, G, rg, inner ? i - 1 : D.ny, jk, inner ? i : 1, jk, jl);
+    }
+    ex[IX(D, ji, jk, jl)] = e;
+  }
+  if (ji <= D.ny && jk <= D.nx + 1) {
+    const int k = (D.periodic && jk == D.nx + 1) ? 1 : jk;
+    const bool inner = k >= 2 && k <= D.nx;
+    F64 e = 0.0;
+    if (jl == D.NL) {
+      e = eta_y_at<F64>(D, G, S, ji, k, jl);
+    } else {
+      const long long b = IX(D, ji, inner ? k : 1, lev), a = IX(D, ji, inner ? k - 1 : D.nx, lev), q = IX(D, ji, k, lev);
+      if (!D.llinear && (inner || D.periodic))
+        e = div_rn(-(G.dz[b] * S.w[b]) - cx[b] + G.dz[a] * S.w[a] + cx[b - D.plane], G.area_dual_y[q], X.rady[q]);
+      if (D.lcorio) e = e + G.fvec_y[IX(D, ji, k, 1)];
+      if (inner || D.periodic) e = e / rho_avg_h<F64>(D, G, rg, ji, inner ? k - 1 : D.nx, ji, inner ? k : 1, jl);
+    }
+    ey[IX(D, ji, jk, jl)] = e;
+  }
+}
+// mass flux densities, mo_vector_tend_expl.F90:64-80: at u and v points, and of the vertical one its
+// two products with half the inner-product weights of a layer, which the layer's four faces share:
+// q5 = 0.5*W5*(rho*w)(l), q6 = 0.5*W6*(rho*w)(l+1) (free-slip value at the surface, 0 at the top)
+__global__ void k64_mass_flux(Dims D, Grid<F64> G, StateT<F64> S, F64* uph, F64* vph, F64* q5, F64* q6) {
+  LG_IDX3;
+  const F64* rg = S.rho + (long long)(D.g - 1) * D.fstride;
+  const long long q = IX(D, ji, jk, jl);
+  F64 f;
+  if (ji <= D.ny && jk <= D.nx + 1 && stv_h_x<F64>(D, rg, S.u, ji, jk, jl, &f)) uph[q] = f;
+  if (ji <= D.ny + 1 && jk <= D.nx && stv_h_y<F64>(D, rg, S.v, ji, jk, jl, &f)) vph[q] = f;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long b = q + D.plane;
+  F64 up = 0.0, lo = 0.0;
+  if (jl >= 2) up = half(rg[q - D.plane] + rg[q]) * S.w[q];
+  if (jl < D.nl) {
+    lo = half(rg[q] + rg[b]) * S.w[b];
+  } else if (D.freeslip) {
+    const long long a = q - D.plane;
+    lo = (rg[q] + (rg[a] - rg[q]) / (G.z_scalar[a] - G.z_scalar[q]) * (G.z_w[b] - G.z_scalar[q])) * S.w[b];
+  }
+  q5[q] = half(G.ipw[4][q]) * up;
+  q6[q] = half(G.ipw[5][q]) * lo;
+}
+// calc_vorticity_flux_term, mo_vorticity_flux.F90:16-171
+__global__ void k64_vort_flux(Dims D, Grid<F64> G, const F64* ex, const F64* ey, const F64* ez, const F64* uph, const F64* vph,
+                              const F64* q5, const F64* q6, F64* px, F64* py, F64* pz) {
+  LG_IDX3;
+  const long long q = IX(D, ji, jk, jl), pl = D.plane;
+  if (ji <= D.ny && jk <= D.nx + 1) {
+    const bool inner = jk >= 2 && jk <= D.nx;
+    if (inner || D.periodic) {
+      const int kk = inner ? jk : 1, km = inner ? jk - 1 : D.nx;
+      const long long a = IX(D, ji, km, jl), b = IX(D, ji, kk, jl);
+      const F64 e0 = ey[b], e1 = ey[b + pl];
+      px[q] = trsk_u<F64>(D, G, vph, uph, ez, ji, km, kk, kk + 1, jl) - q5[a] * e0 - q6[a] * e1 - q5[b] * e0 - q6[b] * e1;
+    }
+  }
+  if (ji <= D.ny + 1 && jk <= D.nx) {
+    const bool inner = ji >= 2 && ji <= D.ny;
+    if (inner || D.periodic) {
+      const int ii = inner ? ji : 1, im = inner ? ji - 1 : D.ny;
+      const long long a = IX(D, im, jk, jl), b = IX(D, ii, jk, jl);
+      const F64 e0 = ex[b], e1 = ex[b + pl];
+      py[q] = trsk_v<F64>(D, G, uph, ez, im, ii, jk, jl) + q5[a] * e0 + q6[a] * e1 + q5[b] * e0 + q6[b] * e1;
+    }
+  }
+  if (jl >= 2 && ji <= D.ny && jk <= D.nx) {
+    const long long a = q - pl, e = q + D.P, s = q + 1;
+    pz[q] = half(G.ipw[0][a] * uph[e - pl] * ey[e] - G.ipw[1][a] * vph[a] * ex[q] + G.ipw[2][a] * uph[a] * ey[q]
+                 - G.ipw[3][a] * vph[s - pl] * ex[s] + G.ipw[0][q] * uph[e] * ey[e] - G.ipw[1][q] * vph[q] * ex[q]
+                 + G.ipw[2][q] * uph[q] * ey[q] - G.ipw[3][q] * vph[s] * ex[s]);
+  }
+}
+
+// combination of the explicit wind tendencies, mo_vector_tend_expl.F90:258-310, and the forward step
+// of the horizontal wind, mo_manage_pchevi.F90:86-89; at the first substep the old tendency has
+// weight 0 and is not read
+__global__ void k64_tend_wind(Dims D, StateT<F64> So, StateT<F64> Sn, Tend<F64> Tn, CarriedF C, int rk_step) {
+  LG_IDX3;
+  const F64 chw = 0.5 + kIMPL_THERMO_WEIGHT, ohw = 1.0 - (0.5 + kIMPL_THERMO_WEIGHT), cvw = 1.0 - kIMPL_THERMO_WEIGHT;
+  const long long q = IX(D, ji, jk, jl);
+  auto weigh = [&](F64 f, F64* t) {
+    if (rk_step == 2) f = half(*t) + half(f);
+    *t = f;
+    return f;
+  };
+  if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
+    F64 f = ohw * C.old_u[q] - chw * (C.nl_u[q] + C.l_u[q]) - half(C.vsg_x[q]) + C.pvt_x[q];
+    if (C.mdt_x) f = f + C.mdt_x[q];
+    Sn.u[q] = So.u[q] + F64(D.dtime) * weigh(f, Tn.u + q);
+  }
+  if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
+    F64 f = ohw * C.old_v[q] - chw * (C.nl_v[q] + C.l_v[q]) - half(C.vsg_y[q]) + C.pvt_y[q];
+    if (C.mdt_y) f = f + C.mdt_y[q];
+    Sn.v[q] = So.v[q] + F64(D.dtime) * weigh(f, Tn.v + q);
+  }
+  if (ji <= D.ny && jk <= D.nx) {
+    const F64 l = C.l_w[q];
+    F64 f = -(cvw * (C.nl_w[q] + l));
+    if (!D.luse_bg) f = f - (1.0 - (1.0 - kIMPL_THERMO_WEIGHT)) * l;
+    f = f - half(C.vsg_z[q]) + C.pvt_z[q] + C.pgcw[q];
+    if (C.mdt_z) f = f + C.mdt_z[q];
+    weigh(f, Tn.w + q);
+  }
+}
+
 }  // namespace
+
+void launch64_rot_grid(const Dims& D, const Grid<double>& G, double* const* a, cudaStream_t st) {
+  k64_rot_grid<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), f64(a[0]), f64(a[1]), f64(a[2]), f64(a[3]),
+                                                                           f64(a[4]), f64(a[5]), f64(a[6]), f64(a[7]), f64(a[8]));
+}
+void launch64_zeta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* zz, cudaStream_t st) {
+  k64_zeta_z<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), X, f64(S), f64(zz));
+}
+void launch64_eta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* ez, cudaStream_t st) {
+  k64_eta_z<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), X, f64(S), f64(ez));
+}
+void launch64_covariant(const Dims& D, const Grid<double>& G, const State& S, double* cx, double* cy, cudaStream_t st) {
+  k64_covariant<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(cx), f64(cy));
+}
+void launch64_eta_xy(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, const double* cx, const double* cy,
+                     double* ex, double* ey, cudaStream_t st) {
+  k64_eta_xy<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), X, f64(S), f64(cx), f64(cy), f64(ex), f64(ey));
+}
+void launch64_mass_flux(const Dims& D, const Grid<double>& G, const State& S, double* uph, double* vph, double* q5, double* q6,
+                        cudaStream_t st) {
+  k64_mass_flux<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(uph), f64(vph), f64(q5), f64(q6));
+}
+void launch64_vort_flux(const Dims& D, const Grid<double>& G, const double* ex, const double* ey, const double* ez,
+                        const double* uph, const double* vph, const double* q5, const double* q6, double* px, double* py,
+                        double* pz, cudaStream_t st) {
+  k64_vort_flux<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(ex), f64(ey), f64(ez), f64(uph), f64(vph),
+                                                                           f64(q5), f64(q6), f64(px), f64(py), f64(pz));
+}
+void launch64_tend_wind(const Dims& D, const State& So, const State& Sn, const Tend<double>& Tn, const Carried<double>& C,
+                        int rk_step, cudaStream_t st) {
+  const Tend<F64> T{f64(Tn.rho), f64(Tn.rt), f64(Tn.u), f64(Tn.v), f64(Tn.w)};
+  const CarriedF K{f64(C.nl_u), f64(C.nl_v), f64(C.nl_w), f64(C.l_u), f64(C.l_v), f64(C.l_w), f64(C.old_u), f64(C.old_v),
+                   f64(C.pgcw), f64(C.vsg_x), f64(C.vsg_y), f64(C.vsg_z), f64(C.pvt_x), f64(C.pvt_y), f64(C.pvt_z),
+                   f64(C.mdt_x), f64(C.mdt_y), f64(C.mdt_z)};
+  k64_tend_wind<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(So), f64(Sn), T, K, rk_step);
+}
 
 void launch64_pgrad_cells(const Dims& D, const Grid<double>& G, const State& S, double* th, double* decel, double* cond,
                           cudaStream_t st) {

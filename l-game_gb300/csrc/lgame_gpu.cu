@@ -94,6 +94,8 @@ struct lgame_gpu {
   // flux or gradient
   double *rdx = nullptr, *rdy = nullptr, *rdz = nullptr;
   Recip recip{};
+  double* rotg[9] = {};  // the arrays of RotGrid
+  RotGrid rot{};
   double* fc[8] = {};
   Faces fcm{}, fct{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
@@ -511,16 +513,10 @@ int preload_budget_scratch() {
 namespace kd {
 const auto k_temperature = lg::k_temperature<F64, F64>;
 const auto k_theta = lg::k_theta<double>;
-const auto k_eta_xy = lg::k_eta_xy<F64, F64>;
-const auto k_eta_z = lg::k_eta_z<F64, F64>;
-const auto k_mass_flux = lg::k_mass_flux<F64, F64>;
-const auto k_vort_flux = lg::k_vort_flux<F64, F64>;
 const auto k_ke = lg::k_ke<F64, F64>;
-const auto k_tend_wind = lg::k_tend_wind<double>;
 const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
 const auto k_diff_visc = lg::k_diff_visc<double, double>;
-const auto k_diff_zeta = lg::k_diff_zeta<double, double>;
 const auto k_diff_vz = lg::k_diff_vz<double, double>;
 const auto k_mom_diff_h = lg::k_mom_diff_h<double, double>;
 const auto k_mom_diff_v = lg::k_mom_diff_v<double, double>;
@@ -589,11 +585,13 @@ int gradient(lgame_gpu* c, const double* f, double* gx, double* gy, double* gz) 
 int advection(lgame_gpu* c, const State& S) {
   const Dims& D = c->D;
   if (!(!D.llinear || D.lcorio)) return LGAME_OK;
-  LAUNCH(kd::k_eta_xy, grd(D, D.ny + 1, D.nx + 1, D.NL), D, f64(c->G), f64(S), f64(c->ex), f64(c->ey));
-  LAUNCH(kd::k_eta_z, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->ez));
-  LAUNCH(kd::k_mass_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->uph), f64(c->vph), f64(c->wph));
-  LAUNCH(kd::k_vort_flux, grd(D, D.ny + 1, D.nx + 1, D.nl), D, f64(c->G), f64(S), f64(c->ex), f64(c->ey),
-         f64(c->ez), f64(c->uph), f64(c->vph), f64(c->wph), f64(c->pvt_x), f64(c->pvt_y), f64(c->pvt_z));
+  // (the covariant winds in fcm; the vertical mass flux's products in wph and divf)
+  if (!D.llinear) LAUNCH_FN("k_covariant", launch64_covariant(D, c->G, S, c->fc[0], c->fc[1], c->stream));
+  LAUNCH_FN("k_eta_xy", launch64_eta_xy(D, c->G, c->rot, S, c->fc[0], c->fc[1], c->ex, c->ey, c->stream));
+  LAUNCH_FN("k_eta_z", launch64_eta_z(D, c->G, c->rot, S, c->ez, c->stream));
+  LAUNCH_FN("k_mass_flux", launch64_mass_flux(D, c->G, S, c->uph, c->vph, c->wph, c->divf, c->stream));
+  LAUNCH_FN("k_vort_flux", launch64_vort_flux(D, c->G, c->ex, c->ey, c->ez, c->uph, c->vph, c->wph, c->divf, c->pvt_x, c->pvt_y,
+                                              c->pvt_z, c->stream));
   if (!D.llinear) {
     LAUNCH(kd::k_ke, grd(D, D.ny, D.nx, D.nl), D, f64(c->G), f64(S), f64(c->vsq));
     // (the vorticity flux above was the last to read ex and ey, which carry the column products here)
@@ -612,7 +610,7 @@ int diffusion_vector(lgame_gpu* c, const State& So) {
   const DiffBuf<double>& B = c->dbuf;
   if (c->diff_mom_h) {
     LAUNCH(kd::k_diff_tke, grd(D, D.ny, D.nx, D.nl), D, G, So, B, c->dpar);
-    LAUNCH(kd::k_diff_zeta, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So, B);
+    LAUNCH_FN("k_diff_zeta", launch64_zeta_z(D, G, c->rot, So, B.zz, c->stream));
     LAUNCH(kd::k_diff_visc, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature, B, c->dpar);
     LAUNCH(kd::k_diff_vz, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So, B);
     LAUNCH(kd::k_mom_diff_h, grd(D, D.ny, D.nx, D.nl), D, G, So, B);
@@ -697,7 +695,7 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
     }
     Tend<double> T = c->tend;
     if (c->diff_mom_h) { C.mdt_x = c->dbuf.mdtx; C.mdt_y = c->dbuf.mdty; C.mdt_z = c->dbuf.mdtz; }
-    LAUNCH(kd::k_tend_wind, grd(D, D.ny + 1, D.nx + 1, D.NL), D, So, Sn, T, C, rk, (float*)nullptr, (float*)nullptr);
+    LAUNCH_FN("k_tend_wind", launch64_tend_wind(D, So, Sn, T, C, rk, c->stream));
     // scalar_tend_expl (mo_scalar_tend_expl.F90:24-181)
     const State& Ss = (rk == 1) ? So : Sn;
     if (rk == 1) {
@@ -958,6 +956,9 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
     if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
     c->colg = ColumnGrid{c->rvol, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz,
                          1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
+    for (double*& p : c->rotg) if ((rc = dalloc(c, &p, F)) != LGAME_OK) return fail(rc);
+    c->rot = RotGrid{f64(c->rotg[0]), f64(c->rotg[1]), f64(c->rotg[2]), f64(c->rotg[3]), f64(c->rotg[4]),
+                     f64(c->rotg[5]), f64(c->rotg[6]), f64(c->rotg[7]), f64(c->rotg[8])};
     c->fcm = Faces{f64(c->fc[0]), f64(c->fc[1]), f64(c->fc[2]), f64(c->fc[3])};
     c->fct = Faces{f64(c->fc[4]), f64(c->fc[5]), f64(c->fc[6]), f64(c->fc[7])};
     c->recip = Recip{f64(c->rvol), f64(c->rdx), f64(c->rdy), f64(c->rdz)};
@@ -1131,6 +1132,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     if (c->split) split_set_diff_par(c->split, c->dpar);
   }
   if (c->rvol) {
+    launch64_rot_grid(D, c->G, c->rotg, c->stream);
     launch64_recip(D, c->G, c->rdx, c->rdy, c->rdz, c->stream);
     launch_column_grid(D, c->G, c->rvol, c->itwdtv, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz, c->stream);
     CK(cudaGetLastError());
