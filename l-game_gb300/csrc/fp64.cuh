@@ -197,11 +197,15 @@ void launch64_pgrad(const Dims& D, const Grid<double>& G, const State& S, const 
 // impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -
 // exner_bg(jl), 1/area_z; 1/c_imp2 and 1/dtime
 struct ColumnGrid {
-  const double *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
+  const F64 *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
   double rc_imp2, rdt;
 };
 void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
                         double* zs_c1h, double* hdeb, double* raz, cudaStream_t st);
+// once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
+// and c_p of ice and water
+void launch_moist_aux(const Dims& D, const Grid<double>& G, const State& So, const double* T, double* vcloud, double* cpi,
+                      double* cpw, cudaStream_t st);
 int column_prepare();
 void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,
                        const Tend<double>& Tn, int rk_step, cudaStream_t st);

@@ -450,9 +450,4 @@ __global__ void k_ke(Dims D, Grid<T> G, StateT<V> S, T* out) {
   out[IX(D, ji, jk, jl)] = inner_product_at<T>(D, G, S.u, S.v, S.w, ji, jk, jl);
 }
 
-// ---- FP64-only kernels (column_fp64.cu; the others: fp64.cuh) --------------------------
-// once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
-// and c_p of ice and water
-__global__ void k_moist_aux(Dims D, Grid<double> G, State So, const double* T, double* vcloud, double* cpi, double* cpw);
-
 }  // namespace lg

@@ -430,17 +430,17 @@ __global__ void k_output(Dims D, Grid<double> G, State A, State B, double c1, do
 // top level and wherever z_w lies below the layer, where the deceleration is then 0 as in the
 // reference's loop bounds.  One thread per scalar point of layers 1..min(nl, n_damping_levels);
 // the deeper layers stay 0.
-__global__ void k_heating_diss(Dims D, Grid<double> G, State S, double* hd) {
+__global__ void k_heating_diss(Dims D, Grid<F64> G, StateT<F64> S, F64* hd) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx || jl > D.nl) return;
   const long long q = IX(D, ji, jk, jl), b = q + D.plane;
-  auto decel = [&](long long p, int lev) -> double {
+  auto decel = [&](long long p, int lev) -> F64 {
     if (lev < 2 || lev > D.ndamp) return 0.0;
-    const double w = S.w[p];
-    return 0.0 + (w / G.damp[p] - w) / D.dtime;  // mom_diff_tend_z (0) plus the swamp layer's part
+    const F64 w = S.w[p];
+    return (w / G.damp[p] - w) / D.dtime;  // mom_diff_tend_z (0) plus the swamp layer's part
   };
-  const double ip = G.ipw[4][q] * S.w[q] * decel(q, jl) + G.ipw[5][q] * S.w[b] * decel(b, jl + 1);
-  hd[q] = -rho_sum_cond_gas<double, double>(D, S.rho, q) * ip;
+  const F64 ip = G.ipw[4][q] * S.w[q] * decel(q, jl) + G.ipw[5][q] * S.w[b] * decel(b, jl + 1);
+  hd[q] = -rho_sum_cond_gas<F64, F64>(D, S.rho, q) * ip;
 }
 
 // deterministic FP64 sums: every block sums a fixed strided subset in a fixed order;
@@ -514,7 +514,6 @@ namespace kd {
 const auto k_temperature = lg::k_temperature<F64, F64>;
 const auto k_theta = lg::k_theta<double>;
 const auto k_ke = lg::k_ke<F64, F64>;
-const auto k_moist_aux = lg::k_moist_aux;
 const auto k_diff_tke = lg::k_diff_tke<double, double>;
 const auto k_diff_visc = lg::k_diff_visc<double, double>;
 const auto k_diff_vz = lg::k_diff_vz<double, double>;
@@ -620,7 +619,7 @@ int diffusion_vector(lgame_gpu* c, const State& So) {
     if (c->sfc_pbl) LAUNCH(kd::k_pbl, grd(D, D.ny, D.nx, 1), D, G, So, c->vsq, c->sbuf, c->spar, B.mdtx, B.mdty);
     LAUNCH(kd::k_diss_rate, grd(D, D.ny, D.nx, D.nl), D, G, So, B, G.damp, (const double*)nullptr);
   } else if (D.lklemp && D.ndamp > 0) {
-    LAUNCH(k_heating_diss, grd(D, D.ny, D.nx, std::min(D.nl, D.ndamp)), D, G, So, c->hdiss);
+    LAUNCH(k_heating_diss, grd(D, D.ny, D.nx, std::min(D.nl, D.ndamp)), D, f64(G), f64(So), f64(c->hdiss));
   }
   return LGAME_OK;
 }
@@ -682,7 +681,7 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
                                           c->tpv, P, step == 0 ? 1 : 0, c->stream));
       // into the edge arrays of theta', which nothing reads after k_pgrad, and cpw
       if (D.ncons > 1)
-        LAUNCH(kd::k_moist_aux, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature, c->tpu, c->tpv, c->cpw);
+        LAUNCH_FN("k_moist_aux", launch_moist_aux(D, G, So, c->temperature, c->tpu, c->tpv, c->cpw, c->stream));
     }
     if (rk == 2 || step == 0) {
       int rc = advection(c, Sv);
@@ -954,7 +953,7 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
                        &c->fc[0], &c->fc[1], &c->fc[2], &c->fc[3], &c->fc[4], &c->fc[5], &c->fc[6], &c->fc[7]};
     for (double** p : colg) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
     if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
-    c->colg = ColumnGrid{c->rvol, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz,
+    c->colg = ColumnGrid{f64(c->rvol), f64(c->zs), f64(c->zs_c2), f64(c->zs_c1h), f64(c->hdeb), f64(c->raz),
                          1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
     for (double*& p : c->rotg) if ((rc = dalloc(c, &p, F)) != LGAME_OK) return fail(rc);
     c->rot = RotGrid{f64(c->rotg[0]), f64(c->rotg[1]), f64(c->rotg[2]), f64(c->rotg[3]), f64(c->rotg[4]),
