@@ -243,24 +243,21 @@ void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X
   else k_column_ver<2><<<nb, kCvCols * kCvChunks, sm, st>>>(D, f64(G), X, f64(So), f64(Sn), T);
 }
 
-// v_fall_liquid, mo_derived.F90:218-263 (state_old, diag%temperature) with calc_diff_coeff (:189-216)
+// v_fall_liquid, mo_derived.F90:218-263 (state_old, diag%temperature)
 __device__ __forceinline__ F64 v_fall_liquid(const Dims& D, const Grid<F64>& G, const F64* rho_g, const F64* T,
                                              double radius, int ji, int jk, int jl) {
-  constexpr double pm = kM_D / kN_A, c1 = kPI * pm, cross_section = 4.0 * kPI * (130e-12 * 130e-12);
   const long long i = IX(D, ji, jk, jl), b = i + D.plane;
   F64 g;
   if (jl == 1) g = G.gm[b];
   else if (jl == D.nl) g = G.gm[i];
   else g = G.ipw[4][i] * G.gm[i] + G.ipw[5][i] * G.gm[b];
   const F64 rg = rho_g[i];
-  const F64 tv = sqrt(div_rn(8.0 * kK_B * T[i], c1, 1.0 / c1).v);
-  const F64 mfp = rcp(1.4142135623730951 * div_rn(rg, pm, 1.0 / pm) * cross_section);
-  const F64 nu = 1.0 / 3.0 * tv * mfp;
+  const F64 nu = calc_diff_coeff(T[i], rg);
   F64 v = 2.0 * (radius * radius) * (kRHO_H2O - rg) * g / (9.0 * rg * nu);
   // v*radius/nu > 10, the quotient formed only where v*radius is not clearly below 10 nu
   const F64 vr = v * radius;
   if (__double2hiint(vr.v) >= __double2hiint((9.99 * nu).v) && (vr / nu) > 10.0)
-    v = sqrt((8.0 * radius * kRHO_H2O * g / (3.0 * rg * 0.8)).v);
+    v = root(8.0 * radius * kRHO_H2O * g / (3.0 * rg * 0.8));
   return v;
 }
 // c_p_water and c_p_ice, mo_dictionary.F90:112-173

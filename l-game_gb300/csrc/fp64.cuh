@@ -126,6 +126,15 @@ __device__ __forceinline__ F64 div_rn(F64 a, F64 b, F64 y) {
 __device__ __forceinline__ double quot(double a, double b) { return div_rn(a, b, rcp_near(b)); }
 __device__ __forceinline__ F64 operator/(F64 a, F64 b) { return div_rn(a, b, rcp_near(b)); }
 
+__device__ __forceinline__ F64 root(F64 a) { return sqrt(a.v); }
+// calc_diff_coeff, mo_derived.F90:189-216
+__device__ __forceinline__ F64 calc_diff_coeff(F64 temperature, F64 density) {
+  constexpr double pm = kM_D / kN_A, c1 = kPI * pm, cross_section = 4.0 * kPI * (130e-12 * 130e-12);
+  const F64 tv = root(div_rn(8.0 * kK_B * temperature, c1, 1.0 / c1));
+  const F64 mfp = rcp(1.4142135623730951 * div_rn(density, pm, 1.0 / pm) * cross_section);
+  return 1.0 / 3.0 * tv * mfp;
+}
+
 // the same arrays, read as F64
 inline const F64* f64(const double* p) { return reinterpret_cast<const F64*>(p); }
 inline F64* f64(double* p) { return reinterpret_cast<F64*>(p); }
@@ -190,6 +199,28 @@ void launch64_pgrad_cells(const Dims& D, const Grid<double>& G, const State& S, 
 void launch64_pgrad(const Dims& D, const Grid<double>& G, const State& S, const double* gx, const double* gy, const double* gz,
                     const double* th, const double* decel, const double* cond, const double* tvu, const double* tvv,
                     const double* tpu, const double* tpv, const PGrad<double>& P, int lfirst, cudaStream_t st);
+
+// the diffusion closure; of DiffBuf's flux arrays one field each is used, for the coefficients at the
+// faces and interfaces
+template <class T>
+struct DiffBuf;
+struct DiffPar;
+void launch64_diff_tke(const Dims& D, const Grid<double>& G, const Recip& R, const State& S, const DiffBuf<double>& B,
+                       const double* gx, const double* gy, const double* gz, double mva, cudaStream_t st);
+void launch64_diff_coeffs(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, int kind, int vertical,
+                          double* ch, double* cv, cudaStream_t st);
+void launch64_diff_face_coeffs(const Dims& D, const double* ch, const double* cv, int vertical, const DiffBuf<double>& B,
+                               cudaStream_t st);
+void launch64_diff_faces(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
+                         const double* w6, const DiffBuf<double>& B, const Faces& F, cudaStream_t st);
+void launch64_diff_div(const Dims& D, const Grid<double>& G, const Recip& R, const Faces& F, const DiffBuf<double>& B,
+                       const double* gz, int vertical, double* out, cudaStream_t st);
+void launch64_diff_visc(const Dims& D, const Grid<double>& G, const State& S, const double* T, const DiffBuf<double>& B,
+                        const DiffPar& P, cudaStream_t st);
+void launch64_diff_vz(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st);
+void launch64_mom_diff_h(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st);
+void launch64_mom_diff_v(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st);
+void launch64_diss_rate(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st);
 
 // the column solves (column_fp64.cu)
 // grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of

@@ -6,10 +6,13 @@
 // column), metrics divide by their stored reciprocals, halves are taken in the exponent, and sums do
 // not start with 0 + x.
 #include "fp64.cuh"
+#include "diffusion.cuh"
 
 #include <algorithm>
 
 namespace lg {
+
+template <> __device__ __forceinline__ F64 dsqrt<F64>(F64 x) { return root(x); }
 
 namespace {
 
@@ -686,7 +689,157 @@ __global__ void k64_tend_wind(Dims D, StateT<F64> So, StateT<F64> Sn, Tend<F64> 
   }
 }
 
+// ---- diffusion closure (diffusion.cuh) --------------------------------------------------------------
+// update_n_squared and tke_update, mo_eff_diff_coeffs.F90:620-669, mo_tke.F90:19-66, marching down the
+// levels (theta_v, its reciprocal and the interface's n_squared are carried); gx, gy, gz: the gradient
+// of the TKE (0 at non-periodic boundary edges and at the first and last level); decay_c =
+// 8*pi^2/mean_velocity_area
+__global__ void __launch_bounds__(128) k64_diff_tke(Dims D, Grid<F64> G, const F64* rdz, StateT<F64> S, DiffBuf<F64> B,
+                                                    const F64* gx, const F64* gy, const F64* gz, double decay_c) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = march_first(D, blockIdx.z), l1 = march_first(D, blockIdx.z + 1) - 1;
+  if (l0 > l1) return;
+  long long q = IX(D, ji, jk, l0);
+  auto theta = [&](long long p) { return G.theta_v_bg[p] + S.tp[p]; };
+  // g * 0.5*(1/theta(l-1) + 1/theta(l)) * dtheta/dz at the interface above layer p
+  auto nz = [&](F64 tha, F64 ra, F64 thb, F64 rb, long long p) {
+    return G.gm[p] * (half(ra + rb) * div_rn(tha - thb, G.dz[p], rdz[p]));
+  };
+  F64 th = theta(q), rth = rcp(th), n_up = 0.0;
+  if (l0 >= 2) {
+    const F64 ta = theta(q - D.plane);
+    n_up = nz(ta, rcp(ta), th, rth, q);
+  }
+  for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
+    const long long b = q + D.plane, e = q + D.P, s = q + 1;
+    F64 n_lo = 0.0;
+    if (jl < D.nl) {
+      const F64 tb = theta(b), rb = rcp(tb);
+      n_lo = nz(th, rth, tb, rb, b);
+      th = tb;
+      rth = rb;
+    }
+    F64 nsq = 0.0;
+    if (jl > 1 && jl < D.nl) nsq = G.ipw[4][q] * n_up + G.ipw[5][q] * n_lo;
+    B.nsq[q] = nsq;
+    n_up = n_lo;
+    const F64 adv = G.ipw[0][q] * S.u[e] * gx[e] + G.ipw[1][q] * S.v[q] * gy[q] + G.ipw[2][q] * S.u[q] * gx[q]
+                  + G.ipw[3][q] * S.v[s] * gy[s] + G.ipw[4][q] * S.w[q] * gz[q] + G.ipw[5][q] * S.w[b] * gz[b];
+    const F64 rg = S.rho[q + (long long)(D.g - 1) * D.fstride], y = rcp_near(rg);
+    const F64 decay_constant = div_rn(decay_c * B.visc[q], rg, y), tke = B.tke[q];
+    F64 t = tke + D.dtime * (-adv + div_rn(B.hd[q], rg, y) - decay_constant * tke);
+    if (negative(t)) t = 0.0;
+    B.tke_new[q] = t;
+  }
+}
+// the coefficients of the scalar diffusion (scalar_diff_coeffs, mo_eff_diff_coeffs.F90:526-618) at a
+// cell: kind 0 mass, 1 temperature (c_g_v = rho_g/rho_g*c_d_v is c_d_v)
+__global__ void k64_diff_cells(Dims D, Grid<F64> G, StateT<F64> S, DiffBuf<F64> B, int kind, int vertical, F64* ch, F64* cv) {
+  LG_IDX3;
+  if (ji > D.ny || jk > D.nx) return;
+  const long long q = IX(D, ji, jk, jl);
+  const F64 rg = S.rho[q + (long long)(D.g - 1) * D.fstride];
+  ch[q] = kind == 0 ? B.visc[q] / rg : kC_D_V * B.visc[q];
+  if (!vertical) return;
+  const F64 t2v = B.vmol[q] + tke2vert<F64>(B.tke[q], B.nsq[q], G.layer_thickness[q]);
+  cv[q] = kind == 0 ? t2v : rg * kC_D_V * t2v;
+}
+// at the faces and interfaces: the mean of the two cells
+__global__ void k64_diff_face_coeffs(Dims D, const F64* ch, const F64* cv, int vertical, F64* hx, F64* hy, F64* hw) {
+  LG_IDX3;
+  const long long q = IX(D, ji, jk, jl);
+  if (ji <= D.ny && jk <= D.nx + 1) {
+    const bool inner = jk >= 2 && jk <= D.nx;
+    hx[q] = half(ch[inner ? q - D.P : IX(D, ji, D.nx, jl)] + ch[inner ? q : IX(D, ji, 1, jl)]);
+  }
+  if (ji <= D.ny + 1 && jk <= D.nx) {
+    const bool inner = ji >= 2 && ji <= D.ny;
+    hy[q] = half(ch[inner ? q - 1 : IX(D, D.ny, jk, jl)] + ch[inner ? q : IX(D, 1, jk, jl)]);
+  }
+  if (vertical && jl >= 2 && ji <= D.ny && jk <= D.nx) hw[q] = half(cv[q - D.plane] + cv[q]);
+}
+// the diffusive flux of a scalar through the faces: coefficient times gradient
+__global__ void k64_diff_faces(Dims D, Grid<F64> G, Recip R, const F64* s, const F64* w5, const F64* w6, const F64* hx,
+                               const F64* hy, Faces F) {
+  LG_IDX3;
+  const long long q = IX(D, ji, jk, jl);
+  F64 r;
+  if (ji <= D.ny && jk <= D.nx + 1)
+    face_x(D, G, grad_x64(D, G, R.dx, s, w5, w6, ji, jk, jl, &r) ? hx[q] * r : F64(0.0), F, jl, q);
+  if (ji <= D.ny + 1 && jk <= D.nx)
+    face_y(D, G, grad_y64(D, G, R.dy, s, w5, w6, ji, jk, jl, &r) ? hy[q] * r : F64(0.0), F, jl, q);
+}
+// its divergence, with the vertical part (add_vertical_div, mo_divergence_operators.F90:149-186)
+__global__ void __launch_bounds__(128) k64_diff_div(Dims D, Grid<F64> G, const F64* rvol, Faces F, const F64* hw, const F64* gz,
+                                                    int vertical, F64* out) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1, jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const int l0 = march_first(D, blockIdx.z), l1 = march_first(D, blockIdx.z + 1) - 1;
+  if (l0 > l1) return;
+  long long q = IX(D, ji, jk, l0);
+  ColumnDiv c;
+  c.start(D, G, F, q, l0);
+  F64 up = 0.0;
+  if (vertical && l0 >= 2) up = hw[q] * gz[q] * G.area_z[q];
+  for (int jl = l0; jl <= l1; ++jl, q += D.plane) {
+    const F64 V = G.volume[q], rV = rvol[q];
+    F64 r = c.step(D, G, F, V, rV, q, jl);
+    if (vertical) {
+      const long long b = q + D.plane;
+      F64 lo = 0.0;
+      if (jl < D.nl) lo = hw[b] * gz[b] * G.area_z[b];
+      r = r + div_rn(up - lo, V, rV);
+      up = lo;
+    }
+    out[q] = r;
+  }
+}
+
 }  // namespace
+
+const DiffBuf<F64>& f64(const DiffBuf<double>& b) { return reinterpret_cast<const DiffBuf<F64>&>(b); }
+void launch64_diff_tke(const Dims& D, const Grid<double>& G, const Recip& R, const State& S, const DiffBuf<double>& B,
+                       const double* gx, const double* gy, const double* gz, double mva, cudaStream_t st) {
+  k64_diff_tke<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), R.dz, f64(S), f64(B), f64(gx), f64(gy), f64(gz),
+                                                      8.0 * (kPI * kPI) / mva);
+}
+void launch64_diff_coeffs(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, int kind, int vertical,
+                          double* ch, double* cv, cudaStream_t st) {
+  k64_diff_cells<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(B), kind, vertical, f64(ch), f64(cv));
+}
+void launch64_diff_face_coeffs(const Dims& D, const double* ch, const double* cv, int vertical, const DiffBuf<double>& B,
+                               cudaStream_t st) {
+  k64_diff_face_coeffs<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(ch), f64(cv), vertical, f64(B.flx),
+                                                                                   f64(B.fly), f64(B.flw));
+}
+void launch64_diff_faces(const Dims& D, const Grid<double>& G, const Recip& R, const double* s, const double* w5,
+                         const double* w6, const DiffBuf<double>& B, const Faces& F, cudaStream_t st) {
+  k64_diff_faces<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), R, f64(s), f64(w5), f64(w6), f64(B.flx),
+                                                                             f64(B.fly), F);
+}
+void launch64_diff_div(const Dims& D, const Grid<double>& G, const Recip& R, const Faces& F, const DiffBuf<double>& B,
+                       const double* gz, int vertical, double* out, cudaStream_t st) {
+  k64_diff_div<<<march_grid(D), kMarchBlock, 0, st>>>(D, f64(G), R.vol, F, f64(B.flw), f64(gz), vertical, f64(out));
+}
+// the closure's other kernels are the templates of diffusion.cuh
+void launch64_diff_visc(const Dims& D, const Grid<double>& G, const State& S, const double* T, const DiffBuf<double>& B,
+                        const DiffPar& P, cudaStream_t st) {
+  k_diff_visc<F64, F64><<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(T), f64(B), P);
+}
+void launch64_diff_vz(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st) {
+  k_diff_vz<F64, F64><<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(B));
+}
+void launch64_mom_diff_h(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st) {
+  k_mom_diff_h<F64, F64><<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(B));
+}
+void launch64_mom_diff_v(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st) {
+  k_mom_diff_v<F64, F64><<<cell_grid(D.ny, D.nx, D.nl - 1), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(B));
+}
+void launch64_diss_rate(const Dims& D, const Grid<double>& G, const State& S, const DiffBuf<double>& B, cudaStream_t st) {
+  k_diss_rate<F64, F64><<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(B), f64(G.damp),
+                                                                           (const F64*)nullptr);
+}
 
 void launch64_rot_grid(const Dims& D, const Grid<double>& G, double* const* a, cudaStream_t st) {
   k64_rot_grid<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), f64(a[0]), f64(a[1]), f64(a[2]), f64(a[3]),

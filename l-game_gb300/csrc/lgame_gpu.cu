@@ -514,16 +514,6 @@ namespace kd {
 const auto k_temperature = lg::k_temperature<F64, F64>;
 const auto k_theta = lg::k_theta<double>;
 const auto k_ke = lg::k_ke<F64, F64>;
-const auto k_diff_tke = lg::k_diff_tke<double, double>;
-const auto k_diff_visc = lg::k_diff_visc<double, double>;
-const auto k_diff_vz = lg::k_diff_vz<double, double>;
-const auto k_mom_diff_h = lg::k_mom_diff_h<double, double>;
-const auto k_mom_diff_v = lg::k_mom_diff_v<double, double>;
-const auto k_diss_rate = lg::k_diss_rate<double, double>;
-const auto k_diff_fluxes1 = lg::k_diff_fluxes<double, double, double, 1>;
-const auto k_diff_fluxes7 = lg::k_diff_fluxes<double, double, double, 7>;
-const auto k_diff_divs1 = lg::k_diff_divs<double, 1>;
-const auto k_diff_divs7 = lg::k_diff_divs<double, 7>;
 const auto k_sfc_turb = lg::k_sfc_turb<double>;
 const auto k_pbl = lg::k_pbl<double, double>;
 const auto k_sfc_column = lg::k_sfc_column<double>;
@@ -608,16 +598,19 @@ int diffusion_vector(lgame_gpu* c, const State& So) {
   const Grid<double>& G = c->G;
   const DiffBuf<double>& B = c->dbuf;
   if (c->diff_mom_h) {
-    LAUNCH(kd::k_diff_tke, grd(D, D.ny, D.nx, D.nl), D, G, So, B, c->dpar);
+    // (the gradient of the TKE in gx, gy, gz, which nothing reads after the pressure gradient)
+    const int rc = gradient(c, B.tke, c->gx, c->gy, c->gz);
+    if (rc != LGAME_OK) return rc;
+    LAUNCH_FN("k_diff_tke", launch64_diff_tke(D, G, c->recip, So, B, c->gx, c->gy, c->gz, c->dpar.mva, c->stream));
     LAUNCH_FN("k_diff_zeta", launch64_zeta_z(D, G, c->rot, So, B.zz, c->stream));
-    LAUNCH(kd::k_diff_visc, grd(D, D.ny, D.nx, D.nl), D, G, So, c->temperature, B, c->dpar);
-    LAUNCH(kd::k_diff_vz, grd(D, D.ny + 1, D.nx + 1, D.nl), D, G, So, B);
-    LAUNCH(kd::k_mom_diff_h, grd(D, D.ny, D.nx, D.nl), D, G, So, B);
-    if (c->diff_mom_v) LAUNCH(kd::k_mom_diff_v, grd(D, D.ny, D.nx, D.nl - 1), D, G, So, B);
+    LAUNCH_FN("k_diff_visc", launch64_diff_visc(D, G, So, c->temperature, B, c->dpar, c->stream));
+    LAUNCH_FN("k_diff_vz", launch64_diff_vz(D, G, So, B, c->stream));
+    LAUNCH_FN("k_mom_diff_h", launch64_mom_diff_h(D, G, So, B, c->stream));
+    if (c->diff_mom_v) LAUNCH_FN("k_mom_diff_v", launch64_mom_diff_v(D, G, So, B, c->stream));
     // pbl_wind_tendency (mo_vector_tend_expl.F90:119-121), before the dissipation reads the
     // momentum diffusion acceleration
     if (c->sfc_pbl) LAUNCH(kd::k_pbl, grd(D, D.ny, D.nx, 1), D, G, So, c->vsq, c->sbuf, c->spar, B.mdtx, B.mdty);
-    LAUNCH(kd::k_diss_rate, grd(D, D.ny, D.nx, D.nl), D, G, So, B, G.damp, (const double*)nullptr);
+    LAUNCH_FN("k_diss_rate", launch64_diss_rate(D, G, So, B, c->stream));
   } else if (D.lklemp && D.ndamp > 0) {
     LAUNCH(k_heating_diss, grd(D, D.ny, D.nx, std::min(D.nl, D.ndamp)), D, f64(G), f64(So), f64(c->hdiss));
   }
@@ -631,23 +624,31 @@ int diffusion_scalar(lgame_gpu* c, const State& So) {
   const Dims& D = c->D;
   const Grid<double>& G = c->G;
   const DiffBuf<double>& B = c->dbuf;
-  const dim3 gs = grd(D, D.ny, D.nx, D.nl), ge = grd(D, D.ny + 1, D.nx + 1, D.nl);
+  // the coefficients (kind 0 mass, 1 temperature; of the cells in theta and divf), then every field's
+  // gradient (column products in ex, ey), faces (fct) and divergence
+  auto coeffs = [&](int kind, int vert) -> int {
+    LAUNCH_FN("k_diff_coeffs", launch64_diff_coeffs(D, G, So, B, kind, vert, c->theta, c->divf, c->stream));
+    LAUNCH_FN("k_diff_coeffs", launch64_diff_face_coeffs(D, c->theta, c->divf, vert, B, c->stream));
+    return LGAME_OK;
+  };
+  auto field = [&](const double* f, int vert, double* out) -> int {
+    LAUNCH_FN("k_grad_vert", launch64_grad_vert(D, G, c->recip, f, c->gz, c->ex, c->ey, c->stream));
+    LAUNCH_FN("k_diff_faces", launch64_diff_faces(D, G, c->recip, f, c->ex, c->ey, B, c->fct, c->stream));
+    LAUNCH_FN("k_diff_div", launch64_diff_div(D, G, c->recip, c->fct, B, c->gz, vert, out, c->stream));
+    return LGAME_OK;
+  };
+  int rc = LGAME_OK;
   if (c->diff_temp_h) {
     const int vert = c->diff_temp_v ? 1 : 0;
-    LAUNCH(kd::k_diff_fluxes1, ge, D, G, So, B, (const double*)c->temperature, 1, vert, B.flx, B.fly, B.flw);
-    LAUNCH(kd::k_diff_divs1, gs, D, G, B.flx, B.fly, B.flw, vert, B.tdh);
+    if ((rc = coeffs(1, vert)) || (rc = field(c->temperature, vert, B.tdh))) return rc;
   }
-  if (c->diff_mass_h) {  // every constituent in one launch each (1 dry, 7 moist)
+  if (c->diff_mass_h) {
     const int vert = c->diff_mass_v ? 1 : 0;
-    if (D.ncons == 7) {
-      LAUNCH(kd::k_diff_fluxes7, ge, D, G, So, B, (const double*)So.rho, 0, vert, B.flx, B.fly, B.flw);
-      LAUNCH(kd::k_diff_divs7, gs, D, G, B.flx, B.fly, B.flw, vert, B.mdt);
-    } else {
-      LAUNCH(kd::k_diff_fluxes1, ge, D, G, So, B, (const double*)So.rho, 0, vert, B.flx, B.fly, B.flw);
-      LAUNCH(kd::k_diff_divs1, gs, D, G, B.flx, B.fly, B.flw, vert, B.mdt);
-    }
+    if ((rc = coeffs(0, vert))) return rc;
+    for (int jc = 0; jc < D.ncons; ++jc)
+      if ((rc = field(So.rho + (long long)jc * D.fstride, vert, B.mdt + (long long)jc * D.fstride))) return rc;
   }
-  return LGAME_OK;
+  return rc;
 }
 
 int step_fp64(lgame_gpu* c, int so, int sn, int step) {
@@ -982,9 +983,7 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
       double** work[] = {&B.tke_new, &B.vmol, &B.nsq, &B.vz, &B.zz, &B.vdiv};
       for (double** p : work) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
       if (c->diff_temp_h || c->diff_mass_h) {
-        const size_t nf = c->diff_mass_h ? (size_t)D.ncons : 1;
-        if ((rc = dalloc(c, &B.flx, F * nf)) || (rc = dalloc(c, &B.fly, F * nf)) || (rc = dalloc(c, &B.flw, F * nf)))
-          return fail(rc);
+        if ((rc = dalloc(c, &B.flx, F)) || (rc = dalloc(c, &B.fly, F)) || (rc = dalloc(c, &B.flw, F))) return fail(rc);
       }
     }
     DiffPar& P = c->dpar;
