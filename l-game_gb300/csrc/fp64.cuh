@@ -46,6 +46,30 @@ __device__ __forceinline__ double mul_int(double x, double y) {
   return __hiloint2double((int)(((uint32_t)(r >> 32) + e) ^ ((xh ^ yh) & 0x80000000u)), (int)(uint32_t)r);
 }
 
+// The same with a single-precision factor x, whose 24 bits leave two of the four partial products;
+// subnormal and non-finite x take the hardware's.
+__device__ __forceinline__ double mul_int(float x, double y) {
+  const uint32_t xu = __float_as_uint(x), yh = (uint32_t)__double2hiint(y), yl = (uint32_t)__double2loint(y);
+  const uint32_t xe = xu & 0x7F800000u, ye = yh & 0x7FF00000u;
+  if ((xe - (1u << 23) >= (254u << 23)) | (ye - (513u << 20) >= (1022u << 20))) {
+    const bool x0 = xu << 1 == 0u, y0 = ((yh << 1) | yl) == 0u;
+    if ((x0 && ye < 0x7FF00000u) || (y0 && xe < 0x7F800000u)) return __hiloint2double((int)((xu ^ yh) & 0x80000000u), 0);
+    return mul_hw(wide(x), y);
+  }
+  // mantissas as a < 2^32 and b < 2^54: the product is in [2^84, 2^86), its upper 64 bits hold 53 or 54
+  const uint32_t a = (xu << 8) | 0x80000000u;
+  const uint32_t bh = (__funnelshift_l(yl, yh, 1) & 0x1FFFFFu) | 0x200000u, bl = yl << 1;
+  const uint64_t low = (uint64_t)a * bl, up = (uint64_t)a * bh + (low >> 32);
+  uint32_t hh = (uint32_t)(up >> 32), hl = (uint32_t)up;
+  const uint32_t big = hh >> 21, sh = 1u - big, mid = (uint32_t)low;
+  hh = __funnelshift_l(hl, hh, sh);
+  hl = __funnelshift_l(mid, hl, sh);
+  const uint32_t t = ((hl >> 1) & 1u) | ((mid << sh) != 0u ? 1u : 0u);
+  const uint64_t r = ((((uint64_t)hh << 32) | hl) + t) >> 1;
+  const uint32_t e = (xe >> 3) + (896u << 20) + ye - 0x3FF00000u - 0x00100000u + (big << 20);
+  return __hiloint2double((int)(((uint32_t)(r >> 32) + e) ^ ((xu ^ yh) & 0x80000000u)), (int)(uint32_t)r);
+}
+
 // x < 0 by the bits (a comparison issues on the FP64 pipe); -0 counts as negative, NaN does not
 __device__ __forceinline__ bool negative(double x) {
   const unsigned u = (unsigned)__double2hiint(x) - 0x80000000u;

@@ -85,3 +85,36 @@ def test_quotient_is_the_rounded_quotient():
         q = x * r
         assert fma(fma(-y, q, x), r, q) == x / y
         assert fma(fma(-y, r, 1.0), r, r) == 1.0 / y
+
+
+def mul_int_single(x, y):
+    """mul_int of csrc/fp64.cuh with a single-precision factor x; None where it takes the hardware's product."""
+    xu = struct.unpack("<I", struct.pack("<f", x))[0]
+    yh, yl = bits(y) >> 32, bits(y) & M32
+    xe, ye = xu & 0x7F800000, yh & 0x7FF00000
+    if (xe - (1 << 23)) & M32 >= 254 << 23 or (ye - (513 << 20)) & M32 >= 1022 << 20:
+        return None
+    a = (xu << 8) & M32 | 0x80000000
+    bh, bl = (((yh << 32 | yl) << 1) >> 32 & 0x1FFFFF) | 0x200000, (yl << 1) & M32
+    low = a * bl
+    up = a * bh + (low >> 32)
+    assert max(low, up) < 1 << 64
+    hh, hl, mid = up >> 32, up & M32, low & M32
+    big = hh >> 21
+    assert big in (0, 1)
+    sh = 1 - big
+    hh, hl = (((hh << 32 | hl) << sh) >> 32) & M32, (((hl << 32 | mid) << sh) >> 32) & M32
+    t = (hl >> 1 & 1) | (1 if (mid << sh) & M32 else 0)
+    r = (((hh << 32 | hl) + t) & ((1 << 64) - 1)) >> 1
+    e = (xe >> 3) + (896 << 20) + ye - 0x3FF00000 - 0x00100000 + (big << 20)
+    return of_bits((((((r >> 32) + e) & M32) ^ ((xu >> 31 ^ yh >> 31) << 31)) << 32) | (r & M32))
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "window", "ties", "ones"])
+def test_integer_product_with_a_single_precision_factor(kind):
+    for x, y in pairs(kind):
+        x = float(np.float32(x)) if 2.0 ** -126 <= abs(float(x)) < 2.0 ** 127 else 1.0 + float(x) % 1.0
+        x = float(np.float32(x))
+        assert bits(mul_int_single(x, float(y))) == bits(x * float(y)), (x, y)
+    for x, y in [(0.0, 1.0), (2.0 ** -127, 1.0), (float("inf"), 1.0), (float("nan"), 1.0), (1.0, 2.0 ** 512), (1.0, 0.0)]:
+        assert mul_int_single(x, y) is None
