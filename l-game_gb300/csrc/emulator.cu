@@ -138,22 +138,24 @@ __device__ __forceinline__ float gelu_grad(float z) {
 //   warp 1 (lane 0)  MMA issuer: four tcgen05.mma per K block into one of two accumulators in
 //                    tensor memory, alternating per tile; the stage is released by a commit to its
 //                    "empty" barrier, the finished accumulator by a commit to its "full" barrier;
-//   warps 2-5        epilogue: warp w reads tensor-memory lanes 32*(w%4).. (tile rows) of the
+//   warps 2-...      epilogue, in groups of four warps that take 32 columns of the tile at a time
+//                    in turn: warp w reads tensor-memory lanes 32*(w%4).. (tile rows) of the
 //                    finished accumulator, applies the fused epilogue, and arrives on the
 //                    accumulator's "empty" barrier, so that the MMAs of the next tile run while
-//                    the previous one drains.
+//                    the previous one drains.  (One group of four left each scheduler a single warp
+//                    with its chain of erff: 24.5 against 20.3 us for 8192 x 512 x 512.)
 // Every wait is bounded and also ends when another role has given up (a shared abort flag);
 // the CTA then waits (bounded) for its own copies and MMAs before freeing tensor memory.
-constexpr int kGemmThreads = 192;
-
 template <int BN>
 struct GemmCfg {
   static constexpr uint32_t kCols = (BN <= 32) ? 32 : (BN <= 64) ? 64 : (BN <= 128) ? 128 : 256;  // one accumulator
   static constexpr uint32_t kA = 128 * 64 * 2, kB = BN * 64 * 2, kStage = kA + kB;             // bytes per stage
-  static constexpr int kStages = (BN <= 128) ? 6 : 4;
+  static constexpr int kStages = (BN <= 64) ? 6 : (BN <= 128) ? 4 : 3;  // what the staging tiles leave room for
+  static constexpr int kGroups = (BN / 32 < 4) ? BN / 32 : (BN % 128 ? 3 : 4);  // epilogue groups: divide BN/32
+  static constexpr int kThreads = 64 + 128 * kGroups;
   // per epilogue warp a 32 x 32 FP32 staging tile (4 KB, 128-byte swizzle) for the TMA store
   static constexpr uint32_t kStg = 32 * 32 * 4;
-  static constexpr size_t kSmem = (size_t)kStages * kStage + 4 * kStg + 1024;  // + alignment slack of the atoms
+  static constexpr size_t kSmem = (size_t)kStages * kStage + 4 * kGroups * kStg + 1024;  // + alignment slack of the atoms
 };
 
 // TMA tensor store of a 3-D box from shared memory (bulk group), and its completion waits
@@ -192,6 +194,19 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t mbar, uint32_t parit
   return false;
 }
 
+// barrier of the four warps of an epilogue group, and whether all of them pass ok
+__device__ __forceinline__ bool group_all(int group, bool ok) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u), "r"(group + 1)
+      : "memory");
+  return r != 0;
+}
+
 // the fused epilogue of 16 accumulator columns (nb..nb+15) of tile row m: the FP32 output
 // values into f (stored by the caller), the BF16 outputs written here
 __device__ __forceinline__ void epilogue16(const Epi& ep, int m, int nb, const float* v, float* f) {
@@ -219,7 +234,7 @@ __device__ __forceinline__ void epilogue16(const Epi& ep, int m, int nb, const f
 #pragma unroll
         for (int j = 0; j < 16; ++j) f[j] = v[j] + ep.bias[nb + j];
       } else {
-        const float4* zp = reinterpret_cast<const float4*>(ep.zprev + (size_t)m * ep.ldc + nb);
+        const float4* zp = reinterpret_cast<const float4*>(ep.zprev + (size_t)m * ep.ldh + nb);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 t = zp[q];
@@ -245,7 +260,7 @@ __device__ __forceinline__ void epilogue16(const Epi& ep, int m, int nb, const f
 }
 
 template <int BN>
-__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(const __grid_constant__ CUtensorMap tmA,
+__global__ void __launch_bounds__(GemmCfg<BN>::kThreads, 1) k_gemm(const __grid_constant__ CUtensorMap tmA,
                                                           const __grid_constant__ CUtensorMap tmB,
                                                           const __grid_constant__ CUtensorMap tmC, int K, int kchunk,
                                                           int tiles_n, int tiles_m, int splits, Epi ep, int* err) {
@@ -277,7 +292,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&acc_full[i]), 1);
-      mbar_init(smem_u32(&acc_empty[i]), 4);  // one arrival per epilogue warp
+      mbar_init(smem_u32(&acc_empty[i]), 4 * Cfg::kGroups);  // one arrival per epilogue warp
     }
     mbar_init(smem_u32(&done), 1);
     abort_flag = 0;
@@ -360,40 +375,65 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(const __grid_constant_
       tc_commit(smem_u32(&done));
     }
   } else {
-    const int qw = warp & 3;  // tensor-memory lanes 32*qw.. = tile rows
-    // this warp's staging tile, after the stages (1024-byte aligned: 128-byte swizzle atoms)
-    const uint32_t stg = sbase + (uint32_t)S * kStage + (uint32_t)qw * Cfg::kStg;
+    const int qw = warp & 3, group = (warp - 2) >> 2;  // tensor-memory lanes 32*qw.. = tile rows
+    // this warp's staging tile, after the stages (1024-byte aligned: 128-byte swizzle atoms), and
+    // the group's four
+    const uint32_t stg = sbase + (uint32_t)S * kStage + (uint32_t)(4 * group + qw) * Cfg::kStg;
     uint8_t* stg_ptr = smem_raw + (stg - smem_u32(smem_raw));
+    const uint8_t* grp_ptr = stg_ptr - qw * Cfg::kStg;
     int lt = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
       int tn, tm, z;
       tile_of(t, &tn, &tm, &z);
       const int b = lt & 1;
       bool ok = mbar_wait_or_abort(smem_u32(&acc_full[b]), (uint32_t)((lt / 2) & 1), abort_v);
-      ok = __all_sync(0xffffffffu, ok);  // the tensor-memory loads below need the whole warp
+      ok = group_all(group, ok);  // the loads below need the whole warp, the barriers the group
       if (!ok) {
         failed = true;
         break;
       }
       tc_fence_after();
       const int m0 = tm * 128 + qw * 32, m = m0 + lane;
-      for (int c = 0; c < BN; c += 32) {
-        float v[32], f[32];
+      for (int c = 32 * group; c < BN; c += 32 * Cfg::kGroups) {
         const uint32_t ta = tmem + (uint32_t)b * kCols + ((uint32_t)(qw * 32) << 16) + (uint32_t)c;
-        tc_ld16(ta, v);
-        tc_ld16(ta + 16, v + 16);
         const int nb = tn * BN + c;
-        epilogue16(ep, m, nb, v, f);
-        epilogue16(ep, m, nb + 16, v + 16, f + 16);
-        if (ep.kind == kEpiBiasGeluH) continue;  // no FP32 output
+        const bool inf = ep.kind == kEpiBiasGeluH, store = !inf && ep.kind != kEpiGeluBwd;
         // the FP32 values through the staging tile: row `lane` in the 128-byte swizzle (its
         // 16-byte chunk j at position j ^ (row % 8), so the warp's stores hit distinct banks),
         // then one TMA store of the 32 x 32 box; the previous box's read of the tile first
-        if (lane == 0) bulk_wait_read0();
+        if (store && lane == 0) bulk_wait_read0();
         __syncwarp();
         float4* row = reinterpret_cast<float4*>(stg_ptr + lane * 128);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) row[j ^ (lane & 7)] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+        for (int h = 0; h < 2; ++h) {
+          float v[16], f[16];
+          tc_ld16(ta + 16 * h, v);
+          epilogue16(ep, m, nb + 16 * h, v, f);
+          if (inf) continue;  // no FP32 output
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            row[(4 * h + j) ^ (lane & 7)] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+        }
+        if (inf) continue;
+        if (!store) {
+          // the column sums of the tile's 128 rows, in the order of k_loss_dy: eight chains of every
+          // eighth row, then the chains.  Lane: chain lane/4 of the warp's columns 8*qw + lane%4 and + 4
+          group_all(group, true);
+          const int j = lane >> 2, c4 = lane & 3;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint8_t* col = grp_ptr + j * 128 + (((2 * qw + h) ^ j) << 4) + 4 * c4;
+            float a = 0.f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) a += *reinterpret_cast<const float*>(col + 1024 * r);
+            float sum = __shfl_sync(0xffffffffu, a, c4);
+#pragma unroll
+            for (int k = 1; k < 8; ++k) sum += __shfl_sync(0xffffffffu, a, 4 * k + c4);
+            if (j == 0) ep.colsum[(size_t)tm * ep.ldh + nb + 8 * qw + 4 * h + c4] = sum;
+          }
+          group_all(group, true);  // before the tiles are written again
+          continue;
+        }
         fence_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -504,7 +544,7 @@ int launch_gemm_bn(const bf16* A, int lda, const bf16* B, int ldb, int M, int N,
   int rc = tensor_map(&ma, A, M, K, lda, 128);
   if (rc == LGAME_OK) rc = tensor_map(&mb, B, N, K, ldb, BN);
   if (rc == LGAME_OK) {
-    if (ep.kind == kEpiBiasGeluH) mc = ma;  // no FP32 output; the map is not used
+    if (ep.kind == kEpiBiasGeluH || ep.kind == kEpiGeluBwd) mc = ma;  // no FP32 output; the map is not used
     else rc = tensor_map_c(&mc, ep.c, N, M, ep.kind == kEpiF32 ? zs : 1, ep.ldc, ep.split_stride);
   }
   if (rc != LGAME_OK) return rc;
@@ -514,7 +554,7 @@ int launch_gemm_bn(const bf16* A, int lda, const bf16* B, int ldb, int M, int N,
   // programmatic dependent launch: see griddepcontrol in k_gemm
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kGemmThreads);
+  cfg.blockDim = dim3(GemmCfg<BN>::kThreads);
   cfg.dynamicSmemBytes = shm;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -554,14 +594,15 @@ int launch_gemm(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, in
 // through shared memory, so that both sides are coalesced.
 //
 // standardised, zero-padded BF16 inputs, row-major and transposed; grid (nin_pad/32, batch/32);
-// rows >= valid (padding of the last batch) are zero and not read
-__global__ void __launch_bounds__(256) k_prep_x(const float* __restrict__ x, int nin, int nin_pad, int batch,
-                                                int valid, const float* mean, const float* istd, bf16* X, bf16* XT) {
+// rows >= valid (padding of the last batch) are zero and not read; with idx, row r is row idx[r] of x
+__global__ void __launch_bounds__(256) k_prep_x(const float* __restrict__ x, const long long* __restrict__ idx, int nin,
+                                                int nin_pad, int batch, int valid, const float* mean, const float* istd, bf16* X, bf16* XT) {
   __shared__ bf16 t[32][34];
   const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
   for (int j = threadIdx.y; j < 32; j += 8) {
     const int r = r0 + j;
-    const float v = (c < nin && r < valid) ? (x[(size_t)r * nin + c] - mean[c]) * istd[c] : 0.f;
+    const float v =
+        (c < nin && r < valid) ? (x[(size_t)(idx ? idx[r] : r) * nin + c] - mean[c]) * istd[c] : 0.f;
     const bf16 b = __float2bfloat16_rn(v);
     X[(size_t)r * nin_pad + c] = b;
     t[j][threadIdx.x] = b;
@@ -571,103 +612,120 @@ __global__ void __launch_bounds__(256) k_prep_x(const float* __restrict__ x, int
   for (int j = threadIdx.y; j < 32; j += 8)
     XT[(size_t)(blockIdx.x * 32 + j) * batch + r0 + threadIdx.x] = t[threadIdx.x][j];
 }
-__global__ void k_prep_y(const float* __restrict__ y, int nout, int nout_pad, int batch, const float* mean,
-                         const float* istd, float* Yt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= batch * nout_pad) return;
-  const int r = i / nout_pad, c = i % nout_pad;
-  Yt[i] = (c < nout) ? (y[(size_t)r * nout + c] - mean[c]) * istd[c] : 0.f;
-}
-// loss partial sums per tile and the output gradient dL/dY = 2 (Y - Yt) / (batch * nout),
-// in FP32, BF16 and transposed BF16; grid (nout_pad/32, batch/32), one partial per block
-__global__ void __launch_bounds__(256) k_loss_dy(const float* Y, const float* Yt, int nout, int nout_pad, int batch,
-                                                 float* d32, bf16* db, bf16* dbt, float* part) {
-  __shared__ bf16 t[32][34];
-  __shared__ float sh[256];
-  const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
-  const float scale = 2.f / (float)((double)batch * nout);
-  float l = 0.f;
-  for (int j = threadIdx.y; j < 32; j += 8) {
-    const size_t i = (size_t)(r0 + j) * nout_pad + c;
-    float d = 0.f;
-    if (c < nout) {
-      const float e = Y[i] - Yt[i];
-      l += e * e;
-      d = e * scale;
-    }
-    d32[i] = d;
-    const bf16 b = __float2bfloat16_rn(d);
-    db[i] = b;
-    t[j][threadIdx.x] = b;
-  }
+// the loss's partial sums, one per 32 x 32 tile, and the output gradient dL/dY = 2 (Y - Yt) / (batch *
+// nout) in BF16 and transposed BF16, with its column sums over the block's 128 rows (the output layer's
+// bias gradient): chains of every eighth row, then the chains; Yt the standardised targets, row r of
+// them row idx[r] of y where idx is given; grid (nout_pad/32, batch/128)
+__global__ void __launch_bounds__(256) k_loss_dy(const float* Y, const float* __restrict__ y,
+                                                 const long long* __restrict__ idx, const float* mean,
+                                                 const float* istd, int nout, int nout_pad, int batch, bf16* db,
+                                                 bf16* dbt, float* part, float* colsum) {
+  __shared__ bf16 t[128][34];
+  __shared__ float sh[4][256];
+  const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 128;
   const int tid = threadIdx.y * 32 + threadIdx.x;
-  sh[tid] = l;
+  const float scale = 2.f / (float)((double)batch * nout);
+  const bool col = c < nout;
+  const float mu = col ? mean[c] : 0.f, is = col ? istd[c] : 0.f;
+  float s = 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float l = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = 32 * q + 8 * k + threadIdx.y;
+      const size_t i = (size_t)(r0 + j) * nout_pad + c;
+      float d = 0.f;
+      if (col) {
+        const float yt = __fmul_rn(y[(size_t)(idx ? idx[r0 + j] : r0 + j) * nout + c] - mu, is);
+        const float e = __fsub_rn(Y[i], yt);
+        l += e * e;
+        d = __fmul_rn(e, scale);
+      }
+      s = __fadd_rn(s, d);
+      const bf16 b = __float2bfloat16_rn(d);
+      db[i] = b;
+      t[j][threadIdx.x] = b;
+    }
+    sh[q][tid] = l;
+  }
   __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += 8)
-    dbt[(size_t)(blockIdx.x * 32 + j) * batch + r0 + threadIdx.x] = t[threadIdx.x][j];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {  // 32 columns x 128 rows: a warp writes 32 rows of a column
+    const int e = 8 * k + threadIdx.y, r = 32 * (e & 3) + threadIdx.x;
+    dbt[(size_t)(blockIdx.x * 32 + (e >> 2)) * batch + r0 + r] = t[r][e >> 2];
+  }
   for (int w = 128; w > 0; w >>= 1) {
-    if (tid < w) sh[tid] += sh[tid + w];
+    if (tid < w)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sh[q][tid] += sh[q][tid + w];
     __syncthreads();
   }
-  if (tid == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = sh[0];
-}
-// deterministic column sums of a rows x cols matrix in two passes: partial sums of 32
-// columns over one chunk of rows per block (grid (cols/32, chunks), warps read rows), then
-// the chunks' partials summed in order
-__global__ void __launch_bounds__(256) k_colsum_part(const float* a, int rows, int cols, float* part) {
-  __shared__ float sh[8][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  const int per = rows / gridDim.y, r0 = blockIdx.y * per;
-  float s = 0.f;
-  for (int r = r0 + threadIdx.y; r < r0 + per; r += 8) s += a[(size_t)r * cols + c];
-  sh[threadIdx.y][threadIdx.x] = s;
+  if (tid < 4) part[(4 * blockIdx.y + tid) * gridDim.x + blockIdx.x] = sh[tid][0];
+  __syncthreads();
+  sh[0][tid] = s;
   __syncthreads();
   if (threadIdx.y == 0) {
-    float t = sh[0][threadIdx.x];
-    for (int k = 1; k < 8; ++k) t += sh[k][threadIdx.x];
-    part[(size_t)blockIdx.y * cols + c] = t;
+    float a = sh[0][threadIdx.x];
+    for (int k = 1; k < 8; ++k) a += sh[0][32 * k + threadIdx.x];
+    colsum[(size_t)blockIdx.y * nout_pad + c] = a;
   }
 }
-__global__ void k_colsum_fin(const float* part, int chunks, int cols, float* out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int k = 0; k < chunks; ++k) s += part[(size_t)k * cols + c];
-  out[c] = s;
+
+// one Adam update
+struct Adam {
+  float lr, b1, b2, c1, c2, eps;
+};
+__device__ __forceinline__ float adam_at(const Adam& A, float gi, float* p, float* m, float* v) {
+  const float mi = A.b1 * *m + (1.f - A.b1) * gi;
+  const float vi = A.b2 * *v + (1.f - A.b2) * gi * gi;
+  *m = mi;
+  *v = vi;
+  const float pi = *p - A.lr * (mi * A.c1) / (sqrtf(vi * A.c2) + A.eps);
+  *p = pi;
+  return pi;
 }
-// split-K partials of dW^T (in x out) summed and written transposed as dW (out x in)
-__global__ void k_splitk_reduce_t(const float* part, int splits, int rows_in, int cols_out, float* gw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows_in * cols_out) return;
-  const int r = i / cols_out, c = i % cols_out;
+// a layer's parameters: weights W (out x in), their BF16 copies (row-major and transposed), biases
+struct Layer {
+  float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb;
+  bf16 *wb, *wtb;
+};
+// the gradient of a layer and (ADAM) its update: the split-K partials of dW^T (in x out) summed in order,
+// a 32 x 32 tile per block that is read along the outputs and written along the inputs; the blocks of
+// the last row sum the bias gradient's partials.  One pass over the partials bounds it: 32 MB for a
+// 512 x 512 layer, which are still in L2.  grid (out/32, in/32 + 1)
+template <bool ADAM>
+__global__ void __launch_bounds__(1024) k_update(const float* part, int splits, int nin, int nout, const float* colsum,
+                                                 int chunks, Layer L, Adam A) {
+  __shared__ float t[32][33];
+  __shared__ bf16 tb[32][34];
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  if (blockIdx.y == gridDim.y - 1) {
+    if (threadIdx.y > 0) return;
+    float s = 0.f;
+#pragma unroll 16
+    for (int k = 0; k < chunks; ++k) s += colsum[(size_t)k * nout + c];
+    L.gb[c] = s;
+    if constexpr (ADAM) adam_at(A, s, L.b + c, L.mb + c, L.vb + c);
+    return;
+  }
+  const int r0 = blockIdx.y * 32;
+  const float* q = part + (size_t)(r0 + threadIdx.y) * nout + c;
+  const size_t n = (size_t)nin * nout;
   float s = 0.f;
-  for (int z = 0; z < splits; ++z) s += part[(size_t)z * rows_in * cols_out + i];
-  gw[(size_t)c * rows_in + r] = s;
-}
-__global__ void k_splitk_reduce(const float* part, int splits, long long n, float* out) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int z = 0; z < splits; ++z) s += part[(size_t)z * n + i];
-  out[i] = s;
-}
-// Adam update of one parameter matrix (rows x cols) and its BF16 copies (row-major, transposed)
-__global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, int cols, float lr, float b1, float b2,
-                       float c1, float c2, float eps, bf16* pb, bf16* pbt, int rows) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  p[i] = pi;
-  if (pb) {
-    const bf16 b = __float2bfloat16_rn(pi);
-    pb[i] = b;
-    const long long r = i / cols, c = i % cols;
-    pbt[(size_t)c * rows + r] = b;
+#pragma unroll 16
+  for (int z = 0; z < splits; ++z) s += q[z * n];
+  t[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  const size_t i = (size_t)(blockIdx.x * 32 + threadIdx.y) * nin + r0 + threadIdx.x;
+  const float g = t[threadIdx.x][threadIdx.y];
+  L.gw[i] = g;
+  if constexpr (ADAM) {
+    const bf16 b = __float2bfloat16_rn(adam_at(A, g, L.w + i, L.mw + i, L.vw + i));
+    L.wb[i] = b;
+    tb[threadIdx.y][threadIdx.x] = b;
+    __syncthreads();
+    L.wtb[(size_t)(r0 + threadIdx.y) * nout + c] = tb[threadIdx.x][threadIdx.y];
   }
 }
 __global__ void k_to_bf16_t(const float* p, long long n, int cols, int rows, bf16* pb, bf16* pbt) {
@@ -685,16 +743,11 @@ __global__ void k_denorm(const float* Y, int nout, int nout_pad, int batch, cons
   const int r = i / nout, c = i % nout;
   y[i] = Y[(size_t)r * nout_pad + c] * std_[c] + mean[c];
 }
-__global__ void k_gather_rows(const float* src, const long long* idx, int batch, int ncol, float* dst) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)batch * ncol) return;
-  const long long r = i / ncol, c = i % ncol;
-  dst[i] = src[idx[r] * ncol + c];
-}
-
-// the loss partials of one batch summed in FP64 into out[0] (one block of 256 threads),
-// so that an epoch keeps every batch's loss on the device until its end
+// the loss partials of the batches (n each) summed in FP64 into out, a block of 256 threads per batch:
+// an epoch keeps every batch's loss on the device until its end
 __global__ void k_loss_total(const float* part, int n, double* out) {
+  part += (size_t)blockIdx.x * n;
+  out += blockIdx.x;
   __shared__ double sh[256];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -726,7 +779,7 @@ struct lgame_emu {
   float *W[4], *b[4], *gW[4], *gb[4], *mW[4], *vW[4], *mb[4], *vb[4];
   bf16 *Wb[4], *WTb[4];
   float *xmean, *xistd, *ymean, *ystd, *yistd;
-  float *xraw, *yraw, *Yt, *Y, *Z[3], *dZ32[4], *part, *lpart, *cpart, *yout;
+  float *xraw, *yraw, *Y, *Z[3], *part, *lpart, *cpart[2], *yout;
   bf16 *X, *XT, *H[3], *HT[3], *dZb[4], *dZT[4];
   int* err = nullptr;
   long long adam_t = 0;
@@ -736,6 +789,7 @@ struct lgame_emu {
   long long dsn = 0;
   long long* idx = nullptr;  // one epoch's shuffled order (dsn entries)
   double* lsum = nullptr;    // per-batch loss sums of one epoch (dsn / 128 entries)
+  float* lparts = nullptr;   // and their partials
   // statistics
   long long gemm_launches = 0;
   double gemm_flop = 0.0;
@@ -811,22 +865,22 @@ int forward(lgame_emu* e, int batch, bool infer = false) {
 
 // prepared inputs of `batch` rows (a multiple of 128) from raw rows the GPU can read (device
 // memory or page-locked host memory), of which the first `valid` hold data
-int prep_x(lgame_emu* e, const float* xraw_dev, int batch, int valid, bool infer = false) {
-  k_prep_x<<<dim3(e->nin_pad / 32, batch / 32), dim3(32, 8), 0, e->st>>>(xraw_dev, e->nin, e->nin_pad, batch, valid,
-                                                                        e->xmean, e->xistd, e->X,
+int prep_x(lgame_emu* e, const float* xraw_dev, int batch, int valid, bool infer = false, const long long* idx = nullptr) {
+  k_prep_x<<<dim3(e->nin_pad / 32, batch / 32), dim3(32, 8), 0, e->st>>>(xraw_dev, idx, e->nin, e->nin_pad, batch,
+                                                                        valid, e->xmean, e->xistd, e->X,
                                                                         infer ? nullptr : e->XT);
   ECK(cudaGetLastError());
   return LGAME_OK;
 }
 
-// loss and gradients of one prepared batch (X, XT, Yt); grads in gW, gb; loss partials in lpart
-int backward(lgame_emu* e, int batch, int* nparts) {
+// loss and gradients of one prepared batch (X, XT) and its raw targets y (row r: row idx[r] where idx is
+// given); loss partials in lpart, grads in gW, gb; with A the parameters are updated layer by layer, each
+// after the product that reads its weights
+int backward(lgame_emu* e, int batch, const float* y, const long long* idx, float* lpart, const Adam* A) {
   const int Hd = e->hidden, no = e->nout_pad;
-  const int np = (no / 32) * (batch / 32);
-  k_loss_dy<<<dim3(no / 32, batch / 32), dim3(32, 8), 0, e->st>>>(e->Y, e->Yt, e->nout, no, batch, e->dZ32[3], e->dZb[3],
-                                                                  e->dZT[3], e->lpart);
+  k_loss_dy<<<dim3(no / 32, batch / 128), dim3(32, 8), 0, e->st>>>(e->Y, y, idx, e->ymean, e->yistd, e->nout, no, batch,
+                                                                   e->dZb[3], e->dZT[3], lpart, e->cpart[1]);
   ECK(cudaGetLastError());
-  *nparts = np;
   for (int l = 3; l >= 0; --l) {
     // dW_l^T (in x out) = act_{l-1}^T (in x batch) * dZ_l^T (out x batch)^T, split over the batch
     const bf16* actT = (l == 0) ? e->XT : e->HT[l - 1];
@@ -841,43 +895,37 @@ int backward(lgame_emu* e, int batch, int* nparts) {
     if (rc) return rc;
     const int kchunk = ((batch / splits + 63) / 64) * 64;
     const int zs = (batch + kchunk - 1) / kchunk;
-    k_splitk_reduce_t<<<blocks((long long)nin_l * nout_l), 256, 0, e->st>>>(e->part, zs, nin_l, nout_l, e->gW[l]);
+    if (l > 0) {
+      // dZ_{l-1} = (dZ_l * W_l) .* gelu'(Z_{l-1}): A = dZ_l (batch x out), B = W_l^T (in x out)
+      Epi eb{};
+      eb.kind = kEpiGeluBwd;
+      eb.zprev = e->Z[l - 1];
+      eb.colsum = e->cpart[(l - 1) & 1];
+      eb.h = e->dZb[l - 1];
+      eb.ldh = Hd;
+      eb.ht = e->dZT[l - 1];
+      eb.ldt = batch;
+      rc = gemm(e, e->dZb[l], nout_l, e->WTb[l], nout_l, batch, Hd, nout_l, 1, eb);
+      if (rc) return rc;
+    }
+    const Layer L{e->W[l], e->gW[l], e->mW[l], e->vW[l], e->b[l], e->gb[l], e->mb[l], e->vb[l], e->Wb[l], e->WTb[l]};
+    const dim3 g(nout_l / 32, nin_l / 32 + 1), t(32, 32);
+    if (A) k_update<true><<<g, t, 0, e->st>>>(e->part, zs, nin_l, nout_l, e->cpart[l & 1], batch / 128, L, *A);
+    else k_update<false><<<g, t, 0, e->st>>>(e->part, zs, nin_l, nout_l, e->cpart[l & 1], batch / 128, L, Adam{});
     ECK(cudaGetLastError());
-    const int chunks = batch / 128;  // rows per chunk: 128
-    k_colsum_part<<<dim3(nout_l / 32, chunks), dim3(32, 8), 0, e->st>>>(e->dZ32[l], batch, nout_l, e->cpart);
-    k_colsum_fin<<<blocks(nout_l), 256, 0, e->st>>>(e->cpart, chunks, nout_l, e->gb[l]);
-    ECK(cudaGetLastError());
-    if (l == 0) break;
-    // dZ_{l-1} = (dZ_l * W_l) .* gelu'(Z_{l-1}): A = dZ_l (batch x out), B = W_l^T (in x out)
-    Epi eb{};
-    eb.kind = kEpiGeluBwd;
-    eb.zprev = e->Z[l - 1];
-    eb.c = e->dZ32[l - 1];
-    eb.ldc = Hd;
-    eb.h = e->dZb[l - 1];
-    eb.ldh = Hd;
-    eb.ht = e->dZT[l - 1];
-    eb.ldt = batch;
-    rc = gemm(e, e->dZb[l], nout_l, e->WTb[l], nout_l, batch, Hd, nout_l, 1, eb);
-    if (rc) return rc;
   }
   return LGAME_OK;
 }
 
-int adam(lgame_emu* e, float lr) {
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+// loss partials of a batch
+int loss_parts(const lgame_emu* e, int batch) { return (e->nout_pad / 32) * (batch / 32); }
+
+// the next Adam step's factors
+Adam adam(lgame_emu* e, float lr) {
   e->adam_t++;
   const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)e->adam_t)));
   const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)e->adam_t)));
-  for (int l = 0; l < 4; ++l) {
-    const long long n = (long long)e->rows[l] * e->cols[l];
-    k_adam<<<blocks(n), 256, 0, e->st>>>(e->W[l], e->gW[l], e->mW[l], e->vW[l], n, e->cols[l], lr, b1, b2, c1, c2, eps,
-                                         e->Wb[l], e->WTb[l], e->rows[l]);
-    k_adam<<<blocks(e->rows[l]), 256, 0, e->st>>>(e->b[l], e->gb[l], e->mb[l], e->vb[l], e->rows[l], 1, lr, b1, b2, c1,
-                                                  c2, eps, nullptr, nullptr, 1);
-    ECK(cudaGetLastError());
-  }
-  return LGAME_OK;
+  return Adam{lr, 0.9f, 0.999f, c1, c2, 1e-8f};
 }
 
 int loss_from_parts(lgame_emu* e, int nparts, int batch, float* loss) {
@@ -894,12 +942,7 @@ int upload_batch(lgame_emu* e, const float* x, const float* y, int batch) {
   ECK(cudaMemcpyAsync(e->xraw, x, sizeof(float) * (size_t)batch * e->nin, cudaMemcpyHostToDevice, e->st));
   int rc = prep_x(e, e->xraw, batch, batch);
   if (rc) return rc;
-  if (y) {
-    ECK(cudaMemcpyAsync(e->yraw, y, sizeof(float) * (size_t)batch * e->nout, cudaMemcpyHostToDevice, e->st));
-    k_prep_y<<<blocks((long long)batch * e->nout_pad), 256, 0, e->st>>>(e->yraw, e->nout, e->nout_pad, batch, e->ymean,
-                                                                         e->yistd, e->Yt);
-    ECK(cudaGetLastError());
-  }
+  if (y) ECK(cudaMemcpyAsync(e->yraw, y, sizeof(float) * (size_t)batch * e->nout, cudaMemcpyHostToDevice, e->st));
   return LGAME_OK;
 }
 
@@ -980,7 +1023,7 @@ extern "C" int lgame_emu_create(int nlev, int hidden, int batch_max, unsigned lo
   if ((rc = ealloc(e, &e->xmean, e->nin)) || (rc = ealloc(e, &e->xistd, e->nin)) || (rc = ealloc(e, &e->ymean, e->nout)) ||
       (rc = ealloc(e, &e->ystd, e->nout)) || (rc = ealloc(e, &e->yistd, e->nout)) ||
       (rc = ealloc(e, &e->xraw, B * e->nin)) || (rc = ealloc(e, &e->yraw, B * e->nout)) ||
-      (rc = ealloc(e, &e->Yt, B * e->nout_pad)) || (rc = ealloc(e, &e->Y, B * e->nout_pad)) ||
+      (rc = ealloc(e, &e->Y, B * e->nout_pad)) ||
       (rc = ealloc(e, &e->X, B * e->nin_pad)) || (rc = ealloc(e, &e->XT, B * e->nin_pad)) ||
       (rc = ealloc(e, &e->yout, B * e->nout)) || (rc = ealloc(e, &e->err, 1)))
     return fail(rc);
@@ -989,13 +1032,14 @@ extern "C" int lgame_emu_create(int nlev, int hidden, int batch_max, unsigned lo
       return fail(rc);
   for (int l = 0; l < 4; ++l) {
     const size_t w = (l == 3) ? e->nout_pad : Hd;
-    if ((rc = ealloc(e, &e->dZ32[l], B * w)) || (rc = ealloc(e, &e->dZb[l], B * w)) || (rc = ealloc(e, &e->dZT[l], B * w)))
+    if ((rc = ealloc(e, &e->dZb[l], B * w)) || (rc = ealloc(e, &e->dZT[l], B * w)))
       return fail(rc);
   }
   size_t pmax = 0;
   for (int l = 0; l < 4; ++l) pmax = std::max(pmax, (size_t)rows[l] * cols[l]);
   if ((rc = ealloc(e, &e->part, pmax * e->splits)) || (rc = ealloc(e, &e->lpart, B * e->nout_pad / 256 + 1)) ||
-      (rc = ealloc(e, &e->cpart, (B / 128) * std::max((size_t)Hd, (size_t)e->nout_pad))))
+      (rc = ealloc(e, &e->cpart[0], (B / 128) * std::max((size_t)Hd, (size_t)e->nout_pad))) ||
+      (rc = ealloc(e, &e->cpart[1], (B / 128) * std::max((size_t)Hd, (size_t)e->nout_pad))))
     return fail(rc);
   // identity normalisation, Xavier-uniform weights (splitmix64), zero biases
   std::vector<float> one(std::max(e->nin, e->nout), 1.f);
@@ -1033,6 +1077,7 @@ extern "C" void lgame_emu_destroy(lgame_emu* e) {
   if (e->dsy) cudaFree(e->dsy);
   if (e->idx) cudaFree(e->idx);
   if (e->lsum) cudaFree(e->lsum);
+  if (e->lparts) cudaFree(e->lparts);
   if (e->st) cudaStreamDestroy(e->st);
   delete e;
 }
@@ -1107,9 +1152,8 @@ extern "C" int lgame_emu_loss_grad(lgame_emu* e, const float* x, const float* y,
     return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_loss_grad: bad arguments (batch a multiple of 128 <= batch_max)");
   int rc = upload_batch(e, x, y, batch);
   if (!rc) rc = forward(e, batch);
-  int np = 0;
-  if (!rc) rc = backward(e, batch, &np);
-  if (!rc) rc = loss_from_parts(e, np, batch, loss);
+  if (!rc) rc = backward(e, batch, e->yraw, nullptr, e->lpart, nullptr);
+  if (!rc) rc = loss_from_parts(e, loss_parts(e, batch), batch, loss);
   if (!rc) rc = check_err(e);
   if (rc) return rc;
   if (grads) {
@@ -1132,10 +1176,11 @@ extern "C" int lgame_emu_train_step(lgame_emu* e, const float* x, const float* y
     return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_train_step: bad arguments");
   int rc = upload_batch(e, x, y, batch);
   if (!rc) rc = forward(e, batch);
-  int np = 0;
-  if (!rc) rc = backward(e, batch, &np);
-  if (!rc) rc = adam(e, lr);
-  if (!rc) rc = loss_from_parts(e, np, batch, loss);
+  if (!rc) {
+    const Adam A = adam(e, lr);
+    rc = backward(e, batch, e->yraw, nullptr, e->lpart, &A);
+  }
+  if (!rc) rc = loss_from_parts(e, loss_parts(e, batch), batch, loss);
   if (!rc) rc = check_err(e);
   return rc;
 }
@@ -1146,13 +1191,16 @@ extern "C" int lgame_emu_set_dataset(lgame_emu* e, const float* x, const float* 
   if (e->dsy) cudaFree(e->dsy);
   if (e->idx) cudaFree(e->idx);
   if (e->lsum) cudaFree(e->lsum);
+  if (e->lparts) cudaFree(e->lparts);
   e->dsx = e->dsy = nullptr;
   e->idx = nullptr;
   e->lsum = nullptr;
+  e->lparts = nullptr;
   ECK(cudaMalloc(&e->dsx, sizeof(float) * (size_t)n * e->nin));
   ECK(cudaMalloc(&e->dsy, sizeof(float) * (size_t)n * e->nout));
   ECK(cudaMalloc(&e->idx, sizeof(long long) * (size_t)n));
   ECK(cudaMalloc(&e->lsum, sizeof(double) * (size_t)(n / 128 + 1)));
+  ECK(cudaMalloc(&e->lparts, sizeof(float) * (size_t)(n / 32 + 1) * (e->nout_pad / 32)));
   ECK(cudaMemcpy(e->dsx, x, sizeof(float) * (size_t)n * e->nin, cudaMemcpyHostToDevice));
   ECK(cudaMemcpy(e->dsy, y, sizeof(float) * (size_t)n * e->nout, cudaMemcpyHostToDevice));
   e->dsn = n;
@@ -1178,21 +1226,19 @@ extern "C" int lgame_emu_train_epoch(lgame_emu* e, int batch, float lr, unsigned
   // the whole order goes up once and every batch's loss stays on the device: the batches are
   // enqueued back to back with one synchronisation at the end of the epoch
   ECK(cudaMemcpyAsync(e->idx, perm.data(), sizeof(long long) * (size_t)e->dsn, cudaMemcpyHostToDevice, e->st));
+  const int np = loss_parts(e, batch);
   for (long long k = 0; k < nb; ++k) {
     const long long* idx = e->idx + k * batch;
-    k_gather_rows<<<blocks((long long)batch * e->nin), 256, 0, e->st>>>(e->dsx, idx, batch, e->nin, e->xraw);
-    k_gather_rows<<<blocks((long long)batch * e->nout), 256, 0, e->st>>>(e->dsy, idx, batch, e->nout, e->yraw);
-    ECK(cudaGetLastError());
-    int rc = prep_x(e, e->xraw, batch, batch);
+    int rc = prep_x(e, e->dsx, batch, batch, false, idx);
+    if (!rc) rc = forward(e, batch);
+    if (!rc) {
+      const Adam A = adam(e, lr);
+      rc = backward(e, batch, e->dsy, idx, e->lparts + (size_t)k * np, &A);
+    }
     if (rc) return rc;
-    k_prep_y<<<blocks((long long)batch * e->nout_pad), 256, 0, e->st>>>(e->yraw, e->nout, e->nout_pad, batch, e->ymean,
-                                                                         e->yistd, e->Yt);
-    rc = forward(e, batch);
-    int np = 0;
-    if (!rc) rc = backward(e, batch, &np);
-    if (!rc) rc = adam(e, lr);
-    if (rc) return rc;
-    k_loss_total<<<1, 256, 0, e->st>>>(e->lpart, np, e->lsum + k);
+  }
+  if (nb) {
+    k_loss_total<<<(unsigned)nb, 256, 0, e->st>>>(e->lparts, np, e->lsum);
     ECK(cudaGetLastError());
   }
   std::vector<double> ls((size_t)nb);

@@ -14,7 +14,8 @@ enum EpiKind { kEpiF32 = 0, kEpiBias = 1, kEpiBiasGelu = 2, kEpiGeluBwd = 3, kEp
 //   kEpiF32      c[z*split_stride + m*ldc + n] = acc               (split-K partials)
 //   kEpiBias     c[m*ldc + n] = acc + bias[n]
 //   kEpiBiasGelu c[m*ldc + n] = z = acc + bias[n]; h[m*ldh + n] = ht[n*ldt + m] = bf16(gelu(z))
-//   kEpiGeluBwd  c[m*ldc + n] = d = acc * gelu'(zprev[m*ldc + n]); h, ht = bf16(d)
+//   kEpiGeluBwd  d = acc * gelu'(zprev[m*ldh + n]); h, ht = bf16(d); colsum[(m/128)*ldh + n] = the sum
+//                of d over the tile's 128 rows
 //   kEpiBiasGeluH h[m*ldh + n] = bf16(gelu(acc + bias[n])) alone (inference)
 struct Epi {
   int kind;
@@ -27,6 +28,7 @@ struct Epi {
   int ldh;
   __nv_bfloat16* ht;
   int ldt;
+  float* colsum;
 };
 
 // heating rates (device, n x nout) of n rows of raw features (device, n x nin)

@@ -45,6 +45,8 @@ int set_err(int code, const std::string& msg) {
 // longitude per column, the feature rows and the heating rates of every column
 struct RadBuffers {
   double *albedo = nullptr, *lat = nullptr, *lon = nullptr;
+  double* o3 = nullptr;     // ozone density over the dry air's
+  bool o3_set = false;      // of the grid now set
   float *features = nullptr, *heating = nullptr;
   long long ncol = 0;
   int nlev = 0;
@@ -1142,6 +1144,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
   }
   CK(cudaStreamSynchronize(c->stream));
   c->grid_set = true;
+  c->radbuf.o3_set = false;
   return LGAME_OK;
 }
 
@@ -1858,61 +1861,110 @@ namespace {
 
 
 // coszenith, mo_rterrtmgp_coupler.F90:550-629 (the sun's direction from the Earth's rotation
-// and revolution relative to the winter solstice 2019-12-20 12:00 UTC), 0 at night
-__device__ double coszenith(double lat, double lon, double t) {
+// and revolution relative to the winter solstice 2019-12-20 12:00 UTC), 0 at night.  Sun: what
+// depends on the time alone
+struct Sun {
+  double cos_rot, sin_rot, cos_rev, sin_rev, cos_ob, sin_ob;
+};
+Sun sun_at(double t) {
   const double omega = 7.292115e-5, omega_rev = 1.99099e-7, obliquity = 0.409092592843564;
   const double tt = t - 1576843200.0;
   const double rot = omega * tt;
+  return Sun{cos(rot), sin(rot), cos(omega_rev * tt), sin(omega_rev * tt), cos(obliquity), sin(obliquity)};
+}
+__device__ double coszenith(const Sun& s, double lat, double lon) {
   const double n1 = cos(lat) * cos(lon), n2 = cos(lat) * sin(lon), n3 = sin(lat);
-  const double s1 = -cos(rot) * cos(obliquity) * n1 + sin(rot) * cos(obliquity) * n2 + sin(obliquity) * n3;
-  const double s2 = -sin(rot) * n1 - cos(rot) * n2;
-  const double s3 = cos(rot) * sin(obliquity) * n1 - sin(rot) * sin(obliquity) * n2 + cos(obliquity) * n3;
-  (void)s3;
-  const double c = -(s1 * cos(omega_rev * tt) + s2 * sin(omega_rev * tt));
+  const double s1 = -s.cos_rot * s.cos_ob * n1 + s.sin_rot * s.cos_ob * n2 + s.sin_ob * n3;
+  const double s2 = -s.sin_rot * n1 - s.cos_rot * n2;
+  const double c = -(s1 * s.cos_rev + s2 * s.sin_rev);
   return c < 0.0 ? 0.0 : c;
 }
 
-// one thread per column: T, dry-air pressure, vapour and ozone densities of every layer,
-// albedo and cos(zenith); column index ji + ny*(jk-1), 4*nl+2 floats per column
-__global__ void k_rad_features(Dims D, Grid<double> G, State S, const double* albedo, const double* lat,
-                               const double* lon, double t, float* X) {
-  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+// the ozone density over the dry air's, of the grid alone: the volume mixing ratio (calc_o3_vmr: FWHM
+// 20 km, maximum 8.5e-6 at 34 km) times the molar masses' ratio
+__global__ void k_rad_ozone(Dims D, Grid<double> G, double* o3) {
+  LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
-  const long long col = (ji - 1) + (long long)D.ny * (jk - 1);
-  const int nl = D.nl, nf = 4 * nl + 2;
-  float* x = X + col * nf;
-  const double sigma = 20e3 / sqrt(8.0 * log(2.0));  // calc_o3_vmr: FWHM 20 km, maximum 8.5e-6 at 34 km
-  const double m_o3 = 0.0479982;                       // kg/mol
-  for (int jl = 1; jl <= nl; ++jl) {
-    const long long i = IX(D, ji, jk, jl);
-    const double rd = S.rho[i + (long long)(D.g - 1) * D.fstride];
-    const double rv = D.lmoist ? S.rho[i + (long long)D.g * D.fstride] : 0.0;
-    double T = (G.theta_v_bg[i] + S.tp[i]) * (G.exner_bg[i] + S.ep[i]);  // temperature_diagnostics
-    if (D.lmoist) T = T / (1.0 + rv / rd * (kM_D / kM_V - 1.0));
-    const double dz = G.z_scalar[i] - 34e3;
-    const double vmr = 8.5e-6 * exp(-dz * dz / (2.0 * sigma * sigma));
-    x[jl - 1] = (float)T;
-    x[nl + jl - 1] = (float)(kR_D * rd * T);
-    x[2 * nl + jl - 1] = (float)rv;
-    x[3 * nl + jl - 1] = (float)(vmr * rd * m_o3 / kM_D);
-  }
-  x[4 * nl] = (float)albedo[col];
-  x[4 * nl + 1] = (float)coszenith(lat[col], lon[col], t);
+  const long long i = IX(D, ji, jk, jl);
+  const double sigma = 20e3 / sqrt(8.0 * log(2.0));
+  const double dz = G.z_scalar[i] - 34e3;
+  const double m_o3 = 0.0479982;  // kg/mol
+  o3[i] = 8.5e-6 * exp(-dz * dz / (2.0 * sigma * sigma)) * m_o3 / kM_D;
 }
 
-// radiation_tendency (W m^-3) = (shortwave + longwave heating rate)/86400 * rho_gas * c_d_p
-__global__ void k_rad_apply(Dims D, State S, const float* heat, double* rad, float* rad_f) {
-  LG_IDX3;
-  if (ji > D.ny || jk > D.nx || jl > D.nl) return;
-  const long long col = (ji - 1) + (long long)D.ny * (jk - 1);
-  const long long i = IX(D, ji, jk, jl);
-  const float hr = heat[col * 2 * D.nl + (jl - 1)] + heat[col * 2 * D.nl + D.nl + (jl - 1)];
-  double rho = S.rho[i + (long long)(D.g - 1) * D.fstride];
-  if (D.lmoist) rho += S.rho[i + (long long)D.g * D.fstride];
-  const double q = (double)hr / 86400.0 * rho * kC_D_P;
-  rad[i] = q;
-  if (rad_f) rad_f[i] = (float)q;
+// a quotient whose numerator may be infinite or NaN, as the hardware gives it
+__device__ __forceinline__ F64 quot_any(F64 a, F64 b, F64 y) {
+  if (((unsigned)__double2hiint(a.v) & 0x7FF00000u) == 0x7FF00000u) return a.v / b.v;
+  return div_rn(a, b, y);
+}
+
+// T, dry-air pressure, vapour and ozone densities of every layer, albedo and cos(zenith); column index
+// ji + ny*(jk-1), 4*nl+2 floats per column.  A block takes 32 columns and 32 layers: the state is read
+// along ji, and the features go out along the layers, through shared memory.  (One thread per column
+// wrote single floats 1288 bytes apart and formed the ozone's exp and four quotients a cell on the FP64
+// pipe: 821 us at 256x256x80, here 135 us.)
+constexpr int kRadTile = 32;
+__global__ void __launch_bounds__(256) k_rad_features(Dims D, Grid<F64> G, StateT<F64> S, const F64* o3,
+                                                      const double* albedo, const double* lat, const double* lon,
+                                                      Sun sun, float* X) {
+  __shared__ float tile[4][kRadTile][kRadTile + 1];
+  const int ji = blockIdx.y * kRadTile + threadIdx.x + 1, jk = blockIdx.x + 1, l0 = blockIdx.z * kRadTile;
+  const int nl = D.nl, nf = 4 * nl + 2;
+  if (ji <= D.ny) {
+#pragma unroll
+    for (int r = 0; r < kRadTile / 8; ++r) {
+      const int k = threadIdx.y + 8 * r;
+      if (l0 + k >= nl) break;
+      const long long i = IX(D, ji, jk, l0 + k + 1);
+      const F64 rd = S.rho[i + (long long)(D.g - 1) * D.fstride];
+      const F64 rv = D.lmoist ? S.rho[i + (long long)D.g * D.fstride] : F64(0.0);
+      F64 T = (G.theta_v_bg[i] + S.tp[i]) * (G.exner_bg[i] + S.ep[i]);  // temperature_diagnostics
+      if (D.lmoist) {  // T/(1 + rv/rd*(M_d/M_v - 1)) in one quotient
+        const F64 f = rd + rv * (kM_D / kM_V - 1.0);
+        T = quot_any(T * rd, f, rcp_near(f));
+      }
+      tile[0][k][threadIdx.x] = narrow(T.v);
+      tile[1][k][threadIdx.x] = narrow((kR_D * rd * T).v);
+      tile[2][k][threadIdx.x] = narrow(rv.v);
+      tile[3][k][threadIdx.x] = narrow((o3[i] * rd).v);
+    }
+    if (l0 == 0 && threadIdx.y == 7) {
+      const long long col = (ji - 1) + (long long)D.ny * (jk - 1);
+      X[col * nf + 4 * nl] = (float)albedo[col];
+      X[col * nf + 4 * nl + 1] = (float)coszenith(sun, lat[col], lon[col]);
+    }
+  }
+  __syncthreads();
+  const int ncol = min(kRadTile, D.ny - (int)blockIdx.y * kRadTile);
+  float* x = X + ((long long)blockIdx.y * kRadTile + (long long)D.ny * (jk - 1)) * nf + l0 + threadIdx.x;
+  if (l0 + (int)threadIdx.x < nl)
+    for (int r = threadIdx.y; r < 4 * ncol; r += 8) x[(long long)(r >> 2) * nf + (r & 3) * nl] = tile[r & 3][threadIdx.x][r >> 2];
+}
+
+// radiation_tendency (W m^-3) = (shortwave + longwave heating rate)/86400 * rho_gas * c_d_p, in the
+// same blocks with the heating rates read along the layers (118 us with a thread per cell that read
+// them 640 bytes apart, at 256x256x80)
+__global__ void __launch_bounds__(256) k_rad_apply(Dims D, StateT<F64> S, const float* heat, double* rad, float* rad_f) {
+  __shared__ float tile[kRadTile][kRadTile + 1];
+  const int ji = blockIdx.y * kRadTile + threadIdx.x + 1, jk = blockIdx.x + 1, l0 = blockIdx.z * kRadTile;
+  const int nl = D.nl, ncol = min(kRadTile, D.ny - (int)blockIdx.y * kRadTile);
+  const float* h = heat + ((long long)blockIdx.y * kRadTile + (long long)D.ny * (jk - 1)) * 2 * nl + l0 + threadIdx.x;
+  if (l0 + (int)threadIdx.x < nl)
+    for (int r = threadIdx.y; r < ncol; r += 8)
+      tile[threadIdx.x][r] = h[(long long)r * 2 * nl] + h[(long long)r * 2 * nl + nl];
+  __syncthreads();
+  if (ji > D.ny) return;
+#pragma unroll
+  for (int r = 0; r < kRadTile / 8; ++r) {
+    const int k = threadIdx.y + 8 * r;
+    if (l0 + k >= nl) break;
+    const long long i = IX(D, ji, jk, l0 + k + 1);
+    F64 rho = S.rho[i + (long long)(D.g - 1) * D.fstride];
+    if (D.lmoist) rho = rho + S.rho[i + (long long)D.g * D.fstride];
+    const F64 q = quot_any(wide(tile[k][threadIdx.x]), 86400.0, 1.0 / 86400.0) * rho * kC_D_P;
+    rad[i] = q.v;
+    if (rad_f) rad_f[i] = narrow(q.v);
+  }
 }
 
 // the context's radiation buffers, allocated at the first radiation call (they live and die
@@ -1927,15 +1979,17 @@ int rad_buffers(lgame_gpu* c, RadBuffers** out) {
     if (cudaMalloc(&r->albedo, sizeof(double) * r->ncol) != cudaSuccess ||
         cudaMalloc(&r->lat, sizeof(double) * r->ncol) != cudaSuccess ||
         cudaMalloc(&r->lon, sizeof(double) * r->ncol) != cudaSuccess ||
+        cudaMalloc(&r->o3, sizeof(double) * D.fstride) != cudaSuccess ||
         cudaMalloc(&r->features, sizeof(float) * r->ncol * nf) != cudaSuccess ||
         cudaMalloc(&r->heating, sizeof(float) * r->ncol * 2 * D.nl) != cudaSuccess)
       return set_err(LGAME_ERR_ALLOC, "radiation buffers: cudaMalloc failed");
     c->allocations.push_back(r->albedo);
     c->allocations.push_back(r->lat);
     c->allocations.push_back(r->lon);
+    c->allocations.push_back(r->o3);
     c->allocations.push_back(r->features);
     c->allocations.push_back(r->heating);
-    c->bytes += (long long)(sizeof(double) * 3 * r->ncol + sizeof(float) * r->ncol * (nf + 2 * D.nl));
+    c->bytes += (long long)(sizeof(double) * (3 * r->ncol + D.fstride) + sizeof(float) * r->ncol * (nf + 2 * D.nl));
     cudaMemset(r->albedo, 0, sizeof(double) * r->ncol);
     cudaMemset(r->lat, 0, sizeof(double) * r->ncol);
     cudaMemset(r->lon, 0, sizeof(double) * r->ncol);
@@ -1944,10 +1998,19 @@ int rad_buffers(lgame_gpu* c, RadBuffers** out) {
   return LGAME_OK;
 }
 
+dim3 rad_grid(const Dims& D) {
+  return dim3((unsigned)D.nx, (unsigned)((D.ny + kRadTile - 1) / kRadTile), (unsigned)((D.nl + kRadTile - 1) / kRadTile));
+}
+
 int rad_features_dev(lgame_gpu* c, RadBuffers* r, int slot, double t) {
   const Dims& D = c->D;
-  k_rad_features<<<dim3((unsigned)((D.ny + 31) / 32), (unsigned)((D.nx + 3) / 4)), dim3(32, 4), 0, c->stream>>>(
-      D, c->G, c->st[slot], r->albedo, r->lat, r->lon, t, r->features);
+  if (!r->o3_set) {
+    k_rad_ozone<<<grd(D, D.ny, D.nx, D.nl), blk(), 0, c->stream>>>(D, c->G, r->o3);
+    CK(cudaGetLastError());
+    r->o3_set = true;
+  }
+  k_rad_features<<<rad_grid(D), dim3(kRadTile, 8), 0, c->stream>>>(D, f64(c->G), f64(c->st[slot]), f64(r->o3), r->albedo,
+                                                                  r->lat, r->lon, sun_at(t), r->features);
   CK(cudaGetLastError());
   return LGAME_OK;
 }
@@ -1955,7 +2018,7 @@ int rad_features_dev(lgame_gpu* c, RadBuffers* r, int slot, double t) {
 int rad_apply_dev(lgame_gpu* c, RadBuffers* r, int slot) {
   const Dims& D = c->D;
   float* rad_f = c->split ? split_carried(c->split).rad : nullptr;
-  k_rad_apply<<<grd(D, D.ny, D.nx, D.nl), blk(), 0, c->stream>>>(D, c->st[slot], r->heating, c->rad, rad_f);
+  k_rad_apply<<<rad_grid(D), dim3(kRadTile, 8), 0, c->stream>>>(D, f64(c->st[slot]), r->heating, c->rad, rad_f);
   CK(cudaGetLastError());
   return LGAME_OK;
 }

@@ -73,3 +73,31 @@ def test_features_match_oracle(key):
         # far from 34 km underflow into float subnormals, where one unit is 1.4e-45
         np.testing.assert_allclose(x[:, :-1], ref[:, :-1].astype(np.float32), rtol=2.4e-7, atol=1.5e-45)
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(33, 34, 33), (64, 4, 32), (31, 65, 20), (4, 32, 65)])
+def test_features_and_tendency_at_tile_edges(shape):
+    """Column and layer counts around the 32 x 32 tiles of the two kernels: the features as above, and
+    the tendency of given heating rates, (sw + lw)/86400*rho_gas*c_d_p with the sum formed in float, to
+    the rounding of that sum and three FP64 operations."""
+    from lgame_gpu import emulator as E
+    ny, nx, nl = shape
+    n = cases.namelist(cases.SMALL["jet"][0], **{**cases.SMALL["jet"][1], "ny": ny, "nx": nx, "n_layers": nl, "n_oro_layers": nl - 5})
+    hm = L.HostModel(n)
+    g = L.GpuModel(L.config_from_namelist(n), hm.grid)
+    g.set_state(0, hm.state)
+    g.set_diag(hm.diag)
+    rng = np.random.default_rng(6)
+    lat, lon, alb = rng.uniform(-1.5, 1.5, (ny, nx)), rng.uniform(-3.0, 3.0, (ny, nx)), rng.uniform(0.1, 0.9, (ny, nx))
+    E.rad_set_surface(g, alb, lat, lon)
+    x = E.rad_features(g, 0, T_SOLSTICE)
+    ref = R.features(hm.state, hm.grid, alb, lat, lon, T_SOLSTICE, bool(n.lmoist))
+    np.testing.assert_allclose(x[:, -1], ref[:, -1], rtol=0, atol=1e-7)
+    np.testing.assert_allclose(x[:, :-1], ref[:, :-1].astype(np.float32), rtol=2.4e-7, atol=1.5e-45)
+    h = rng.normal(size=(ny * nx, 2 * nl)).astype(np.float32)
+    E.rad_apply_heating(g, 0, h)
+    rho = (hm.state["rho"][..., -2] + hm.state["rho"][..., -1]).reshape(ny * nx, nl, order="F")
+    out = g.get_diag()["radiation_tendency"].reshape(ny * nx, nl, order="F")
+    np.testing.assert_allclose(out, (h[:, :nl] + h[:, nl:]).astype(np.float64) / 86400.0 * rho * 1005.0, rtol=1e-14)
+    g.close()
