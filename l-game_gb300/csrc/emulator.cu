@@ -588,6 +588,243 @@ int launch_gemm(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, in
   }
 }
 
+// ---- inference in one launch -----------------------------------------------------------------
+// All four layers of 128 columns of the atmosphere (a tile) by one CTA, for a network whose layers are at
+// most 512 wide: the activations of a layer stay in shared memory as the next product's A operand
+// (128 x 512 BF16, in the 128-byte swizzle's layout), its 128 x 512 FP32 accumulator is the whole
+// tensor memory, and only the weights stream through a ring of stages.  Layer by layer every product
+// was a launch of about one tile per SM, whose operands, epilogue and tail followed one another:
+// 85 us for 8192 columns with preparation and result (three products of 20 us, 13, 10 and 7 us).
+//   warp 0       weights: 256 x 64 blocks by TMA, half a layer's outputs after the other
+//   warp 1       tcgen05.mma, 128 x 256 (the last layer: x nout_pad) per half
+//   warps 2-17   standardise the tile's inputs into A; after each half's products bias, GELU and BF16:
+//                the first half's results wait in registers, as the second half still reads A; after
+//                the last layer the heating rates, through shared memory to whole rows
+// The waits are bounded and end on the abort flag as in k_gemm.
+constexpr int kMlpThreads = 64 + 512, kMlpStages = 3, kMlpWidth = 512;
+constexpr uint32_t kMlpA = 128 * 64 * 2, kMlpStage = 256 * 64 * 2;  // a K block of A, of the weights
+constexpr size_t kMlpSmem = (size_t)(kMlpWidth / 64) * kMlpA + (size_t)kMlpStages * kMlpStage + 1024;
+struct Mlp {
+  const float* x;
+  float* y;
+  const float *xmean, *xistd, *ymean, *ystd, *bias[4];
+  long long n;
+  int nin, nin_pad, hidden, nout, nout_pad;
+};
+
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp(const __grid_constant__ CUtensorMap w0,
+                                                        const __grid_constant__ CUtensorMap w1,
+                                                        const __grid_constant__ CUtensorMap w2,
+                                                        const __grid_constant__ CUtensorMap w3, const Mlp P, int ntiles,
+                                                        int* err) {
+  constexpr int S = kMlpStages;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full[S], empty[S], acc_full[2], act_ready, out_done, done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+  const volatile int* abort_v = &abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t act = (smem_u32(smem_raw) + 1023u) & ~1023u, ring = act + (kMlpWidth / 64) * kMlpA;
+  if (warp == 0) tc_alloc(smem_u32(&tmem_base), 512);
+  if (tid == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(smem_u32(&full[i]), 1);
+      mbar_init(smem_u32(&empty[i]), 1);
+    }
+    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&acc_full[i]), 1);
+    mbar_init(smem_u32(&act_ready), 16);
+    mbar_init(smem_u32(&out_done), 16);
+    mbar_init(smem_u32(&done), 1);
+    abort_flag = 0;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+  const int halves = P.hidden / 256;
+  auto nk_of = [&](int l) { return (l == 0 ? P.nin_pad : P.hidden) / 64; };
+  bool failed = false;
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;  // weight blocks issued
+      for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x)
+        for (int l = 0; l < 4 && !failed; ++l) {
+          const CUtensorMap* map = l == 0 ? &w0 : l == 1 ? &w1 : l == 2 ? &w2 : &w3;
+          const int nh = l < 3 ? halves : 1, nk = nk_of(l);
+          const uint32_t bytes = (uint32_t)(l < 3 ? 256 : P.nout_pad) * 128u;
+          for (int b = 0; b < nh * nk; ++b, ++it) {
+            const int st = it % S;
+            if (it >= S && !mbar_wait_or_abort(smem_u32(&empty[st]), (uint32_t)((it / S - 1) & 1), abort_v)) {
+              failed = true;
+              break;
+            }
+            mbar_arrive_expect_tx(smem_u32(&full[st]), bytes);
+            tma_load_2d(ring + st * kMlpStage, map, 64 * (b % nk), 256 * (b / nk), smem_u32(&full[st]));
+          }
+        }
+      if (failed) {
+        abort_flag = 1;
+        // the copies still in flight land before the CTA exits (bounded)
+        for (int j = max(0, it - S); j < it; ++j) mbar_wait(smem_u32(&full[j % S]), (uint32_t)((j / S) & 1));
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int it = 0, lt = 0;  // weight blocks consumed, layers begun
+      for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x)
+        for (int l = 0; l < 4 && !failed; ++l, ++lt) {
+          // the layer's inputs are in shared memory, and the accumulator has been read out
+          if (!mbar_wait_or_abort(smem_u32(&act_ready), (uint32_t)(lt & 1), abort_v)) {
+            failed = true;
+            break;
+          }
+          tc_fence_after();
+          const int nh = l < 3 ? halves : 1, nk = nk_of(l);
+          const uint32_t idesc = instr_desc(128, l < 3 ? 256 : P.nout_pad);
+          for (int h = 0; h < nh && !failed; ++h) {
+            for (int kb = 0; kb < nk; ++kb, ++it) {
+              const int st = it % S;
+              if (!mbar_wait_or_abort(smem_u32(&full[st]), (uint32_t)((it / S) & 1), abort_v)) {
+                failed = true;
+                break;
+              }
+              tc_fence_after();
+              const uint32_t a = act + kb * kMlpA, w = ring + st * kMlpStage;
+#pragma unroll
+              for (int s = 0; s < 4; ++s)
+                tc_mma(tmem + 256 * h, smem_desc_sw128(a + s * 32), smem_desc_sw128(w + s * 32), idesc,
+                       (kb > 0 || s > 0) ? 1u : 0u);
+              tc_commit(smem_u32(&empty[st]));
+            }
+            if (!failed) tc_commit(smem_u32(&acc_full[h]));
+          }
+        }
+      if (failed) abort_flag = 1;
+      tc_commit(smem_u32(&done));
+    }
+  } else {
+    const int qw = warp & 3, ew = warp - 2, group = ew >> 2, m = 32 * qw + lane;  // tensor-memory lane = tile row
+    uint8_t* act_ptr = smem_raw + (act - smem_u32(smem_raw));
+    uint32_t phase[2] = {0u, 0u};
+    // the warp's part of half h is ready to be read
+    auto acc_wait = [&](int h) -> bool {
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_or_abort(smem_u32(&acc_full[h]), phase[h], abort_v));
+      phase[h] ^= 1u;
+      tc_fence_after();
+      return ok;
+    };
+    auto ready = [&]() {  // the warp's part of A is written, its part of the accumulator read
+      tc_fence_before();
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&act_ready));
+    };
+    uint8_t* row = act_ptr + m * 128;
+    auto put = [&](int col, const uint4& v) {  // eight activations of this row, columns col..
+      *reinterpret_cast<uint4*>(row + (col >> 6) * kMlpA + ((((col & 63) >> 3) ^ (m & 7)) << 4)) = v;
+    };
+    auto gelu16 = [&](const float* bias, int col, uint4* out) {  // columns col..col+15 of this row
+      float v[16];
+      tc_ld16(tmem + ((uint32_t)(32 * qw) << 16) + (uint32_t)col, v);
+      __align__(16) bf16 hb[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) hb[j] = __float2bfloat16_rn(gelu(v[j] + bias[col + j]));
+      out[0] = reinterpret_cast<const uint4*>(hb)[0];
+      out[1] = reinterpret_cast<const uint4*>(hb)[1];
+    };
+    int tiles = 0;
+    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x, ++tiles) {
+      const long long r0 = (long long)t * 128;
+      const int rows = (int)min(128LL, P.n - r0);
+      // the last tile's results have left the memory of A
+      if (tiles > 0 && !__all_sync(0xffffffffu, mbar_wait_or_abort(smem_u32(&out_done), (uint32_t)((tiles - 1) & 1), abort_v))) {
+        failed = true;
+        break;
+      }
+      // inputs: rows ew, ew + 16, ...; lanes along the features
+      for (int c = lane; c < P.nin_pad; c += 32) {
+        const bool in = c < P.nin;
+        const float mu = in ? P.xmean[c] : 0.f, is = in ? P.xistd[c] : 0.f;
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = ew + 16 * k;
+          v[k] = (in && r < rows) ? (P.x[(size_t)(r0 + r) * P.nin + c] - mu) * is : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = ew + 16 * k;
+          *reinterpret_cast<bf16*>(act_ptr + (c >> 6) * kMlpA + r * 128 + ((((c & 63) >> 3) ^ (r & 7)) << 4) + (c & 7) * 2) =
+              __float2bfloat16_rn(v[k]);
+        }
+      }
+      ready();
+      for (int l = 0; l < 3; ++l) {
+        const float* bias = P.bias[l];
+        uint4 first[8];
+        const int col = 64 * group;
+        if (!acc_wait(0)) { failed = true; break; }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gelu16(bias, col + 16 * q, first + 2 * q);
+        if (halves == 2 && !acc_wait(1)) { failed = true; break; }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) put(col + 8 * q, first[q]);
+        if (halves == 2) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 o[2];
+            gelu16(bias, 256 + col + 16 * q, o);
+            put(256 + col + 16 * q, o[0]);
+            put(256 + col + 16 * q + 8, o[1]);
+          }
+        }
+        ready();
+      }
+      if (failed || !acc_wait(0)) { failed = true; break; }
+      // heating rates: the warp's 32 rows x 64 columns through its 8 KB of the memory of A
+      const int col = 64 * group;
+      if (col < P.nout_pad) {
+        uint8_t* stg = act_ptr + ew * 8192;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float v[16];
+          tc_ld16(tmem + ((uint32_t)(32 * qw) << 16) + (uint32_t)(col + 16 * q), v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int c = col + 16 * q + j;
+            v[j] = c < P.nout ? fmaf(v[j] + P.bias[3][c], P.ystd[c], P.ymean[c]) : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(stg + lane * 256 + (((4 * q + j) ^ (lane & 15)) << 4)) =
+                make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        }
+        __syncwarp();
+        const int last = min(32, rows - 32 * qw);
+        for (int r = 0; r < last; ++r)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int c = lane + 32 * k;
+            if (col + c < P.nout)
+              P.y[(size_t)(r0 + 32 * qw + r) * P.nout + col + c] =
+                  *reinterpret_cast<const float*>(stg + r * 256 + (((c >> 2) ^ (r & 15)) << 4) + (c & 3) * 4);
+          }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&out_done));
+    }
+    if (failed && lane == 0) abort_flag = 1;
+  }
+  __syncwarp();
+  const bool ok = mbar_wait(smem_u32(&done), 0);
+  tc_fence_after();
+  if (__syncthreads_or(failed || !ok) && tid == 0) atomicExch(err, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc_dealloc(tmem, 512);
+}
+
 // ---- element-wise and reduction kernels ------------------------------------------------------
 // Kernels that write a matrix and its transpose work on 32 x 32 tiles (blocks of 32 x 8
 // threads): a warp reads and writes a row of the tile, and the transposed copy goes out
@@ -772,7 +1009,7 @@ inline unsigned blocks(long long n, int t = 256) { return (unsigned)((n + t - 1)
 using namespace emu;
 
 struct lgame_emu {
-  int nlev = 0, nin = 0, nin_pad = 0, hidden = 0, nout = 0, nout_pad = 0, bmax = 0, device = 0;
+  int nlev = 0, nin = 0, nin_pad = 0, hidden = 0, nout = 0, nout_pad = 0, bmax = 0, device = 0, nsm = 0;
   cudaStream_t st = nullptr;
   std::vector<void*> allocs;
   int rows[4], cols[4];              // layer l: rows = outputs (padded), cols = inputs (padded)
@@ -863,6 +1100,15 @@ int forward(lgame_emu* e, int batch, bool infer = false) {
   return gemm(e, in, Hd, e->Wb[3], Hd, batch, e->nout_pad, Hd, 1, ep);
 }
 
+// whether k_mlp runs the inference of n columns: where the widths fit shared and tensor memory, and the
+// layers' own launches would take more than one batch or have filled the SMs.  k_mlp takes about 75 us
+// for every 152 tiles of 128 columns (512 wide, 80 layers); layer by layer a batch takes 50 us for one
+// tile and 85 us for 8192 columns.  A radiation update of 4096 columns: 105 us by layers, 121 us in one
+// launch; 9216 columns 180 and 131 us; 65536 columns 804 and 495 us.
+bool mlp_pays(const lgame_emu* e, long long n) {
+  return e->hidden <= kMlpWidth && e->nin_pad <= kMlpWidth && (n > e->bmax || n >= 8192) && n <= (1LL << 37);
+}
+
 // prepared inputs of `batch` rows (a multiple of 128) from raw rows the GPU can read (device
 // memory or page-locked host memory), of which the first `valid` hold data
 int prep_x(lgame_emu* e, const float* xraw_dev, int batch, int valid, bool infer = false, const long long* idx = nullptr) {
@@ -870,6 +1116,38 @@ int prep_x(lgame_emu* e, const float* xraw_dev, int batch, int valid, bool infer
                                                                         valid, e->xmean, e->xistd, e->X,
                                                                         infer ? nullptr : e->XT);
   ECK(cudaGetLastError());
+  return LGAME_OK;
+}
+
+// heating rates (n x nout) of n columns' features, both readable by the GPU, in batches of bmax; mlp: in one
+// launch (the rule stands at mlp_pays)
+int predict(lgame_emu* e, const float* x, long long n, float* y) {
+  if (mlp_pays(e, n)) {
+    CUtensorMap w[4];
+    for (int l = 0; l < 4; ++l) {
+      const int rc = tensor_map(&w[l], e->Wb[l], e->rows[l], e->cols[l], e->cols[l], l < 3 ? 256 : e->nout_pad);
+      if (rc) return emu_fail(rc, "emulator: tensor map of the weights");
+    }
+    ECK(cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem));
+    const Mlp P{x, y, e->xmean, e->xistd, e->ymean, e->ystd, {e->b[0], e->b[1], e->b[2], e->b[3]}, n, e->nin, e->nin_pad,
+                e->hidden, e->nout, e->nout_pad};
+    const int ntiles = (int)((n + 127) / 128);
+    k_mlp<<<std::min(ntiles, e->nsm), kMlpThreads, kMlpSmem, e->st>>>(w[0], w[1], w[2], w[3], P, ntiles, e->err);
+    ECK(cudaGetLastError());
+    e->gemm_launches++;
+    for (int l = 0; l < 4; ++l) e->gemm_flop += 2.0 * (128.0 * ntiles) * e->rows[l] * (double)e->cols[l];
+    return LGAME_OK;
+  }
+  for (long long r0 = 0; r0 < n; r0 += e->bmax) {
+    const int b = (int)std::min<long long>(e->bmax, n - r0);
+    const int bp = ((b + 127) / 128) * 128;
+    int rc = prep_x(e, x + r0 * e->nin, bp, b, true);
+    if (!rc) rc = forward(e, bp, true);
+    if (rc) return rc;
+    k_denorm<<<blocks((long long)b * e->nout), 256, 0, e->st>>>(e->Y, e->nout, e->nout_pad, b, e->ymean, e->ystd,
+                                                                 y + r0 * e->nout);
+    ECK(cudaGetLastError());
+  }
   return LGAME_OK;
 }
 
@@ -959,20 +1237,11 @@ int refresh_bf16(lgame_emu* e) {
 
 namespace emu {
 // device-side inference for the coupling code: n rows of raw features (device) -> heating
-// rates (device, n x nout), in batches of bmax
+// rates (device, n x nout)
 int infer_device(lgame_emu* e, const float* x_dev, long long n, float* y_dev, cudaStream_t st) {
   if (cudaStreamSynchronize(st) != cudaSuccess) return LGAME_ERR_CUDA;
-  for (long long r0 = 0; r0 < n; r0 += e->bmax) {
-    const int b = (int)std::min<long long>(e->bmax, n - r0);
-    const int bp = ((b + 127) / 128) * 128;
-    int rc = prep_x(e, x_dev + r0 * e->nin, bp, b, true);
-    if (rc) return rc;
-    rc = forward(e, bp, true);
-    if (rc) return rc;
-    k_denorm<<<blocks((long long)b * e->nout), 256, 0, e->st>>>(e->Y, e->nout, e->nout_pad, b, e->ymean, e->ystd,
-                                                                 y_dev + r0 * e->nout);
-    ECK(cudaGetLastError());
-  }
+  const int rc = predict(e, x_dev, n, y_dev);
+  if (rc) return rc;
   ECK(cudaStreamSynchronize(e->st));
   return check_err(e);
 }
@@ -1005,6 +1274,7 @@ extern "C" int lgame_emu_create(int nlev, int hidden, int batch_max, unsigned lo
   e->nout_pad = ((e->nout + 63) / 64) * 64;
   e->bmax = batch_max;
   e->device = device;
+  e->nsm = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking) != cudaSuccess) return fail(LGAME_ERR_CUDA);
   const int Hd = hidden;
   const int rows[4] = {Hd, Hd, Hd, e->nout_pad}, cols[4] = {e->nin_pad, Hd, Hd, Hd};
@@ -1268,18 +1538,14 @@ extern "C" int lgame_emu_infer(lgame_emu* e, const float* x, long long n, float*
   if (!e || !x || !y || n < 0) return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_infer: bad arguments");
   const float* xv = (const float*)mapped_view(x);
   float* yv = (float*)mapped_view(y);
-  for (long long r0 = 0; r0 < n; r0 += e->bmax) {
-    const int b = (int)std::min<long long>(e->bmax, n - r0);
-    const int bp = ((b + 127) / 128) * 128;
-    const float* src = xv ? xv + r0 * e->nin : e->xraw;
+  // what the GPU cannot address goes through the device buffers, bmax rows at a time
+  const long long step = (xv && yv) ? std::max<long long>(n, 1) : e->bmax;
+  for (long long r0 = 0; r0 < n; r0 += step) {
+    const long long b = std::min(step, n - r0);
     if (!xv)
       ECK(cudaMemcpyAsync(e->xraw, x + r0 * e->nin, sizeof(float) * (size_t)b * e->nin, cudaMemcpyHostToDevice, e->st));
-    int rc = prep_x(e, src, bp, b, true);
-    if (!rc) rc = forward(e, bp, true);
+    const int rc = predict(e, xv ? xv + r0 * e->nin : e->xraw, b, yv ? yv + r0 * e->nout : e->yout);
     if (rc) return rc;
-    k_denorm<<<blocks((long long)b * e->nout), 256, 0, e->st>>>(e->Y, e->nout, e->nout_pad, b, e->ymean, e->ystd,
-                                                                 yv ? yv + r0 * e->nout : e->yout);
-    ECK(cudaGetLastError());
     if (!yv)
       ECK(cudaMemcpyAsync(y + r0 * e->nout, e->yout, sizeof(float) * (size_t)b * e->nout, cudaMemcpyDeviceToHost, e->st));
   }

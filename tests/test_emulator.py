@@ -249,3 +249,25 @@ def test_lrad_update_drives_attached_emulator():
     a.close()
     b.close()
     emu.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nlev, hidden, n", [(3, 256, 129), (20, 256, 1000), (20, 512, 255), (125, 512, 700),
+                                             (64, 512, 20001), (126, 512, 257)])
+def test_inference_in_one_launch_equals_the_layers(nlev, hidden, n):
+    """More columns than a batch run in one launch where the layers are at most 512 wide (126 layers of the
+    atmosphere make 506 inputs, padded to 512), one batch at a time in the layers' own: the same
+    products in the same order, so the same bits, for the smallest and largest widths, ragged last tiles
+    and more tiles than SMs."""
+    rng = np.random.default_rng(nlev + n)
+    emu = E.Emulator(nlev=nlev, hidden=hidden, batch_max=128, seed=7)
+    emu.set_normalization(rng.normal(size=emu.nin), rng.uniform(0.5, 2.0, emu.nin), rng.normal(size=emu.nout),
+                          rng.uniform(0.5, 2.0, emu.nout))
+    x = rng.normal(size=(n, emu.nin)).astype(np.float32)
+    torch = pytest.importorskip("torch")
+    xp = torch.empty((n, emu.nin), dtype=torch.float32, pin_memory=True).numpy()
+    yp = torch.zeros((n, emu.nout), dtype=torch.float32, pin_memory=True).numpy()
+    xp[...] = x
+    emu.infer(xp, out=yp)  # page-locked: all columns in one call
+    np.testing.assert_array_equal(yp, emu.infer(x))  # pageable: a batch at a time
+    emu.close()
