@@ -66,6 +66,7 @@ struct SplitCtx {
   double* rmz = nullptr;
   // sediment heating of each condensate (nc planes), summed into the carried csh
   float* csh_part = nullptr;
+  float* cw = nullptr;  // contravariant wind correction times the interface area (moist)
   // divergence of the gradient of theta_bg (the third-order theta chain of the background),
   // and the background's x and y edge averages as FP32 pairs
   float* dbg = nullptr;
@@ -571,47 +572,131 @@ __global__ void __launch_bounds__(128) ks_div_h(Dims D, Grid<float> GF, GridX X,
   }
 }
 
+constexpr int kTracers = 6;  // moist: five condensates and water vapour (the gas has its own kernels)
 // divergences of the gas and theta_v fluxes and the diabatic rho*theta_v term,
-// mo_scalar_tend_expl.F90:106-177 (the gas has old_weight 0, new_weight 1), column-marching
-__global__ void __launch_bounds__(128) ks_gas_div(Dims D, Grid<float> GF, GridX X, StateF Ss, const float* fu,
+// mo_scalar_tend_expl.F90:106-177 (the gas has old_weight 0, new_weight 1), column-marching.  A layer's
+// fluxes, metrics and heating rates are loaded two layers ahead, and what only a layer with heating needs
+// (its temperature, densities and exner) one layer ahead, so that a layer waits for memory once:
+// 1053 us at 768x768x80 with six resident blocks (five 1252, and 1680 with each layer's loads in its own
+// turn), with cw 1145 us.
+// TRACERS: also cw, the contravariant correction of the wind through the interfaces nf+1..nl times their
+// area, for ks_tracers, from the slopes and weights that are here already.
+struct GasLoads {  // fluxes through the faces (layer_faces' order), metrics, the layer's heating
+  float f[4], t[4], u[4], area[4], slope[4], w[4], az, iv, heat;
+};
+struct GasLayer {  // of a layer: horizontal parts, half the slope-weighted sums, upper area
+  float fh, th, fs, ts, us, az, iv, heat;
+};
+struct GasHeat {  // of a layer with heating
+  float T, rho[kTracers + 1], exner;
+};
+template <bool TRACERS>
+__global__ void __launch_bounds__(128, 6) ks_gas_div(Dims D, Grid<float> GF, GridX X, StateF Ss, const float* fu,
                                                   const float* fv, const float* gu, const float* gv, const float* Tm,
                                                   const float* hd, const float* rad, const float* csh, float* t_rho,
                                                   float* t_rt, const float* mdt, const float* tdh,
-                                                  const float* ptr, const float* pth) {
+                                                  const float* ptr, const float* pth, const float* u_new,
+                                                  const float* v_new, float* cw) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
   const LevelChunk lc = level_chunk(D);
   const long long goff = (long long)(D.g - 1) * D.fstride;
-  auto fx = [&](int i, int j, int k) { return fu[IX(D, i, j, k)]; };
-  auto fy = [&](int i, int j, int k) { return fv[IX(D, i, j, k)]; };
-  auto gx = [&](int i, int j, int k) { return gu[IX(D, i, j, k)]; };
-  auto gy = [&](int i, int j, int k) { return gv[IX(D, i, j, k)]; };
-  LayerFaces mc = layer_faces(D, GF, fx, fy, ji, jk, lc.l0), mn{};
-  LayerFaces tc = layer_faces(D, GF, gx, gy, ji, jk, lc.l0), tn{};
-  float mh_prev = 0.f, th_prev = 0.f;
+  auto load = [&](int l) {
+    GasLoads R{};
+    if (l > D.nl) return R;
+    const long long p = IX(D, ji, jk, l), e = IX(D, ji, jk + 1, l), s = IX(D, ji + 1, jk, l);
+    R.f[0] = fu[e]; R.f[1] = fv[p]; R.f[2] = fu[p]; R.f[3] = fv[s];
+    R.t[0] = gu[e]; R.t[1] = gv[p]; R.t[2] = gu[p]; R.t[3] = gv[s];
+    R.area[0] = GF.area_x[e]; R.area[1] = GF.area_y[p]; R.area[2] = GF.area_x[p]; R.area[3] = GF.area_y[s];
+    if (l > D.nf) {
+      R.slope[0] = GF.slope_x[e]; R.slope[1] = GF.slope_y[p]; R.slope[2] = GF.slope_x[p]; R.slope[3] = GF.slope_y[s];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) R.w[k] = GF.ipw[k][p];
+      R.az = GF.area_z[p];
+      if constexpr (TRACERS) {
+        R.u[0] = u_new[e]; R.u[1] = v_new[p]; R.u[2] = u_new[p]; R.u[3] = v_new[s];
+      }
+    }
+    R.iv = X.inv_volume_f[p];
+    R.heat = hd[p] + rad[p];                 // dissipative, radiative heating
+    if (pth) R.heat = R.heat + pth[p];       // phase transitions
+    R.heat = R.heat + csh[p];                // sediment heating
+    if (tdh) R.heat = R.heat + tdh[p];       // temperature diffusion
+    return R;
+  };
+  auto reduce = [&](const GasLoads& R, int l) {
+    GasLayer L;
+    auto hor = [&](const float* f) {
+      return fmaf(-f[3], R.area[3], fmaf(-f[2], R.area[2], fmaf(f[0], R.area[0], f[1] * R.area[1])));
+    };
+    L.fh = hor(R.f);
+    L.th = hor(R.t);
+    auto slopes = [&](const float* v) {
+      return fmaf(0.5f * v[3] * R.slope[3], R.w[3],
+                  fmaf(0.5f * v[2] * R.slope[2], R.w[2],
+                       fmaf(0.5f * v[0] * R.slope[0], R.w[0], 0.5f * v[1] * R.slope[1] * R.w[1])));
+    };
+    L.fs = l > D.nf ? slopes(R.f) : 0.f;
+    L.ts = l > D.nf ? slopes(R.t) : 0.f;
+    L.us = TRACERS && l > D.nf ? slopes(R.u) : 0.f;
+    L.az = R.az;
+    L.iv = R.iv;
+    L.heat = R.heat;
+    return L;
+  };
+  auto heat_loads = [&](const GasLayer& L, int l) {
+    GasHeat H{};
+    if (l <= D.nl && L.heat != 0.f) {
+      const long long p = IX(D, ji, jk, l);
+      H.T = Tm[p];
+#pragma unroll
+      for (int k = 0; k < kTracers + 1; ++k)
+        if (k < D.ncons) H.rho[k] = Ss.rho[p + (long long)k * D.fstride];
+      H.exner = GF.exner_bg[p] + Ss.ep[p];
+    }
+    return H;
+  };
+  float fs_prev = 0.f, ts_prev = 0.f;
   if (lc.l0 - 1 >= D.nf + 1) {
-    mh_prev = layer_faces(D, GF, fx, fy, ji, jk, lc.l0 - 1).h;
-    th_prev = layer_faces(D, GF, gx, gy, ji, jk, lc.l0 - 1).h;
+    const GasLayer P = reduce(load(lc.l0 - 1), lc.l0 - 1);
+    fs_prev = P.fs;
+    ts_prev = P.ts;
   }
+  GasLoads R = load(lc.l0 + 1);
+  GasLayer cur = reduce(load(lc.l0), lc.l0);
+  GasHeat H = heat_loads(cur, lc.l0);
   for (int jl = lc.l0; jl <= lc.l1; ++jl) {
     const long long q = IX(D, ji, jk, jl);
-    mn.h = 0.f;
-    tn.h = 0.f;
-    if (jl < D.nl || jl == D.nf) {
-      mn = layer_faces(D, GF, fx, fy, ji, jk, jl + 1);
-      tn = layer_faces(D, GF, gx, gy, ji, jk, jl + 1);
+    const GasLayer nxt = reduce(R, jl + 1);
+    if (jl < lc.l1) R = load(jl + 2);
+    const GasHeat Hn = heat_loads(nxt, jl + 1);
+    const VertFaces vm = vert_faces(D, fs_prev, cur.fs, nxt.fs, jl), vt = vert_faces(D, ts_prev, cur.ts, nxt.ts, jl);
+    float cm = 0.f, ct = 0.f;
+    if (vm.up) {
+      cm += vm.cu * cur.az;
+      ct += vt.cu * cur.az;
     }
-    float heat = hd[q] + rad[q];           // dissipative, radiative heating
-    if (pth) heat = heat + pth[q];         // phase transitions
-    heat = heat + csh[q];                  // sediment heating
-    if (tdh) heat = heat + tdh[q];         // temperature diffusion
-    const float div_m = div_col(D, GF, X, mc, vert_faces(D, mh_prev, mc.h, mn.h, jl), ji, jk, jl);
-    const float div_t = div_col(D, GF, X, tc, vert_faces(D, th_prev, tc.h, tn.h, jl), ji, jk, jl);
+    if (vm.lo) {
+      cm -= vm.cl * nxt.az;
+      ct -= vt.cl * nxt.az;
+    }
+    if (TRACERS && vm.lo) cw[q + D.plane] = ((jl == D.nf) ? -nxt.us : -(cur.us + nxt.us)) * nxt.az;
+    const float div_m = (cur.fh + cm) * cur.iv, div_t = (cur.th + ct) * cur.iv;
     float x = 0.f;
-    if (heat != 0.f) {
-      const float cv = c_v_mass_weighted_air<float>(D, Ss.rho, Tm, q);
-      x = float(kC_D_V) * Ss.rho[q + goff] / cv * heat / (float(kC_D_P) * (GF.exner_bg[q] + Ss.ep[q]));
+    if (cur.heat != 0.f) {
+      float cv = 0.f, rg;  // c_v_mass_weighted_air, mo_derived.F90:157-187
+      if (D.lmoist) {
+#pragma unroll
+        for (int jc = 1; jc < kTracers; ++jc) cv = cv + H.rho[jc - 1] * c_p_cond(jc, H.T);
+        cv = cv + (H.rho[kTracers - 1] - H.rho[kTracers]) * float(kC_D_V);
+        cv = cv + H.rho[kTracers] * float(kC_V_V);
+        rg = H.rho[kTracers - 1];
+      } else {
+        rg = H.rho[0];
+        cv = rg * float(kC_D_V);
+      }
+      x = float(kC_D_V) * rg / cv * cur.heat / (float(kC_D_P) * H.exner);
     }
     if (ptr) {  // phase transitions' vapour rate and mass diffusion of the gas
       const float mdg = mdt ? mdt[q + goff] : 0.f, ptg = ptr[q + goff];
@@ -625,79 +710,50 @@ __global__ void __launch_bounds__(128) ks_gas_div(Dims D, Grid<float> GF, GridX 
       t_rho[q + goff] = -div_m;
       t_rt[q] = -div_t + x;
     }
-    mh_prev = mc.h;
-    th_prev = tc.h;
-    mc = mn;
-    tc = tn;
+    fs_prev = cur.fs;
+    ts_prev = cur.ts;
+    cur = nxt;
+    H = Hn;
   }
 }
 
 // scalar_tend_expl for the tracers, mo_scalar_tend_expl.F90:24-104 (upstream fluxes,
 // mo_scalar_tend_expl.F90:56-82; vertical upstream term with the contravariant correction,
-// mo_averaging.F90:16-54), split step.  The velocity through each of the six faces of the
-// cell, times the face area, and the index of the face's upwind cell are found once per
-// cell; the tracer loop then only loads densities at known addresses, and every tracer's
-// divergence is formed before the first tendency is stored, so no load waits on a velocity
-// or on an earlier store.  The first substep (new weight 1) does not read the old tendency.
-// Five resident blocks of 256 threads per SM (48 registers) ran 4 % faster than four.
-constexpr int kTracers = 6;  // moist: five condensates and water vapour (the gas has its own kernel)
-__global__ void __launch_bounds__(256, 5) ks_tracers(Dims D, Grid<float> GF, GridX X, StateF Ss, const float* u_new,
-                                                     const float* v_new, float* t_rho, int rk_step,
+// mo_averaging.F90:16-54, whose product with the area ks_gas_div left in cw), split step.  The
+// velocities through the six faces of the cell, times the face areas, and the indices of the
+// faces' upwind cells are found once per cell; the tracer loop then only loads densities at known
+// addresses, and every tracer's divergence is formed before the first tendency is stored, so no load
+// waits on an earlier store.  The first substep (new weight 1) does not read the old tendency.
+// 873 us at 768x768x80 with six resident blocks (five 918, four 951).  Forming the corrections here took
+// half of the kernel's loads (1687 us); a column-marching form keeps too many values a tracer (1839 us).
+__global__ void __launch_bounds__(256, 6) ks_tracers(Dims D, Grid<float> GF, GridX X, StateF Ss, const float* u_new,
+                                                     const float* v_new, const float* cw, float* t_rho, int rk_step,
                                                      const float* mdt, const float* ptr) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
   const long long q = IX(D, ji, jk, jl);
-  // horizontal faces: flux = rho(upwind cell) * velocity, 0 on a non-periodic boundary
-  auto face_x = [&](int kf, float* a, long long* up) {
-    int kk = kf, ka = kf - 1, kb = kf;
-    if (kf < 2 || kf > D.nx) {
-      if (!D.periodic) { *a = 0.f; *up = q; return; }
-      kk = 1; ka = D.nx; kb = 1;
-    }
-    const float u = u_new[IX(D, ji, kk, jl)];
-    *a = u * GF.area_x[IX(D, ji, kf, jl)];
-    *up = IX(D, ji, (u >= 0.f) ? ka : kb, jl);
-  };
-  auto face_y = [&](int i_f, float* a, long long* up) {
-    int ii = i_f, ia = i_f, ib = i_f - 1;
-    if (i_f < 2 || i_f > D.ny) {
-      if (!D.periodic) { *a = 0.f; *up = q; return; }
-      ii = 1; ia = 1; ib = D.ny;
-    }
-    const float v = v_new[IX(D, ii, jk, jl)];
-    *a = v * GF.area_y[IX(D, i_f, jk, jl)];
-    *up = IX(D, (v >= 0.f) ? ia : ib, jk, jl);
-  };
-  float a_e, a_n, a_w, a_s, a_u = 0.f, a_l = 0.f;
-  long long i_e, i_n, i_w, i_s, i_u = q, i_l = q;
-  face_x(jk + 1, &a_e, &i_e);
-  face_y(ji, &a_n, &i_n);
-  face_x(jk, &a_w, &i_w);
-  face_y(ji + 1, &a_s, &i_s);
-  // vertical faces: the contravariant vertical velocity correction at the upper (jl) and
-  // lower (jl+1) interface inside the terrain-following layers; the upwind cell by its sign
-  auto wx = [&](int i, int j, int k) { return u_new[IX(D, i, j, k)]; };
-  auto wy = [&](int i, int j, int k) { return v_new[IX(D, i, j, k)]; };
-  // (the top terrain-following layer nf has only its lower face, the lowest layer nl only
-  // its upper one, unless it is layer nf itself)
-  if (jl > D.nf) {
-    const float cu = vcc<float>(D, GF, wx, wy, ji, jk, jl);
-    a_u = cu * GF.area_z[IX(D, ji, jk, jl)];
-    i_u = (cu <= 0.f) ? IX(D, ji, jk, jl - 1) : q;
-  }
-  if (jl == D.nf || (jl > D.nf && jl < D.nl)) {
-    const float cl = vcc<float>(D, GF, wx, wy, ji, jk, jl + 1);
-    a_l = cl * GF.area_z[IX(D, ji, jk, jl + 1)];
-    i_l = (cl <= 0.f) ? q : IX(D, ji, jk, jl + 1);
-  }
+  // horizontal faces: flux = rho(upwind cell) * velocity, 0 on a non-periodic boundary; the periodic
+  // wrap edges take the velocity at the first edge
+  const Edge w = edge_x(D, ji, jk, jl), e = edge_x(D, ji, jk + 1, jl), n = edge_y(D, ji, jk, jl), so = edge_y(D, ji + 1, jk, jl);
+  const bool up = jl > D.nf, lo = jl >= D.nf && jl < D.nl;  // the interfaces of the terrain-following layers
+  const float ue = u_new[e.b], uw = u_new[w.b], vn = v_new[n.b], vs = v_new[so.b];
+  const float ae = GF.area_x[e.q], aw = GF.area_x[w.q], an = GF.area_y[n.q], as = GF.area_y[so.q];
+  float a_u = 0.f, a_l = 0.f;
+  if (up) a_u = cw[q];
+  if (lo) a_l = cw[q + D.plane];
+  const float a_e = e.flux ? ue * ae : 0.f, a_w = w.flux ? uw * aw : 0.f;
+  const float a_n = n.flux ? vn * an : 0.f, a_s = so.flux ? vs * as : 0.f;
+  const long long i_e = ue >= 0.f ? e.a : e.b, i_w = uw >= 0.f ? w.a : w.b;
+  const long long i_n = vn >= 0.f ? n.b : n.a, i_s = vs >= 0.f ? so.b : so.a;
+  const long long i_u = up && a_u <= 0.f ? q - D.plane : q, i_l = lo && a_l > 0.f ? q + D.plane : q;
   const float iv = X.inv_volume_f[q];
   float dv[kTracers];
 #pragma unroll
   for (int t = 0; t < kTracers; ++t) {
     const int jc = t + 1 + (t + 1 >= D.g ? 1 : 0);
     const float* r = Ss.rho + (long long)(jc - 1) * D.fstride;
-    const float comp = r[i_e] * a_e + r[i_n] * a_n - r[i_w] * a_w - r[i_s] * a_s + r[i_u] * a_u - r[i_l] * a_l;
-    dv[t] = comp * iv;
+    const float hor = fmaf(-r[i_s], a_s, fmaf(-r[i_w], a_w, fmaf(r[i_e], a_e, r[i_n] * a_n)));
+    dv[t] = fmaf(-r[i_l], a_l, fmaf(r[i_u], a_u, hor)) * iv;
   }
   if (mdt) {  // mass diffusion: -div + mass_diff_tendency
 #pragma unroll
@@ -1672,8 +1728,9 @@ dim3 cblk() { return dim3(32, 4, 1); }
 dim3 cgrd(int rows, int cols) { return dim3((unsigned)((rows + 31) / 32), (unsigned)((cols + 3) / 4), 1u); }
 // the marching divergences: the column in as many chunks as give the device about 128 warps an SM,
 // of at least 4 levels.  (One chunk: ks_gas_div 187, 421, 505, 1772 us at 4x256x60, 128x128x80,
-// 256x256x80, 768x768x80; so: 24, 62, 245, 1718 us.  64 warps an SM: 72 us at 128x128x80, 1899 us at
-// 768x768x80; two levels a chunk at least: 64 us at 128x128x80.)
+// 256x256x80, 768x768x80; so: 24, 62, 245, 1718 us, and 50, 198, 1145 us at the last three since it
+// loads layers ahead.  64 warps an SM: 72 us at 128x128x80, 1899 us at 768x768x80; two levels a chunk at
+// least: 64 us at 128x128x80, both before that.)
 dim3 cgrd_levels(const Dims& D) {
   dim3 g = cgrd(D.ny, D.nx);
   const long long warps = 4LL * g.x * g.y;
@@ -1734,6 +1791,7 @@ int split_create(const Dims& D, bool column_fp64, const SplitDiff& diff, const S
   else if ((rc = salloc(s, &s->vsq, F, bytes))) return fail(rc);
   if ((rc = salloc(s, &s->gzd, F, bytes)) || (rc = salloc(s, &s->rmz, F, bytes))) return fail(rc);
   if (D.nc > 0 && (rc = salloc(s, &s->csh_part, F * D.nc, bytes))) return fail(rc);
+  if (D.ncons > 1 && (rc = salloc(s, &s->cw, F, bytes))) return fail(rc);
   if ((rc = salloc(s, &s->dbg, F, bytes)) || (rc = salloc(s, &s->tbu, F, bytes)) || (rc = salloc(s, &s->tbv, F, bytes)))
     return fail(rc);
   float** fl[] = {&s->fu, &s->fv, &s->gu, &s->gv};
@@ -2174,15 +2232,6 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
       SYNC(vector_terms(Sn, Mn, true));
     }
     SL("ks_tend_wind", ks_tend_wind, sgrd(D.ny + 1, D.nx + 1, D.NL), B, D, So, Sn, T, CC, C, rk, Mn.u, Mn.v);
-    // side: the tracer tendencies (read the tracer densities of Ms and the new u, v; write the
-    // tracer fields of T.rho), beside the gas fluxes, divergence and vertical solve, which write
-    // the gas field of T.rho, T.rt, the gas density, theta', exner', rhotheta_v and w
-    if (tracers) {
-      SYNC(after(side, stream, EV_B));
-      cur = side;
-      SL("ks_tracers", ks_tracers, sgrd(D.ny, D.nx, D.nl), B, D, GF, s->GX, Ms, Mn.u, Mn.v, T.rho, rk, mdt, ptr);
-      cur = stream;
-    }
     // third-order theta edges of the state used here; in the first substep that is the old
     // state, whose edges the pressure gradient's call above already left in tvu/tvv (nothing
     // in between writes the old mirror or tvu/tvv), so only the second substep recomputes them
@@ -2200,8 +2249,17 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
         return LGAME_ERR_CUDA;
       }
     }
-    SL("ks_gas_div", ks_gas_div, cgrd_levels(D), cblk(), D, GF, s->GX, Ms, s->fu, s->fv, s->gu, s->gv,
-       C.temperature, C.hdiss, C.rad, C.csh, T.rho, T.rt, mdt, tdh, ptr, pth);
+    SL("ks_gas_div", (tracers ? ks_gas_div<true> : ks_gas_div<false>), cgrd_levels(D), cblk(), D, GF, s->GX, Ms, s->fu,
+       s->fv, s->gu, s->gv, C.temperature, C.hdiss, C.rad, C.csh, T.rho, T.rt, mdt, tdh, ptr, pth, Mn.u, Mn.v, s->cw);
+    // side: the tracer tendencies (read the tracer densities of Ms and the new u, v; write the
+    // tracer fields of T.rho), after the gas divergence, which leaves cw, beside the vertical solve, which
+    // writes the gas density, theta', exner', rhotheta_v and w
+    if (tracers) {
+      SYNC(after(side, stream, EV_B));
+      cur = side;
+      SL("ks_tracers", ks_tracers, sgrd(D.ny, D.nx, D.nl), B, D, GF, s->GX, Ms, Mn.u, Mn.v, s->cw, T.rho, rk, mdt, ptr);
+      cur = stream;
+    }
     if (SF.sens || SF.soil)
       SL("ks_sfc_column", k_sfc_column_split<float>, sgrd(D.ny, D.nx, 1), B, D, G, So, rk == 1 ? So : Sn, T.rt,
          SF.buf, SF.par, SF.tsoil[so], SF.tsoil[rk == 1 ? so : sn], SF.tsoil[sn]);
