@@ -790,87 +790,294 @@ __global__ void __launch_bounds__(256, 6) ks_tracers(Dims D, Grid<float> GF, Gri
   }
 }
 
-// the potential vorticity and its flux (calc_pot_vort, mo_vorticities.F90:189-421; vorticity
-// flux, mo_vorticity_flux.F90:16-171) of the split step: the FP32 bodies of k_eta_xy, k_eta_z
-// and k_vort_flux with register caps that keep six blocks of 256 threads resident
-// eta_x, eta_y, eta_z and the mass flux densities (mo_vector_tend_expl.F90:64-66) in one
-// launch: they read the same u, v, w and gas density around a point, which then come through
-// the cache once
-__global__ void __launch_bounds__(256, 6) ks_eta(Dims D, Grid<float> G, StateF S, float* ex, float* ey, float* ez,
+// ---- potential vorticity and its flux, marching down the levels ------------------------------
+// A thread walks a chunk of levels of one plane point (ji, jk).  Everything a level reads is loaded
+// before anything is stored, at addresses that are valid everywhere (the edge kernels' reason), and what two
+// levels share is carried.  The periodic copies at ny+1 and nx+1 evaluate the point they copy.
+struct Around {  // the point (I, K) evaluated and its neighbours' plane offsets at level 1
+  int I, K;
+  bool fi, fk;  // not a non-periodic boundary row, column
+  long long c, n, s, w, e, nw, sw, se, ne;
+};
+__device__ __forceinline__ Around around(const Dims& D, int ji, int jk) {
+  Around A;
+  A.fi = D.periodic || (ji >= 2 && ji <= D.ny);
+  A.fk = D.periodic || (jk >= 2 && jk <= D.nx);
+  A.I = D.periodic && ji == D.ny + 1 ? 1 : ji;
+  A.K = D.periodic && jk == D.nx + 1 ? 1 : jk;
+  const int im = A.I == 1 ? D.ny : A.I - 1, km = A.K == 1 ? D.nx : A.K - 1;
+  const int ip = min(A.I + 1, D.ny + 1), kp = min(A.K + 1, D.nx + 1);
+  A.c = IX(D, A.I, A.K, 1);
+  A.n = IX(D, im, A.K, 1);
+  A.s = IX(D, ip, A.K, 1);
+  A.w = IX(D, A.I, km, 1);
+  A.e = IX(D, A.I, kp, 1);
+  A.nw = IX(D, im, km, 1);
+  A.sw = IX(D, ip, km, 1);
+  A.se = IX(D, ip, kp, 1);
+  A.ne = IX(D, im, kp, 1);
+  return A;
+}
+
+// calc_pot_vort (mo_vorticities.F90:19-421, with rel_vort and rel_vort_z_local) and the mass flux
+// densities (mo_vector_tend_expl.F90:64-66).  Carried from level to level: the winds and heights at the
+// dual point's four sides, w, the products length times covariant wind of the x and y vorticity, and the
+// sums of the density.  One quotient a component, (zeta + f*A)/(A*rho), zeta before its division by the dual
+// area A; the rescaled length (r_e + zd)/(r_e + z) of a dual point's side as 1 + (zd - z)/(r_e + z), since
+// r_e + z has half a metre's resolution in FP32.  The last block in z does ex and ey at level 1 and at the
+// surface, whose formulas are their own.  A thread a point, each term with its own branches, loads and
+// quotients, took 3.37 ms at 1024x1024x80; so 1.80 ms (1.03 ms of memory traffic at the copy rate).
+__global__ void __launch_bounds__(128, 4) ks_eta(Dims D, Grid<float> G, StateF S, float* ex, float* ey, float* ez,
                                                  float* uph, float* vph, float* wph) {
-  LG_IDX3;
-  if (jl > D.NL) return;
-  if (ji <= D.ny + 1 && jk <= D.nx) ex[IX(D, ji, jk, jl)] = eta_x_at<float>(D, G, S, ji, jk, jl);
-  if (ji <= D.ny && jk <= D.nx + 1) ey[IX(D, ji, jk, jl)] = eta_y_at<float>(D, G, S, ji, jk, jl);
-  if (jl > D.nl) return;
-  if (ji <= D.ny + 1 && jk <= D.nx + 1) ez[IX(D, ji, jk, jl)] = eta_z_at<float>(D, G, S, ji, jk, jl);
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny + 1 || jk > D.nx + 1) return;
+  const bool px = jk <= D.nx, py = ji <= D.ny;
+  const int chunks = (int)gridDim.z - 1;
+  if ((int)blockIdx.z == chunks) {
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      const int jl = k ? D.NL : 1;
+      if (px) ex[IX(D, ji, jk, jl)] = eta_x_at<float>(D, G, S, ji, jk, jl);
+      if (py) ey[IX(D, ji, jk, jl)] = eta_y_at<float>(D, G, S, ji, jk, jl);
+    }
+    return;
+  }
+  const int len = (D.nl + chunks - 1) / chunks, l0 = (int)blockIdx.z * len + 1, l1 = min(D.nl, l0 + len - 1);
+  const Around A = around(D, ji, jk);
   const float* rg = S.rho + (long long)(D.g - 1) * D.fstride;
-  if (ji <= D.ny && jk <= D.nx + 1) {
-    float f;
-    if (stv_h_x<float>(D, rg, S.u, ji, jk, jl, &f)) uph[IX(D, ji, jk, jl)] = f;
+  const long long pl = D.plane, q1 = IX(D, ji, jk, 1);
+  const bool zeta = !D.llinear;
+  const float fx = D.lcorio ? G.fvec_x[A.c] : 0.f, fy = D.lcorio ? G.fvec_y[A.c] : 0.f, fz = D.lcorio ? G.fvec_z[A.c] : 0.f;
+  // the dual point's sides: v at (I,K), u at (im,K), v at (I,km), u at (I,K); wind and height at the
+  // level above, here and below
+  float ua[4], ub[4], uc[4], za[4], zb[4], zc[4];
+  auto sides = [&](long long o, float* u, float* z) {
+    u[0] = S.v[A.c + o]; u[1] = S.u[A.n + o]; u[2] = S.v[A.w + o]; u[3] = S.u[A.c + o];
+    z[0] = G.z_v[A.c + o]; z[1] = G.z_u[A.n + o]; z[2] = G.z_v[A.w + o]; z[3] = G.z_u[A.c + o];
+  };
+  struct W { float c, n, w; };
+  auto cells = [&](const float* p, long long o) { return W{p[A.c + o], p[A.n + o], p[A.w + o]}; };
+  // dx (dy) times the covariant wind at the u (v) point of layer l, horizontal_covariant_x/y
+  // (mo_averaging.F90:56-176): wu, wl are w at the layer's upper and lower interface
+  struct Cov { float x, y; };
+  auto covariant = [&](int l, long long o, float u, float v, float dx, float dy, const W& wu, const W& wl) {
+    Cov r{dx * u, dy * v};
+    if (l > D.nf) {
+      const W w5 = cells(G.ipw[4], o), w6 = cells(G.ipw[5], o);
+      const float sx = G.slope_x[A.c + o], sy = G.slope_y[A.c + o];
+      float mx = w5.w * wu.w + w5.c * wu.c, my = w5.n * wu.n + w5.c * wu.c;
+      if (l < D.nl || D.freeslip) {
+        mx = mx + w6.w * wl.w + w6.c * wl.c;
+        my = my + w6.n * wl.n + w6.c * wl.c;
+      }
+      r.x = dx * (u + sx * (0.5f * mx));
+      r.y = dy * (v + sy * (0.5f * my));
+    }
+    return r;
+  };
+  long long o = (long long)(l0 - 1) * pl;
+  W w0 = cells(S.w, o);
+  sides(o, ub, zb);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) { ua[m] = ub[m]; za[m] = zb[m]; }
+  Cov cp{0.f, 0.f};
+  float rx = 0.f, ry = 0.f, rc0 = 0.f;  // density of the layer above: the u (v) point's two cells, the cell
+  if (l0 > 1) {
+    const long long a = o - pl;
+    sides(a, ua, za);
+    const W wa = cells(S.w, a), r = cells(rg, a);
+    cp = covariant(l0 - 1, a, ua[3], ua[0], G.dx[A.c + a], G.dy[A.c + a], wa, w0);
+    rx = r.w + r.c;
+    ry = r.n + r.c;
+    rc0 = r.c;
   }
-  if (ji <= D.ny + 1 && jk <= D.nx) {
-    float f;
-    if (stv_h_y<float>(D, rg, S.v, ji, jk, jl, &f)) vph[IX(D, ji, jk, jl)] = f;
-  }
-  if (jl >= 2 && ji <= D.ny && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    wph[q] = 0.5f * (rg[IX(D, ji, jk, jl - 1)] + rg[q]) * S.w[q];
+  for (int l = l0; l <= l1; ++l, o += pl) {
+    sides(o + pl, uc, zc);  // below the lowest layer: the padding level, not used
+    const W w1 = cells(S.w, o + pl), r = cells(rg, o), dz = cells(G.dz, o);
+    const float rnw = rg[A.nw + o], zd = G.z_area_dual_z[A.c + o];
+    const float dxc = G.dx[A.c + o], dxn = G.dx[A.n + o], dyc = G.dy[A.c + o], dyw = G.dy[A.w + o];
+    const float ax = G.area_dual_x[A.c + o], ay = G.area_dual_y[A.c + o], az = G.area_dual_z[A.c + o];
+    const Cov cv = covariant(l, o, ub[3], ub[0], dxc, dyc, w0, w1);
+    const float length[4] = {dyc, -dxn, -dyw, dxc};
+    float zz = 0.f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (l <= D.nf) {
+        zz += length[m] * ub[m];
+      } else {
+        const float d = zd - zb[m];
+        const bool up = (d > 0.f || l == D.nl) && l > 1;
+        const float zs = up ? za[m] : zc[m], us = up ? ua[m] : uc[m];
+        const float rescaled = fmaf(length[m], d / (float(kR_E) + zb[m]), length[m]);
+        zz += rescaled * (ub[m] + (ub[m] - us) * (d / (zb[m] - zs)));
+      }
+    }
+    if (!zeta) zz = 0.f;
+    const float ez_ = A.fi && A.fk ? (zz + fz * az) / (az * (0.25f * (r.w + r.c + r.n + rnw))) : fz;
+    float ex_ = 0.f, ey_ = 0.f;
+    if (l > 1) {
+      const float zx = zeta ? dz.n * w0.n - cp.y - dz.c * w0.c + cv.y : 0.f;
+      const float zy = zeta ? dz.w * w0.w + cp.x - dz.c * w0.c - cv.x : 0.f;
+      ex_ = A.fi ? (zx + fx * ax) / (ax * (0.25f * (ry + r.n + r.c))) : fx;
+      ey_ = A.fk ? (zy + fy * ay) / (ay * (0.25f * (rx + r.w + r.c))) : fy;
+    }
+    const long long q = q1 + o;
+    ez[q] = ez_;
+    if (l > 1 && px) ex[q] = ex_;
+    if (l > 1 && py) ey[q] = ey_;
+    if (py && A.fk) uph[q] = 0.5f * (r.w + r.c) * ub[3];
+    if (px && A.fi) vph[q] = 0.5f * (r.n + r.c) * ub[0];
+    if (l > 1 && px && py) wph[q] = 0.5f * (rc0 + r.c) * w0.c;
+    cp = cv;
+    w0 = w1;
+    rx = r.w + r.c;
+    ry = r.n + r.c;
+    rc0 = r.c;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) { ua[m] = ub[m]; ub[m] = uc[m]; za[m] = zb[m]; zb[m] = zc[m]; }
   }
 }
-__global__ void __launch_bounds__(256, 6) ks_vort_flux(Dims D, Grid<float> G, StateF S, const float* ex,
+
+// calc_vorticity_flux_term, mo_vorticity_flux.F90:16-171.  Carried from level to level: the vertical mass
+// flux, eta_x and eta_y at the interface between, and the products weight times horizontal mass flux of the layer
+// above, which the vertical component adds to this layer's before the vorticity multiplies both.
+// 1.92 -> 1.18 ms at 1024x1024x80 against a thread a point (0.74 ms of memory traffic).
+__global__ void __launch_bounds__(128, 4) ks_vort_flux(Dims D, Grid<float> G, StateF S, const float* ex,
                                                        const float* ey, const float* ez, const float* uph,
                                                        const float* vph, const float* wph, float* px, float* py,
                                                        float* pz) {
-  vort_flux_body<float, float>(D, G, S, ex, ey, ez, uph, vph, wph, px, py, pz);
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny + 1 || jk > D.nx + 1) return;
+  const LevelChunk lc = level_chunk(D);
+  if (lc.l0 > D.nl) return;
+  const Around A = around(D, ji, jk);
+  const bool out_x = ji <= D.ny && A.fk, out_y = jk <= D.nx && A.fi, cell = ji <= D.ny && jk <= D.nx;
+  const long long pl = D.plane, q1 = IX(D, ji, jk, 1);
+  const int row = min(A.I, D.ny) - 1;
+  const float u1 = 0.25f * G.trsk_u[0][row], u2 = 0.25f * G.trsk_u[1][row], u3 = 0.25f * G.trsk_u[2][row];
+  const float v1 = 0.25f * G.trsk_v[0][row], v2 = 0.25f * G.trsk_v[1][row];
+  // vertical mass flux at the surface: free slip, mo_vector_tend_expl.F90:68-80
+  auto surface = [&](long long p1) {
+    if (!D.freeslip) return 0.f;
+    const float* rg = S.rho + (long long)(D.g - 1) * D.fstride;
+    const long long b = p1 + (long long)(D.nl - 1) * pl, a = b - pl;
+    const float dv = rg[b] + (rg[a] - rg[b]) / (G.z_scalar[a] - G.z_scalar[b]) * (G.z_w[b + pl] - G.z_scalar[b]);
+    return dv * S.w[b + pl];
+  };
+  long long o = (long long)(lc.l0 - 1) * pl;
+  float wc = wph[A.c + o], wn = wph[A.n + o], ww = wph[A.w + o], xc = ex[A.c + o], yc = ey[A.c + o];
+  float fe = 0.f, fn = 0.f, fw = 0.f, fs = 0.f;  // weight times flux through the layer above's faces
+  if (lc.l0 > 1) {
+    const long long a = A.c + o - pl;
+    fe = G.ipw[0][a] * uph[A.e + o - pl];
+    fn = G.ipw[1][a] * vph[a];
+    fw = G.ipw[2][a] * uph[a];
+    fs = G.ipw[3][a] * vph[A.s + o - pl];
+  }
+  for (int l = lc.l0; l <= lc.l1; ++l, o += pl) {
+    const float uc = uph[A.c + o], uw = uph[A.w + o], ue = uph[A.e + o], un = uph[A.n + o], une = uph[A.ne + o];
+    const float vc = vph[A.c + o], vw = vph[A.w + o], vs = vph[A.s + o], vsw = vph[A.sw + o];
+    const float zc = ez[A.c + o], zn = ez[A.n + o], zs = ez[A.s + o], zw = ez[A.w + o], ze = ez[A.e + o];
+    const float zsw = ez[A.sw + o], zse = ez[A.se + o], zne = ez[A.ne + o];
+    const float w1 = G.ipw[0][A.c + o], w2 = G.ipw[1][A.c + o], w3 = G.ipw[2][A.c + o], w4 = G.ipw[3][A.c + o];
+    const float w5c = G.ipw[4][A.c + o], w5n = G.ipw[4][A.n + o], w5w = G.ipw[4][A.w + o];
+    const float w6c = G.ipw[5][A.c + o], w6n = G.ipw[5][A.n + o], w6w = G.ipw[5][A.w + o];
+    const float ye = ey[A.e + o], xs = ex[A.s + o], xd = ex[A.c + o + pl], yd = ey[A.c + o + pl];
+    float dc, dn, dw;
+    if (l < D.nl) {
+      dc = wph[A.c + o + pl];
+      dn = wph[A.n + o + pl];
+      dw = wph[A.w + o + pl];
+    } else {
+      dc = surface(A.c);
+      dn = surface(A.n);
+      dw = surface(A.w);
+    }
+    // the TRSK terms, mo_vorticity_flux.F90:33-45, :72-80
+    const float cs = zc + zs, ce = zc + ze;
+    const float tx = u1 * vw * (zw + zc + cs) + u2 * uw * (zw + zsw + cs) + u3 * vsw * (zsw + zs + cs)
+                   + u3 * vs * (zs + zse + cs) + u2 * ue * (zse + ze + cs) + u1 * vc * (zc + ze + cs);
+    const float ty = v1 * uc * (zc + zs + ce) + v1 * ue * (ze + zse + ce) + v2 * une * (zne + ze + ce)
+                   + v2 * un * (zn + zc + ce);
+    const float rx = tx - 0.5f * (w5w * ww + w5c * wc) * yc - 0.5f * (w6w * dw + w6c * dc) * yd;
+    const float ry = ty + 0.5f * (w5n * wn + w5c * wc) * xc + 0.5f * (w6n * dn + w6c * dc) * xd;
+    const float ge = w1 * ue, gn = w2 * vc, gw = w3 * uc, gs = w4 * vs;
+    const float rz = 0.5f * ((fe + ge) * ye - (fn + gn) * xc + (fw + gw) * yc - (fs + gs) * xs);
+    const long long q = q1 + o;
+    if (out_x) px[q] = rx;
+    if (out_y) py[q] = ry;
+    if (cell && l > 1) pz[q] = rz;
+    wc = dc; wn = dn; ww = dw; xc = xd; yc = yd;
+    fe = ge; fn = gn; fw = gw; fs = gs;
+  }
 }
 
 // combination of the explicit wind tendencies, mo_vector_tend_expl.F90:258-310, and the
-// forward step of the horizontal wind, mo_manage_pchevi.F90:86-89 (FP64 state), split step:
-// the body of k_tend_wind<float> with the pressure-gradient terms of a background state read
-// in the FP32 form ks_pgrad keeps for it (net nl + l and the previous substep's -(nl + l), the
-// values k_tend_wind rounds to FP32 itself); without a background state the FP64 arrays.
-// mu, mv: the FP32 mirrors of the new u, v.
-__global__ void ks_tend_wind(Dims D, State So, State Sn, Tend<float> Tn, Carried<float> C, SplitCarriedF PF,
-                             int rk_step, float* mu, float* mv) {
+// forward step of the horizontal wind, mo_manage_pchevi.F90:86-89 (FP64 state), split step,
+// with the pressure-gradient terms of a background state read in the FP32 form ks_pgrad keeps for it
+// (net nl + l and the previous substep's -(nl + l)); without a background state the FP64 arrays.
+// The three components' loads come first (the edge kernels' reason); the first substep (old weight 0) does
+// not read the old tendency: 1.85 -> 1.49 ms at 1024x1024x80 (1.33 ms of memory traffic).  mu, mv: the FP32 mirrors of the new u, v.
+__global__ void __launch_bounds__(256, 5) ks_tend_wind(Dims D, State So, State Sn, Tend<float> Tn, Carried<float> C,
+                                                       SplitCarriedF PF, int rk_step, float* mu, float* mv) {
   LG_IDX3;
-  const float new_weight = (rk_step == 2) ? 0.5f : 1.f;
-  const float old_weight = 1.f - new_weight;
+  if (ji > D.ny + 1 || jk > D.nx + 1) return;
   const double chw_d = 0.5 + kIMPL_THERMO_WEIGHT, ohw_d = 1.0 - (0.5 + kIMPL_THERMO_WEIGHT);
-  const double cvw_d = 1.0 - kIMPL_THERMO_WEIGHT, no_bg_d = D.luse_bg ? 0.0 : 1.0;
-  auto pg_h = [&](const float* old_f, const float* net_f, const double* old, const double* nl, const double* l,
-                  long long q) -> float {
-    if (D.luse_bg) return float(ohw_d) * old_f[q] - float(chw_d) * net_f[q];
-    return narrow(ohw_d * old[q] - chw_d * (nl[q] + l[q]));
-  };
-  if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
-    const long long q = IX(D, ji, jk, jl);
-    float f = pg_h(PF.pold_u, PF.pnet_u, C.old_u, C.nl_u, C.l_u, q) - 0.5f * C.vsg_x[q] + C.pvt_x[q];
-    if (C.mdt_x) f = f + C.mdt_x[q];
-    const float t = old_weight * Tn.u[q] + new_weight * f;
-    Tn.u[q] = t;
-    const double un = So.u[q] + D.dtime * wide(t);
-    Sn.u[q] = un;
-    mu[q] = narrow(un);
+  const double cvw_d = 1.0 - kIMPL_THERMO_WEIGHT;
+  const int i = min(ji, D.ny), k = min(jk, D.nx), l = min(jl, D.nl);
+  const long long qu = IX(D, i, jk, l), qv = IX(D, ji, k, l), qw = IX(D, i, k, jl);
+  float gu, gv, gw;
+  if (D.luse_bg) {
+    const float ou = PF.pold_u[qu], nu = PF.pnet_u[qu], ov = PF.pold_v[qv], nv = PF.pnet_v[qv], nw = PF.pnet_w[qw];
+    gu = float(ohw_d) * ou - float(chw_d) * nu;
+    gv = float(ohw_d) * ov - float(chw_d) * nv;
+    gw = -(float(cvw_d) * nw);
+  } else {
+    const double ou = C.old_u[qu], nu = C.nl_u[qu], lu = C.l_u[qu], ov = C.old_v[qv], nv = C.nl_v[qv], lv = C.l_v[qv];
+    const double nw = C.nl_w[qw], lw = C.l_w[qw];
+    gu = narrow(ohw_d * ou - chw_d * (nu + lu));
+    gv = narrow(ohw_d * ov - chw_d * (nv + lv));
+    gw = narrow(-(cvw_d * (nw + lw)) - (1.0 - cvw_d) * lw);
   }
-  if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    float f = pg_h(PF.pold_v, PF.pnet_v, C.old_v, C.nl_v, C.l_v, q) - 0.5f * C.vsg_y[q] + C.pvt_y[q];
-    if (C.mdt_y) f = f + C.mdt_y[q];
-    const float t = old_weight * Tn.v[q] + new_weight * f;
-    Tn.v[q] = t;
-    const double vn = So.v[q] + D.dtime * wide(t);
-    Sn.v[q] = vn;
-    mv[q] = narrow(vn);
+  const float ku = C.vsg_x[qu], kv = C.vsg_y[qv], kw = C.vsg_z[qw];
+  const float vu = C.pvt_x[qu], vv = C.pvt_y[qv], vw = C.pvt_z[qw], cw = C.pgcw[qw];
+  const double uo = So.u[qu], vo = So.v[qv];
+  float du = 0.f, dv = 0.f, dw = 0.f, tu = 0.f, tv = 0.f, tw = 0.f;
+  if (C.mdt_x) {
+    du = C.mdt_x[qu];
+    dv = C.mdt_y[qv];
+    dw = C.mdt_z[qw];
   }
-  if (jl <= D.NL && ji <= D.ny && jk <= D.nx) {
-    const long long q = IX(D, ji, jk, jl);
-    const float pg = D.luse_bg ? -(float(cvw_d) * PF.pnet_w[q])
-                               : narrow(-(cvw_d * (C.nl_w[q] + C.l_w[q])) - no_bg_d * (1.0 - cvw_d) * C.l_w[q]);
-    float f = pg - 0.5f * C.vsg_z[q] + C.pvt_z[q] + C.pgcw[q];
-    if (C.mdt_z) f = f + C.mdt_z[q];
-    Tn.w[q] = old_weight * Tn.w[q] + new_weight * f;
+  if (rk_step == 2) {
+    tu = Tn.u[qu];
+    tv = Tn.v[qv];
+    tw = Tn.w[qw];
   }
+  float fu = gu - 0.5f * ku + vu, fv = gv - 0.5f * kv + vv, fw = gw - 0.5f * kw + vw + cw;
+  if (C.mdt_x) {
+    fu = fu + du;
+    fv = fv + dv;
+    fw = fw + dw;
+  }
+  if (rk_step == 2) {
+    fu = 0.5f * tu + 0.5f * fu;
+    fv = 0.5f * tv + 0.5f * fv;
+    fw = 0.5f * tw + 0.5f * fw;
+  }
+  const double un = uo + D.dtime * wide(fu), vn = vo + D.dtime * wide(fv);
+  if (jl <= D.nl && ji <= D.ny) {
+    Tn.u[qu] = fu;
+    Sn.u[qu] = un;
+    mu[qu] = narrow(un);
+  }
+  if (jl <= D.nl && jk <= D.nx) {
+    Tn.v[qv] = fv;
+    Sn.v[qv] = vn;
+    mv[qv] = narrow(vn);
+  }
+  if (ji <= D.ny && jk <= D.nx) Tn.w[qw] = fw;
 }
 
 // ---- three_band_solver_ver, mo_column_solvers.F90:21-351 --------------------------------
@@ -1731,8 +1938,8 @@ dim3 cgrd(int rows, int cols) { return dim3((unsigned)((rows + 31) / 32), (unsig
 // 256x256x80, 768x768x80; so: 24, 62, 245, 1718 us, and 50, 198, 1145 us at the last three since it
 // loads layers ahead.  64 warps an SM: 72 us at 128x128x80, 1899 us at 768x768x80; two levels a chunk at
 // least: 64 us at 128x128x80, both before that.)
-dim3 cgrd_levels(const Dims& D) {
-  dim3 g = cgrd(D.ny, D.nx);
+dim3 cgrd_levels(const Dims& D, int rows, int cols) {
+  dim3 g = cgrd(rows, cols);
   const long long warps = 4LL * g.x * g.y;
   const int chunks = (int)std::min<long long>((kSMs * 128LL + warps - 1) / warps, D.nl);
   const int len = std::max((D.nl + chunks - 1) / chunks, 4);
@@ -2113,7 +2320,7 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
                      float* pv) -> int {
     SL("ks_grad_vert", (k_grad_vert<float, float>), sgrd(D.ny, D.nx, D.nl - 1), B, D, GF, tp, s->gz);
     SL("ks_grad_hor", ks_grad_hor<float>, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, tp, s->gz, s->gx, s->gy);
-    SL("ks_div_h", ks_div_h, cgrd_levels(D), cblk(), D, GF, s->GX, s->gx, s->gy, s->divf);
+    SL("ks_div_h", ks_div_h, cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, s->GX, s->gx, s->gy, s->divf);
     SL("ks_theta_edges", ks_theta_edges, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, tp, s->divf, s->dbg, s->tbu, s->tbv, u,
        v, ou, ov, pu, pv);
     return LGAME_OK;
@@ -2149,9 +2356,10 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
          C.vsg_x, C.vsg_y);
     }
     cur = stream;
-    SL("ks_eta", ks_eta, sgrd(D.ny + 1, D.nx + 1, D.NL), B, D, GF, Mv, s->ex, s->ey, s->ez, s->uph, s->vph, s->wph);
-    SL("ks_vort_flux", ks_vort_flux, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, Mv, s->ex, s->ey,
-       s->ez, s->uph, s->vph, s->wph, C.pvt_x, C.pvt_y, C.pvt_z);
+    const dim3 gp = cgrd_levels(D, D.ny + 1, D.nx + 1), ge(gp.x, gp.y, gp.z + 1);
+    SL("ks_eta", ks_eta, ge, cblk(), D, GF, Mv, s->ex, s->ey, s->ez, s->uph, s->vph, s->wph);
+    SL("ks_vort_flux", ks_vort_flux, gp, cblk(), D, GF, Mv, s->ex, s->ey, s->ez, s->uph, s->vph, s->wph, C.pvt_x,
+       C.pvt_y, C.pvt_z);
     if (ke && branch) SYNC(after(stream, side2, EV_JKE));
     return LGAME_OK;
   };
@@ -2249,7 +2457,7 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
         return LGAME_ERR_CUDA;
       }
     }
-    SL("ks_gas_div", (tracers ? ks_gas_div<true> : ks_gas_div<false>), cgrd_levels(D), cblk(), D, GF, s->GX, Ms, s->fu,
+    SL("ks_gas_div", (tracers ? ks_gas_div<true> : ks_gas_div<false>), cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, s->GX, Ms, s->fu,
        s->fv, s->gu, s->gv, C.temperature, C.hdiss, C.rad, C.csh, T.rho, T.rt, mdt, tdh, ptr, pth, Mn.u, Mn.v, s->cw);
     // side: the tracer tendencies (read the tracer densities of Ms and the new u, v; write the
     // tracer fields of T.rho), after the gas divergence, which leaves cw, beside the vertical solve, which
