@@ -115,86 +115,8 @@ __device__ __forceinline__ T div_wind_at(const Dims& D, const Grid<T>& G, const 
   return div_h_at<T>(D, G, fx, fy, ji, jk, jl);
 }
 
-// ---- 1. update_n_squared and tke_update (first substep, any horizontal diffusion on) ----------
-// One thread per scalar point.  Reads the old TKE, viscosity and heating_diss; writes the
-// updated TKE to tke_new (the old one is still read by neighbours) and n_squared.
-template <class T, class V>
-__global__ void k_diff_tke(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, DiffPar P) {
-  LG_IDX3;
-  if (ji > D.ny || jk > D.nx) return;
-  const long long q = IX(D, ji, jk, jl);
-  // update_n_squared, mo_eff_diff_coeffs.F90:620-669: g * 0.5*(1/theta(l-1) + 1/theta(l)) *
-  // dtheta/dz at w level l in 2..nl, zero at levels 1 and nl+1
-  auto nz = [&](int l) -> T {
-    if (l < 2 || l > D.nl) return T(0);
-    const long long a = IX(D, ji, jk, l - 1), b = IX(D, ji, jk, l);
-    const T th_a = G.theta_v_bg[a] + T(S.tp[a]), th_b = G.theta_v_bg[b] + T(S.tp[b]);
-    const T grad = (th_a - th_b) / G.dz[b];
-    return G.gm[b] * (half_of(T(1) / th_a + T(1) / th_b) * grad);
-  };
-  T nsq;
-  if (jl == 1) nsq = nz(1);
-  else if (jl == D.nl) nsq = nz(D.nl + 1);
-  else nsq = W_(5, ji, jk, jl) * nz(jl) + W_(6, ji, jk, jl) * nz(jl + 1);
-  B.nsq[q] = nsq;
-  // tke_update, mo_tke.F90:19-66: the inner product of the wind with grad(tke)
-  const T* tke = B.tke;
-  auto gz = [&](int i, int j, int l) -> T {  // grad_vert(tke), zero at levels 1 and nl+1
-    if (l < 2 || l > D.nl) return T(0);
-    return (tke[IX(D, i, j, l - 1)] - tke[IX(D, i, j, l)]) / G.dz[IX(D, i, j, l)];
-  };
-  auto remap_gx = [&](int i, int j, int l) -> T {  // remap_ver2hor_x of gz
-    T r = T(0);
-    if (j == 1 || j == D.nx + 1) {
-      if (!D.periodic) return r;
-      r = r + W_(5, i, D.nx, l) * gz(i, D.nx, l);
-      r = r + W_(5, i, 1, l) * gz(i, 1, l);
-      if (l < D.nl || D.freeslip) { r = r + W_(6, i, D.nx, l) * gz(i, D.nx, l + 1); r = r + W_(6, i, 1, l) * gz(i, 1, l + 1); }
-    } else {
-      r = r + W_(5, i, j - 1, l) * gz(i, j - 1, l);
-      r = r + W_(5, i, j, l) * gz(i, j, l);
-      if (l < D.nl || D.freeslip) { r = r + W_(6, i, j - 1, l) * gz(i, j - 1, l + 1); r = r + W_(6, i, j, l) * gz(i, j, l + 1); }
-    }
-    return half_of(r);
-  };
-  auto remap_gy = [&](int i, int j, int l) -> T {  // remap_ver2hor_y of gz
-    T r = T(0);
-    if (i == 1 || i == D.ny + 1) {
-      if (!D.periodic) return r;
-      r = r + W_(5, D.ny, j, l) * gz(D.ny, j, l);
-      r = r + W_(5, 1, j, l) * gz(1, j, l);
-      if (l < D.nl || D.freeslip) { r = r + W_(6, D.ny, j, l) * gz(D.ny, j, l + 1); r = r + W_(6, 1, j, l) * gz(1, j, l + 1); }
-    } else {
-      r = r + W_(5, i - 1, j, l) * gz(i - 1, j, l);
-      r = r + W_(5, i, j, l) * gz(i, j, l);
-      if (l < D.nl || D.freeslip) { r = r + W_(6, i - 1, j, l) * gz(i - 1, j, l + 1); r = r + W_(6, i, j, l) * gz(i, j, l + 1); }
-    }
-    return half_of(r);
-  };
-  auto gx = [&](int i, int j, int l) -> T {  // grad_hor x at a u point; non-periodic boundary: 0
-    T r;
-    if (!grad_x_cov<T, T>(D, G, tke, i, j, l, &r)) return T(0);
-    if (l > D.nf) r = r - G.slope_x[IX(D, i, j, l)] * remap_gx(i, j, l);
-    return r;
-  };
-  auto gy = [&](int i, int j, int l) -> T {
-    T r;
-    if (!grad_y_cov<T, T>(D, G, tke, i, j, l, &r)) return T(0);
-    if (l > D.nf) r = r - G.slope_y[IX(D, i, j, l)] * remap_gy(i, j, l);
-    return r;
-  };
-  const T adv = W_(1, ji, jk, jl) * T(S.u[IX(D, ji, jk + 1, jl)]) * gx(ji, jk + 1, jl)
-              + W_(2, ji, jk, jl) * T(S.v[q]) * gy(ji, jk, jl)
-              + W_(3, ji, jk, jl) * T(S.u[q]) * gx(ji, jk, jl)
-              + W_(4, ji, jk, jl) * T(S.v[IX(D, ji + 1, jk, jl)]) * gy(ji + 1, jk, jl)
-              + W_(5, ji, jk, jl) * T(S.w[q]) * gz(ji, jk, jl)
-              + W_(6, ji, jk, jl) * T(S.w[q + D.plane]) * gz(ji, jk, jl + 1);
-  const T rg = T(S.rho[q + (long long)(D.g - 1) * D.fstride]);
-  const T decay_constant = T(8.0 * (kPI * kPI)) / T(P.mva) * B.visc[q] / rg;
-  T t = tke[q] + T(D.dtime) * (-adv + B.hd[q] / rg - decay_constant * tke[q]);
-  if (t < T(0)) t = T(0);
-  B.tke_new[q] = t;
-}
+// ---- 1. update_n_squared and tke_update (first substep, any horizontal diffusion on): ks_diff_tke in
+// split.cu, k64_diff_tke in kernels_fp64.cu
 
 // ---- 2. hor_viscosity (mo_eff_diff_coeffs.F90:24-159) -------------------------------------
 // One thread per scalar point: viscosity_molecular, the eddy viscosity (Smagorinsky from the

@@ -266,26 +266,6 @@ __device__ __forceinline__ T eta_y_at(const Dims& D, const Grid<T>& G, const Sta
   return e;
 }
 
-// eta_z at (ji,jk,jl), mo_vorticities.F90:176-186 and :377-419
-template <class T, class V>
-__device__ __forceinline__ T eta_z_at(const Dims& D, const Grid<T>& G, const StateT<V>& S, int ji, int jk, int jl) {
-  if (D.periodic) {
-    if (ji == D.ny + 1) ji = 1;
-    if (jk == D.nx + 1) jk = 1;
-  }
-  T z = T(0);
-  if (!D.llinear) z = rel_vort_z_local<T, V>(D, G, S.u, S.v, ji, jk, jl) / G.area_dual_z[IX(D, ji, jk, jl)];
-  T e = D.lcorio ? z + G.fvec_z[IX(D, ji, jk, 1)] : z;
-  const bool inner = ji >= 2 && ji <= D.ny && jk >= 2 && jk <= D.nx;
-  if (inner || D.periodic) {
-    const V* rg = S.rho + (long long)(D.g - 1) * D.fstride;
-    const int km = (jk == 1) ? D.nx : jk - 1, im = (ji == 1) ? D.ny : ji - 1;
-    e = e / (quarter_of(T(rg[IX(D, ji, km, jl)]) + T(rg[IX(D, ji, jk, jl)]) + T(rg[IX(D, im, jk, jl)]) +
-                        T(rg[IX(D, im, km, jl)])));
-  }
-  return e;
-}
-
 // TRSK term for u, mo_vorticity_flux.F90:33-45 (km, kk, kp: columns jk-1, jk, jk+1)
 template <class T>
 __device__ __forceinline__ T trsk_u(const Dims& D, const Grid<T>& G, const T* vp, const T* up, const T* ez,
@@ -385,61 +365,6 @@ __global__ void k_div_h(Dims D, Grid<T> G, const T* vx, const T* vy, T* out) {
   auto fx = [&](int i, int j, int k) { return vx[IX(D, i, j, k)]; };
   auto fy = [&](int i, int j, int k) { return vy[IX(D, i, j, k)]; };
   out[IX(D, ji, jk, jl)] = div_h_at<T>(D, G, fx, fy, ji, jk, jl);
-}
-
-// calc_vorticity_flux_term, mo_vorticity_flux.F90:16-171
-template <class T, class V = double>
-__device__ __forceinline__ void vort_flux_body(const Dims& D, const Grid<T>& G, const StateT<V>& S, const T* ex,
-                                               const T* ey, const T* ez, const T* uph, const T* vph, const T* wph,
-                                               T* px, T* py, T* pz) {
-  LG_IDX3;
-  // vertical mass flux with the free-slip surface value, mo_vector_tend_expl.F90:68-80
-  auto wp = [&](int i, int j, int k) -> T {
-    if (k == D.NL) {
-      if (!D.freeslip) return T(0);
-      const V* rg = S.rho + (long long)(D.g - 1) * D.fstride;
-      const T dv = T(rg[IX(D, i, j, D.nl)]) + (T(rg[IX(D, i, j, D.nl - 1)]) - T(rg[IX(D, i, j, D.nl)]))
-                   / (G.z_scalar[IX(D, i, j, D.nl - 1)] - G.z_scalar[IX(D, i, j, D.nl)])
-                   * (G.z_w[IX(D, i, j, D.NL)] - G.z_scalar[IX(D, i, j, D.nl)]);
-      return dv * T(S.w[IX(D, i, j, D.NL)]);
-    }
-    return wph[IX(D, i, j, k)];
-  };
-  if (jl <= D.nl && ji <= D.ny && jk <= D.nx + 1) {
-    const bool inner = jk >= 2 && jk <= D.nx;
-    if (inner || D.periodic) {
-      const int kk = inner ? jk : 1, km = inner ? jk - 1 : D.nx, kp = kk + 1;
-      T r = trsk_u<T>(D, G, vph, uph, ez, ji, km, kk, kp, jl);
-      r = r - half_of(W_(5, ji, km, jl)) * wp(ji, km, jl) * ey[IX(D, ji, kk, jl)]
-            - half_of(W_(6, ji, km, jl)) * wp(ji, km, jl + 1) * ey[IX(D, ji, kk, jl + 1)]
-            - half_of(W_(5, ji, kk, jl)) * wp(ji, kk, jl) * ey[IX(D, ji, kk, jl)]
-            - half_of(W_(6, ji, kk, jl)) * wp(ji, kk, jl + 1) * ey[IX(D, ji, kk, jl + 1)];
-      px[IX(D, ji, jk, jl)] = r;
-    }
-  }
-  if (jl <= D.nl && ji <= D.ny + 1 && jk <= D.nx) {
-    const bool inner = ji >= 2 && ji <= D.ny;
-    if (inner || D.periodic) {
-      const int ii = inner ? ji : 1, im = inner ? ji - 1 : D.ny;
-      T r = trsk_v<T>(D, G, uph, ez, im, ii, jk, jl);
-      r = r + half_of(W_(5, im, jk, jl)) * wp(im, jk, jl) * ex[IX(D, ii, jk, jl)]
-            + half_of(W_(6, im, jk, jl)) * wp(im, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)]
-            + half_of(W_(5, ii, jk, jl)) * wp(ii, jk, jl) * ex[IX(D, ii, jk, jl)]
-            + half_of(W_(6, ii, jk, jl)) * wp(ii, jk, jl + 1) * ex[IX(D, ii, jk, jl + 1)];
-      py[IX(D, ji, jk, jl)] = r;
-    }
-  }
-  if (jl >= 2 && jl <= D.nl && ji <= D.ny && jk <= D.nx) {
-    pz[IX(D, ji, jk, jl)] = half_of(
-        W_(1, ji, jk, jl - 1) * uph[IX(D, ji, jk + 1, jl - 1)] * ey[IX(D, ji, jk + 1, jl)]
-      - W_(2, ji, jk, jl - 1) * vph[IX(D, ji, jk, jl - 1)] * ex[IX(D, ji, jk, jl)]
-      + W_(3, ji, jk, jl - 1) * uph[IX(D, ji, jk, jl - 1)] * ey[IX(D, ji, jk, jl)]
-      - W_(4, ji, jk, jl - 1) * vph[IX(D, ji + 1, jk, jl - 1)] * ex[IX(D, ji + 1, jk, jl)]
-      + W_(1, ji, jk, jl) * uph[IX(D, ji, jk + 1, jl)] * ey[IX(D, ji, jk + 1, jl)]
-      - W_(2, ji, jk, jl) * vph[IX(D, ji, jk, jl)] * ex[IX(D, ji, jk, jl)]
-      + W_(3, ji, jk, jl) * uph[IX(D, ji, jk, jl)] * ey[IX(D, ji, jk, jl)]
-      - W_(4, ji, jk, jl) * vph[IX(D, ji + 1, jk, jl)] * ex[IX(D, ji + 1, jk, jl)]);
-  }
 }
 
 // inner_product of the wind with itself, mo_inner_product.F90:16-50

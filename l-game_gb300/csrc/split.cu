@@ -1014,6 +1014,218 @@ __global__ void __launch_bounds__(128, 4) ks_vort_flux(Dims D, Grid<float> G, St
   }
 }
 
+// ---- update_n_squared and tke_update of the diffusion closure -----------------------------------
+// (mo_eff_diff_coeffs.F90:620-669, mo_tke.F90:19-66; diffusion.cuh says what the reference's work arrays
+// hold), marching like ks_eta: the vertical gradients of the TKE at the interfaces of the cell and its
+// four neighbours are formed once and carried, and so are theta_v and its part of n_squared.  Reads the old
+// TKE, viscosity and heating_diss; writes tke_new (neighbours still read the old one) and n_squared.
+// A thread a cell formed the gradients at each of its four faces anew: 3.11 -> 1.52 ms at 1024x1024x80.
+__global__ void __launch_bounds__(128, 4) ks_diff_tke(Dims D, Grid<float> G, StateF S, DiffBuf<float> B, DiffPar P) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const LevelChunk lc = level_chunk(D);
+  if (lc.l0 > D.nl) return;
+  // the cell, then its west, east, north and south neighbours (across the periodic edges), and whether the
+  // edge towards them is a non-periodic boundary's, whose gradient is 0
+  const bool per = D.periodic;
+  const long long pl = D.plane, q1 = IX(D, ji, jk, 1);
+  const long long p1[5] = {q1, IX(D, ji, jk == 1 ? D.nx : jk - 1, 1), IX(D, ji, jk == D.nx ? 1 : jk + 1, 1),
+                           IX(D, ji == 1 ? D.ny : ji - 1, jk, 1), IX(D, ji == D.ny ? 1 : ji + 1, jk, 1)};
+  const bool in_w = per || jk > 1, in_e = per || jk < D.nx, in_n = per || ji > 1, in_s = per || ji < D.ny;
+  const long long e1 = q1 + D.P, s1 = q1 + 1;  // the east u point, the south v point
+  const float* rg = S.rho + (long long)(D.g - 1) * D.fstride;
+  const float decay = float(8.0 * (kPI * kPI)) / float(P.mva);
+  auto theta = [&](long long p) { return G.theta_v_bg[p] + S.tp[p]; };
+  long long o = (long long)(lc.l0 - 1) * pl;
+  // t: TKE of layer l; g: its gradient at the layer's upper interface, 0 at the top
+  float t[5], g[5], th = theta(q1 + o), nz = 0.f, w = S.w[q1 + o];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    t[m] = B.tke[p1[m] + o];
+    g[m] = 0.f;
+  }
+  // g*0.5*(1/theta(l-1) + 1/theta(l))*dtheta/dz at the interface p between theta_v a and b
+  auto n_squared = [&](long long p, float a, float b, float dz) {
+    return G.gm[p] * (0.5f * (1.f / a + 1.f / b) * ((a - b) / dz));
+  };
+  if (lc.l0 > 1) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) g[m] = (B.tke[p1[m] + o - pl] - t[m]) / G.dz[p1[m] + o];
+    nz = n_squared(q1 + o, theta(q1 + o - pl), th, G.dz[q1 + o]);
+  }
+  for (int l = lc.l0; l <= lc.l1; ++l, o += pl) {
+    const bool below = l < D.nl;
+    const long long d = below ? o + pl : o;
+    float tn[5], dz[5], w5[5], w6[5], gn[5], h[5], sw = 0.f, se = 0.f, sn = 0.f, ss = 0.f;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      tn[m] = B.tke[p1[m] + d];
+      dz[m] = G.dz[p1[m] + d];
+      w5[m] = m == 0 || l > D.nf ? G.ipw[4][p1[m] + o] : 0.f;
+      w6[m] = m == 0 || l > D.nf ? G.ipw[5][p1[m] + o] : 0.f;
+    }
+    if (l > D.nf) {
+      sw = G.slope_x[q1 + o];
+      se = G.slope_x[e1 + o];
+      sn = G.slope_y[q1 + o];
+      ss = G.slope_y[s1 + o];
+    }
+    const long long q = q1 + o;
+    const float dxw = G.dx[q], dxe = G.dx[p1[2] + o], dyn = G.dy[q], dys = G.dy[p1[4] + o];
+    const float w1 = G.ipw[0][q], w2 = G.ipw[1][q], w3 = G.ipw[2][q], w4 = G.ipw[3][q];
+    const float ue = S.u[e1 + o], uw = S.u[q], vn = S.v[q], vs = S.v[s1 + o], wn = S.w[q + pl];
+    const float visc = B.visc[q], rho = rg[q], hd = B.hd[q], thn = theta(q1 + d), gm = G.gm[q1 + d];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      gn[m] = below ? (t[m] - tn[m]) / dz[m] : 0.f;
+      h[m] = w5[m] * g[m] + w6[m] * gn[m];  // the column's part of the remap to its faces
+    }
+    const float nzn = below ? gm * (0.5f * (1.f / th + 1.f / thn) * ((th - thn) / dz[0])) : 0.f;
+    const float gw = in_w ? (t[0] - t[1]) / dxw - sw * (0.5f * (h[1] + h[0])) : 0.f;
+    const float ge = in_e ? (t[2] - t[0]) / dxe - se * (0.5f * (h[0] + h[2])) : 0.f;
+    const float gN = in_n ? (t[3] - t[0]) / dyn - sn * (0.5f * (h[3] + h[0])) : 0.f;
+    const float gS = in_s ? (t[0] - t[4]) / dys - ss * (0.5f * (h[0] + h[4])) : 0.f;
+    const float adv = w1 * ue * ge + w2 * vn * gN + w3 * uw * gw + w4 * vs * gS + w5[0] * w * g[0] + w6[0] * wn * gn[0];
+    const float r = t[0] + float(D.dtime) * (-adv + hd / rho - decay * visc / rho * t[0]);
+    B.nsq[q] = l == 1 || l == D.nl ? 0.f : w5[0] * nz + w6[0] * nzn;
+    B.tke_new[q] = r < 0.f ? 0.f : r;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      t[m] = tn[m];
+      g[m] = gn[m];
+    }
+    th = thn;
+    nz = nzn;
+    w = wn;
+  }
+}
+
+// hor_viscosity (k_diff_visc, diffusion.cuh) with the divergence of the wind formed as in ks_div_h: 2.14 ->
+// 1.13 ms at 1024x1024x80
+__global__ void __launch_bounds__(128) ks_diff_visc(Dims D, Grid<float> G, GridX X, StateF S, const float* Tm,
+                                                    DiffBuf<float> B, DiffPar P) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const LevelChunk lc = level_chunk(D);
+  if (lc.l0 > D.nl) return;
+  auto fx = [&](int i, int j, int k) { return S.u[IX(D, i, j, k)]; };
+  auto fy = [&](int i, int j, int k) { return S.v[IX(D, i, j, k)]; };
+  const float* rho = S.rho + (long long)(D.g - 1) * D.fstride;
+  LayerFaces cur = layer_faces(D, G, fx, fy, ji, jk, lc.l0), nxt{};
+  float h_prev = 0.f;
+  if (lc.l0 - 1 >= D.nf + 1) h_prev = layer_faces(D, G, fx, fy, ji, jk, lc.l0 - 1).h;
+  for (int jl = lc.l0; jl <= lc.l1; ++jl) {
+    const long long q = IX(D, ji, jk, jl);
+    const float rg = rho[q], t = Tm[q], tke = B.tke_new[q];
+    float vac = 0.f;
+    if (!P.tke_h) vac = 0.25f * (B.zz[q] + B.zz[q + D.P] + B.zz[q + 1] + B.zz[q + D.P + 1]);
+    nxt.h = 0.f;
+    if (jl < D.nl || jl == D.nf) nxt = layer_faces(D, G, fx, fy, ji, jk, jl + 1);
+    const float dv = div_col(D, G, X, cur, vert_faces(D, h_prev, cur.h, nxt.h, jl), ji, jk, jl);
+    const float vmol = diff_coeff_t<float>(t, rg);
+    float eddy;
+    if (P.tke_h) {
+      eddy = tke2hor<float>(P, tke);
+    } else {
+      const float a = vac * vac + dv * dv, b = float(P.bg_shear) * float(P.bg_shear);
+      eddy = float(P.c_s) * float(P.mva) * sqrtf(a > b ? a : b);
+    }
+    const float visc = rg * (vmol + eddy);
+    B.vmol[q] = vmol;
+    B.visc[q] = visc;
+    B.vdiv[q] = visc * dv;
+    B.tke[q] = tke;
+    h_prev = cur.h;
+    cur = nxt;
+  }
+}
+
+// mom_diff_h (mo_momentum_diff_diss.F90:25-160; k_mom_diff_h, diffusion.cuh), marching like ks_eta: the
+// dual points' viscosity times vorticity and heights, and the w points' accelerations, are carried: 2.32 ->
+// 1.95 ms at 1024x1024x80.
+__global__ void __launch_bounds__(128, 5) ks_mom_diff_h(Dims D, Grid<float> G, StateF S, DiffBuf<float> B) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const LevelChunk lc = level_chunk(D);
+  if (lc.l0 > D.nl) return;
+  const bool in_x = D.periodic || jk >= 2, in_y = D.periodic || ji >= 2;
+  const long long pl = D.plane, c1 = IX(D, ji, jk, 1), w1 = IX(D, ji, jk >= 2 ? jk - 1 : D.nx, 1),
+                  n1 = IX(D, ji >= 2 ? ji - 1 : D.ny, jk, 1);
+  const long long d1[3] = {c1, c1 + 1, c1 + D.P};  // dual points (ji, jk), (ji+1, jk), (ji, jk+1)
+  const long long x1 = IX(D, ji, D.nx + 1, 1), y1 = IX(D, D.ny + 1, jk, 1);
+  const float* zd = G.z_area_dual_z;
+  struct W { float c, w, n; };
+  auto cells = [&](const float* p, long long o) { return W{p[c1 + o], p[w1 + o], p[n1 + o]}; };
+  long long o = (long long)(lc.l0 - 1) * pl;
+  float va[3], vb[3], vc[3], za[3], zb[3], zc[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const long long u = lc.l0 > 1 ? o - pl : o;
+    va[m] = B.vz[d1[m] + u];
+    za[m] = zd[d1[m] + u];
+    vb[m] = B.vz[d1[m] + o];
+    zb[m] = zd[d1[m] + o];
+  }
+  W mu = cells(B.mdtz, o);
+  for (int l = lc.l0; l <= lc.l1; ++l, o += pl) {
+    const long long q = c1 + o, d = l < D.nl ? o + pl : o;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      vc[m] = B.vz[d1[m] + d];
+      zc[m] = zd[d1[m] + d];
+    }
+    const W ml = cells(B.mdtz, o + pl), sd = cells(B.vdiv, o);
+    W r = cells(S.rho, o);
+    for (int jc = 1; jc <= D.nc; ++jc) {
+      const W x = cells(S.rho + (long long)jc * D.fstride, o);
+      r.c = r.c + x.c;
+      r.w = r.w + x.w;
+      r.n = r.n + x.n;
+    }
+    const float dx = G.dx[q], dy = G.dy[q], dyd = G.dy_dual[q], dxd = G.dx_dual[q];
+    float rx = in_x ? 0.f : B.mdtx[q], ry = in_y ? 0.f : B.mdty[q];
+    float mx = 0.f, my = 0.f;
+    if (l > D.nf) {
+      const W w5 = cells(G.ipw[4], o), w6 = cells(G.ipw[5], o);
+      const float sx = G.slope_x[q], sy = G.slope_y[q];
+      mx = w5.w * mu.w + w5.c * mu.c;
+      my = w5.n * mu.n + w5.c * mu.c;
+      if (l < D.nl || D.freeslip) {
+        mx = mx + w6.w * ml.w + w6.c * ml.c;
+        my = my + w6.n * ml.n + w6.c * ml.c;
+      }
+      mx = sx * (0.5f * mx);
+      my = sy * (0.5f * my);
+    }
+    float grad[3];  // half the vertical gradient over the layers above and below
+#pragma unroll
+    for (int m = 0; m < 3; ++m) grad[m] = 0.5f * (va[m] - vc[m]) / (za[m] - zc[m]);
+    if (in_x) {
+      const float up = (vb[1] - vb[0]) / dyd - (zb[1] - zb[0]) / dyd * (grad[1] + grad[0]);
+      rx = ((sd.c - sd.w) / dx - mx + up) / (0.5f * (r.w + r.c));
+    }
+    if (in_y) {
+      const float vp = (vb[2] - vb[0]) / dxd - (zb[2] - zb[0]) / dxd * (grad[2] + grad[0]);
+      ry = ((sd.n - sd.c) / dy - my + vp) / (0.5f * (r.n + r.c));
+    }
+    B.mdtx[q] = rx;
+    B.mdty[q] = ry;
+    if (jk == 1) B.mdtx[x1 + o] = rx;
+    if (ji == 1) B.mdty[y1 + o] = ry;
+    mu = ml;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      va[m] = vb[m];
+      vb[m] = vc[m];
+      za[m] = zb[m];
+      zb[m] = zc[m];
+    }
+  }
+}
+
 // combination of the explicit wind tendencies, mo_vector_tend_expl.F90:258-310, and the
 // forward step of the horizontal wind, mo_manage_pchevi.F90:86-89 (FP64 state), split step,
 // with the pressure-gradient terms of a background state read in the FP32 form ks_pgrad keeps for it
@@ -2381,11 +2593,12 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
       }
       if (SD.mom_h) {
         const dim3 gs = sgrd(D.ny, D.nx, D.nl);
-        SL("ks_diff_tke", (k_diff_tke<float, float>), gs, B, D, GF, Mo, DB, SD.par);
+        SL("ks_diff_tke", ks_diff_tke, cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, Mo, DB, SD.par);
         SL("ks_diff_zeta", (k_diff_zeta<float, float>), sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, Mo, DB);
-        SL("ks_diff_visc", (k_diff_visc<float, float>), gs, B, D, GF, Mo, (const float*)C.temperature, DB, SD.par);
+        SL("ks_diff_visc", ks_diff_visc, cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, s->GX, Mo, (const float*)C.temperature,
+           DB, SD.par);
         SL("ks_diff_vz", (k_diff_vz<float, float>), sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, Mo, DB);
-        SL("ks_mom_diff_h", (k_mom_diff_h<float, float>), gs, B, D, GF, Mo, DB);
+        SL("ks_mom_diff_h", ks_mom_diff_h, cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, Mo, DB);
         if (SD.mom_v) SL("ks_mom_diff_v", (k_mom_diff_v<float, float>), sgrd(D.ny, D.nx, D.nl - 1), B, D, GF, Mo, DB);
         if (SF.pbl)
           SL("ks_pbl", (k_pbl<float, float>), sgrd(D.ny, D.nx, 1), B, D, G, So, s->vsq, SF.buf, SF.par, DB.mdtx, DB.mdty);
