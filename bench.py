@@ -122,6 +122,7 @@ def _kernel_fields(ncons: int) -> dict:
         "theta": (1, 2, 0, 0),                         # theta'; theta_bg, out
         "grad_vert": (0, 3, 0, 0),                     # field, dz, out
         "grad_hor": (0, 5, 0, 5),                      # field, dx, dy, 2 out; slopes, dz-gradient, 2 weights
+        "grad": (0, 6, 0, 4),                          # both: field, dx, dy, dz, 2 out; slopes, 2 weights
         "div_h": (0, 6, 0, 7),                         # 2 in, area_x/y, volume, out; area_z, slopes, 4 weights
         "theta_edges": (2, 4, 0, 0),                   # u, v; theta, div, 2 out
         "eta_xy": (4, 11, 0, 0),                       # u, v, w, rho_g; dx,dy,dz,z_u,z_v,z_w,z_scalar,2 dual areas, 2 out

@@ -57,7 +57,7 @@ struct SplitCtx {
   float *ipw[6] = {}, *trsk_u[3] = {}, *trsk_v[2] = {};
   double *inv_dx = nullptr, *inv_dy = nullptr, *inv_dz = nullptr, *inv_volume = nullptr, *inv_area_z = nullptr;
   // FP32 intermediates
-  float *gx, *gy, *gz, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph;
+  float *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph;
   // kinetic energy in FP64: its vertical differences over thin layers cancel most digits
   double* vsq = nullptr;
   // FP64 vertical gradient of exner' at w points (0 at the top and surface levels), and per
@@ -450,36 +450,6 @@ __global__ void ks_heating_diss(Dims D, Grid<float> GF, GridX X, StateF M, float
   hd[q] = -rho_sum_cond_gas<float, float>(D, M.rho, q) * ip;
 }
 
-// grad_hor, mo_gradient_operators.F90:17-63 + :85-130, at the u and v points of layer jl, S the type
-// of the scalar (FP64: the kinetic energy; its differences are taken in FP64 and rounded)
-template <class S>
-__global__ void ks_grad_hor(Dims D, Grid<float> G, const S* s, const float* rz, float* rx, float* ry) {
-  LG_IDX3;
-  if (ji > D.ny + 1 || jk > D.nx + 1) return;
-  const long long q = IX(D, ji, jk, jl), pl = D.plane;
-  const Edge x = edge_x(D, ji, jk, jl), y = edge_y(D, ji, jk, jl);
-  const S xa = s[x.a], xb = s[x.b], ya = s[y.a], yb = s[y.b];
-  const float dx = G.dx[x.b], dy = G.dy[y.b];
-  float r, t;
-  if (jl > D.nf) {
-    const bool lower = jl < D.nl || D.freeslip;
-    const float *w5 = G.ipw[4], *w6 = G.ipw[5];
-    const float sx = G.slope_x[x.q], sy = G.slope_y[y.q];
-    float mx = w5[x.a] * rz[x.a] + w5[x.b] * rz[x.b], my = w5[y.a] * rz[y.a] + w5[y.b] * rz[y.b];
-    if (lower) {
-      mx = mx + w6[x.a] * rz[x.a + pl] + w6[x.b] * rz[x.b + pl];
-      my = my + w6[y.a] * rz[y.a + pl] + w6[y.b] * rz[y.b + pl];
-    }
-    r = cvt<float>(xb - xa) / dx - sx * (0.5f * mx);
-    t = cvt<float>(ya - yb) / dy - sy * (0.5f * my);
-  } else {
-    r = cvt<float>(xb - xa) / dx;
-    t = cvt<float>(ya - yb) / dy;
-  }
-  if (x.flux) rx[q] = r;
-  if (y.flux) ry[q] = t;
-}
-
 // ---- column-marching divergences -------------------------------------------------------
 // div_h with the contravariant vertical correction (div_h_at above: div_h,
 // mo_divergence_operators.F90:16-68, and vertical_contravariant_corr, mo_averaging.F90:16-54)
@@ -817,6 +787,73 @@ __device__ __forceinline__ Around around(const Dims& D, int ji, int jk) {
   A.se = IX(D, ip, kp, 1);
   A.ne = IX(D, im, kp, 1);
   return A;
+}
+
+// grad_vert and grad_hor, mo_gradient_operators.F90:17-130, S the type of the scalar (FP64: the kinetic
+// energy; its differences are taken in FP64 and rounded).  The vertical gradients at the interfaces of an
+// edge's cells are formed here and carried; with VERT they are kept too (levels 2..nl of rz, whose first
+// and surface levels, which no operator writes, are read as they are).  One kernel for the two, which wrote
+// and read the vertical gradient in between: 3.31 -> 2.38 ms for the three of a step at 1024x1024x80.
+template <class S, bool VERT>
+__global__ void __launch_bounds__(128) ks_grad(Dims D, Grid<float> G, const S* s, float* rx, float* ry, float* rz) {
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny + 1 || jk > D.nx + 1) return;
+  const LevelChunk lc = level_chunk(D);
+  if (lc.l0 > D.nl) return;
+  const Around A = around(D, ji, jk);
+  const bool px = jk <= D.nx, py = ji <= D.ny;
+  const long long pl = D.plane, q1 = IX(D, ji, jk, 1);
+  const long long p[3] = {A.c, A.n, A.w};
+  long long o = (long long)(lc.l0 - 1) * pl;
+  S t[3];
+  float g[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    t[m] = s[p[m] + o];
+    g[m] = lc.l0 > 1 ? cvt<float>(s[p[m] + o - pl] - t[m]) / G.dz[p[m] + o] : VERT ? rz[p[m]] : 0.f;
+  }
+  for (int l = lc.l0; l <= lc.l1; ++l, o += pl) {
+    const bool below = l < D.nl;
+    S tn[3];
+    float dz[3], w5[3], w6[3], gn[3], sx = 0.f, sy = 0.f;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      tn[m] = s[p[m] + (below ? o + pl : o)];
+      dz[m] = below ? G.dz[p[m] + o + pl] : (VERT ? rz[p[m] + o + pl] : 0.f);
+    }
+    const float dx = G.dx[A.c + o], dy = G.dy[A.c + o];
+    if (l > D.nf) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        w5[m] = G.ipw[4][p[m] + o];
+        w6[m] = G.ipw[5][p[m] + o];
+      }
+      sx = G.slope_x[q1 + o];
+      sy = G.slope_y[q1 + o];
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) gn[m] = below ? cvt<float>(t[m] - tn[m]) / dz[m] : dz[m];
+    float x = cvt<float>(t[0] - t[2]) / dx, y = cvt<float>(t[1] - t[0]) / dy;
+    if (l > D.nf) {
+      float mx = w5[2] * g[2] + w5[0] * g[0], my = w5[1] * g[1] + w5[0] * g[0];
+      if (below || D.freeslip) {
+        mx = mx + w6[2] * gn[2] + w6[0] * gn[0];
+        my = my + w6[1] * gn[1] + w6[0] * gn[0];
+      }
+      x = x - sx * (0.5f * mx);
+      y = y - sy * (0.5f * my);
+    }
+    const long long q = q1 + o;
+    if (py && A.fk) rx[q] = x;
+    if (px && A.fi) ry[q] = y;
+    if (VERT && px && py && l > 1) rz[q] = g[0];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      t[m] = tn[m];
+      g[m] = gn[m];
+    }
+  }
 }
 
 // calc_pot_vort (mo_vorticities.F90:19-421, with rel_vort and rel_vort_z_local) and the mass flux
@@ -2202,7 +2239,7 @@ int split_create(const Dims& D, bool column_fp64, const SplitDiff& diff, const S
       (rc = salloc(s, &s->inv_dz, F, bytes)) || (rc = salloc(s, &s->inv_volume, F, bytes)) ||
       (rc = salloc(s, &s->inv_area_z, F, bytes)))
     return fail(rc);
-  float** scratch[] = {&s->gx, &s->gy, &s->gz, &s->divf, &s->tvu, &s->tvv, &s->tpu, &s->tpv,
+  float** scratch[] = {&s->gx, &s->gy, &s->divf, &s->tvu, &s->tvv, &s->tpu, &s->tpv,
                        &s->ex, &s->ey, &s->ez, &s->uph, &s->vph, &s->wph};
   for (float** p : scratch) if ((rc = salloc(s, p, F, bytes))) return fail(rc);
   s->sfc = sfc;
@@ -2530,8 +2567,8 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
   // the edges of theta_bg + theta' (and of theta' alone when pu/pv are given)
   auto theta3f = [&](const float* tp, const float* u, const float* v, float* ou, float* ov, float* pu,
                      float* pv) -> int {
-    SL("ks_grad_vert", (k_grad_vert<float, float>), sgrd(D.ny, D.nx, D.nl - 1), B, D, GF, tp, s->gz);
-    SL("ks_grad_hor", ks_grad_hor<float>, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, tp, s->gz, s->gx, s->gy);
+    SL("ks_grad", (ks_grad<float, false>), cgrd_levels(D, D.ny + 1, D.nx + 1), cblk(), D, GF, tp, s->gx, s->gy,
+       (float*)nullptr);
     SL("ks_div_h", ks_div_h, cgrd_levels(D, D.ny, D.nx), cblk(), D, GF, s->GX, s->gx, s->gy, s->divf);
     SL("ks_theta_edges", ks_theta_edges, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, tp, s->divf, s->dbg, s->tbu, s->tbv, u,
        v, ou, ov, pu, pv);
@@ -2563,9 +2600,8 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
     }
     if (ke) {
       SL("ks_ke", ks_ke, sgrd(D.ny, D.nx, D.nl), B, D, G, Sv, s->vsq);
-      SL("ks_grad_vert", (k_grad_vert<float, double>), sgrd(D.ny, D.nx, D.nl - 1), B, D, GF, s->vsq, C.vsg_z);
-      SL("ks_grad_hor", ks_grad_hor<double>, sgrd(D.ny + 1, D.nx + 1, D.nl), B, D, GF, s->vsq, C.vsg_z,
-         C.vsg_x, C.vsg_y);
+      SL("ks_grad", (ks_grad<double, true>), cgrd_levels(D, D.ny + 1, D.nx + 1), cblk(), D, GF, s->vsq, C.vsg_x, C.vsg_y,
+         C.vsg_z);
     }
     cur = stream;
     const dim3 gp = cgrd_levels(D, D.ny + 1, D.nx + 1), ge(gp.x, gp.y, gp.z + 1);
