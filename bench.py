@@ -134,6 +134,7 @@ def _kernel_fields(ncons: int) -> dict:
         "tracers": (ntr + 2, 2 * ntr + 3, 0, 7),       # rho_jc, u, v; tend r/w per tracer, area_x/y, volume
         "gas_theta": (3, 9, 0, 7),                     # rho_g, u, v; 2 theta edges, area_x/y, volume, rad, csh, 2 out
         "gas_flux": (0, 9, 0, 0),                      # rho_g, u, v, 2 theta edges; 4 fluxes out
+        "theta_flux": (0, 14, 0, 0),                   # rho_g, theta', u, v, 2 divergences, 2 pairs of background edges; 4 fluxes
         "gas_div": (0, 11, 0, 7),                      # 4 fluxes, area_x/y, volume, rad, csh; 2 tendencies out
     }
 
