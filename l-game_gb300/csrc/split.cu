@@ -39,14 +39,13 @@ struct GridX {  // FP64 reciprocal metrics and FP32 metric differences of the FP
 // x / d to FP64 accuracy for an FP32 divisor d in the normal range.  r = 1/d correctly
 // rounded in FP32; the residual 1 - d*r of a correctly rounded reciprocal is exact in FP32,
 // so r + (1 - d*r)*r is 1/d to ~2^-48 as an unevaluated pair of FP32 numbers (the
-// correction step of Markstein's division), and x*(r + r_lo) costs two FP64-pipe operations
-// (relative error below 2^-47) instead of a conversion and an FP64 division.
+// correction step of Markstein's division), and x*(r + r_lo) costs one FP64-pipe operation and a
+// product formed beside that pipe (relative error below 2^-47) instead of a conversion and an FP64 division.
 __device__ __forceinline__ double div_f(double x, float d) {
   const float r = __frcp_rn(d);
   const float r_lo = __fmaf_rn(-d, r, 1.f) * r;
-  return fma(x, wide(r_lo), x * wide(r));
+  return fma(x, wide(r_lo), mul_int(r, x));
 }
-
 }  // namespace
 
 struct SplitCtx {
@@ -1371,12 +1370,14 @@ __global__ void __launch_bounds__(256, 5) ks_tend_wind(Dims D, State So, State S
 // FP32).
 //
 // Two kernels (the rule between them stands at their launch in split_step).  Large grids:
-// ks_column_ver, one thread per column, streamed top to bottom and back; every warp issues FP64
-// work all the time, which is what bounds it (about 26 FP64 operations a cell).  Small grids:
-// ks_column_ver_tile below.
+// ks_column_ver, one thread per column, streamed top to bottom and back, bound by about 20 FP64
+// operations a cell and the latency of a level's loads.  Six more products are formed beside the FP64 pipe
+// (fp64.cuh; the hardware's: 1.41 against 1.34 ms at 512x512x80), and the increment of rho*theta_v serves both it
+// and exner'; with each layer's inputs loaded a level ahead (five blocks of 96 registers an SM; six of 80: 1.42
+// ms) 1.57 -> 1.34 ms.  Small grids: ks_column_ver_tile below.
 constexpr int kMaxLayers = 128;  // layers a context may have (lgame_gpu_create)
 template <class C>
-__global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
+__global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
                                                      State Sn, StateF Mo, StateF Mn, Tend<float> Tn, int rk_step) {
   constexpr bool F64 = sizeof(C) == 8;
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
@@ -1412,88 +1413,100 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
   };
   auto W = [](C x) -> double { if constexpr (F64) return x; else return wide(x); };
   auto Nr = [](double x) -> float { return narrow(x); };
+  auto M = [](C a, double x) -> double { if constexpr (F64) return a * x; else return mul_int(a, x); };
   auto quot = [](double x, C d) -> double { if constexpr (F64) return x / d; else return div_f(x, d); };
 
-  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
-  // state, where theta * d(exner')/dz carries the whole hydrostatic balance)
-  struct Lay { C a, b, g, th, ro, iv; double thd; };
-  auto layer = [&](int jl) -> Lay {
+  // what a layer and an interface (w level) read; the layer's is loaded a level ahead of its use (the
+  // interfaces' ahead too spills: 1.35 ms at 512x512x80)
+  struct LayIn { C ro, rt, eb, ep, iv, ru, rtu, epu, tr, trt; double tp, epd; };
+  auto layer_in = [&](int jl) -> LayIn {
+    LayIn R{};
+    if (jl > nl) return R;
     const long long i = IX(D, ji, jk, jl);
-    Lay L;
-    L.thd = D.luse_bg ? 0.0 : Su.rt[i] / Su.rho[goff + i];
-    const C ro = rho_o(i), rto = rt_o(i);
-    const C iro = C(1) / ro, irto = C(1) / rto;
-    L.a = -rto * iro * iro;
-    L.b = iro;
-    L.g = rdcv * irto * (ebg(i) + ep_o(i));
-    if (rk_step == 2) {
-      const C ru = rho_u(i), rtu = rt_u(i);
-      const C iru = C(1) / ru, irtu = C(1) / rtu;
-      L.a = C(0.5) * (L.a - rtu * iru * iru);
-      L.b = C(0.5) * (L.b + iru);
-      L.g = C(0.5) * (L.g + rdcv * irtu * (ebg(i) + ep_u(i)));
-      L.th = rtu * iru;
-    } else {
-      L.th = rto * iro;
-    }
-    L.ro = ro;
-    L.iv = ivol(i);
-    return L;
+    R.ro = rho_o(i); R.rt = rt_o(i); R.eb = ebg(i); R.ep = ep_o(i); R.iv = ivol(i);
+    if (rk_step == 2) { R.ru = rho_u(i); R.rtu = rt_u(i); R.epu = ep_u(i); }
+    R.tr = C(Tn.rho[goff + i]); R.trt = C(Tn.rt[i]);
+    R.tp = So.tp[i]; R.epd = So.ep[i];
+    return R;
   };
-  // explicit predictions of theta_v' and exner' (FP64 state plus increments) and of rho_g
-  auto predict = [&](int jl, const Lay& L, double* tpe, double* epe, C* rhe) {
+  struct ItfIn { C dz, deb, dp, w, iaz, tw; double wd; };
+  auto itf_in = [&](int jl) -> ItfIn {
+    ItfIn R{};
+    if (jl > nl) return R;
     const long long i = IX(D, ji, jk, jl);
-    const C tr = C(Tn.rho[goff + i]), trt = C(Tn.rt[i]);
-    *tpe = So.tp[i] + W(dtf * (L.a * tr + L.b * trt));
-    *epe = So.ep[i] + W(dtf * L.g * trt);
-    *rhe = L.ro + dtf * tr;
+    R.dz = dzs(i); R.deb = debg(i); R.dp = damp(i); R.w = w_o(i); R.iaz = iarz(i); R.tw = C(Tn.w[i]);
+    R.wd = So.w[i];
+    return R;
+  };
+  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
+  // state, where theta * d(exner')/dz carries the whole hydrostatic balance); the explicit predictions of
+  // theta_v' and exner' (FP64 state plus increments) and of rho_g
+  struct Lay { C a, b, g, th, ro, iv, rhe; double thd, tpe, epe; };
+  auto layer = [&](int jl, const LayIn& R) -> Lay {
+    Lay L;
+    const long long i = IX(D, ji, jk, jl);
+    L.thd = D.luse_bg ? 0.0 : Su.rt[i] / Su.rho[goff + i];
+    const C iro = C(1) / R.ro, irto = C(1) / R.rt;
+    L.a = -R.rt * iro * iro;
+    L.b = iro;
+    L.g = rdcv * irto * (R.eb + R.ep);
+    if (rk_step == 2) {
+      const C iru = C(1) / R.ru, irtu = C(1) / R.rtu;
+      L.a = C(0.5) * (L.a - R.rtu * iru * iru);
+      L.b = C(0.5) * (L.b + iru);
+      L.g = C(0.5) * (L.g + rdcv * irtu * (R.eb + R.epu));
+      L.th = R.rtu * iru;
+    } else {
+      L.th = R.rt * iro;
+    }
+    L.ro = R.ro;
+    L.iv = R.iv;
+    L.tpe = R.tp + W(dtf * (L.a * R.tr + L.b * R.trt));
+    L.epe = R.epd + W(dtf * L.g * R.trt);
+    L.rhe = R.ro + dtf * R.tr;
+    return L;
   };
 
   C epr[kMaxLayers + 1];       // elimination multipliers
   double rpr[kMaxLayers + 1];  // substituted right-hand side, then the solution (FP64)
   C tis[kMaxLayers + 1];       // interface theta
   C gs[kMaxLayers + 1];        // gamma of each layer
-  Lay L0 = layer(1), L1 = layer(2), L2{};
-  double tpe0, epe0, tpe1, epe1, tpe2 = 0.0, epe2 = 0.0;
-  C rhe0, rhe1, rhe2 = C(0);
-  predict(1, L0, &tpe0, &epe0, &rhe0);
-  predict(2, L1, &tpe1, &epe1, &rhe1);
+  Lay L0 = layer(1, layer_in(1)), L1 = layer(2, layer_in(2)), L2{};
+  LayIn R = layer_in(3);
   gs[1] = L0.g;
   C cv_prev = C(0), epr_prev = C(0);
   double rpr_prev = 0.0;
+  // at the interface below layer jl: theta, and 2/(rho(jl) + rho(jl+1))
+  C ti = C(0.5) * (L0.th + L1.th), irio = C(2) / (L0.ro + L1.ro);
   for (int jl = 1; jl <= n; ++jl) {  // row jl: level jl+1 between layers jl (a) and jl+1 (b)
-    const long long ib = IX(D, ji, jk, jl + 1);
+    const LayIn Rn = layer_in(jl + 3);
+    const ItfIn I1 = itf_in(jl + 1), I2 = itf_in(jl + 2);
     gs[jl + 1] = L1.g;
-    const C ti = C(0.5) * (L0.th + L1.th);
     tis[jl] = ti;
-    const C irio = C(2) / (L0.ro + L1.ro);
-    const C dz = dzs(ib), deb = debg(ib), dp = damp(ib);
-    const double wo = So.w[ib];
-    const C wof = w_o(ib);
+    const C dz = I1.dz, deb = I1.deb, dp = I1.dp, wof = I1.w;
+    const double wo = I1.wd;
     const C al0 = L0.a * L0.iv, al1 = L1.a * L1.iv, be0 = L0.b * L0.iv, be1 = L1.b * L1.iv;
     const C ga0 = L0.g * L0.iv, ga1 = L1.g * L1.iv;
     const C dv = -(ti * ti) * (ga0 + ga1) + C(0.5) * deb * (al1 - al0 + ti * (be1 - be0))
-                 - dz * ic2 * irio * (C(2) * iarz(ib) + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
-    const C rie = C(0.5) * (rhe0 + rhe1);
+                 - dz * ic2 * irio * (C(2) * I1.iaz + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
+    const C rie = C(0.5) * (L0.rhe + L1.rhe);
     // The products of FP32 coefficients with FP64 values here and in the state update below
     // stay FP64 products of the FP32 factors: merging two FP32 factors into one rounded
     // coefficient (e.g. -dz*ic2*(1 + rie*irio) for w_old) saves two FP64 operations per cell
     // but lets an atmosphere at rest over hills drift about four times faster (1e-8 instead
     // of 3e-9 m/s of spurious wind after 3 h at 256 x 256 x 50).
-    double rv = (wo + W(dtf * C(Tn.w[ib]))) * W(-dz * ic2);
-    rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, epe0 - epe1, rv);
-    rv = fma(W(C(0.5) * idtf * deb), tpe0 + tpe1, rv);
+    double rv = M(-dz * ic2, wo + W(dtf * I1.tw));
+    rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
+    rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
     rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
     // couplings with row jl+1 (layer b's derivatives), which need layer jl+2
-    C cv = C(0), ev = C(0);
+    C cv = C(0), ev = C(0), ti_n = C(0), irio_n = C(0);
     if (jl < n) {
-      L2 = layer(jl + 2);
-      predict(jl + 2, L2, &tpe2, &epe2, &rhe2);
-      const long long ic = IX(D, ji, jk, jl + 2);
-      const C ti_n = C(0.5) * (L1.th + L2.th);
-      const C irio_n = C(2) / (L1.ro + L2.ro);
-      cv = ti_n * ga1 * ti + C(0.5) * debg(ic) * (al1 + be1 * ti)
-           - dzs(ic) * ic1 * C(0.5) * w_o(ic) * L1.iv * irio_n * damp(ic);
+      L2 = layer(jl + 2, R);
+      ti_n = C(0.5) * (L1.th + L2.th);
+      irio_n = C(2) / (L1.ro + L2.ro);
+      cv = ti_n * ga1 * ti + C(0.5) * I2.deb * (al1 + be1 * ti)
+           - I2.dz * ic1 * C(0.5) * I2.w * L1.iv * irio_n * I2.dp;
       ev = ti * ga1 * ti_n - C(0.5) * deb * (al1 + be1 * ti_n) + dz * ic1 * C(0.5) * wof * L1.iv * irio * dp;
     }
     const C piv = dv - epr_prev * cv_prev;
@@ -1504,8 +1517,9 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
     epr[jl] = epr_prev;
     cv_prev = cv;
     L0 = L1; L1 = L2;
-    tpe0 = tpe1; epe0 = epe1; rhe0 = rhe1;
-    tpe1 = tpe2; epe1 = epe2; rhe1 = rhe2;
+    R = Rn;
+    ti = ti_n;
+    irio = irio_n;
   }
   // back substitution fused with the new state, mo_column_solvers.F90:300-345, bottom to top:
   // layer jl needs the solutions of the rows above (w level jl) and below it (w level jl+1),
@@ -1531,6 +1545,7 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
   };
   StateIn in_cur = state_in(nl), in_up{}, in_below{};
   double s1 = 0.0;     // solution at the interface below the layer (w level jl+1)
+  double p1 = 0.0;     // theta there times it
   C rnf_below = C(0);  // new rho_g of the layer below (FP32: rounded)
   for (int jl = nl; jl >= 1; --jl) {
     if (jl > 1) in_up = state_in(jl - 1);
@@ -1538,15 +1553,13 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
     // solution of row jl-1 (w level jl), the interface above the layer
     double s0 = 0.0;
     if (jl >= 2) s0 = (jl - 1 == n) ? rpr[n] : fma(-W(epr[jl - 1]), s1, rpr[jl - 1]);
-    const C t0 = (jl >= 2) ? tis[jl - 1] : C(0);
-    const C t1 = (jl <= n) ? tis[jl] : C(0);
+    const double p0 = (jl >= 2) ? M(tis[jl - 1], s0) : 0.0;
     const double dtv = W(dtf * in_cur.ivf);
-    const double rto = in_cur.rt;
     const double rho_e = in_cur.rho + W(dtf * C(in_cur.trho));
-    const double rt_e = rto + W(dtf * C(in_cur.trt));
     const double rn = fma(dtv, s1 - s0, rho_e);
-    const double rtn = fma(dtv, fma(-W(t0), s0, W(t1) * s1), rt_e);
-    const double epn = fma(W(gs[jl]), rtn - rto, in_cur.ep);
+    const double inc = fma(dtv, p1 - p0, W(dtf * C(in_cur.trt)));
+    const double rtn = in_cur.rt + inc;
+    const double epn = fma(W(gs[jl]), inc, in_cur.ep);
     const float rnf = Nr(rn);
     const C rnc = F64 ? C(rn) : C(rnf);
     if constexpr (F64) {
@@ -1568,11 +1581,12 @@ __global__ void __launch_bounds__(128, 6) ks_column_ver(Dims D, Grid<double> G, 
       const long long ib = i + D.plane;
       const C rin = C(0.5) * (rnc + rnf_below);
       const C irio = C(2) / (in_cur.mro + in_below.mro);
-      const double wn = fma(-W(rin), in_below.w, W(C(2) * in_below.iaz) * s1) * W(irio);
+      const double wn = M(irio, fma(-W(rin), in_below.w, M(C(2) * in_below.iaz, s1)));
       Sn.w[ib] = wn;
       Mn.w[ib] = Nr(wn);
     }
     s1 = s0;
+    p1 = p0;
     rnf_below = rnc;
     in_below = in_cur;
     in_cur = in_up;
@@ -1635,6 +1649,7 @@ struct ColVer {
     if constexpr (F64) return G.exner_bg[i - D.plane] - G.exner_bg[i]; else return X.deb_f[i];
   }
   static __device__ double W(C x) { if constexpr (F64) return x; else return wide(x); }
+  static __device__ double M(C a, double x) { if constexpr (F64) return a * x; else return mul_int(a, x); }
   static __device__ double quot(double x, C d) { if constexpr (F64) return x / d; else return div_f(x, d); }
 
   // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
@@ -1689,7 +1704,7 @@ struct ColVer {
     r.dv = -(ti * ti) * (ga0 + ga1) + C(0.5) * deb * (al1 - al0 + ti * (be1 - be0))
            - dz * ic2 * irio * (C(2) * iarz(ib) + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
     const C rie = C(0.5) * (L0.rhe + L1.rhe);
-    double rv = (wo + W(dtf * C(Tn.w[ib]))) * W(-dz * ic2);
+    double rv = M(-dz * ic2, wo + W(dtf * C(Tn.w[ib])));
     rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
     rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
     r.rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
@@ -1735,9 +1750,9 @@ struct ColVer {
     const long long i = IX(D, ji, jk, jl);
     const double dtv = W(dtf * c.ivf);
     const double rn = new_rho(c, s0, s1);
-    const double rt_e = c.rt + W(dtf * C(c.trt));
-    const double rtn = fma(dtv, fma(-W(t0), s0, W(t1) * s1), rt_e);
-    const double epn = fma(W(g), rtn - c.rt, c.ep);
+    const double inc = fma(dtv, M(t1, s1) - M(t0, s0), W(dtf * C(c.trt)));
+    const double rtn = c.rt + inc;
+    const double epn = fma(W(g), inc, c.ep);
     const float rnf = narrow(rn);
     const C rnc = F64 ? C(rn) : C(rnf);
     if constexpr (F64) {
@@ -1759,7 +1774,7 @@ struct ColVer {
       const long long ib = i + D.plane;
       const C rin = C(0.5) * (rnc + rnc_below);
       const C irio = C(2) / (c.mro + below.mro);
-      const double wn = fma(-W(rin), below.w, W(C(2) * below.iaz) * s1) * W(irio);
+      const double wn = M(irio, fma(-W(rin), below.w, M(C(2) * below.iaz, s1)));
       Sn.w[ib] = wn;
       Mn.w[ib] = narrow(wn);
     }
@@ -1786,10 +1801,10 @@ struct ColVer {
 //   3. every thread its rows' y/p;  4. the first TC threads the back substitution;
 //   5. every thread the new state of its chunk of layers.
 // The chain of levels then waits on shared memory and arithmetic alone, and the levels' loads and
-// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 34 against 280
-// us at 4 x 256 x 60, 150 against 381 us at 128 x 128 x 80; equal (460 us) at 256 x 256 x 80, and
-// slower above (3.6 against 3.2 ms at 768 x 768 x 80), where the phases in which one warp works
-// cost more than the latency they hide.
+// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 33 against 280
+// us at 4 x 256 x 60, 140 against 381 us at 128 x 128 x 80, 279 against 376 us at 180 x 210 x 80, equal (415 us)
+// at 230 x 236 x 80, and slower above, where the phases in which one warp works cost more than the
+// latency they hide.
 template <class C, int TC, int NW>
 __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
     ks_column_ver_tile(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So, State Sn, StateF Mo, StateF Mn,
@@ -2750,8 +2765,8 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
     // The vertical solve by the number of columns: up to 8 columns an SM, 8 a block with 32 chunks of
     // levels (34 us at 1,024 columns of 60 layers; 54 with 32 x 12); up to the size that gives
     // every SM sub-partition three warps of columns, 32 a block with 12 chunks (150 us at 16,384
-    // columns of 80 layers; 216 with 8 x 32); above, a thread a column (461 us at 65,536 columns
-    // of 80 layers; 502 with 32 x 12).  The FP64-coefficient solve keeps twice the shared memory
+    // columns of 80 layers; 216 with 8 x 32); above, a thread a column (equal, 415 us, at 54,280 columns of
+    // 80 layers; 199 against 354 at 22,500).  The FP64-coefficient solve keeps twice the shared memory
     // a column and takes 16 columns a block.
     const long long cols = (long long)D.ny * D.nx;
 #define CV_ARGS D, G, GF, s->GX, So, Sn, Mo, Mn, T, rk
