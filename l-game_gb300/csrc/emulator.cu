@@ -146,12 +146,16 @@ __device__ __forceinline__ float gelu_grad(float z) {
 //                    with its chain of erff: 24.5 against 20.3 us for 8192 x 512 x 512.)
 // Every wait is bounded and also ends when another role has given up (a shared abort flag);
 // the CTA then waits (bounded) for its own copies and MMAs before freeing tensor memory.
-template <int BN>
+// PLAIN: FP32 results without a fused epilogue or split K, whose epilogue two groups keep up with; what the
+// other groups' staging tiles would take holds the full ring (65536 x 512 x 512: three stages and four groups
+// 47.2 us, four and two 40.8 us; 8192 x 512 x 512 9.2 and 8.8 us).
+template <int BN, bool PLAIN>
 struct GemmCfg {
   static constexpr uint32_t kCols = (BN <= 32) ? 32 : (BN <= 64) ? 64 : (BN <= 128) ? 128 : 256;  // one accumulator
   static constexpr uint32_t kA = 128 * 64 * 2, kB = BN * 64 * 2, kStage = kA + kB;             // bytes per stage
-  static constexpr int kStages = (BN <= 64) ? 6 : (BN <= 128) ? 4 : 3;  // what the staging tiles leave room for
-  static constexpr int kGroups = (BN / 32 < 4) ? BN / 32 : (BN % 128 ? 3 : 4);  // epilogue groups: divide BN/32
+  static constexpr int kStages =  // what the staging tiles leave room for
+      PLAIN ? (BN <= 128 ? 6 : 4) : (BN <= 64) ? 6 : (BN <= 128) ? 4 : 3;
+  static constexpr int kGroups = PLAIN ? 2 : (BN / 32 < 4) ? BN / 32 : (BN % 128 ? 3 : 4);  // epilogue groups: divide BN/32
   static constexpr int kThreads = 64 + 128 * kGroups;
   // per epilogue warp a 32 x 32 FP32 staging tile (4 KB, 128-byte swizzle) for the TMA store
   static constexpr uint32_t kStg = 32 * 32 * 4;
@@ -259,12 +263,12 @@ __device__ __forceinline__ void epilogue16(const Epi& ep, int m, int nb, const f
   }
 }
 
-template <int BN>
-__global__ void __launch_bounds__(GemmCfg<BN>::kThreads, 1) k_gemm(const __grid_constant__ CUtensorMap tmA,
+template <int BN, bool PLAIN>
+__global__ void __launch_bounds__(GemmCfg<BN, PLAIN>::kThreads, 1) k_gemm(const __grid_constant__ CUtensorMap tmA,
                                                           const __grid_constant__ CUtensorMap tmB,
                                                           const __grid_constant__ CUtensorMap tmC, int K, int kchunk,
                                                           int tiles_n, int tiles_m, int splits, Epi ep, int* err) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, PLAIN>;
   constexpr int S = Cfg::kStages;
   constexpr uint32_t kCols = Cfg::kCols, kA = Cfg::kA, kStage = Cfg::kStage;
   extern __shared__ uint8_t smem_raw[];
@@ -524,14 +528,14 @@ int tensor_map_c(CUtensorMap* map, const float* base, int cols, int rows, int sp
   return encode_cached(map, k);
 }
 
-template <int BN>
+template <int BN, bool PLAIN>
 int launch_gemm_bn(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K, int splits, const Epi& ep,
                    int* err, cudaStream_t st) {
-  const size_t shm = GemmCfg<BN>::kSmem;
+  const size_t shm = GemmCfg<BN, PLAIN>::kSmem;
   static bool attr_set = false;
   static int nsm = 0;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(k_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_gemm<BN, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm) != cudaSuccess)
       return LGAME_ERR_CUDA;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -554,7 +558,7 @@ int launch_gemm_bn(const bf16* A, int lda, const bf16* B, int ldb, int M, int N,
   // programmatic dependent launch: see griddepcontrol in k_gemm
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(GemmCfg<BN>::kThreads);
+  cfg.blockDim = dim3(GemmCfg<BN, PLAIN>::kThreads);
   cfg.dynamicSmemBytes = shm;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -562,7 +566,7 @@ int launch_gemm_bn(const bf16* A, int lda, const bf16* B, int ldb, int M, int N,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, k_gemm<BN>, ma, mb, mc, K, kchunk, tiles_n, tiles_m, zs, ep, err) != cudaSuccess)
+  if (cudaLaunchKernelEx(&cfg, k_gemm<BN, PLAIN>, ma, mb, mc, K, kchunk, tiles_n, tiles_m, zs, ep, err) != cudaSuccess)
     return LGAME_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? LGAME_OK : LGAME_ERR_CUDA;
 }
@@ -580,12 +584,19 @@ int launch_gemm(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, in
   if (!bn)
     for (int c : {64, 128, 192, 256})
       if (N % c == 0) { bn = c; break; }
+  // the short split-K products of a weight gradient (a few K blocks a tile, many tiles) keep the four groups: an
+  // epoch of 65536 columns 2.67 ms, 2.84 with the plain form
+  const bool plain = ep.kind == kEpiF32 && splits == 1;
+#define GEMM_BN(BN)                                                                            \
+  (plain ? launch_gemm_bn<BN, true>(A, lda, B, ldb, M, N, K, splits, ep, err, st) \
+         : launch_gemm_bn<BN, false>(A, lda, B, ldb, M, N, K, splits, ep, err, st))
   switch (bn) {
-    case 256: return launch_gemm_bn<256>(A, lda, B, ldb, M, N, K, splits, ep, err, st);
-    case 192: return launch_gemm_bn<192>(A, lda, B, ldb, M, N, K, splits, ep, err, st);
-    case 128: return launch_gemm_bn<128>(A, lda, B, ldb, M, N, K, splits, ep, err, st);
-    default: return launch_gemm_bn<64>(A, lda, B, ldb, M, N, K, splits, ep, err, st);
+    case 256: return GEMM_BN(256);
+    case 192: return GEMM_BN(192);
+    case 128: return GEMM_BN(128);
+    default: return GEMM_BN(64);
   }
+#undef GEMM_BN
 }
 
 // ---- inference in one launch -----------------------------------------------------------------
