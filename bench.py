@@ -146,10 +146,10 @@ def _kernel_fields(ncons: int) -> dict:
 # moved per launch of the dominant kernel); traffic above the algorithmic bytes is re-reads and
 # per-thread stacks.
 MEASURED_DRAM_BYTES_PER_CELL = {
-    "ks_column_tracers": 206.0, "ks_column_ver": 228.4, "ks_tracers": 98.5, "ks_pgrad": 213.6,
-    "ks_tend_wind": 109.8, "ks_gas_div": 98.7, "ks_eta": 82.9, "ks_vort_flux": 59.6, "ks_div_h": 45.0,
-    "ks_ke": 78.6, "ks_theta_edges": 44.7, "ks_gas_flux": 29.4, "ks_gzp": 36.4,
-    "ks_temperature": 25.4, "ks_csh_sum": 21.0, "ks_heating_diss": 16.1,
+    "ks_column_ver": 229.0, "ks_column_tracers": 200.2, "ks_pgrad": 192.9, "ks_gas_div": 106.4,
+    "ks_tend_wind": 103.2, "ks_eta": 86.5, "ks_ke": 78.7, "ks_tracers": 78.3, "ks_gzp": 65.1,
+    "ks_vort_flux": 59.2, "ks_theta_flux": 52.0, "ks_theta_edges": 47.5, "ks_div_h": 47.1, "ks_grad": 36.5,
+    "ks_gas_flux": 29.1, "ks_temperature": 25.4, "ks_heating_diss": 16.2, "ks_csh_sum": 8.0,
 }
 
 
@@ -415,9 +415,9 @@ def profile_kernels(g, steps: int, first_step: int, ncons: int, cells: int, peak
 
 # FP64 thread instructions per cell of one launch of the split step's FP64-heavy kernels:
 # sm__inst_executed_pipe_fp64.sum x 32 / cells from an ncu capture of the moist jet at
-# 192x192x80 (ks_column_ver: 2,597,768 warp instructions, 2,949,120 cells).  The FP64 pipe
+# 256x256x80 (ks_column_ver: the mean of a step's two launches, 5,242,880 cells).  The FP64 pipe
 # issues 1.68 operations per clock per SM on this GPU (register-only probe; FMA and add alike).
-FP64_INST_PER_CELL = {"ks_column_ver": 28.2}
+FP64_INST_PER_CELL = {"ks_column_ver": 25.2}
 FP64_OPS_PER_CLK_SM = 1.68
 
 
@@ -431,7 +431,7 @@ def fp64_pipe_roofline(kernel: str, avg_ms: float, cells: int, clocks) -> dict |
     peak = FP64_OPS_PER_CLK_SM * 152 * mhz * 1e6
     achieved = per * cells / (avg_ms * 1e-3)
     return {"achieved_ops_per_s": achieved, "peak_ops_per_s": peak, "frac": achieved / peak,
-            "fp64_inst_per_cell": per, "src": "ncu sm__inst_executed_pipe_fp64 at 192x192x80; 1.68 FP64 ops/clk/SM "
+            "fp64_inst_per_cell": per, "src": "ncu sm__inst_executed_pipe_fp64 at 256x256x80; 1.68 FP64 ops/clk/SM "
                                               "(probe) at the sampled SM clock"}
 
 

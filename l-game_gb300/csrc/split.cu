@@ -1371,7 +1371,7 @@ __global__ void __launch_bounds__(256, 5) ks_tend_wind(Dims D, State So, State S
 //
 // Two kernels (the rule between them stands at their launch in split_step).  Large grids:
 // ks_column_ver, one thread per column, streamed top to bottom and back, bound by about 20 FP64
-// operations a cell and the latency of a level's loads.  Six more products are formed beside the FP64 pipe
+// operations a cell and the latency of a level's loads.  Five more products are formed beside the FP64 pipe
 // (fp64.cuh; the hardware's: 1.41 against 1.34 ms at 512x512x80), and the increment of rho*theta_v serves both it
 // and exner'; with each layer's inputs loaded a level ahead (five blocks of 96 registers an SM; six of 80: 1.42
 // ms) 1.57 -> 1.34 ms.  Small grids: ks_column_ver_tile below.
