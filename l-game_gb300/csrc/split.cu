@@ -1374,9 +1374,10 @@ __global__ void __launch_bounds__(256, 5) ks_tend_wind(Dims D, State So, State S
 // operations a cell and the latency of a level's loads.  Five more products are formed beside the FP64 pipe
 // (fp64.cuh; the hardware's: 1.41 against 1.34 ms at 512x512x80), and the increment of rho*theta_v serves both it
 // and exner'; with each layer's inputs loaded a level ahead (five blocks of 96 registers an SM; six of 80: 1.42
-// ms) 1.57 -> 1.34 ms.  Small grids: ks_column_ver_tile below.
+// ms) 1.57 -> 1.34 ms; compiled with and without a background state (BG), whose absence costs two
+// registers a layer and three FP64 operations, 1.27 ms.  Small grids: ks_column_ver_tile below.
 constexpr int kMaxLayers = 128;  // layers a context may have (lgame_gpu_create)
-template <class C>
+template <class C, bool BG>
 __global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
                                                      State Sn, StateF Mo, StateF Mn, Tend<float> Tn, int rk_step) {
   constexpr bool F64 = sizeof(C) == 8;
@@ -1445,7 +1446,8 @@ __global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, 
   auto layer = [&](int jl, const LayIn& R) -> Lay {
     Lay L;
     const long long i = IX(D, ji, jk, jl);
-    L.thd = D.luse_bg ? 0.0 : Su.rt[i] / Su.rho[goff + i];
+    L.thd = 0.0;
+    if constexpr (!BG) L.thd = Su.rt[i] / Su.rho[goff + i];
     const C iro = C(1) / R.ro, irto = C(1) / R.rt;
     L.a = -R.rt * iro * iro;
     L.b = iro;
@@ -1496,7 +1498,7 @@ __global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, 
     // but lets an atmosphere at rest over hills drift about four times faster (1e-8 instead
     // of 3e-9 m/s of spurious wind after 3 h at 256 x 256 x 50).
     double rv = M(-dz * ic2, wo + W(dtf * I1.tw));
-    rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
+    rv = fma(BG ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
     rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
     rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
     // couplings with row jl+1 (layer b's derivatives), which need layer jl+2
@@ -2777,11 +2779,13 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
     if (s->column_fp64) {
       if (tiny) CV_TILE(double, 8, 32);
       else if (small) CV_TILE(double, 16, 16);
-      else SL("ks_column_ver", ks_column_ver<double>, cgrd(D.ny, D.nx), cblk(), CV_ARGS);
+      else SL("ks_column_ver", (D.luse_bg ? ks_column_ver<double, true> : ks_column_ver<double, false>), cgrd(D.ny, D.nx),
+              cblk(), CV_ARGS);
     } else {
       if (tiny) CV_TILE(float, 8, 32);
       else if (small) CV_TILE(float, 32, 12);
-      else SL("ks_column_ver", ks_column_ver<float>, cgrd(D.ny, D.nx), cblk(), CV_ARGS);
+      else SL("ks_column_ver", (D.luse_bg ? ks_column_ver<float, true> : ks_column_ver<float, false>), cgrd(D.ny, D.nx),
+              cblk(), CV_ARGS);
     }
 #undef CV_TILE
 #undef CV_ARGS

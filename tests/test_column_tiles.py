@@ -39,3 +39,27 @@ def test_split_close_to_fp64_at_the_tilings_borders(grid, precision):
         g.close()
     errs = field_errors(states[1], states[0])
     assert max(errs.values()) <= 1e-5, errs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grid", [(19, 65, 13, 12), (243, 240, 5, 4)])
+def test_split_close_to_fp64_without_a_background_state(grid):
+    """Both column kernels without a background state (the thread-per-column one is compiled for each), one
+    step, at test_split's bar for it."""
+    ny, nx, nl, no = grid
+    n = cases.namelist("jet_1024x1024x80", ny=ny, nx=nx, n_layers=nl, n_oro_layers=no, theta_adv_order=2,
+                       luse_bg_state=False, lklemp=False)
+    hm = L.HostModel(n)
+    states = []
+    for prec in (L.PRECISION_FP64, L.PRECISION_SPLIT):
+        cfg = L.config_from_namelist(n)
+        cfg.precision = prec
+        g = L.GpuModel(cfg, hm.grid)
+        for slot in (0, 1):
+            g.set_state(slot, hm.state)
+        g.set_diag(hm.diag)
+        g.pchevi(0, 1, 0)
+        states.append(g.get_state(1))
+        g.close()
+    errs = field_errors(states[1], states[0])
+    assert max(errs.values()) <= 1e-5, errs
