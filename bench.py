@@ -417,7 +417,7 @@ def profile_kernels(g, steps: int, first_step: int, ncons: int, cells: int, peak
 # sm__inst_executed_pipe_fp64.sum x 32 / cells from an ncu capture of the moist jet at
 # 256x256x80 (ks_column_ver: the mean of a step's two launches, 5,242,880 cells).  The FP64 pipe
 # issues 1.68 operations per clock per SM on this GPU (register-only probe; FMA and add alike).
-FP64_INST_PER_CELL = {"ks_column_ver": 25.2}
+FP64_INST_PER_CELL = {"ks_column_ver": 23.2}
 FP64_OPS_PER_CLK_SM = 1.68
 
 
