@@ -87,7 +87,7 @@ struct SplitCtx {
   SplitSfc sfc{};
   // the step's concurrent branches: two side streams and the events of their forks and joins
   cudaStream_t br[2] = {nullptr, nullptr};
-  cudaEvent_t ev[8] = {};
+  cudaEvent_t ev[9] = {};
 };
 
 namespace {
@@ -2571,16 +2571,17 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
   // into `stream` by events:
   //   first substep:  the closure, swamp-layer heating and phase transitions (FP32 and
   //                   latency-bound) beside the theta edges and the FP64 pressure gradient;
-  //   both substeps:  the tracer tendencies beside the gas fluxes, divergences and vertical solve;
+  //   both substeps:  the tracer tendencies beside the vertical solve;
   //   between them:   the first substep's tracer solver beside the second substep's vorticity,
-  //                   kinetic energy (FP64, on a second side stream) and wind update.
-  // Every pair was checked for the arrays one writes and the other reads (the comments at each
-  // fork); with `serial` (per-kernel tracing, and the caller's graph capture, where the serial
-  // order measured faster) everything runs on `stream` in the same order.
+  //                   kinetic energy (FP64, on a second side stream) and wind update, which waits
+  //                   for the first substep's tracer tendencies (they read the wind it overwrites).
+  // Every two kernels of which one writes what the other reads or writes are ordered
+  // (tests/test_split_order.py); with `serial` (per-kernel tracing, and the caller's graph capture,
+  // where the serial order measured faster) everything runs on `stream` in the same order.
   const bool conc = !serial;
   cudaStream_t cur = stream;
   cudaStream_t side = conc ? s->br[0] : stream, side2 = conc ? s->br[1] : stream;
-  enum { EV_A = 0, EV_JA, EV_B, EV_C, EV_CSH, EV_KE, EV_JKE, EV_END };
+  enum { EV_A = 0, EV_JA, EV_B, EV_C, EV_CSH, EV_KE, EV_JKE, EV_END, EV_TR };
   // `to` starts after everything enqueued on `from` so far
   auto after = [&](cudaStream_t to, cudaStream_t from, int k) -> int {
     if (!conc || to == from) return LGAME_OK;
@@ -2727,8 +2728,13 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
     } else {
       // main: vorticity of the new state; side 2: its kinetic energy (FP64); both read the state
       // of the first substep (u, v from its wind update, w and rho_g from its vertical solve),
-      // which the tracer solver still running on the side stream does not write
+      // which the tracer tendencies and the tracer solver still running on the side stream do not write
       SYNC(vector_terms(Sn, Mn, true));
+      // the first substep's tracer tendencies, on the side stream, read the wind written next
+      if (tracers && conc && cudaStreamWaitEvent(stream, s->ev[EV_TR], 0) != cudaSuccess) {
+        lgame_set_error("split step: join event failed");
+        return LGAME_ERR_CUDA;
+      }
     }
     SL("ks_tend_wind", ks_tend_wind, sgrd(D.ny + 1, D.nx + 1, D.NL), B, D, So, Sn, T, CC, C, rk, Mn.u, Mn.v);
     // gas fluxes with third-order theta edges of the state used here; in the first substep that is the
@@ -2759,6 +2765,10 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
       SYNC(after(side, stream, EV_B));
       cur = side;
       SL("ks_tracers", ks_tracers, sgrd(D.ny, D.nx, D.nl), B, D, GF, s->GX, Ms, Mn.u, Mn.v, s->cw, T.rho, rk, mdt, ptr);
+      if (rk == 1 && conc && cudaEventRecord(s->ev[EV_TR], side) != cudaSuccess) {
+        lgame_set_error("split step: event record failed");
+        return LGAME_ERR_CUDA;
+      }
       cur = stream;
     }
     if (SF.sens || SF.soil)
