@@ -1206,6 +1206,14 @@ int backward(lgame_emu* e, int batch, const float* y, const long long* idx, floa
   return LGAME_OK;
 }
 
+// whether the weight gradients' products take the network's widths, asked before a batch begins: its updates
+// go layer by layer, so a product refused at the last layer would leave the others' updates behind
+int trainable(const lgame_emu* e) {
+  if (e->nin_pad % 128)
+    return emu_fail(LGAME_ERR_INVALID_ARG, "emulator: training needs 4*nlev+2 inputs that round up to an even multiple of 64");
+  return LGAME_OK;
+}
+
 // loss partials of a batch
 int loss_parts(const lgame_emu* e, int batch) { return (e->nout_pad / 32) * (batch / 32); }
 
@@ -1431,7 +1439,8 @@ extern "C" int lgame_emu_set_normalization(lgame_emu* e, const float* xm, const 
 extern "C" int lgame_emu_loss_grad(lgame_emu* e, const float* x, const float* y, int batch, float* loss, float* grads) {
   if (!e || !x || !y || batch < 128 || batch % 128 || batch > e->bmax)
     return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_loss_grad: bad arguments (batch a multiple of 128 <= batch_max)");
-  int rc = upload_batch(e, x, y, batch);
+  int rc = trainable(e);
+  if (!rc) rc = upload_batch(e, x, y, batch);
   if (!rc) rc = forward(e, batch);
   if (!rc) rc = backward(e, batch, e->yraw, nullptr, e->lpart, nullptr);
   if (!rc) rc = loss_from_parts(e, loss_parts(e, batch), batch, loss);
@@ -1455,7 +1464,8 @@ extern "C" int lgame_emu_loss_grad(lgame_emu* e, const float* x, const float* y,
 extern "C" int lgame_emu_train_step(lgame_emu* e, const float* x, const float* y, int batch, float lr, float* loss) {
   if (!e || !x || !y || batch < 128 || batch % 128 || batch > e->bmax)
     return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_train_step: bad arguments");
-  int rc = upload_batch(e, x, y, batch);
+  int rc = trainable(e);
+  if (!rc) rc = upload_batch(e, x, y, batch);
   if (!rc) rc = forward(e, batch);
   if (!rc) {
     const Adam A = adam(e, lr);
@@ -1491,6 +1501,7 @@ extern "C" int lgame_emu_set_dataset(lgame_emu* e, const float* x, const float* 
 extern "C" int lgame_emu_train_epoch(lgame_emu* e, int batch, float lr, unsigned long long seed, float* mean_loss) {
   if (!e || !e->dsx || batch < 128 || batch % 128 || batch > e->bmax)
     return emu_fail(LGAME_ERR_INVALID_ARG, "lgame_emu_train_epoch: no dataset or bad batch");
+  if (const int rc = trainable(e)) return rc;
   // shuffled order (Fisher-Yates with splitmix64), whole batches only
   std::vector<long long> perm(e->dsn);
   for (long long i = 0; i < e->dsn; ++i) perm[i] = i;

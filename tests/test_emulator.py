@@ -271,3 +271,20 @@ def test_inference_in_one_launch_equals_the_layers(nlev, hidden, n):
     emu.infer(xp, out=yp)  # page-locked: all columns in one call
     np.testing.assert_array_equal(yp, emu.infer(x))  # pageable: a batch at a time
     emu.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nlev", [8, 40, 96])
+def test_refused_training_leaves_the_network_as_it_was(nlev):
+    """Inputs padded to an odd multiple of 64 have no weight gradient product: a step and an epoch are refused,
+    and no layer has been updated by then."""
+    emu, x, y, _ = _emu_and_data(nlev=nlev, batch=128)
+    emu.set_dataset(x, y)
+    p, out = emu.get_params(), emu.infer(x)
+    for train in (lambda: emu.train_step(x, y, 1e-2), lambda: emu.train_epoch(128, 1e-2, 1), lambda: emu.loss_grad(x, y)):
+        with pytest.raises(L.LgameError) as err:
+            train()
+        assert err.value.code == L.ERR_INVALID_ARG
+        np.testing.assert_array_equal(emu.get_params(), p)
+        np.testing.assert_array_equal(emu.infer(x), out)
+    emu.close()
