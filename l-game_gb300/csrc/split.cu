@@ -17,6 +17,7 @@
 #include "common.h"
 #include "fp64.cuh"
 #include "lgame_gpu.h"
+#include "tile_sweep.cuh"
 
 #include <algorithm>
 #include <string>
@@ -1798,13 +1799,13 @@ struct ColVer {
 // Small grids: a block owns TC columns and NW chunks of levels (a lane per column, chunk w of a
 // column in thread w*TC + lane), in phases:
 //   1. every thread forms the rows of its chunk (matrix, right-hand side) into shared memory;
-//   2. the first TC threads run the factorisation (pivot p, upper factor e/p, lower factor c/p,
-//      type C) and the forward substitution y = r - (c/p)*y, one multiply-add a row in the chain;
+//   2. the first TC threads run the factorisation (pivot p, upper factor e/p, type C) and the forward
+//      substitution y = r - (c/p)*y, c/p held in FP64 (tile_sweep.cuh), one multiply-add a row in the chain;
 //   3. every thread its rows' y/p;  4. the first TC threads the back substitution;
 //   5. every thread the new state of its chunk of layers.
 // The chain of levels then waits on shared memory and arithmetic alone, and the levels' loads and
-// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 33 against 280
-// us at 4 x 256 x 60, 140 against 381 us at 128 x 128 x 80, 279 against 376 us at 180 x 210 x 80, equal (415 us)
+// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 34 against 280
+// us at 4 x 256 x 60, 141 against 381 us at 128 x 128 x 80, 279 against 376 us at 180 x 210 x 80, equal (415 us)
 // at 230 x 236 x 80, and slower above, where the phases in which one warp works cost more than the
 // latency they hide.
 template <class C, int TC, int NW>
@@ -1812,7 +1813,7 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
     ks_column_ver_tile(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So, State Sn, StateF Mo, StateF Mn,
                        Tend<float> Tn, int rk_step) {
   using Cv = ColVer<C>;
-  constexpr int kRow = 5 * TC;  // coefficients of one level of the block's columns in shared memory
+  constexpr int kRow = kTileCoef * TC;  // coefficients of one level of the block's columns in shared memory
   const int lane = threadIdx.x % TC, w = threadIdx.x / TC;
   const int col = blockIdx.x * TC + lane;
   const bool valid = col < D.ny * D.nx;
@@ -1845,37 +1846,12 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
     }
   }
   __syncthreads();
-  if (w == 0 && valid) {
-    C cv_prev = C(0), epr_prev = C(0), f = C(0);
-    double y = 0.0;
-    C* row = sc;
-    double* r = sr;
-#pragma unroll 4
-    for (int jl = 1; jl <= n; ++jl, row += kRow, r += TC) {
-      const C piv = row[0] - epr_prev * cv_prev;
-      y = fma(-Cv::W(f), y, r[0]);
-      r[0] = y;
-      epr_prev = row[2 * TC] / piv;
-      cv_prev = row[TC];
-      f = cv_prev / piv;
-      row[0] = piv;
-      row[2 * TC] = epr_prev;
-    }
-  }
+  if (w == 0 && valid) tile_forward<C, TC>(sc, sr, n);
   __syncthreads();
   if (valid)
     for (int jl = r0; jl <= r1; ++jl) sr[TC * (jl - 1)] = Cv::quot(sr[TC * (jl - 1)], sc[kRow * (jl - 1)]);
   __syncthreads();
-  if (w == 0 && valid) {
-    C* row = sc + kRow * (n - 2);
-    double* r = sr + TC * (n - 2);
-    double s = r[TC];
-#pragma unroll 4
-    for (int jl = n - 1; jl >= 1; --jl, row -= kRow, r -= TC) {
-      s = fma(-Cv::W(row[2 * TC]), s, r[0]);
-      r[0] = s;
-    }
-  }
+  if (w == 0 && valid) tile_back<C, TC>(sc, sr, n);
   __syncthreads();
   // the new state, each chunk of layers bottom to top; the chunk's first layer needs the new
   // density of the layer below it, formed anew
@@ -1902,7 +1878,7 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
   if (D.freeslip && l1 == nl) V.free_slip();
 }
 template <class C, int TC>
-constexpr size_t column_ver_smem(int nl) { return (size_t)nl * TC * (sizeof(double) + 5 * sizeof(C)); }
+constexpr size_t column_ver_smem(int nl) { return (size_t)nl * TC * (sizeof(double) + kTileCoef * sizeof(C)); }
 
 // ---- three_band_solver_gen_densities, mo_column_solvers.F90:353-604 ----------------------
 // The reference's system per (column, tracer)  d_l s_l + e_l s_{l+1} + c_{l-1} s_{l-1} = rho_l + inc_l
