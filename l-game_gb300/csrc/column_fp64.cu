@@ -24,15 +24,15 @@ constexpr int kMaxLayers = 128;
 // fourteen arrays in local memory took 788, 2116 us a launch at 65x97x33, 192x192x80; two blocks an SM 158,
 // 1591 us; three (80 registers) 139, 1523 us.
 constexpr int kCvCols = 16, kCvChunks = 16;
-constexpr int kCvArrays = 7;  // c (then c of the row above), d, e (then e/den), r (then the solution), interface
-                              // theta, gamma, 1/(interface density)
+constexpr int kCvArrays = 7;  // c, d, e (then e/den), r (then the solution), interface theta, gamma,
+                              // 1/(interface density)
 
 template <int RK>
 __global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
     k_column_ver(Dims D, Grid<F64> G, ColumnGrid X, StateT<F64> So, StateT<F64> Sn, Tend<F64> Tn) {
   extern __shared__ __align__(16) double sm_raw[];
   F64* const sm_cv = reinterpret_cast<F64*>(sm_raw);
-    constexpr int S = kCvCols;
+  constexpr int S = kCvCols;
   const int lane = threadIdx.x % S, w = threadIdx.x / S;
   const int col = blockIdx.x * S + lane;
   const bool valid = col < D.ny * D.nx;

@@ -1,8 +1,8 @@
 // fp64.cuh -- FP64 arithmetic of the FP64 step in fewer operations of the FP64 pipe, which issues
 // 1.6 operations per clock and SM on this GPU against 64 integer ones: with plain expressions every
 // kernel of the step had that pipe at 80-88 % and everything else below 10 %, so its time was the
-// number of these operations.  Every function returns the bits of the plain expression (exceptions
-// as stated).
+// number of these operations.  Every function returns the bits of the plain expression, with the exceptions
+// stated beside it (tests/test_fp64_device.py compares them on the GPU).
 #pragma once
 
 #include <cstdint>
@@ -117,38 +117,55 @@ __device__ __forceinline__ bool negative(F64 a) { return negative(a.v); }
 __device__ __forceinline__ bool nonzero(F64 a) { return nonzero(a.v); }
 __device__ __forceinline__ bool upwind(F64 a) { return upwind(a.v); }
 __device__ __forceinline__ bool positive(F64 a) { return positive(a.v); }
-// 1/b to about a unit of the last place: the single-precision reciprocal of b's leading bits (to
-// 2^-22) and one step of Halley's iteration, y(1 + e + e^2) with e = 1 - b*y: three operations of the
-// FP64 pipe
-static __device__ __noinline__ double rcp_hw(double b) { return 1.0 / b; }
-__device__ __forceinline__ double rcp_near(double b) {
+// 1/b to about a unit of the last place, b within 2^-100..2^99: the single-precision reciprocal of b's leading
+// 24 bits (to 2^-21: the cut and two units of __fdividef) and one step of Halley's iteration, y(1 + e + e^2)
+// with e = 1 - b*y, to e^3: three operations of the FP64 pipe
+__device__ __forceinline__ bool near_range(double b) {
+  return ((uint32_t)__double2hiint(b) & 0x7FF00000u) - (923u << 20) < (200u << 20);
+}
+__device__ __forceinline__ double rcp_start(double b) {
   const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
-  if ((hi & 0x7FF00000u) - (923u << 20) >= (200u << 20)) return rcp_hw(b);  // not within 2^-100..2^99
   const float f = __uint_as_float((hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29)));
   const double y = wide(__fdividef(1.f, f));
   const double e = fma(-b, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
-// 1/b and a/b rounded to nearest for y within two units of the last place of 1/b: value, remainder,
-// correction (Markstein, IBM J. Res. Dev. 34, 1990).  The result is the correctly rounded one, except
-// that a value within 2^-50 of its last place from the middle of two doubles may round the other
-// way; a zero quotient's sign is not kept, and an infinite a gives NaN.
+static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
+// the same for any b, the hardware's quotient outside that range
+__device__ __forceinline__ double rcp_near(double b) { return near_range(b) ? rcp_start(b) : div_hw(1.0, b); }
+// a remainder that is not finite (infinite or NaN operands, a zero divisor, overflow) corrects nothing: the
+// quotient as it is then is the hardware's
+__device__ __forceinline__ double corrected(double q, double r, double y) {
+  return ((uint32_t)__double2hiint(r) & 0x7FF00000u) == 0x7FF00000u ? q : fma(r, y, q);
+}
+// 1/b and a/b rounded to nearest: value, remainder, correction (Markstein, IBM J. Res. Dev. 34, 1990).
+// div_rn: b within 2^-100..2^99, 0, infinite or NaN, and y its reciprocal to 2^-50 (four units of the last
+// place: also a product of two such reciprocals, for a rounded product of two divisors); the corrected quotient
+// is off by the product of y's and q's errors, at most 2^-99, before it is rounded.  So the result is the
+// correctly rounded one, except that
+//   a value within 2^-46 of its last place from the middle of two doubles may round the other way;
+//   a quotient below 2^-1022, and one of a dividend below 2^-960, whose remainder is not exact, may be off by
+//   a unit of its last place;
+//   a zero quotient's sign is not kept.
 __device__ __forceinline__ double rcp(double b) {
   const double y = rcp_near(b);
-  return fma(fma(-b, y, 1.0), y, y);
+  return corrected(y, fma(-b, y, 1.0), y);
 }
 __device__ __forceinline__ F64 rcp(F64 b) { return rcp(b.v); }
 __device__ __forceinline__ F64 rcp_near(F64 b) { return rcp_near(b.v); }
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
   const double q = a * y;
-  return fma(fma(-b, q, a), y, q);
+  return corrected(q, fma(-b, q, a), y);
 }
 __device__ __forceinline__ F64 div_rn(F64 a, F64 b, F64 y) {
   const double q = mul_int(a.v, y.v);
-  return fma(fma(-b.v, q, a.v), y.v, q);
+  return corrected(q, fma(-b.v, q, a.v), y.v);
 }
-__device__ __forceinline__ double quot(double a, double b) { return div_rn(a, b, rcp_near(b)); }
-__device__ __forceinline__ F64 operator/(F64 a, F64 b) { return div_rn(a, b, rcp_near(b)); }
+__device__ __forceinline__ double quot(double a, double b) { return near_range(b) ? div_rn(a, b, rcp_start(b)) : div_hw(a, b); }
+__device__ __forceinline__ F64 operator/(F64 a, F64 b) {
+  if (near_range(b.v)) return div_rn(a, b, rcp_start(b.v));
+  return div_hw(a.v, b.v);
+}
 
 __device__ __forceinline__ F64 root(F64 a) { return sqrt(a.v); }
 // calc_diff_coeff, mo_derived.F90:189-216

@@ -1,5 +1,5 @@
 // kernels_fp64.cu -- explicit kernels of the FP64 step (compiled with -fmad=false: only the fma
-// written out are fused), in the reference's operand order, so with its bits.
+// written out are fused), in the reference's operand order, so with its bits (the exceptions: fp64.cuh).
 //
 // All are bound by the FP64 pipe (fp64.cuh), so each is written for few of its operations: a
 // product that two cells or two interfaces share is formed once (at the face, or carried down the

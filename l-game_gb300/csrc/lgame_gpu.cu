@@ -1894,12 +1894,6 @@ __global__ void k_rad_ozone(Dims D, Grid<double> G, double* o3) {
   o3[i] = 8.5e-6 * exp(-dz * dz / (2.0 * sigma * sigma)) * m_o3 / kM_D;
 }
 
-// a quotient whose numerator may be infinite or NaN, as the hardware gives it
-__device__ __forceinline__ F64 quot_any(F64 a, F64 b, F64 y) {
-  if (((unsigned)__double2hiint(a.v) & 0x7FF00000u) == 0x7FF00000u) return a.v / b.v;
-  return div_rn(a, b, y);
-}
-
 // T, dry-air pressure, vapour and ozone densities of every layer, albedo and cos(zenith); column index
 // ji + ny*(jk-1), 4*nl+2 floats per column.  A block takes 32 columns and 32 layers: the state is read
 // along ji, and the features go out along the layers, through shared memory.  (One thread per column
@@ -1923,7 +1917,7 @@ __global__ void __launch_bounds__(256) k_rad_features(Dims D, Grid<F64> G, State
       F64 T = (G.theta_v_bg[i] + S.tp[i]) * (G.exner_bg[i] + S.ep[i]);  // temperature_diagnostics
       if (D.lmoist) {  // T/(1 + rv/rd*(M_d/M_v - 1)) in one quotient
         const F64 f = rd + rv * (kM_D / kM_V - 1.0);
-        T = quot_any(T * rd, f, rcp_near(f));
+        T = T * rd / f;
       }
       tile[0][k][threadIdx.x] = narrow(T.v);
       tile[1][k][threadIdx.x] = narrow((kR_D * rd * T).v);
@@ -1963,7 +1957,7 @@ __global__ void __launch_bounds__(256) k_rad_apply(Dims D, StateT<F64> S, const 
     const long long i = IX(D, ji, jk, l0 + k + 1);
     F64 rho = S.rho[i + (long long)(D.g - 1) * D.fstride];
     if (D.lmoist) rho = rho + S.rho[i + (long long)D.g * D.fstride];
-    const F64 q = quot_any(wide(tile[k][threadIdx.x]), 86400.0, 1.0 / 86400.0) * rho * kC_D_P;
+    const F64 q = div_rn(F64(wide(tile[k][threadIdx.x])), 86400.0, 1.0 / 86400.0) * rho * kC_D_P;
     rad[i] = q.v;
     if (rad_f) rad_f[i] = narrow(q.v);
   }
