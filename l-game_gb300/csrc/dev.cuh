@@ -348,15 +348,4 @@ __device__ __forceinline__ double c_p_cond(int jc, double temperature) {
   return ((jc - 1) % 2 == 0) ? c_p_ice(temperature) : c_p_water(temperature);
 }
 
-// calc_diff_coeff, mo_derived.F90:189-216
-__device__ __forceinline__ double calc_diff_coeff(double temperature, double density) {
-  const double particle_radius = 130e-12;
-  const double particle_mass = kM_D / kN_A;
-  const double thermal_velocity = sqrt(8.0 * kK_B * temperature / (kPI * particle_mass));
-  const double particle_density = density / particle_mass;
-  const double cross_section = 4.0 * kPI * (particle_radius * particle_radius);
-  const double mean_free_path = 1.0 / (1.4142135623730951 * particle_density * cross_section);
-  return 1.0 / 3.0 * thermal_velocity * mean_free_path;
-}
-
 }  // namespace lg

@@ -312,27 +312,9 @@ __global__ void k_diss_rate(Dims D, Grid<T> G, StateT<V> S, DiffBuf<T> B, const 
 // ---- 7. temperature and mass diffusion (mo_scalar_tend_expl.F90:60-101) ----------------------------
 // The effective coefficients of scalar_diff_coeffs (mo_eff_diff_coeffs.F90:526-618) at a scalar
 // point: horizontal and vertical, for mass (kind 0) and temperature (kind 1).  The specific
-// heat c_g_v of spec_heat_cap_diagnostics_v (mo_derived.F90:40-68) is rho_g/rho_g*c_d_v.
-template <class T, class V>
-__device__ __forceinline__ T diff_coeff_h(const Dims& D, const StateT<V>& S, const DiffBuf<T>& B, int kind, long long p) {
-  const T rg = T(S.rho[p + (long long)(D.g - 1) * D.fstride]);
-  if (kind == 0) return B.visc[p] / rg;
-  const T c_g_v = T(0) + rg / rg * T(kC_D_V);
-  return c_g_v * B.visc[p];
-}
-template <class T, class V>
-__device__ __forceinline__ T diff_coeff_v(const Dims& D, const Grid<T>& G, const StateT<V>& S, const DiffBuf<T>& B,
-                                          int kind, long long p) {
-  const T t2v = B.vmol[p] + tke2vert<T>(B.tke[p], B.nsq[p], G.layer_thickness[p]);
-  if (kind == 0) return t2v;
-  const T rg = T(S.rho[p + (long long)(D.g - 1) * D.fstride]);
-  const T c_g_v = T(0) + rg / rg * T(kC_D_V);
-  return rg * c_g_v * t2v;
-}
-
-// (the FP64 step's scalar diffusion: k64_diff_* in kernels_fp64.cu)
-
-// ---- 7b. temperature and mass diffusion of the split step, fluxes and divergence fused ----------
+// heat c_g_v of spec_heat_cap_diagnostics_v (mo_derived.F90:40-68) is rho_g/rho_g*c_d_v.  The FP64 step's
+// kernels are k64_diff_* in kernels_fp64.cu; below, the split step's, fluxes and divergence fused.
+//
 // The diffusive flux densities and their divergence, for the NM mass fields and (HT) the temperature
 // together, in FP32, in one launch that marches down the levels: the flux densities never reach
 // HBM and the metrics and coefficients are read once for all fields.  A block owns a tile of
@@ -500,7 +482,7 @@ k_diff_scalar_col(Dims D, Grid<float> G, StateF S, DiffBuf<float> B, const float
       const float idz = g_lo ? 1.f / ai.dz1 : 0.f;
       if (NM > 0) sh_c[slot] = ai.vi / ai.rg;
       if (HT > 0) sh_c[NS + slot] = float(kC_D_V) * ai.vi;
-      if (vm || vt) {  // diff_coeff_v at the cell; the interface above takes the mean with the layer above
+      if (vm || vt) {  // the vertical coefficients at the cell; the interface above takes the mean with the layer above
         const float t2v = ai.vmol + tke2vert<float>(ai.tke, ai.nsq, ai.lt);
         const float cv1 = ai.rg * float(kC_D_V) * t2v;
         hv0 = 0.5f * (cvp0 + t2v);

@@ -115,20 +115,6 @@ __device__ __forceinline__ float c_p_cond(int jc, float temperature) {
   return ((jc - 1) % 2 == 0) ? c_p_ice(temperature) : c_p_water(temperature);
 }
 
-// c_v_mass_weighted_air, mo_derived.F90:157-187
-template <class T, class V>
-__device__ __forceinline__ T c_v_mass_weighted_air(const Dims& D, const V* rho, const T* Tm, long long q) {
-  T c = T(0);
-  for (int jc = 1; jc <= D.nc; ++jc) c = c + T(rho[q + (long long)(jc - 1) * D.fstride]) * c_p_cond(jc, Tm[q]);
-  if (D.lmoist) {
-    c = c + (T(rho[q + (long long)D.nc * D.fstride]) - T(rho[q + (long long)(D.nc + 1) * D.fstride])) * T(kC_D_V);
-    c = c + T(rho[q + (long long)(D.nc + 1) * D.fstride]) * T(kC_V_V);
-  } else {
-    c = T(rho[q + (long long)D.nc * D.fstride]) * T(kC_D_V);
-  }
-  return c;
-}
-
 // inner_product, mo_inner_product.F90:16-50 (both vectors the state wind)
 template <class T, class V>
 __device__ __forceinline__ T inner_product_at(const Dims& D, const Grid<T>& G, const V* u, const V* v,

@@ -2185,7 +2185,6 @@ __global__ void ks_csh_sum(Dims D, const float* csh_part, float* csh) {
 // dynamic shared memory of ks_column_tracers: alpha, beta and e' of three tracers, 32 columns
 size_t tracer_smem(int nl) { return (size_t)nl * kTrRow * sizeof(float); }
 
-// dynamic shared memory of ks_column_ver: right-hand side and five coefficients per level, 32 columns
 // the tile kernel's shared memory is allowed for the most layers a context may have: contexts of
 // different heights share the function's attribute
 template <class C, int TC, int NW>
