@@ -96,9 +96,12 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
     Lay L0 = layer(r0, true), L1 = layer(r0 + 1, true), L2{};
     F64 rio = 0.5 * (L0.ro + L1.ro), yrio = rcp_near(rio);
     F64 t = 0.5 * (L0.th + L1.th);
+    // half of exner_bg(jl-1) - exner_bg(jl) at the interface above layer p
+    auto half_deb = [&](long long p) { return half(G.exner_bg[p - pl] - G.exner_bg[p]); };
+    F64 hdeb = half_deb(c0 + (long long)r0 * pl);
     for (int jl = r0; jl <= r1; ++jl) {
       const long long b = c0 + (long long)jl * pl;  // layer jl+1 and w level jl+1
-      const F64 zs = X.zs[b], hdeb = X.hdeb[b], dp = G.damp[b], wo = So.w[b];
+      const F64 zs = G.z_scalar[b - pl] - G.z_scalar[b], dp = G.damp[b], wo = So.w[b];
       const F64 rie = 0.5 * (L0.rhe + L1.rhe);
       const F64 dv = -(t * t) * (L0.ga + L1.ga) + hdeb * (L1.al - L0.al + t * (L1.be - L0.be))
                       - div_rn(zs, c_imp2 * rio, X.rc_imp2 * yrio)
@@ -107,15 +110,16 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
       const F64 rv = div_rn(-(wo + dtime * Tn.w[b]) * zs, c_imp2, X.rc_imp2)
                       + div_rn(t * (L0.epe - L1.epe), dtime, rdt)
                       + 2.0 * (0.5 / dtime) * (L0.tpe + L1.tpe) * hdeb
-                      - div_rn(X.zs_c2[b] * wo * rie, rio, yrio);
-      F64 cv = 0.0, ev = 0.0, rio_n = 0.0, yrio_n = 0.0, tn = 0.0;
+                      - div_rn(div_rn(zs, c_imp2, X.rc_imp2) * wo * rie, rio, yrio);
+      F64 cv = 0.0, ev = 0.0, rio_n = 0.0, yrio_n = 0.0, tn = 0.0, hdeb_n = 0.0;
       if (jl < n) {
         L2 = layer(jl + 2, jl < r1);
         const long long cc = b + pl;
         tn = 0.5 * (L1.th + L2.th);
         rio_n = 0.5 * (L1.ro + L2.ro);
         yrio_n = rcp_near(rio_n);
-        cv = tn * L1.ga * t + X.hdeb[cc] * (L1.al + L1.be * t)
+        hdeb_n = half_deb(cc);
+        cv = tn * L1.ga * t + hdeb_n * (L1.al + L1.be * t)
            - div_rn(X.zs_c1h[cc] * So.w[cc], L1.V * rio_n, L1.rV * yrio_n) * G.damp[cc];
         ev = t * L1.ga * tn - hdeb * (L1.al + L1.be * tn)
            + div_rn(X.zs_c1h[b] * wo, L1.V * rio, L1.rV * yrio) * dp;
@@ -133,6 +137,7 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
       rio = rio_n;
       yrio = yrio_n;
       t = tn;
+      hdeb = hdeb_n;
     }
   }
   __syncthreads();
@@ -208,30 +213,22 @@ __global__ void __launch_bounds__(kCvCols* kCvChunks, 3)
   }
 }
 
-// the grid-only factors of the vertical solve, at w level jl = 2..nl (index of layer jl) and, the
-// reciprocal of the volume, at every layer
-__global__ void k_column_grid(Dims D, Grid<double> G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
-                              double* zs_c1h, double* hdeb, double* raz) {
+// the grid-only factors of the column solves (ColumnGrid; itwdtv may be null)
+__global__ void k_column_grid(Dims D, Grid<double> G, double* rvol, double* itwdtv, double* zs_c1h, double* raz) {
   LG_IDX3;
   if (ji > D.ny || jk > D.nx) return;
-  const long long q = IX(D, ji, jk, jl), a = q - D.plane;
+  const long long q = IX(D, ji, jk, jl);
   rvol[q] = 1.0 / G.volume[q];
-  itwdtv[q] = 0.5 * D.dtime / G.volume[q];
+  if (itwdtv) itwdtv[q] = 0.5 * D.dtime / G.volume[q];
   if (jl == 1) return;
-  const double c_imp2 = kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P;
-  const double c_imp1 = kIMPL_THERMO_WEIGHT * D.dtime * kC_D_P;
-  const double z = G.z_scalar[a] - G.z_scalar[q];
-  zs[q] = z;
-  zs_c2[q] = z / c_imp2;
-  zs_c1h[q] = z / c_imp1 * 0.5;
-  hdeb[q] = 0.5 * (G.exner_bg[a] - G.exner_bg[q]);
+  zs_c1h[q] = (G.z_scalar[q - D.plane] - G.z_scalar[q]) / (kIMPL_THERMO_WEIGHT * D.dtime * kC_D_P) * 0.5;
   raz[q] = 1.0 / G.area_z[q];
 }
 
-void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
-                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st) {
+void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs_c1h, double* raz,
+                        cudaStream_t st) {
   const dim3 g((unsigned)((D.ny + 31) / 32), (unsigned)D.nl, (unsigned)((D.nx + 7) / 8));
-  k_column_grid<<<g, dim3(32, 8), 0, st>>>(D, G, rvol, itwdtv, zs, zs_c2, zs_c1h, hdeb, raz);
+  k_column_grid<<<g, dim3(32, 8), 0, st>>>(D, G, rvol, itwdtv, zs_c1h, raz);
 }
 
 void launch_column_ver(const Dims& D, const Grid<double>& G, const ColumnGrid& X, const State& So, const State& Sn,

@@ -192,11 +192,10 @@ struct Faces {
   F64 *px, *py, *hx, *hy;
 };
 
-// grid-only factors of the vorticity: reciprocals of the dual areas (x and y to level nl+1); in the
-// terrain-following layers, for each side of a dual point, (r_e + z_dual)/(r_e + z_side) times its
-// length, with the side's sign; reciprocals of z(l) - z(l+1) at v and u points
+// grid-only factors of the vorticity: in the terrain-following layers, for each side of a dual point,
+// (r_e + z_dual)/(r_e + z_side) times its length, with the side's sign
 struct RotGrid {
-  const F64 *radx, *rady, *radz, *m0, *m1, *m2, *m3, *ryv, *ryu;
+  const F64 *m0, *m1, *m2, *m3;
 };
 
 // the explicit kernels (kernels_fp64.cu)
@@ -204,8 +203,8 @@ void launch64_rot_grid(const Dims& D, const Grid<double>& G, double* const* a, c
 void launch64_zeta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* zz, cudaStream_t st);
 void launch64_eta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* ez, cudaStream_t st);
 void launch64_covariant(const Dims& D, const Grid<double>& G, const State& S, double* cx, double* cy, cudaStream_t st);
-void launch64_eta_xy(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, const double* cx, const double* cy,
-                     double* ex, double* ey, cudaStream_t st);
+void launch64_eta_xy(const Dims& D, const Grid<double>& G, const State& S, const double* cx, const double* cy, double* ex,
+                     double* ey, cudaStream_t st);
 void launch64_mass_flux(const Dims& D, const Grid<double>& G, const State& S, double* uph, double* vph, double* q5, double* q6,
                         cudaStream_t st);
 void launch64_vort_flux(const Dims& D, const Grid<double>& G, const double* ex, const double* ey, const double* ez,
@@ -265,15 +264,15 @@ void launch64_diss_rate(const Dims& D, const Grid<double>& G, const State& S, co
 
 // the column solves (column_fp64.cu)
 // grid-only factors of the column solves: 1/volume at the layers; at w level jl = 2..nl (index of
-// layer jl) z_scalar(jl-1) - z_scalar(jl), that over c_imp2 and half of it over c_imp1 (c_imp2 =
-// impl_thermo_weight*dtime^2*c_d_p, c_imp1 the same with dtime), half of exner_bg(jl-1) -
-// exner_bg(jl), 1/area_z; 1/c_imp2 and 1/dtime
+// layer jl) half of z_scalar(jl-1) - z_scalar(jl) over c_imp1 (= impl_thermo_weight*dtime*c_d_p), 1/area_z;
+// 1/c_imp2 (c_imp2 = c_imp1*dtime) and 1/dtime
 struct ColumnGrid {
-  const F64 *rvol, *zs, *zs_c2, *zs_c1h, *hdeb, *raz;
+  const F64 *rvol, *zs_c1h, *raz;
   double rc_imp2, rdt;
 };
-void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs, double* zs_c2,
-                        double* zs_c1h, double* hdeb, double* raz, cudaStream_t st);
+// itwdtv: 0.5*dtime/volume, of moist runs (null: not formed)
+void launch_column_grid(const Dims& D, const Grid<double>& G, double* rvol, double* itwdtv, double* zs_c1h, double* raz,
+                        cudaStream_t st);
 // once per step of a moist run, from state_old and its temperature: the cloud droplets' fall speed
 // and c_p of ice and water
 void launch_moist_aux(const Dims& D, const Grid<double>& G, const State& So, const double* T, double* vcloud, double* cpi,

@@ -478,29 +478,17 @@ __global__ void k64_pgrad(Dims D, Grid<F64> G, StateT<F64> S, const F64* gx, con
 
 // ---- potential vorticity and its flux, mo_vorticities.F90, mo_vorticity_flux.F90 -------------------
 // grid-only factors (RotGrid)
-__global__ void k64_rot_grid(Dims D, Grid<F64> G, F64* radx, F64* rady, F64* radz, F64* m0, F64* m1, F64* m2, F64* m3,
-                             F64* ryv, F64* ryu) {
+__global__ void k64_rot_grid(Dims D, Grid<F64> G, F64* m0, F64* m1, F64* m2, F64* m3) {
   LG_IDX3;
+  if (ji > D.ny + 1 || jk > D.nx + 1 || jl <= D.nf) return;
   const long long q = IX(D, ji, jk, jl);
-  const F64 one = 1.0;
-  if (ji <= D.ny + 1 && jk <= D.nx) radx[q] = one / G.area_dual_x[q];
-  if (ji <= D.ny && jk <= D.nx + 1) rady[q] = one / G.area_dual_y[q];
-  if (jl > D.nl || ji > D.ny + 1 || jk > D.nx + 1) return;
-  radz[q] = one / G.area_dual_z[q];
-  if (jl < D.nl) {
-    if (jk <= D.nx) ryv[q] = one / (G.z_v[q] - G.z_v[q + D.plane]);
-    if (ji <= D.ny) ryu[q] = one / (G.z_u[q] - G.z_u[q + D.plane]);
-  }
-  if (jl > D.nf) {
-    const RotSides n = rot_sides(D, ji, jk, jl);
-    if (n.in) {
-      const F64 up = F64(kR_E) + G.z_area_dual_z[q];
-      m0[q] = up / (F64(kR_E) + G.z_v[n.v0]) * G.dy[n.v0];
-      m1[q] = -(up / (F64(kR_E) + G.z_u[n.u1])) * G.dx[n.u1];
-      m2[q] = -(up / (F64(kR_E) + G.z_v[n.v2])) * G.dy[n.v2];
-      m3[q] = up / (F64(kR_E) + G.z_u[n.u3]) * G.dx[n.u3];
-    }
-  }
+  const RotSides n = rot_sides(D, ji, jk, jl);
+  if (!n.in) return;
+  const F64 up = F64(kR_E) + G.z_area_dual_z[q];
+  m0[q] = up / (F64(kR_E) + G.z_v[n.v0]) * G.dy[n.v0];
+  m1[q] = -(up / (F64(kR_E) + G.z_u[n.u1])) * G.dx[n.u1];
+  m2[q] = -(up / (F64(kR_E) + G.z_v[n.v2])) * G.dy[n.v2];
+  m3[q] = up / (F64(kR_E) + G.z_u[n.u3]) * G.dx[n.u3];
 }
 // rel_vort_z_local, mo_vorticities.F90:423-538, over the dual area: the wind of each of the four sides
 // extrapolated to the dual point's height
@@ -514,17 +502,15 @@ __device__ __forceinline__ F64 zeta_z64(const Dims& D, const Grid<F64>& G, const
     r = G.dy[n.v0] * v[n.v0] - G.dx[n.u1] * u[n.u1] - G.dy[n.v2] * v[n.v2] + G.dx[n.u3] * u[n.u3];
   } else {
     const F64 zd = G.z_area_dual_z[q];
-    auto side = [&](const F64* x, const F64* z, const F64* ry, const F64* m, long long i) {
+    auto side = [&](const F64* x, const F64* z, const F64* m, long long i) {
       const F64 z0 = z[i], x0 = x[i], dz = zd - z0;
       const bool above = (positive(dz) || jl == D.nl) && jl != 1;
       const long long o = above ? i - pl : i + pl;
-      const F64 y = above ? -ry[o] : ry[i];
-      return m[q] * (x0 + dz * div_rn(x0 - x[o], z0 - z[o], y));
+      return m[q] * (x0 + dz * ((x0 - x[o]) / (z0 - z[o])));
     };
-    r = side(v, G.z_v, X.ryv, X.m0, n.v0) + side(u, G.z_u, X.ryu, X.m1, n.u1) + side(v, G.z_v, X.ryv, X.m2, n.v2)
-      + side(u, G.z_u, X.ryu, X.m3, n.u3);
+    r = side(v, G.z_v, X.m0, n.v0) + side(u, G.z_u, X.m1, n.u1) + side(v, G.z_v, X.m2, n.v2) + side(u, G.z_u, X.m3, n.u3);
   }
-  return div_rn(r, G.area_dual_z[q], X.radz[q]);
+  return r / G.area_dual_z[q];
 }
 __global__ void k64_zeta_z(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, F64* zz) {
   LG_IDX3;
@@ -568,7 +554,7 @@ __global__ void k64_covariant(Dims D, Grid<F64> G, StateT<F64> S, F64* cx, F64* 
 }
 // eta_x (ny+1, nx, nl+1) and eta_y (ny, nx+1, nl+1); level 1 takes the vorticity of level 2, and the
 // surface level the general form
-__global__ void k64_eta_xy(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, const F64* cx, const F64* cy, F64* ex, F64* ey) {
+__global__ void k64_eta_xy(Dims D, Grid<F64> G, StateT<F64> S, const F64* cx, const F64* cy, F64* ex, F64* ey) {
   LG_IDX3;
   const int lev = max(jl, 2);
   const F64* rg = S.rho + (long long)(D.g - 1) * D.fstride;
@@ -581,7 +567,7 @@ __global__ void k64_eta_xy(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, const 
     } else {
       const long long b = IX(D, inner ? i : 1, jk, lev), a = IX(D, inner ? i - 1 : D.ny, jk, lev), q = IX(D, i, jk, lev);
       if (!D.llinear && (inner || D.periodic))
-        e = div_rn(G.dz[a] * S.w[a] - cy[b - D.plane] - G.dz[b] * S.w[b] + cy[b], G.area_dual_x[q], X.radx[q]);
+        e = (G.dz[a] * S.w[a] - cy[b - D.plane] - G.dz[b] * S.w[b] + cy[b]) / G.area_dual_x[q];
       if (D.lcorio) e = e + G.fvec_x[IX(D, i, jk, 1)];
       if (inner || D.periodic) e = e / rho_avg_h<F64>(D, G, rg, inner ? i - 1 : D.ny, jk, inner ? i : 1, jk, jl);
     }
@@ -596,7 +582,7 @@ __global__ void k64_eta_xy(Dims D, Grid<F64> G, RotGrid X, StateT<F64> S, const 
     } else {
       const long long b = IX(D, ji, inner ? k : 1, lev), a = IX(D, ji, inner ? k - 1 : D.nx, lev), q = IX(D, ji, k, lev);
       if (!D.llinear && (inner || D.periodic))
-        e = div_rn(-(G.dz[b] * S.w[b]) - cx[b] + G.dz[a] * S.w[a] + cx[b - D.plane], G.area_dual_y[q], X.rady[q]);
+        e = (-(G.dz[b] * S.w[b]) - cx[b] + G.dz[a] * S.w[a] + cx[b - D.plane]) / G.area_dual_y[q];
       if (D.lcorio) e = e + G.fvec_y[IX(D, ji, k, 1)];
       if (inner || D.periodic) e = e / rho_avg_h<F64>(D, G, rg, ji, inner ? k - 1 : D.nx, ji, inner ? k : 1, jl);
     }
@@ -610,9 +596,9 @@ __global__ void k64_mass_flux(Dims D, Grid<F64> G, StateT<F64> S, F64* uph, F64*
   LG_IDX3;
   const F64* rg = S.rho + (long long)(D.g - 1) * D.fstride;
   const long long q = IX(D, ji, jk, jl);
-  F64 f;
-  if (ji <= D.ny && jk <= D.nx + 1 && stv_h_x<F64>(D, rg, S.u, ji, jk, jl, &f)) uph[q] = f;
-  if (ji <= D.ny + 1 && jk <= D.nx && stv_h_y<F64>(D, rg, S.v, ji, jk, jl, &f)) vph[q] = f;
+  F64 f;  // (0 at a non-periodic boundary, which the reference leaves untouched: the arrays serve others in turn)
+  if (ji <= D.ny && jk <= D.nx + 1) uph[q] = stv_h_x<F64>(D, rg, S.u, ji, jk, jl, &f) ? f : F64(0.0);
+  if (ji <= D.ny + 1 && jk <= D.nx) vph[q] = stv_h_y<F64>(D, rg, S.v, ji, jk, jl, &f) ? f : F64(0.0);
   if (ji > D.ny || jk > D.nx) return;
   const long long b = q + D.plane;
   F64 up = 0.0, lo = 0.0;
@@ -842,8 +828,7 @@ void launch64_diss_rate(const Dims& D, const Grid<double>& G, const State& S, co
 }
 
 void launch64_rot_grid(const Dims& D, const Grid<double>& G, double* const* a, cudaStream_t st) {
-  k64_rot_grid<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), f64(a[0]), f64(a[1]), f64(a[2]), f64(a[3]),
-                                                                           f64(a[4]), f64(a[5]), f64(a[6]), f64(a[7]), f64(a[8]));
+  k64_rot_grid<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(a[0]), f64(a[1]), f64(a[2]), f64(a[3]));
 }
 void launch64_zeta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, double* zz, cudaStream_t st) {
   k64_zeta_z<<<cell_grid(D.ny + 1, D.nx + 1, D.nl), kCellBlock, 0, st>>>(D, f64(G), X, f64(S), f64(zz));
@@ -854,9 +839,9 @@ void launch64_eta_z(const Dims& D, const Grid<double>& G, const RotGrid& X, cons
 void launch64_covariant(const Dims& D, const Grid<double>& G, const State& S, double* cx, double* cy, cudaStream_t st) {
   k64_covariant<<<cell_grid(D.ny, D.nx, D.nl), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(cx), f64(cy));
 }
-void launch64_eta_xy(const Dims& D, const Grid<double>& G, const RotGrid& X, const State& S, const double* cx, const double* cy,
-                     double* ex, double* ey, cudaStream_t st) {
-  k64_eta_xy<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), X, f64(S), f64(cx), f64(cy), f64(ex), f64(ey));
+void launch64_eta_xy(const Dims& D, const Grid<double>& G, const State& S, const double* cx, const double* cy, double* ex,
+                     double* ey, cudaStream_t st) {
+  k64_eta_xy<<<cell_grid(D.ny + 1, D.nx + 1, D.NL), kCellBlock, 0, st>>>(D, f64(G), f64(S), f64(cx), f64(cy), f64(ex), f64(ey));
 }
 void launch64_mass_flux(const Dims& D, const Grid<double>& G, const State& S, double* uph, double* vph, double* q5, double* q6,
                         cudaStream_t st) {

@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -87,23 +88,22 @@ struct lgame_gpu {
   // the phase transitions (lphase_trans extension): rates (nc+1 fields) and heating rate
   bool phase = false;
   double *ptr = nullptr, *pth = nullptr;
+  std::map<int, std::vector<double>> idle_diag;  // diagnostics of a closure that is off, as the caller set them
   // scratch
   // FP64 step: grid-only factors of the column solves (ColumnGrid), 0.5*dtime/volume
-  double *rvol = nullptr, *itwdtv = nullptr, *zs = nullptr, *zs_c2 = nullptr, *zs_c1h = nullptr, *hdeb = nullptr,
-         *raz = nullptr;
+  double *rvol = nullptr, *itwdtv = nullptr, *zs_c1h = nullptr, *raz = nullptr;
   ColumnGrid colg{};
-  // reciprocals of the metrics of the explicit kernels, and the faces of the mass flux and of theta_v's
-  // flux or gradient
+  // reciprocals of the metrics of the explicit kernels
   double *rdx = nullptr, *rdy = nullptr, *rdz = nullptr;
   Recip recip{};
-  double* rotg[9] = {};  // the arrays of RotGrid
+  double* rotg[4] = {};  // the arrays of RotGrid
   RotGrid rot{};
-  double* fc[8] = {};
+  // faces, in scratch arrays that are free by then: of a gradient or of the mass flux (ez, uph, vph, wph: free
+  // but between the vorticity and its flux), of theta_v's flux (ex, ey, theta, divf: free after theta3)
   Faces fcm{}, fct{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
-  double* staging = nullptr;
-  size_t staging_elems = 0;
+  double* staging = nullptr;  // a level of the inner product weights (lgame_gpu_set_grid)
   double* reduce_buf = nullptr;
   int* flag = nullptr;
   Grid<double> G{};
@@ -288,12 +288,11 @@ const double* device_view(const double* host) {
 }
 
 __global__ void k_split_ipw(Dims D, const double* src, double* w1, double* w2, double* w3, double* w4,
-                            double* w5, double* w6) {
+                            double* w5, double* w6, int jl) {
   const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int jk = blockIdx.z * blockDim.y + threadIdx.y + 1;
-  const int jl = blockIdx.y + 1;
   if (ji > D.ny || jk > D.nx) return;
-  const size_t h = 6 * ((size_t)(ji - 1) + (size_t)D.ny * ((size_t)(jk - 1) + (size_t)D.nx * (size_t)(jl - 1)));
+  const size_t h = 6 * ((size_t)(ji - 1) + (size_t)D.ny * (size_t)(jk - 1));
   const long long q = IX(D, ji, jk, jl);
   w1[q] = src[h]; w2[q] = src[h + 1]; w3[q] = src[h + 2]; w4[q] = src[h + 3]; w5[q] = src[h + 4]; w6[q] = src[h + 5];
 }
@@ -561,8 +560,8 @@ int theta3(lgame_gpu* c, const double* tp, int mode, const double* u, const doub
   const Dims& D = c->D;
   LAUNCH(kd::k_theta, grd(D, D.ny, D.nx, D.nl), D, c->G, tp, c->theta, mode);
   LAUNCH_FN("k_grad_vert", launch64_grad_vert(D, c->G, c->recip, c->theta, c->gz, c->ex, c->ey, c->stream));
-  LAUNCH_FN("k_grad_faces", launch64_grad_faces(D, c->G, c->recip, c->theta, c->ex, c->ey, c->fct, c->stream));
-  LAUNCH_FN("k_div_h", launch64_div(D, c->G, c->recip, c->fct, c->divf, c->stream));
+  LAUNCH_FN("k_grad_faces", launch64_grad_faces(D, c->G, c->recip, c->theta, c->ex, c->ey, c->fcm, c->stream));
+  LAUNCH_FN("k_div_h", launch64_div(D, c->G, c->recip, c->fcm, c->divf, c->stream));
   LAUNCH_FN("k_theta_edges", launch64_theta_edges(D, c->theta, c->divf, u, v, ou, ov, c->stream));
   return LGAME_OK;
 }
@@ -578,9 +577,9 @@ int gradient(lgame_gpu* c, const double* f, double* gx, double* gy, double* gz) 
 int advection(lgame_gpu* c, const State& S) {
   const Dims& D = c->D;
   if (!(!D.llinear || D.lcorio)) return LGAME_OK;
-  // (the covariant winds in fcm; the vertical mass flux's products in wph and divf)
-  if (!D.llinear) LAUNCH_FN("k_covariant", launch64_covariant(D, c->G, S, c->fc[0], c->fc[1], c->stream));
-  LAUNCH_FN("k_eta_xy", launch64_eta_xy(D, c->G, c->rot, S, c->fc[0], c->fc[1], c->ex, c->ey, c->stream));
+  // (the covariant winds in uph and vph, before the mass flux; the vertical mass flux's products in wph and divf)
+  if (!D.llinear) LAUNCH_FN("k_covariant", launch64_covariant(D, c->G, S, c->uph, c->vph, c->stream));
+  LAUNCH_FN("k_eta_xy", launch64_eta_xy(D, c->G, S, c->uph, c->vph, c->ex, c->ey, c->stream));
   LAUNCH_FN("k_eta_z", launch64_eta_z(D, c->G, c->rot, S, c->ez, c->stream));
   LAUNCH_FN("k_mass_flux", launch64_mass_flux(D, c->G, S, c->uph, c->vph, c->wph, c->divf, c->stream));
   LAUNCH_FN("k_vort_flux", launch64_vort_flux(D, c->G, c->ex, c->ey, c->ez, c->uph, c->vph, c->wph, c->divf, c->pvt_x, c->pvt_y,
@@ -629,7 +628,7 @@ int diffusion_scalar(lgame_gpu* c, const State& So) {
   const Grid<double>& G = c->G;
   const DiffBuf<double>& B = c->dbuf;
   // the coefficients (kind 0 mass, 1 temperature; of the cells in theta and divf), then every field's
-  // gradient (column products in ex, ey), faces (fct) and divergence
+  // gradient (column products in ex, ey), faces (fcm) and divergence
   auto coeffs = [&](int kind, int vert) -> int {
     LAUNCH_FN("k_diff_coeffs", launch64_diff_coeffs(D, G, So, B, kind, vert, c->theta, c->divf, c->stream));
     LAUNCH_FN("k_diff_coeffs", launch64_diff_face_coeffs(D, c->theta, c->divf, vert, B, c->stream));
@@ -637,8 +636,8 @@ int diffusion_scalar(lgame_gpu* c, const State& So) {
   };
   auto field = [&](const double* f, int vert, double* out) -> int {
     LAUNCH_FN("k_grad_vert", launch64_grad_vert(D, G, c->recip, f, c->gz, c->ex, c->ey, c->stream));
-    LAUNCH_FN("k_diff_faces", launch64_diff_faces(D, G, c->recip, f, c->ex, c->ey, B, c->fct, c->stream));
-    LAUNCH_FN("k_diff_div", launch64_diff_div(D, G, c->recip, c->fct, B, c->gz, vert, out, c->stream));
+    LAUNCH_FN("k_diff_faces", launch64_diff_faces(D, G, c->recip, f, c->ex, c->ey, B, c->fcm, c->stream));
+    LAUNCH_FN("k_diff_div", launch64_diff_div(D, G, c->recip, c->fcm, B, c->gz, vert, out, c->stream));
     return LGAME_OK;
   };
   int rc = LGAME_OK;
@@ -680,9 +679,9 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
         const int rc = gradient(c, So.ep, c->gx, c->gy, c->gz);
         if (rc != LGAME_OK) return rc;
       }
-      // (theta_v and the two quotients of every cell in theta and fcm)
-      LAUNCH_FN("k_pgrad_cells", launch64_pgrad_cells(D, G, So, c->theta, c->fc[0], c->fc[1], c->stream));
-      LAUNCH_FN("k_pgrad", launch64_pgrad(D, G, So, c->gx, c->gy, c->gz, c->theta, c->fc[0], c->fc[1], c->tvu, c->tvv, c->tpu,
+      // (theta_v and the two quotients of every cell in theta, uph and vph)
+      LAUNCH_FN("k_pgrad_cells", launch64_pgrad_cells(D, G, So, c->theta, c->uph, c->vph, c->stream));
+      LAUNCH_FN("k_pgrad", launch64_pgrad(D, G, So, c->gx, c->gy, c->gz, c->theta, c->uph, c->vph, c->tvu, c->tvv, c->tpu,
                                           c->tpv, P, step == 0 ? 1 : 0, c->stream));
       // into the edge arrays of theta', which nothing reads after k_pgrad, and cpw
       if (D.ncons > 1)
@@ -715,9 +714,9 @@ int step_fp64(lgame_gpu* c, int so, int sn, int step) {
              (const double*)c->tsoil[so], c->cfg.lsfc_phase_trans, D.dtime, c->ptr, c->pth);
     const double* ptr = c->phase ? c->ptr : nullptr;
     const double* pth = c->phase ? c->pth : nullptr;
-    if (D.ncons > 1) {  // the slope terms of the new wind in fct, its vertical correction in divf
-      LAUNCH_FN("k_wind_slopes", launch64_wind_slopes(D, G, Sn.u, Sn.v, c->fc[6], c->fc[7], c->stream));
-      LAUNCH_FN("k_contra", launch64_contra(D, G, c->fc[6], c->fc[7], c->divf, c->stream));
+    if (D.ncons > 1) {  // the slope terms of the new wind in uph and vph, its vertical correction in divf
+      LAUNCH_FN("k_wind_slopes", launch64_wind_slopes(D, G, Sn.u, Sn.v, c->uph, c->vph, c->stream));
+      LAUNCH_FN("k_contra", launch64_contra(D, G, c->uph, c->vph, c->divf, c->stream));
       LAUNCH_FN("k_tracers", launch64_tracers(D, G, c->recip, Ss, Sn.u, Sn.v, c->divf, T.rho, rk, mdt, ptr, c->stream));
     }
     // theta_v_adv_3rd_order of the state used here: in the first substep that is state_old,
@@ -907,6 +906,9 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
   for (int f = 0; f < LGAME_GRID_LAND_FRACTION; ++f) {
     if (f == LGAME_GRID_INNER_PRODUCT_WEIGHTS || f == LGAME_GRID_TRSK_WEIGHTS_U || f == LGAME_GRID_TRSK_WEIGHTS_V) continue;
     size_t n = (f == LGAME_GRID_FVEC_X || f == LGAME_GRID_FVEC_Y || f == LGAME_GRID_FVEC_Z) ? (size_t)D.plane : F;
+    // what only the closure (and the phase transitions: the layers' thickness) reads, the FP64 step does without
+    const bool dual = f == LGAME_GRID_DX_DUAL || f == LGAME_GRID_DY_DUAL, thick = f == LGAME_GRID_LAYER_THICKNESS;
+    if (cfg->precision == LGAME_PRECISION_FP64 && !cfg->lmom_diff_h && (dual || (thick && !cfg->lphase_trans))) continue;
     if ((rc = dalloc(c, &c->grid[f], n)) != LGAME_OK) return fail(rc);
   }
   // surface layer and soil: one plane per surface field, nsoillays planes of soil temperature
@@ -954,30 +956,28 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
                         &c->ex, &c->ey, &c->ez, &c->uph, &c->vph, &c->wph, &c->vsq};
   for (double** p : scratch) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
   if (cfg->precision == LGAME_PRECISION_FP64) {
-    double** colg[] = {&c->rvol, &c->itwdtv, &c->zs, &c->zs_c2, &c->zs_c1h, &c->hdeb, &c->raz, &c->rdx, &c->rdy, &c->rdz,
-                       &c->fc[0], &c->fc[1], &c->fc[2], &c->fc[3], &c->fc[4], &c->fc[5], &c->fc[6], &c->fc[7]};
+    double** colg[] = {&c->rvol, &c->zs_c1h, &c->raz, &c->rdx, &c->rdy, &c->rdz, &c->rotg[0], &c->rotg[1], &c->rotg[2],
+                       &c->rotg[3]};
     for (double** p : colg) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
-    if (D.ncons > 1 && (rc = dalloc(c, &c->cpw, F))) return fail(rc);
-    c->colg = ColumnGrid{f64(c->rvol), f64(c->zs), f64(c->zs_c2), f64(c->zs_c1h), f64(c->hdeb), f64(c->raz),
+    if (D.ncons > 1 && ((rc = dalloc(c, &c->cpw, F)) || (rc = dalloc(c, &c->itwdtv, F)))) return fail(rc);
+    c->colg = ColumnGrid{f64(c->rvol), f64(c->zs_c1h), f64(c->raz),
                          1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P), 1.0 / D.dtime};
-    for (double*& p : c->rotg) if ((rc = dalloc(c, &p, F)) != LGAME_OK) return fail(rc);
-    c->rot = RotGrid{f64(c->rotg[0]), f64(c->rotg[1]), f64(c->rotg[2]), f64(c->rotg[3]), f64(c->rotg[4]),
-                     f64(c->rotg[5]), f64(c->rotg[6]), f64(c->rotg[7]), f64(c->rotg[8])};
-    c->fcm = Faces{f64(c->fc[0]), f64(c->fc[1]), f64(c->fc[2]), f64(c->fc[3])};
-    c->fct = Faces{f64(c->fc[4]), f64(c->fc[5]), f64(c->fc[6]), f64(c->fc[7])};
+    c->rot = RotGrid{f64(c->rotg[0]), f64(c->rotg[1]), f64(c->rotg[2]), f64(c->rotg[3])};
+    c->fcm = Faces{f64(c->ez), f64(c->uph), f64(c->vph), f64(c->wph)};
+    c->fct = Faces{f64(c->ex), f64(c->ey), f64(c->theta), f64(c->divf)};
     c->recip = Recip{f64(c->rvol), f64(c->rdx), f64(c->rdy), f64(c->rdz)};
     if (column_prepare()) return fail(set_err(LGAME_ERR_CUDA, "shared memory of the column solvers refused"));
   }
-  // diffusion closure: the carried diagnostics always, the work arrays when a part is on
+  // diffusion closure (without it, its carried diagnostics stay on the host: idle_diag)
   {
     DiffBuf<double>& B = c->dbuf;
-    double** carried_d[] = {&B.tke, &B.visc, &B.mdtx, &B.mdty, &B.mdtz};
-    for (double** p : carried_d) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
     B.hd = c->hdiss;
     c->diff_mom_h = cfg->lmom_diff_h; c->diff_mom_v = cfg->lmom_diff_v;
     c->diff_temp_h = cfg->ltemp_diff_h; c->diff_temp_v = cfg->ltemp_diff_v;
     c->diff_mass_h = cfg->lmass_diff_h; c->diff_mass_v = cfg->lmass_diff_v;
     if (c->diff_mom_h) {
+      double** carried_d[] = {&B.tke, &B.visc, &B.mdtx, &B.mdty, &B.mdtz};
+      for (double** p : carried_d) if ((rc = dalloc(c, p, F)) != LGAME_OK) return fail(rc);
       // temp_diff_heating and mass_diff_tendency in both modes (the C ABI's diagnostics), the work
       // arrays for the FP64 step only (the split step keeps FP32 ones)
       if (c->diff_temp_h && (rc = dalloc(c, &B.tdh, F)) != LGAME_OK) return fail(rc);
@@ -997,8 +997,7 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
     P.mom_v = cfg->lmom_diff_v;
     P.mva = 0.0;  // set with the grid
   }
-  c->staging_elems = 6 * (size_t)D.ny * D.nx * D.nl;
-  if ((rc = dalloc(c, &c->staging, c->staging_elems)) != LGAME_OK) return fail(rc);
+  if ((rc = dalloc(c, &c->staging, 6 * (size_t)D.ny * D.nx)) != LGAME_OK) return fail(rc);
   if ((rc = dalloc(c, &c->reduce_buf, (size_t)kRedBlocks * LGAME_BUDGETS_MAX + LGAME_BUDGETS_MAX)) != LGAME_OK) return fail(rc);
   {
     void* q = nullptr;
@@ -1050,7 +1049,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
   const Dims& D = c->D;
   int rc;
   for (int i = 0; i < LGAME_GRID_LAND_FRACTION; ++i) {
-    if (i == LGAME_GRID_INNER_PRODUCT_WEIGHTS || i == LGAME_GRID_TRSK_WEIGHTS_U || i == LGAME_GRID_TRSK_WEIGHTS_V) continue;
+    if (!c->grid[i]) continue;  // the weights, below; fields this run does not read
     if ((rc = copy_h2d(c, c->grid[i], f[i], grid_ext(D, i))) != LGAME_OK) return rc;
   }
   // surface planes, the soil grid (parameters of the surface kernels), and the carried
@@ -1071,12 +1070,15 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     P.i2dzt = P.ns > 0 ? 1.0 / (2.0 * (P.zc[P.ns - 1] - P.z_t_const)) : 0.0;
     if (c->split) split_set_sfc_par(c->split, P);
   }
-  // inner product weights: (6,ny,nx,nl) -> six padded fields
-  CK(cudaMemcpyAsync(c->staging, f[LGAME_GRID_INNER_PRODUCT_WEIGHTS], 6 * sizeof(double) * (size_t)D.ny * D.nx * D.nl,
-                     cudaMemcpyHostToDevice, c->stream));
-  k_split_ipw<<<grd(D, D.ny, D.nx, D.nl), blk(), 0, c->stream>>>(D, c->staging, c->ipw[0], c->ipw[1], c->ipw[2],
-                                                                  c->ipw[3], c->ipw[4], c->ipw[5]);
-  CK(cudaGetLastError());
+  // inner product weights: (6,ny,nx,nl) -> six padded fields, a level at a time
+  for (int jl = 1; jl <= D.nl; ++jl) {
+    const size_t n = 6 * (size_t)D.ny * D.nx;
+    CK(cudaMemcpyAsync(c->staging, f[LGAME_GRID_INNER_PRODUCT_WEIGHTS] + n * (size_t)(jl - 1), n * sizeof(double),
+                       cudaMemcpyHostToDevice, c->stream));
+    k_split_ipw<<<grd(D, D.ny, D.nx, 1), blk(), 0, c->stream>>>(D, c->staging, c->ipw[0], c->ipw[1], c->ipw[2], c->ipw[3],
+                                                                 c->ipw[4], c->ipw[5], jl);
+    CK(cudaGetLastError());
+  }
   // TRSK weights (3,ny) and (2,ny+1)
   std::vector<double> tmp((size_t)D.P, 0.0);
   for (int k = 0; k < 3; ++k) {
@@ -1136,7 +1138,7 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
   if (c->rvol) {
     launch64_rot_grid(D, c->G, c->rotg, c->stream);
     launch64_recip(D, c->G, c->rdx, c->rdy, c->rdz, c->stream);
-    launch_column_grid(D, c->G, c->rvol, c->itwdtv, c->zs, c->zs_c2, c->zs_c1h, c->hdeb, c->raz, c->stream);
+    launch_column_grid(D, c->G, c->rvol, c->itwdtv, c->zs_c1h, c->raz, c->stream);
     CK(cudaGetLastError());
   }
   if (c->split) {
@@ -1257,12 +1259,22 @@ double* diag_dev(lgame_gpu* c, int f) {
 }
 }  // namespace
 
+namespace {
+// the diffusion closure's carried diagnostics, which a run without it does not touch: they are kept on the host
+// as they were set
+bool idle_diag(const lgame_gpu* c, int i) {
+  return !c->diff_mom_h && (i == LGAME_DIAG_TKE || i == LGAME_DIAG_VISCOSITY || i == LGAME_DIAG_MOM_DIFF_TEND_X ||
+                            i == LGAME_DIAG_MOM_DIFF_TEND_Y || i == LGAME_DIAG_MOM_DIFF_TEND_Z);
+}
+}  // namespace
+
 extern "C" int lgame_gpu_set_diag(lgame_gpu* c, const double* const* f, int nfields) {
   if (!c || !f || nfields != LGAME_DIAG_NFIELDS) return set_err(LGAME_ERR_INVALID_ARG, "lgame_gpu_set_diag: bad arguments");
   const Dims& D = c->D;
   for (int i = 0; i < nfields; ++i) {
-    if (!f[i] || !diag_dev(c, i)) continue;  // not given, or not formed in this run (phase transitions off)
     const Ext e = diag_ext(D, i);
+    if (f[i] && idle_diag(c, i)) c->idle_diag[i].assign(f[i], f[i] + e.n1 * e.n2 * e.n3);
+    if (!f[i] || !diag_dev(c, i)) continue;  // not given, or not formed in this run (phase transitions off)
     const int nrep = diag_nrep(D, i);
     for (int r = 0; r < nrep; ++r) {
       int rc = copy_h2d(c, diag_dev(c, i) + (size_t)r * D.fstride, f[i] + r * e.n1 * e.n2 * e.n3, e);
@@ -1288,8 +1300,10 @@ extern "C" int lgame_gpu_get_diag(lgame_gpu* c, double* const* f, int nfields) {
     if (!f[i]) continue;
     const Ext e = diag_ext(D, i);
     const int nrep = diag_nrep(D, i);
-    if (!diag_dev(c, i)) {  // not formed in this run: the reference's zero
-      std::memset(f[i], 0, sizeof(double) * e.n1 * e.n2 * e.n3 * (size_t)nrep);
+    if (!diag_dev(c, i)) {  // not formed in this run: as it was set, or the reference's zero
+      const auto kept = c->idle_diag.find(i);
+      if (kept != c->idle_diag.end()) std::memcpy(f[i], kept->second.data(), sizeof(double) * kept->second.size());
+      else std::memset(f[i], 0, sizeof(double) * e.n1 * e.n2 * e.n3 * (size_t)nrep);
       continue;
     }
     for (int r = 0; r < nrep; ++r) {

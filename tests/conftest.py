@@ -1,5 +1,6 @@
 """pytest configuration: paths to the package and the oracle, and the gpu marker."""
 import os
+import subprocess
 import sys
 from pathlib import Path
 
@@ -21,3 +22,18 @@ def has_gpu() -> bool:
         return torch.cuda.is_available()
     except Exception:
         return False
+
+
+@pytest.fixture(scope="session")
+def recording_library(tmp_path_factory):
+    """The library's own objects linked with a stand-in for the CUDA runtime (fake_cudart.cpp) that runs no
+    kernel: its host code on the CPU."""
+    import build
+    build.build()
+    objs = sorted(str(p) for p in build.OUT.glob("*.o"))
+    assert len(objs) == len(build.CUDA_UNITS) + len(build.CXX_UNITS)
+    lib = tmp_path_factory.mktemp("fake") / "liblgame_fake.so"
+    cuda = Path(build._nvcc()).resolve().parent.parent
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-fopenmp", f"-I{cuda}/include",
+                    str(ROOT / "tests" / "fake_cudart.cpp"), *objs, "-o", str(lib)], check=True)
+    return lib

@@ -15,8 +15,6 @@ from pathlib import Path
 
 import pytest
 
-import build
-
 HERE = Path(__file__).resolve().parent
 STATE = ("u", "v", "w", "gas", "tr", "th")  # th: rho*theta_v, theta', exner'
 FLUX = ["fu", "fv", "gu", "gv"]
@@ -123,18 +121,6 @@ for step in range(2):
     g.pchevi(step % 2, (step + 1) % 2, step)
 print(lib.fake_log().decode())
 """
-
-
-@pytest.fixture(scope="module")
-def recording_library(tmp_path_factory):
-    build.build()
-    objs = sorted(str(p) for p in build.OUT.glob("*.o"))
-    assert len(objs) == len(build.CUDA_UNITS) + len(build.CXX_UNITS)
-    lib = tmp_path_factory.mktemp("fake") / "liblgame_fake.so"
-    cuda = Path(build._nvcc()).resolve().parent.parent
-    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-fopenmp", f"-I{cuda}/include", str(HERE / "fake_cudart.cpp"), *objs,
-                    "-o", str(lib)], check=True)
-    return lib
 
 
 PHYSICS = dict(lmom_diff_h=True, lmom_diff_v=True, ltemp_diff_h=True, ltemp_diff_v=True, lmass_diff_h=True,
