@@ -1372,242 +1372,17 @@ __global__ void __launch_bounds__(256, 5) ks_tend_wind(Dims D, State So, State S
 //
 // Two kernels (the rule between them stands at their launch in split_step).  Large grids:
 // ks_column_ver, one thread per column, streamed top to bottom and back, bound by about 20 FP64
-// operations a cell and the latency of a level's loads.  Five more products are formed beside the FP64 pipe
-// (fp64.cuh; the hardware's: 1.41 against 1.34 ms at 512x512x80), and the increment of rho*theta_v serves both it
-// and exner'; with each layer's inputs loaded a level ahead (five blocks of 96 registers an SM; six of 80: 1.42
-// ms) 1.57 -> 1.34 ms; compiled with and without a background state (BG), whose absence costs two
-// registers a layer and three FP64 operations, 1.27 ms.  Small grids: ks_column_ver_tile below.
+// operations a cell and the latency of a level's loads: five more products are formed beside the FP64 pipe
+// (fp64.cuh), the increment of rho*theta_v serves both it and exner', each layer's inputs are loaded a level
+// ahead (five blocks of 96 registers an SM), and it is compiled with and without a background state (BG),
+// whose absence costs two registers a layer and three FP64 operations: 1.57 -> 1.21 ms a launch at
+// 512x512x80.  Small grids: ks_column_ver_tile below.
 constexpr int kMaxLayers = 128;  // layers a context may have (lgame_gpu_create)
-template <class C, bool BG>
-__global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
-                                                     State Sn, StateF Mo, StateF Mn, Tend<float> Tn, int rk_step) {
-  constexpr bool F64 = sizeof(C) == 8;
-  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (ji > D.ny || jk > D.nx) return;
-  const int nl = D.nl, n = nl - 1;
-  const C dtf = C(D.dtime), idtf = C(1.0 / D.dtime);
-  const double idtd = 1.0 / D.dtime;
-  const long long goff = (long long)(D.g - 1) * D.fstride;
-  const C rdcv = C(kR_D / kC_D_V);
-  const C ic2 = C(1.0 / (kIMPL_THERMO_WEIGHT * (D.dtime * D.dtime) * kC_D_P));
-  const C ic1 = C(1.0 / (kIMPL_THERMO_WEIGHT * D.dtime * kC_D_P));
-  const StateF& Mu = (rk_step == 1) ? Mo : Mn;  // state_new_used, mo_column_solvers.F90:69-73
-  const State& Su = (rk_step == 1) ? So : Sn;
-  // the inputs of the coefficients, from the FP32 mirror or the FP64 state and metrics
-  auto rho_o = [&](long long i) -> C { if constexpr (F64) return So.rho[goff + i]; else return Mo.rho[goff + i]; };
-  auto rt_o = [&](long long i) -> C { if constexpr (F64) return So.rt[i]; else return Mo.rt[i]; };
-  auto ep_o = [&](long long i) -> C { if constexpr (F64) return So.ep[i]; else return Mo.ep[i]; };
-  auto rho_u = [&](long long i) -> C { if constexpr (F64) return Su.rho[goff + i]; else return Mu.rho[goff + i]; };
-  auto rt_u = [&](long long i) -> C { if constexpr (F64) return Su.rt[i]; else return Mu.rt[i]; };
-  auto ep_u = [&](long long i) -> C { if constexpr (F64) return Su.ep[i]; else return Mu.ep[i]; };
-  auto w_o = [&](long long i) -> C { if constexpr (F64) return So.w[i]; else return Mo.w[i]; };
-  auto ebg = [&](long long i) -> C { if constexpr (F64) return G.exner_bg[i]; else return GF.exner_bg[i]; };
-  auto ivol = [&](long long i) -> C { if constexpr (F64) return X.inv_volume[i]; else return X.inv_volume_f[i]; };
-  auto iarz = [&](long long i) -> C { if constexpr (F64) return X.inv_area_z[i]; else return X.inv_area_z_f[i]; };
-  auto damp = [&](long long i) -> C { if constexpr (F64) return G.damp[i]; else return GF.damp[i]; };
-  // at w level jl (2..nl): z_scalar(jl-1) - z_scalar(jl) and exner_bg(jl-1) - exner_bg(jl)
-  auto dzs = [&](long long i) -> C {
-    if constexpr (F64) return G.z_scalar[i - D.plane] - G.z_scalar[i]; else return X.dzs_f[i];
-  };
-  auto debg = [&](long long i) -> C {
-    if constexpr (F64) return G.exner_bg[i - D.plane] - G.exner_bg[i]; else return X.deb_f[i];
-  };
-  auto W = [](C x) -> double { if constexpr (F64) return x; else return wide(x); };
-  auto Nr = [](double x) -> float { return narrow(x); };
-  auto M = [](C a, double x) -> double { if constexpr (F64) return a * x; else return mul_int(a, x); };
-  auto quot = [](double x, C d) -> double { if constexpr (F64) return x / d; else return div_f(x, d); };
 
-  // what a layer and an interface (w level) read; the layer's is loaded a level ahead of its use (the
-  // interfaces' ahead too spills: 1.35 ms at 512x512x80)
-  struct LayIn { C ro, rt, eb, ep, iv, ru, rtu, epu, tr, trt; double tp, epd; };
-  auto layer_in = [&](int jl) -> LayIn {
-    LayIn R{};
-    if (jl > nl) return R;
-    const long long i = IX(D, ji, jk, jl);
-    R.ro = rho_o(i); R.rt = rt_o(i); R.eb = ebg(i); R.ep = ep_o(i); R.iv = ivol(i);
-    if (rk_step == 2) { R.ru = rho_u(i); R.rtu = rt_u(i); R.epu = ep_u(i); }
-    R.tr = C(Tn.rho[goff + i]); R.trt = C(Tn.rt[i]);
-    R.tp = So.tp[i]; R.epd = So.ep[i];
-    return R;
-  };
-  struct ItfIn { C dz, deb, dp, w, iaz, tw; double wd; };
-  auto itf_in = [&](int jl) -> ItfIn {
-    ItfIn R{};
-    if (jl > nl) return R;
-    const long long i = IX(D, ji, jk, jl);
-    R.dz = dzs(i); R.deb = debg(i); R.dp = damp(i); R.w = w_o(i); R.iaz = iarz(i); R.tw = C(Tn.w[i]);
-    R.wd = So.w[i];
-    return R;
-  };
-  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
-  // state, where theta * d(exner')/dz carries the whole hydrostatic balance); the explicit predictions of
-  // theta_v' and exner' (FP64 state plus increments) and of rho_g
-  struct Lay { C a, b, g, th, ro, iv, rhe; double thd, tpe, epe; };
-  auto layer = [&](int jl, const LayIn& R) -> Lay {
-    Lay L;
-    const long long i = IX(D, ji, jk, jl);
-    L.thd = 0.0;
-    if constexpr (!BG) L.thd = Su.rt[i] / Su.rho[goff + i];
-    const C iro = C(1) / R.ro, irto = C(1) / R.rt;
-    L.a = -R.rt * iro * iro;
-    L.b = iro;
-    L.g = rdcv * irto * (R.eb + R.ep);
-    if (rk_step == 2) {
-      const C iru = C(1) / R.ru, irtu = C(1) / R.rtu;
-      L.a = C(0.5) * (L.a - R.rtu * iru * iru);
-      L.b = C(0.5) * (L.b + iru);
-      L.g = C(0.5) * (L.g + rdcv * irtu * (R.eb + R.epu));
-      L.th = R.rtu * iru;
-    } else {
-      L.th = R.rt * iro;
-    }
-    L.ro = R.ro;
-    L.iv = R.iv;
-    L.tpe = R.tp + W(dtf * (L.a * R.tr + L.b * R.trt));
-    L.epe = R.epd + W(dtf * L.g * R.trt);
-    L.rhe = R.ro + dtf * R.tr;
-    return L;
-  };
-
-  C epr[kMaxLayers + 1];       // elimination multipliers
-  double rpr[kMaxLayers + 1];  // substituted right-hand side, then the solution (FP64)
-  C tis[kMaxLayers + 1];       // interface theta
-  C gs[kMaxLayers + 1];        // gamma of each layer
-  Lay L0 = layer(1, layer_in(1)), L1 = layer(2, layer_in(2)), L2{};
-  LayIn R = layer_in(3);
-  gs[1] = L0.g;
-  C cv_prev = C(0), epr_prev = C(0);
-  double rpr_prev = 0.0;
-  // at the interface below layer jl: theta, and 2/(rho(jl) + rho(jl+1))
-  C ti = C(0.5) * (L0.th + L1.th), irio = C(2) / (L0.ro + L1.ro);
-  for (int jl = 1; jl <= n; ++jl) {  // row jl: level jl+1 between layers jl (a) and jl+1 (b)
-    const LayIn Rn = layer_in(jl + 3);
-    const ItfIn I1 = itf_in(jl + 1), I2 = itf_in(jl + 2);
-    gs[jl + 1] = L1.g;
-    tis[jl] = ti;
-    const C dz = I1.dz, deb = I1.deb, dp = I1.dp, wof = I1.w;
-    const double wo = I1.wd;
-    const C al0 = L0.a * L0.iv, al1 = L1.a * L1.iv, be0 = L0.b * L0.iv, be1 = L1.b * L1.iv;
-    const C ga0 = L0.g * L0.iv, ga1 = L1.g * L1.iv;
-    const C dv = -(ti * ti) * (ga0 + ga1) + C(0.5) * deb * (al1 - al0 + ti * (be1 - be0))
-                 - dz * ic2 * irio * (C(2) * I1.iaz + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
-    const C rie = C(0.5) * (L0.rhe + L1.rhe);
-    // The products of FP32 coefficients with FP64 values here and in the state update below
-    // stay FP64 products of the FP32 factors: merging two FP32 factors into one rounded
-    // coefficient (e.g. -dz*ic2*(1 + rie*irio) for w_old) saves two FP64 operations per cell
-    // but lets an atmosphere at rest over hills drift about four times faster (1e-8 instead
-    // of 3e-9 m/s of spurious wind after 3 h at 256 x 256 x 50).
-    double rv = M(-dz * ic2, wo + W(dtf * I1.tw));
-    rv = fma(BG ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
-    rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
-    rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
-    // couplings with row jl+1 (layer b's derivatives), which need layer jl+2
-    C cv = C(0), ev = C(0), ti_n = C(0), irio_n = C(0);
-    if (jl < n) {
-      L2 = layer(jl + 2, R);
-      ti_n = C(0.5) * (L1.th + L2.th);
-      irio_n = C(2) / (L1.ro + L2.ro);
-      cv = ti_n * ga1 * ti + C(0.5) * I2.deb * (al1 + be1 * ti)
-           - I2.dz * ic1 * C(0.5) * I2.w * L1.iv * irio_n * I2.dp;
-      ev = ti * ga1 * ti_n - C(0.5) * deb * (al1 + be1 * ti_n) + dz * ic1 * C(0.5) * wof * L1.iv * irio * dp;
-    }
-    const C piv = dv - epr_prev * cv_prev;
-    const double x = (jl == 1) ? rv : fma(-W(cv_prev), rpr_prev, rv);
-    rpr_prev = quot(x, piv);
-    rpr[jl] = rpr_prev;
-    epr_prev = ev / piv;
-    epr[jl] = epr_prev;
-    cv_prev = cv;
-    L0 = L1; L1 = L2;
-    R = Rn;
-    ti = ti_n;
-    irio = irio_n;
-  }
-  // back substitution fused with the new state, mo_column_solvers.F90:300-345, bottom to top:
-  // layer jl needs the solutions of the rows above (w level jl) and below it (w level jl+1),
-  // and w at level jl+1 the new densities of layers jl and jl+1, all known once the
-  // substitution has reached row jl-1.  The inputs of the layer above are loaded before the
-  // current layer's results are stored (a store may alias a later load, which stops the
-  // compiler from moving the loads itself).
-  struct StateIn { double rt, rho, ep, bg, w; C ivf, iaz, mro; float trho, trt; };
-  auto state_in = [&](int m) {
-    StateIn r;
-    const long long p = IX(D, ji, jk, m);
-    r.rt = So.rt[p];
-    r.rho = So.rho[goff + p];
-    r.ep = So.ep[p];
-    r.bg = G.theta_v_bg[p];
-    r.w = So.w[p];
-    r.ivf = ivol(p);
-    r.iaz = iarz(p);
-    r.mro = rho_o(p);
-    r.trho = Tn.rho[goff + p];
-    r.trt = Tn.rt[p];
-    return r;
-  };
-  StateIn in_cur = state_in(nl), in_up{}, in_below{};
-  double s1 = 0.0;     // solution at the interface below the layer (w level jl+1)
-  double p1 = 0.0;     // theta there times it
-  C rnf_below = C(0);  // new rho_g of the layer below (FP32: rounded)
-  for (int jl = nl; jl >= 1; --jl) {
-    if (jl > 1) in_up = state_in(jl - 1);
-    const long long i = IX(D, ji, jk, jl);
-    // solution of row jl-1 (w level jl), the interface above the layer
-    double s0 = 0.0;
-    if (jl >= 2) s0 = (jl - 1 == n) ? rpr[n] : fma(-W(epr[jl - 1]), s1, rpr[jl - 1]);
-    const double p0 = (jl >= 2) ? M(tis[jl - 1], s0) : 0.0;
-    const double dtv = W(dtf * in_cur.ivf);
-    const double rho_e = in_cur.rho + W(dtf * C(in_cur.trho));
-    const double rn = fma(dtv, s1 - s0, rho_e);
-    const double inc = fma(dtv, p1 - p0, W(dtf * C(in_cur.trt)));
-    const double rtn = in_cur.rt + inc;
-    const double epn = fma(W(gs[jl]), inc, in_cur.ep);
-    const float rnf = Nr(rn);
-    const C rnc = F64 ? C(rn) : C(rnf);
-    if constexpr (F64) {
-      const double tpn = fma(-in_cur.bg, rn, rtn) / rn;
-      Sn.tp[i] = tpn;
-      Mn.tp[i] = Nr(tpn);
-    } else {
-      const float tpf = narrow(fma(-in_cur.bg, rn, rtn)) / rnf;
-      Sn.tp[i] = wide(tpf);
-      Mn.tp[i] = tpf;
-    }
-    Sn.rho[goff + i] = rn;
-    Sn.rt[i] = rtn;
-    Sn.ep[i] = epn;
-    Mn.rho[goff + i] = rnf;
-    Mn.rt[i] = Nr(rtn);
-    Mn.ep[i] = Nr(epn);
-    if (jl <= n) {  // w at level jl+1 from the increment there, between this layer and the one below
-      const long long ib = i + D.plane;
-      const C rin = C(0.5) * (rnc + rnf_below);
-      const C irio = C(2) / (in_cur.mro + in_below.mro);
-      const double wn = M(irio, fma(-W(rin), in_below.w, M(C(2) * in_below.iaz, s1)));
-      Sn.w[ib] = wn;
-      Mn.w[ib] = Nr(wn);
-    }
-    s1 = s0;
-    p1 = p0;
-    rnf_below = rnc;
-    in_below = in_cur;
-    in_cur = in_up;
-  }
-  if (D.freeslip) {  // w_free_slip, mo_inner_product.F90:52-75, with the new u, v
-    const int m = nl;
-    const double wf =
-        G.ipw[0][IX(D, ji, jk, m)] * Sn.u[IX(D, ji, jk + 1, m)] * G.slope_x[IX(D, ji, jk + 1, m)]
-      + G.ipw[1][IX(D, ji, jk, m)] * Sn.v[IX(D, ji, jk, m)] * G.slope_y[IX(D, ji, jk, m)]
-      + G.ipw[2][IX(D, ji, jk, m)] * Sn.u[IX(D, ji, jk, m)] * G.slope_x[IX(D, ji, jk, m)]
-      + G.ipw[3][IX(D, ji, jk, m)] * Sn.v[IX(D, ji + 1, jk, m)] * G.slope_y[IX(D, ji + 1, jk, m)];
-    Sn.w[IX(D, ji, jk, m + 1)] = wf;
-    Mn.w[IX(D, ji, jk, m + 1)] = narrow(wf);
-  }
-}
-
-// the same operators as functions of the column, for ks_column_ver_tile (in ks_column_ver they
-// stand in the loop: with these functions there it took 3.47 instead of 3.15 ms at 768 x 768 x 80)
+// the operators of the solve as functions of a column, for both kernels; what a level reads (LayIn, ItfIn) is
+// loaded by functions of its own, so that a kernel can load ahead of its use.  (The order of the calls decides
+// how a level's loads and divisions overlap: with the next layer formed before this row the thread-per-column
+// kernel takes 1.37 ms at 512x512x80, with an interface loaded twice 1.30, as it is 1.21.)
 template <class C>
 struct ColVer {
   static constexpr bool F64 = sizeof(C) == 8;
@@ -1618,6 +1393,7 @@ struct ColVer {
   const State &So, &Sn, &Su;  // Su: state_new_used, mo_column_solvers.F90:69-73
   const StateF &Mo, &Mn, &Mu;
   const Tend<float>& Tn;
+  const bool bg;  // a background state
   const int rk_step, ji, jk;
   const long long goff;
   const C dtf, idtf, rdcv, ic2, ic1;
@@ -1625,9 +1401,9 @@ struct ColVer {
 
   __device__ __forceinline__ ColVer(const Dims& D_, const Grid<double>& G_, const Grid<float>& GF_, const GridX& X_,
                                     const State& So_, const State& Sn_, const StateF& Mo_, const StateF& Mn_,
-                                    const Tend<float>& Tn_, int rk, int i, int j)
+                                    const Tend<float>& Tn_, bool bg_, int rk, int i, int j)
       : D(D_), G(G_), GF(GF_), X(X_), So(So_), Sn(Sn_), Su(rk == 1 ? So_ : Sn_), Mo(Mo_), Mn(Mn_),
-        Mu(rk == 1 ? Mo_ : Mn_), Tn(Tn_), rk_step(rk), ji(i), jk(j), goff((long long)(D_.g - 1) * D_.fstride),
+        Mu(rk == 1 ? Mo_ : Mn_), Tn(Tn_), bg(bg_), rk_step(rk), ji(i), jk(j), goff((long long)(D_.g - 1) * D_.fstride),
         dtf(C(D_.dtime)), idtf(C(1.0 / D_.dtime)), rdcv(C(kR_D / kC_D_V)),
         ic2(C(1.0 / (kIMPL_THERMO_WEIGHT * (D_.dtime * D_.dtime) * kC_D_P))),
         ic1(C(1.0 / (kIMPL_THERMO_WEIGHT * D_.dtime * kC_D_P))), idtd(1.0 / D_.dtime) {}
@@ -1655,77 +1431,99 @@ struct ColVer {
   static __device__ double M(C a, double x) { if constexpr (F64) return a * x; else return mul_int(a, x); }
   static __device__ double quot(double x, C d) { if constexpr (F64) return x / d; else return div_f(x, d); }
 
-  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
-  // state, where theta * d(exner')/dz carries the whole hydrostatic balance); with predict() the
-  // explicit predictions of theta_v' and exner' (FP64 state plus increments) and of rho_g
-  struct Lay { C a, b, g, th, ro, iv, rhe; double thd, tpe, epe; };
-  __device__ __forceinline__ Lay layer(int jl) const {
+  // what a layer and an interface (w level) read
+  struct LayIn { C ro, rt, eb, ep, iv, ru, rtu, epu, tr, trt; double tp, epd; };
+  __device__ __forceinline__ LayIn layer_in(int jl) const {
+    LayIn R{};
+    if (jl > D.nl) return R;
     const long long i = IX(D, ji, jk, jl);
-    Lay L{};
-    L.thd = D.luse_bg ? 0.0 : Su.rt[i] / Su.rho[goff + i];
-    const C ro = rho_o(i), rto = rt_o(i);
-    const C iro = C(1) / ro, irto = C(1) / rto;
-    L.a = -rto * iro * iro;
+    R.ro = rho_o(i); R.rt = rt_o(i); R.eb = ebg(i); R.ep = ep_o(i); R.iv = ivol(i);
+    if (rk_step == 2) { R.ru = rho_u(i); R.rtu = rt_u(i); R.epu = ep_u(i); }
+    R.tr = C(Tn.rho[goff + i]); R.trt = C(Tn.rt[i]);
+    R.tp = So.tp[i]; R.epd = So.ep[i];
+    return R;
+  }
+  struct ItfIn { C dz, deb, dp, w, iaz, tw; double wd; };
+  __device__ __forceinline__ ItfIn itf_in(int jl) const {
+    ItfIn R{};
+    if (jl > D.nl) return R;
+    const long long i = IX(D, ji, jk, jl);
+    R.dz = dzs(i); R.deb = debg(i); R.dp = damp(i); R.w = w_o(i); R.iaz = iarz(i); R.tw = C(Tn.w[i]);
+    R.wd = So.w[i];
+    return R;
+  }
+  // unscaled alpha, beta, gamma; theta of state_new_used (type C, and FP64 without a background
+  // state, where theta * d(exner')/dz carries the whole hydrostatic balance); the explicit predictions of
+  // theta_v' and exner' (FP64 state plus increments) and of rho_g
+  struct Lay { C a, b, g, th, ro, iv, rhe; double thd, tpe, epe; };
+  __device__ __forceinline__ Lay layer(int jl, const LayIn& R) const {
+    Lay L;
+    const long long i = IX(D, ji, jk, jl);
+    L.thd = 0.0;
+    if (!bg) L.thd = Su.rt[i] / Su.rho[goff + i];
+    const C iro = C(1) / R.ro, irto = C(1) / R.rt;
+    L.a = -R.rt * iro * iro;
     L.b = iro;
-    L.g = rdcv * irto * (ebg(i) + ep_o(i));
+    L.g = rdcv * irto * (R.eb + R.ep);
     if (rk_step == 2) {
-      const C ru = rho_u(i), rtu = rt_u(i);
-      const C iru = C(1) / ru, irtu = C(1) / rtu;
-      L.a = C(0.5) * (L.a - rtu * iru * iru);
+      const C iru = C(1) / R.ru, irtu = C(1) / R.rtu;
+      L.a = C(0.5) * (L.a - R.rtu * iru * iru);
       L.b = C(0.5) * (L.b + iru);
-      L.g = C(0.5) * (L.g + rdcv * irtu * (ebg(i) + ep_u(i)));
-      L.th = rtu * iru;
+      L.g = C(0.5) * (L.g + rdcv * irtu * (R.eb + R.epu));
+      L.th = R.rtu * iru;
     } else {
-      L.th = rto * iro;
+      L.th = R.rt * iro;
     }
-    L.ro = ro;
-    L.iv = ivol(i);
+    L.ro = R.ro;
+    L.iv = R.iv;
+    L.tpe = R.tp + W(dtf * (L.a * R.tr + L.b * R.trt));
+    L.epe = R.epd + W(dtf * L.g * R.trt);
+    L.rhe = R.ro + dtf * R.tr;
     return L;
   }
-  __device__ __forceinline__ void predict(int jl, Lay& L) const {
-    const long long i = IX(D, ji, jk, jl);
-    const C tr = C(Tn.rho[goff + i]), trt = C(Tn.rt[i]);
-    L.tpe = So.tp[i] + W(dtf * (L.a * tr + L.b * trt));
-    L.epe = So.ep[i] + W(dtf * L.g * trt);
-    L.rhe = L.ro + dtf * tr;
+  // at the interface between layers a and b: theta, and 2/(rho(a) + rho(b))
+  struct Itf { C t, irho; };
+  __device__ __forceinline__ Itf itf(const Lay& a, const Lay& b) const {
+    return Itf{C(0.5) * (a.th + b.th), C(2) / (a.ro + b.ro)};
   }
 
-  // row jl: level jl+1 between layers jl (L0) and jl+1 (L1); the couplings with row jl+1 (layer
-  // jl+1's derivatives) need layer jl+2 (L2) and are 0 in the last row
-  struct Row { C dv, cv, ev, ti; double rv; };
-  __device__ __forceinline__ Row row(int jl, const Lay& L0, const Lay& L1, const Lay& L2) const {
+  // row jl: the interface I (its inputs N) between layers jl (L0) and jl+1 (L1); diagonal and right-hand side
+  struct Row { C dv; double rv; };
+  __device__ __forceinline__ Row row(const Lay& L0, const Lay& L1, const ItfIn& N, const Itf& I) const {
     Row r;
-    const long long ib = IX(D, ji, jk, jl + 1);
-    const C ti = C(0.5) * (L0.th + L1.th);
-    r.ti = ti;
-    const C irio = C(2) / (L0.ro + L1.ro);
-    const C dz = dzs(ib), deb = debg(ib), dp = damp(ib);
-    const double wo = So.w[ib];
-    const C wof = w_o(ib);
+    const C ti = I.t, irio = I.irho;
+    const C dz = N.dz, deb = N.deb, dp = N.dp, wof = N.w;
+    const double wo = N.wd;
     const C al0 = L0.a * L0.iv, al1 = L1.a * L1.iv, be0 = L0.b * L0.iv, be1 = L1.b * L1.iv;
     const C ga0 = L0.g * L0.iv, ga1 = L1.g * L1.iv;
     r.dv = -(ti * ti) * (ga0 + ga1) + C(0.5) * deb * (al1 - al0 + ti * (be1 - be0))
-           - dz * ic2 * irio * (C(2) * iarz(ib) + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
+           - dz * ic2 * irio * (C(2) * N.iaz + dtf * wof * C(0.5) * (L1.iv - L0.iv)) * dp;
     const C rie = C(0.5) * (L0.rhe + L1.rhe);
-    double rv = M(-dz * ic2, wo + W(dtf * C(Tn.w[ib])));
-    rv = fma(D.luse_bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, rv);
-    rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, rv);
-    r.rv = fma(W(-dz * ic2 * rie * irio), wo, rv);
-    r.cv = r.ev = C(0);
-    if (jl < D.nl - 1) {
-      const long long ic = IX(D, ji, jk, jl + 2);
-      const C ti_n = C(0.5) * (L1.th + L2.th);
-      const C irio_n = C(2) / (L1.ro + L2.ro);
-      r.cv = ti_n * ga1 * ti + C(0.5) * debg(ic) * (al1 + be1 * ti)
-             - dzs(ic) * ic1 * C(0.5) * w_o(ic) * L1.iv * irio_n * damp(ic);
-      r.ev = ti * ga1 * ti_n - C(0.5) * deb * (al1 + be1 * ti_n) + dz * ic1 * C(0.5) * wof * L1.iv * irio * dp;
-    }
+    // The products of FP32 coefficients with FP64 values here and in the state update below
+    // stay FP64 products of the FP32 factors: merging two FP32 factors into one rounded
+    // coefficient (e.g. -dz*ic2*(1 + rie*irio) for w_old) saves two FP64 operations per cell
+    // but lets an atmosphere at rest over hills drift about four times faster (1e-8 instead
+    // of 3e-9 m/s of spurious wind after 3 h at 256 x 256 x 50).
+    r.rv = M(-dz * ic2, wo + W(dtf * N.tw));
+    r.rv = fma(bg ? W(ti * idtf) : 0.5 * (L0.thd + L1.thd) * idtd, L0.epe - L1.epe, r.rv);
+    r.rv = fma(W(C(0.5) * idtf * deb), L0.tpe + L1.tpe, r.rv);
+    r.rv = fma(W(-dz * ic2 * rie * irio), wo, r.rv);
     return r;
+  }
+  // and its couplings with row jl+1 by layer jl+1's derivatives, between the interfaces I1 above and I2 below it
+  struct Coupling { C c, e; };
+  __device__ __forceinline__ Coupling coupling(const Lay& L1, const ItfIn& N1, const ItfIn& N2, const Itf& I1,
+                                               const Itf& I2) const {
+    const C al1 = L1.a * L1.iv, be1 = L1.b * L1.iv, ga1 = L1.g * L1.iv;
+    return Coupling{I2.t * ga1 * I1.t + C(0.5) * N2.deb * (al1 + be1 * I1.t)
+                        - N2.dz * ic1 * C(0.5) * N2.w * L1.iv * I2.irho * N2.dp,
+                    I1.t * ga1 * I2.t - C(0.5) * N1.deb * (al1 + be1 * I2.t)
+                        + N1.dz * ic1 * C(0.5) * N1.w * L1.iv * I1.irho * N1.dp};
   }
 
   // the new state, mo_column_solvers.F90:300-345: layer jl from the solutions s0, s1 at the
-  // interfaces above and below it (w levels jl, jl+1) and their interface theta t0, t1; w at level
-  // jl+1 from the new densities of layers jl and jl+1
+  // interfaces above and below it (w levels jl, jl+1) and their products p0, p1 with the interface theta;
+  // w at level jl+1 from the new densities of layers jl and jl+1
   struct StateIn { double rt, rho, ep, bg, w; C ivf, iaz, mro; float trho, trt; };
   __device__ __forceinline__ StateIn state_in(int m) const {
     StateIn r;
@@ -1749,11 +1547,11 @@ struct ColVer {
   static __device__ __forceinline__ C rho_c(double rn) { if constexpr (F64) return rn; else return narrow(rn); }
   // returns rho_c of the layer's new density; below: the layer below and its rho_c
   __device__ __forceinline__ C new_state(int jl, const StateIn& c, const StateIn& below, C rnc_below, double s0,
-                                         double s1, C t0, C t1, C g) const {
+                                         double s1, double p0, double p1, C g) const {
     const long long i = IX(D, ji, jk, jl);
     const double dtv = W(dtf * c.ivf);
     const double rn = new_rho(c, s0, s1);
-    const double inc = fma(dtv, M(t1, s1) - M(t0, s0), W(dtf * C(c.trt)));
+    const double inc = fma(dtv, p1 - p0, W(dtf * C(c.trt)));
     const double rtn = c.rt + inc;
     const double epn = fma(W(g), inc, c.ep);
     const float rnf = narrow(rn);
@@ -1796,6 +1594,78 @@ struct ColVer {
   }
 };
 
+// a thread a column; BG: with a background state
+template <class C, bool BG>
+__global__ void __launch_bounds__(128, 5) ks_column_ver(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So,
+                                                     State Sn, StateF Mo, StateF Mn, Tend<float> Tn, int rk_step) {
+  using Cv = ColVer<C>;
+  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int jk = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  if (ji > D.ny || jk > D.nx) return;
+  const Cv V(D, G, GF, X, So, Sn, Mo, Mn, Tn, BG, rk_step, ji, jk);
+  const int nl = D.nl, n = nl - 1;
+  C epr[kMaxLayers + 1];       // elimination multipliers
+  double rpr[kMaxLayers + 1];  // substituted right-hand side, then the solution (FP64)
+  C tis[kMaxLayers + 1];       // interface theta
+  C gs[kMaxLayers + 1];        // gamma of each layer
+  typename Cv::Lay L0 = V.layer(1, V.layer_in(1)), L1 = V.layer(2, V.layer_in(2)), L2{};
+  typename Cv::LayIn R = V.layer_in(3);
+  gs[1] = L0.g;
+  C cv_prev = C(0), epr_prev = C(0);
+  double rpr_prev = 0.0;
+  typename Cv::Itf I1 = V.itf(L0, L1);
+  typename Cv::ItfIn N1 = V.itf_in(2);
+  for (int jl = 1; jl <= n; ++jl) {  // row jl: level jl+1 between layers jl and jl+1
+    // (a layer's inputs are loaded a level ahead of their use; the interfaces' ahead too spills: 1.35 ms at
+    // 512x512x80)
+    const typename Cv::LayIn Rn = V.layer_in(jl + 3);
+    const typename Cv::ItfIn N2 = V.itf_in(jl + 2);
+    gs[jl + 1] = L1.g;
+    tis[jl] = I1.t;
+    const typename Cv::Row q = V.row(L0, L1, N1, I1);
+    typename Cv::Itf I2{C(0), C(0)};
+    typename Cv::Coupling k{C(0), C(0)};
+    if (jl < n) {
+      L2 = V.layer(jl + 2, R);
+      I2 = V.itf(L1, L2);
+      k = V.coupling(L1, N1, N2, I1, I2);
+    }
+    const C piv = q.dv - epr_prev * cv_prev;
+    const double x = (jl == 1) ? q.rv : fma(-Cv::W(cv_prev), rpr_prev, q.rv);
+    rpr_prev = Cv::quot(x, piv);
+    rpr[jl] = rpr_prev;
+    epr_prev = k.e / piv;
+    epr[jl] = epr_prev;
+    cv_prev = k.c;
+    L0 = L1; L1 = L2;
+    R = Rn;
+    I1 = I2;
+    N1 = N2;
+  }
+  // back substitution fused with the new state, bottom to top: layer jl needs the solutions of the rows above
+  // (w level jl) and below it (w level jl+1), and w at level jl+1 the new densities of layers jl and jl+1,
+  // all known once the substitution has reached row jl-1.  The inputs of the layer above are loaded before
+  // the current layer's results are stored (a store may alias a later load, which stops the
+  // compiler from moving the loads itself).
+  typename Cv::StateIn in_cur = V.state_in(nl), in_up{}, in_below{};
+  double s1 = 0.0;     // solution at the interface below the layer (w level jl+1)
+  double p1 = 0.0;     // theta there times it
+  C rnf_below = C(0);  // new rho_g of the layer below (FP32: rounded)
+  for (int jl = nl; jl >= 1; --jl) {
+    if (jl > 1) in_up = V.state_in(jl - 1);
+    // solution of row jl-1 (w level jl), the interface above the layer
+    double s0 = 0.0;
+    if (jl >= 2) s0 = (jl - 1 == n) ? rpr[n] : fma(-Cv::W(epr[jl - 1]), s1, rpr[jl - 1]);
+    const double p0 = (jl >= 2) ? Cv::M(tis[jl - 1], s0) : 0.0;
+    rnf_below = V.new_state(jl, in_cur, in_below, rnf_below, s0, s1, p0, p1, gs[jl]);
+    s1 = s0;
+    p1 = p0;
+    in_below = in_cur;
+    in_cur = in_up;
+  }
+  if (D.freeslip) V.free_slip();
+}
+
 // Small grids: a block owns TC columns and NW chunks of levels (a lane per column, chunk w of a
 // column in thread w*TC + lane), in phases:
 //   1. every thread forms the rows of its chunk (matrix, right-hand side) into shared memory;
@@ -1804,10 +1674,10 @@ struct ColVer {
 //   3. every thread its rows' y/p;  4. the first TC threads the back substitution;
 //   5. every thread the new state of its chunk of layers.
 // The chain of levels then waits on shared memory and arithmetic alone, and the levels' loads and
-// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 34 against 280
-// us at 4 x 256 x 60, 141 against 381 us at 128 x 128 x 80, 279 against 376 us at 180 x 210 x 80, equal (415 us)
-// at 230 x 236 x 80, and slower above, where the phases in which one warp works cost more than the
-// latency they hide.
+// FP64 operations run side by side.  Measured per launch, against ks_column_ver: 31 against 204
+// us at 4 x 256 x 60, 124 against 275 us at 128 x 128 x 80, 245 against 322 us at 180 x 210 x 80, equal (363 us)
+// at 243 x 240 x 80, and slower above (529 against 413 us at 288 x 288 x 80), where the phases in which one
+// warp works cost more than the latency they hide.
 template <class C, int TC, int NW>
 __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
     ks_column_ver_tile(Dims D, Grid<double> G, Grid<float> GF, GridX X, State So, State Sn, StateF Mo, StateF Mn,
@@ -1817,7 +1687,7 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
   const int lane = threadIdx.x % TC, w = threadIdx.x / TC;
   const int col = blockIdx.x * TC + lane;
   const bool valid = col < D.ny * D.nx;
-  const Cv V(D, G, GF, X, So, Sn, Mo, Mn, Tn, rk_step, valid ? col % D.ny + 1 : 1, valid ? col / D.ny + 1 : 1);
+  const Cv V(D, G, GF, X, So, Sn, Mo, Mn, Tn, D.luse_bg, rk_step, valid ? col % D.ny + 1 : 1, valid ? col / D.ny + 1 : 1);
   const int nl = D.nl, n = nl - 1;
   extern __shared__ __align__(16) unsigned char smem_cv[];
   double* const sr = (double*)smem_cv + lane;             // right-hand side, y, then the solution
@@ -1825,24 +1695,29 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
                                                           // e/p), interface theta, gamma of layer jl
   const int chunk = (n + NW - 1) / NW, r0 = w * chunk + 1, r1 = min(n, (w + 1) * chunk);
   if (valid && r0 <= r1) {
-    typename Cv::Lay L0 = V.layer(r0), L1 = V.layer(r0 + 1), L2{};
-    V.predict(r0, L0);
-    V.predict(r0 + 1, L1);
+    typename Cv::Lay L0 = V.layer(r0, V.layer_in(r0)), L1 = V.layer(r0 + 1, V.layer_in(r0 + 1)), L2{};
+    typename Cv::ItfIn N1 = V.itf_in(r0 + 1), N2{};
+    typename Cv::Itf I1 = V.itf(L0, L1), I2{C(0), C(0)};
     for (int jl = r0; jl <= r1; ++jl) {
+      const typename Cv::Row q = V.row(L0, L1, N1, I1);
+      typename Cv::Coupling k{C(0), C(0)};
       if (jl < n) {
-        L2 = V.layer(jl + 2);
-        if (jl < r1) V.predict(jl + 2, L2);
+        L2 = V.layer(jl + 2, V.layer_in(jl + 2));
+        N2 = V.itf_in(jl + 2);
+        I2 = V.itf(L1, L2);
+        k = V.coupling(L1, N1, N2, I1, I2);
       }
-      const typename Cv::Row q = V.row(jl, L0, L1, L2);
       C* const row = sc + kRow * (jl - 1);
       row[0] = q.dv;
-      row[TC] = q.cv;
-      row[2 * TC] = q.ev;
-      row[3 * TC] = q.ti;
+      row[TC] = k.c;
+      row[2 * TC] = k.e;
+      row[3 * TC] = I1.t;
       row[4 * TC] = L0.g;
       if (jl == n) row[kRow + 4 * TC] = L1.g;
       sr[TC * (jl - 1)] = q.rv;
       L0 = L1; L1 = L2;
+      N1 = N2;
+      I1 = I2;
     }
   }
   __syncthreads();
@@ -1861,7 +1736,7 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
   auto sol = [&](int m) -> double { return (m >= 1 && m <= n) ? sr[TC * (m - 1)] : 0.0; };
   auto tif = [&](int m) -> C { return (m >= 1 && m <= n) ? sc[kRow * (m - 1) + 3 * TC] : C(0); };
   typename Cv::StateIn in_cur = V.state_in(l1), in_up{}, in_below{};
-  double s1 = sol(l1);
+  double s1 = sol(l1), p1 = Cv::M(tif(l1), s1);
   C rnf_below = C(0);
   if (l1 < nl) {
     in_below = V.state_in(l1 + 1);
@@ -1869,9 +1744,10 @@ __global__ void __launch_bounds__(TC * NW, sizeof(C) == 4 ? 768 / (TC * NW) : 1)
   }
   for (int jl = l1; jl >= l0; --jl) {
     if (jl > l0) in_up = V.state_in(jl - 1);
-    const double s0 = sol(jl - 1);
-    rnf_below = V.new_state(jl, in_cur, in_below, rnf_below, s0, s1, tif(jl - 1), tif(jl), sc[kRow * (jl - 1) + 4 * TC]);
+    const double s0 = sol(jl - 1), p0 = Cv::M(tif(jl - 1), s0);
+    rnf_below = V.new_state(jl, in_cur, in_below, rnf_below, s0, s1, p0, p1, sc[kRow * (jl - 1) + 4 * TC]);
     s1 = s0;
+    p1 = p0;
     in_below = in_cur;
     in_cur = in_up;
   }
@@ -2750,10 +2626,10 @@ int split_step(SplitCtx* s, const Dims& D, const Grid<double>& G, const State& S
       SL("ks_sfc_column", k_sfc_column_split<float>, sgrd(D.ny, D.nx, 1), B, D, G, So, rk == 1 ? So : Sn, T.rt,
          SF.buf, SF.par, SF.tsoil[so], SF.tsoil[rk == 1 ? so : sn], SF.tsoil[sn]);
     // The vertical solve by the number of columns: up to 8 columns an SM, 8 a block with 32 chunks of
-    // levels (34 us at 1,024 columns of 60 layers; 54 with 32 x 12); up to the size that gives
-    // every SM sub-partition three warps of columns, 32 a block with 12 chunks (150 us at 16,384
-    // columns of 80 layers; 216 with 8 x 32); above, a thread a column (equal, 415 us, at 54,280 columns of
-    // 80 layers; 199 against 354 at 22,500).  The FP64-coefficient solve keeps twice the shared memory
+    // levels (31 us at 1,024 columns of 60 layers; 45 with 32 x 12); up to the size that gives
+    // every SM sub-partition three warps of columns, 32 a block with 12 chunks (124 us at 16,384
+    // columns of 80 layers; 202 with 8 x 32); above, a thread a column (equal, 363 us, at 58,320 columns of
+    // 80 layers; 171 against 296 at 22,500).  The FP64-coefficient solve keeps twice the shared memory
     // a column and takes 16 columns a block.
     const long long cols = (long long)D.ny * D.nx;
 #define CV_ARGS D, G, GF, s->GX, So, Sn, Mo, Mn, T, rk

@@ -19,10 +19,9 @@ __device__ __forceinline__ double wide_normal(float f) {
 
 // A pivot's reciprocal and the two quotients by it.  FP32: r to a unit of the last place (one instruction; the
 // chain of pivots waits for it), e/p = e*r, and c/p as an FP64 number to 2^-45: c*r as the exact sum of two FP32
-// numbers, the second with c times r's residual correction.  An FP32 multiplier c/p is good to 2^-24 and
-// carries that into the FP64 right-hand sides: 139 instead of 141 us a launch at 128x128x80, but an
-// atmosphere at rest over hills (192x192x50) drifted to 2.9e-11 m/s RMS in 3 h instead of 1.6e-11.  FP64: the
-// rounded quotients.
+// numbers, the second with c times r's residual correction.  An FP32 multiplier c/p would be good to 2^-24 and
+// carry that into right-hand sides that are held in FP64; it would save 1 % of a launch.  FP64: the rounded
+// quotients.
 __device__ __forceinline__ void quotients(float c, float e, float p, double* c_p, float* e_p) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p));
