@@ -103,7 +103,6 @@ struct lgame_gpu {
   Faces fcm{}, fct{};
   double* cpw = nullptr;                      // FP64 step, moist: c_p of water at the step's temperature
   double *theta, *gz, *gx, *gy, *divf, *tvu, *tvv, *tpu, *tpv, *ex, *ey, *ez, *uph, *vph, *wph, *vsq;
-  double* staging = nullptr;  // a level of the inner product weights (lgame_gpu_set_grid)
   double* reduce_buf = nullptr;
   int* flag = nullptr;
   Grid<double> G{};
@@ -287,14 +286,16 @@ const double* device_view(const double* host) {
   return (const double*)a.devicePointer;
 }
 
-__global__ void k_split_ipw(Dims D, const double* src, double* w1, double* w2, double* w3, double* w4,
-                            double* w5, double* w6, int jl) {
-  const int ji = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int jk = blockIdx.z * blockDim.y + threadIdx.y + 1;
-  if (ji > D.ny || jk > D.nx) return;
-  const size_t h = 6 * ((size_t)(ji - 1) + (size_t)D.ny * (size_t)(jk - 1));
+// n points of the inner product weights (6,ny,nx,nl), the first the p0-th, to their places in six padded fields
+__global__ void k_split_ipw(Dims D, const double* src, long long p0, long long n, double* w1, double* w2, double* w3,
+                            double* w4, double* w5, double* w6) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const long long col = (p0 + k) / D.ny;
+  const int ji = (int)((p0 + k) % D.ny) + 1, jk = (int)(col % D.nx) + 1, jl = (int)(col / D.nx) + 1;
+  const double* h = src + 6 * k;
   const long long q = IX(D, ji, jk, jl);
-  w1[q] = src[h]; w2[q] = src[h + 1]; w3[q] = src[h + 2]; w4[q] = src[h + 3]; w5[q] = src[h + 4]; w6[q] = src[h + 5];
+  w1[q] = h[0]; w2[q] = h[1]; w3[q] = h[2]; w4[q] = h[3]; w5[q] = h[4]; w6[q] = h[5];
 }
 
 __global__ void k_check_finite(Dims D, State S, int* flag) {
@@ -997,7 +998,6 @@ extern "C" int lgame_gpu_create(const lgame_config* cfg, lgame_gpu** out) {
     P.mom_v = cfg->lmom_diff_v;
     P.mva = 0.0;  // set with the grid
   }
-  if ((rc = dalloc(c, &c->staging, 6 * (size_t)D.ny * D.nx)) != LGAME_OK) return fail(rc);
   if ((rc = dalloc(c, &c->reduce_buf, (size_t)kRedBlocks * LGAME_BUDGETS_MAX + LGAME_BUDGETS_MAX)) != LGAME_OK) return fail(rc);
   {
     void* q = nullptr;
@@ -1070,13 +1070,14 @@ extern "C" int lgame_gpu_set_grid(lgame_gpu* c, const double* const* f, int nfie
     P.i2dzt = P.ns > 0 ? 1.0 / (2.0 * (P.zc[P.ns - 1] - P.z_t_const)) : 0.0;
     if (c->split) split_set_sfc_par(c->split, P);
   }
-  // inner product weights: (6,ny,nx,nl) -> six padded fields, a level at a time
-  for (int jl = 1; jl <= D.nl; ++jl) {
-    const size_t n = 6 * (size_t)D.ny * D.nx;
-    CK(cudaMemcpyAsync(c->staging, f[LGAME_GRID_INNER_PRODUCT_WEIGHTS] + n * (size_t)(jl - 1), n * sizeof(double),
+  // inner product weights: (6,ny,nx,nl) -> six padded fields, through a work array and so in about six parts
+  const long long points = (long long)D.ny * D.nx * D.nl, part = D.fstride / 6;
+  for (long long p0 = 0; p0 < points; p0 += part) {
+    const long long n = std::min(part, points - p0);
+    CK(cudaMemcpyAsync(c->theta, f[LGAME_GRID_INNER_PRODUCT_WEIGHTS] + 6 * p0, sizeof(double) * 6 * (size_t)n,
                        cudaMemcpyHostToDevice, c->stream));
-    k_split_ipw<<<grd(D, D.ny, D.nx, 1), blk(), 0, c->stream>>>(D, c->staging, c->ipw[0], c->ipw[1], c->ipw[2], c->ipw[3],
-                                                                 c->ipw[4], c->ipw[5], jl);
+    k_split_ipw<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(D, c->theta, p0, n, c->ipw[0], c->ipw[1], c->ipw[2],
+                                                                     c->ipw[3], c->ipw[4], c->ipw[5]);
     CK(cudaGetLastError());
   }
   // TRSK weights (3,ny) and (2,ny+1)
@@ -1273,7 +1274,11 @@ extern "C" int lgame_gpu_set_diag(lgame_gpu* c, const double* const* f, int nfie
   const Dims& D = c->D;
   for (int i = 0; i < nfields; ++i) {
     const Ext e = diag_ext(D, i);
-    if (f[i] && idle_diag(c, i)) c->idle_diag[i].assign(f[i], f[i] + e.n1 * e.n2 * e.n3);
+    if (f[i] && idle_diag(c, i)) {
+      const size_t n = e.n1 * e.n2 * e.n3;
+      if (std::all_of(f[i], f[i] + n, [](double v) { return v == 0.0 && !std::signbit(v); })) c->idle_diag.erase(i);
+      else c->idle_diag[i].assign(f[i], f[i] + n);
+    }
     if (!f[i] || !diag_dev(c, i)) continue;  // not given, or not formed in this run (phase transitions off)
     const int nrep = diag_nrep(D, i);
     for (int r = 0; r < nrep; ++r) {
