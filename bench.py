@@ -146,10 +146,10 @@ def _kernel_fields(ncons: int) -> dict:
 # moved per launch of the dominant kernel); traffic above the algorithmic bytes is re-reads and
 # per-thread stacks.
 MEASURED_DRAM_BYTES_PER_CELL = {
-    "ks_column_ver": 229.0, "ks_column_tracers": 200.2, "ks_pgrad": 192.9, "ks_gas_div": 106.4,
-    "ks_tend_wind": 103.2, "ks_eta": 86.5, "ks_ke": 78.7, "ks_tracers": 78.3, "ks_gzp": 65.1,
-    "ks_vort_flux": 59.2, "ks_theta_flux": 52.0, "ks_theta_edges": 47.5, "ks_div_h": 47.1, "ks_grad": 36.5,
-    "ks_gas_flux": 29.1, "ks_temperature": 25.4, "ks_heating_diss": 16.2, "ks_csh_sum": 8.0,
+    "ks_column_ver": 228.6, "ks_column_tracers": 200.2, "ks_pgrad": 192.9, "ks_gas_div": 106.8,
+    "ks_tend_wind": 103.3, "ks_eta": 86.5, "ks_ke": 78.7, "ks_tracers": 78.3, "ks_gzp": 65.0,
+    "ks_vort_flux": 59.2, "ks_theta_flux": 52.0, "ks_theta_edges": 47.6, "ks_div_h": 47.1, "ks_grad": 36.5,
+    "ks_gas_flux": 29.0, "ks_temperature": 25.5, "ks_heating_diss": 16.1, "ks_csh_sum": 8.0,
 }
 
 
