@@ -29,7 +29,7 @@ def recording_library(tmp_path_factory):
     """The library's own objects linked with a stand-in for the CUDA runtime (fake_cudart.cpp) that runs no
     kernel: its host code on the CPU."""
     import build
-    build.build()
+    build.build(force=not list(build.OUT.glob("*.o")))
     objs = sorted(str(p) for p in build.OUT.glob("*.o"))
     assert len(objs) == len(build.CUDA_UNITS) + len(build.CXX_UNITS)
     lib = tmp_path_factory.mktemp("fake") / "liblgame_fake.so"
