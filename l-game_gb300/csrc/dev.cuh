@@ -242,6 +242,12 @@ __device__ __forceinline__ T div_h_at(const Dims& D, const Grid<T>& G, FX vx, FY
 
 // ---- mo_vorticities.F90 ------------------------------------------------------
 
+// a*b rounded by itself: the terms of a circulation cancel where the flow does not vary, and one of them inside a
+// multiply-add would leave its rounding behind
+__device__ __forceinline__ float apart(float a, float b) { return __fmul_rn(a, b); }
+template <class T>
+__device__ __forceinline__ T apart(T a, T b) { return a * b; }
+
 // rel_vort_z_local, mo_vorticities.F90:423-538
 template <class T, class V>
 __device__ __forceinline__ T rel_vort_z_local(const Dims& D, const Grid<T>& G, const V* u, const V* v, int ji, int jk, int jl) {
@@ -256,10 +262,10 @@ __device__ __forceinline__ T rel_vort_z_local(const Dims& D, const Grid<T>& G, c
     j_i[3] = (ji == D.ny + 1) ? 1 : ji; j_k[3] = jk;
   }
   if (jl <= D.nf) {
-    r = r + G.dy[IX(D, j_i[0], j_k[0], jl)] * T(v[IX(D, j_i[0], j_k[0], jl)])
-          + T(-1) * G.dx[IX(D, j_i[1], j_k[1], jl)] * T(u[IX(D, j_i[1], j_k[1], jl)])
-          + T(-1) * G.dy[IX(D, j_i[2], j_k[2], jl)] * T(v[IX(D, j_i[2], j_k[2], jl)])
-          + G.dx[IX(D, j_i[3], j_k[3], jl)] * T(u[IX(D, j_i[3], j_k[3], jl)]);
+    r = r + apart(G.dy[IX(D, j_i[0], j_k[0], jl)], T(v[IX(D, j_i[0], j_k[0], jl)]))
+          - apart(G.dx[IX(D, j_i[1], j_k[1], jl)], T(u[IX(D, j_i[1], j_k[1], jl)]))
+          - apart(G.dy[IX(D, j_i[2], j_k[2], jl)], T(v[IX(D, j_i[2], j_k[2], jl)]))
+          + apart(G.dx[IX(D, j_i[3], j_k[3], jl)], T(u[IX(D, j_i[3], j_k[3], jl)]));
   } else {
     const T zd = G.z_area_dual_z[IX(D, ji, jk, jl)];
 #pragma unroll
@@ -275,7 +281,7 @@ __device__ __forceinline__ T rel_vort_z_local(const Dims& D, const Grid<T>& G, c
         if (jl == 1) sh = 1;
         const T vv = T(v[IX(D, ii, kk, jl)]);
         const T vg = (vv - T(v[IX(D, ii, kk, jl + sh)])) / (zv - G.z_v[IX(D, ii, kk, jl + sh)]);
-        r = r + sgn * l_rescale * G.dy[IX(D, ii, kk, jl)] * (vv + delta_z * vg);
+        r = r + apart(sgn * l_rescale * G.dy[IX(D, ii, kk, jl)], vv + delta_z * vg);
       } else {
         const T zu = G.z_u[IX(D, ii, kk, jl)];
         const T l_rescale = (T(kR_E) + zd) / (T(kR_E) + zu);
@@ -285,7 +291,7 @@ __device__ __forceinline__ T rel_vort_z_local(const Dims& D, const Grid<T>& G, c
         if (jl == 1) sh = 1;
         const T uu = T(u[IX(D, ii, kk, jl)]);
         const T vg = (uu - T(u[IX(D, ii, kk, jl + sh)])) / (zu - G.z_u[IX(D, ii, kk, jl + sh)]);
-        r = r + sgn * l_rescale * G.dx[IX(D, ii, kk, jl)] * (uu + delta_z * vg);
+        r = r + apart(sgn * l_rescale * G.dx[IX(D, ii, kk, jl)], uu + delta_z * vg);
       }
     }
   }

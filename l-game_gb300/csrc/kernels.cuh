@@ -135,9 +135,9 @@ __device__ __forceinline__ T zeta_x_raw(const Dims& D, const Grid<T>& G, const S
     const bool inner = ji >= 2 && ji <= D.ny;
     if (!inner && !D.periodic) return T(0);
     const int ii = inner ? ji : 1, im = inner ? ji - 1 : D.ny;
-    return G.dz[IX(D, im, jk, jl)] * T(w[IX(D, im, jk, jl)])
+    return apart(G.dz[IX(D, im, jk, jl)], T(w[IX(D, im, jk, jl)]))
          - G.dy[IX(D, ii, jk, jl - 1)] * hcov_y<T, V>(D, G, v, w, ii, jk, jl - 1)
-         - G.dz[IX(D, ii, jk, jl)] * T(w[IX(D, ii, jk, jl)])
+         - apart(G.dz[IX(D, ii, jk, jl)], T(w[IX(D, ii, jk, jl)]))
          + G.dy[IX(D, ii, jk, jl)] * hcov_y<T, V>(D, G, v, w, ii, jk, jl);
   }
   // surface level NL
@@ -148,8 +148,8 @@ __device__ __forceinline__ T zeta_x_raw(const Dims& D, const Grid<T>& G, const S
   T r = -G.dy[IX(D, ii, jk, nl)] * hcov_y<T, V>(D, G, v, w, ii, jk, nl);
   if (D.freeslip && (inner || (D.periodic && ii == 1))) {
     const int im = (ii == 1) ? D.ny : ii - 1;
-    r = r + half_of(G.dz[IX(D, im, jk, NL)]) * T(w[IX(D, im, jk, NL)])
-          - half_of(G.dz[IX(D, ii, jk, NL)]) * T(w[IX(D, ii, jk, NL)])
+    r = r + apart(half_of(G.dz[IX(D, im, jk, NL)]), T(w[IX(D, im, jk, NL)]))
+          - apart(half_of(G.dz[IX(D, ii, jk, NL)]), T(w[IX(D, ii, jk, NL)]))
           + G.dy[IX(D, ii, jk, nl)] * (T(v[IX(D, ii, jk, nl)])
           + (T(v[IX(D, ii, jk, nl - 1)]) - T(v[IX(D, ii, jk, nl)])) / (G.z_v[IX(D, ii, jk, nl - 1)] - G.z_v[IX(D, ii, jk, nl)])
           * (half_of(G.z_w[IX(D, im, jk, NL)] + G.z_w[IX(D, ii, jk, NL)]) - G.z_v[IX(D, ii, jk, nl)])
@@ -167,9 +167,9 @@ __device__ __forceinline__ T zeta_y_raw(const Dims& D, const Grid<T>& G, const S
     const bool inner = jk >= 2 && jk <= D.nx;
     if (!inner && !D.periodic) return T(0);
     const int kk = inner ? jk : 1, km = inner ? jk - 1 : D.nx;
-    return -G.dz[IX(D, ji, kk, jl)] * T(w[IX(D, ji, kk, jl)])
+    return -apart(G.dz[IX(D, ji, kk, jl)], T(w[IX(D, ji, kk, jl)]))
          - G.dx[IX(D, ji, kk, jl)] * hcov_x<T, V>(D, G, u, w, ji, kk, jl)
-         + G.dz[IX(D, ji, km, jl)] * T(w[IX(D, ji, km, jl)])
+         + apart(G.dz[IX(D, ji, km, jl)], T(w[IX(D, ji, km, jl)]))
          + G.dx[IX(D, ji, kk, jl - 1)] * hcov_x<T, V>(D, G, u, w, ji, kk, jl - 1);
   }
   const int nl = D.nl, NL = D.NL;
@@ -179,8 +179,8 @@ __device__ __forceinline__ T zeta_y_raw(const Dims& D, const Grid<T>& G, const S
   T r = G.dx[IX(D, ji, kk, nl)] * hcov_x<T, V>(D, G, u, w, ji, kk, nl);
   if (D.freeslip && (inner || (D.periodic && kk == 1))) {
     const int km = (kk == 1) ? D.nx : kk - 1;
-    r = r + half_of(G.dz[IX(D, ji, km, NL)]) * T(w[IX(D, ji, km, NL)])
-          - half_of(G.dz[IX(D, ji, kk, NL)]) * T(w[IX(D, ji, kk, NL)])
+    r = r + apart(half_of(G.dz[IX(D, ji, km, NL)]), T(w[IX(D, ji, km, NL)]))
+          - apart(half_of(G.dz[IX(D, ji, kk, NL)]), T(w[IX(D, ji, kk, NL)]))
           - G.dx[IX(D, ji, kk, nl)] * (T(u[IX(D, ji, kk, nl)])
           + (T(u[IX(D, ji, kk, nl - 1)]) - T(u[IX(D, ji, kk, nl)])) / (G.z_u[IX(D, ji, kk, nl - 1)] - G.z_u[IX(D, ji, kk, nl)])
           * (half_of(G.z_w[IX(D, ji, km, NL)] + G.z_w[IX(D, ji, kk, NL)]) - G.z_u[IX(D, ji, kk, nl)])

@@ -970,21 +970,21 @@ __global__ void __launch_bounds__(128, 4) ks_eta(Dims D, Grid<float> G, StateF S
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       if (l <= D.nf) {
-        zz += length[m] * ub[m];
+        zz += apart(length[m], ub[m]);
       } else {
         const float d = zd - zb[m];
         const bool up = (d > 0.f || l == D.nl) && l > 1;
         const float zs = up ? za[m] : zc[m], us = up ? ua[m] : uc[m];
         const float rescaled = fmaf(length[m], d / (float(kR_E) + zb[m]), length[m]);
-        zz += rescaled * (ub[m] + (ub[m] - us) * (d / (zb[m] - zs)));
+        zz += apart(rescaled, ub[m] + (ub[m] - us) * (d / (zb[m] - zs)));
       }
     }
     if (!zeta) zz = 0.f;
     const float ez_ = A.fi && A.fk ? (zz + fz * az) / (az * (0.25f * (r.w + r.c + r.n + rnw))) : fz;
     float ex_ = 0.f, ey_ = 0.f;
     if (l > 1) {
-      const float zx = zeta ? dz.n * w0.n - cp.y - dz.c * w0.c + cv.y : 0.f;
-      const float zy = zeta ? dz.w * w0.w + cp.x - dz.c * w0.c - cv.x : 0.f;
+      const float zx = zeta ? apart(dz.n, w0.n) - cp.y - apart(dz.c, w0.c) + cv.y : 0.f;
+      const float zy = zeta ? apart(dz.w, w0.w) + cp.x - apart(dz.c, w0.c) - cv.x : 0.f;
       ex_ = A.fi ? (zx + fx * ax) / (ax * (0.25f * (ry + r.n + r.c))) : fx;
       ey_ = A.fk ? (zy + fy * ay) / (ay * (0.25f * (rx + r.w + r.c))) : fy;
     }
